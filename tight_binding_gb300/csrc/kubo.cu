@@ -203,84 +203,182 @@ __global__ void mu_kernel_scale_kernel(double2* __restrict__ mu, const double* _
 }
 
 // ------------------------------------------------------------------ Gamma contractions (FP64)
-// zeta(e) = sum_mn mu_mn a_m a_n [(e - i n s) e^{i n th} T_m + (e + i m s) e^{-i m th} T_n] / (1-e^2)^2 / vol
-//         = sum_m a_m T_m (sum_n mu_mn P_n) + sum_m P'_m (sum_n mu_mn a_n T_n),
-//   P_n = a_n (e - i n s) e^{i n th},   P'_m = a_m (e + i m s) e^{-i m th}.
-__global__ void bastin_zeta_kernel(const double2* __restrict__ mu, int32_t M, const double* __restrict__ eps,
-                                   double vol, double2* __restrict__ zeta) {
-  extern __shared__ double2 sm[];
-  double2* P = sm;          // P_n
-  double2* Q = sm + M;      // a_n T_n (real, stored as complex)
-  const double e = eps[blockIdx.x];
-  const double s = sqrt(1.0 - e * e), th = acos(e);
-  for (int n = threadIdx.x; n < M; n += blockDim.x) {
-    double sn, cn;
-    sincos(n * th, &sn, &cn);
-    const double an = n == 0 ? 1.0 : 2.0;
-    // (e - i n s)(cn + i sn)
-    P[n] = make_double2(an * (e * cn + n * s * sn), an * (e * sn - n * s * cn));
-    Q[n] = make_double2(an * cn, 0.0);
-  }
-  __syncthreads();
-  double zr = 0.0, zi = 0.0;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    double sm_, cm;
-    sincos(m * th, &sm_, &cm);
-    const double am = m == 0 ? 1.0 : 2.0;
-    double r1 = 0.0, i1 = 0.0, r2 = 0.0, i2 = 0.0;
-    const double2* row = mu + (int64_t)m * M;
-    for (int n = 0; n < M; ++n) {
-      const double2 u = row[n];
-      r1 += u.x * P[n].x - u.y * P[n].y;
-      i1 += u.x * P[n].y + u.y * P[n].x;
-      r2 += u.x * Q[n].x;
-      i2 += u.y * Q[n].x;
+// Both spectra are double trigonometric sums over (m, n).  The product rule
+//   cos(m th) e^{i n th} = (e^{i (n+m) th} + e^{i (n-m) th}) / 2
+// collects them into one series over q = n + m and q = |n - m|: the M^2 moments
+// are summed once along their antidiagonals and diagonals, and each energy then
+// costs a series of 2M - 1 terms instead of M^2.  With w_mn = a_m a_n mu_mn / 2,
+//   U_q = sum_{n+m=q} w,  D_q = sum_{n+m=q} (n - m) w,  V_d = sum_{n-m=d} w,
+//   P_q = V_q + V_-q (V_0 at q = 0),  I_q = V_q - V_-q,  A = U + P,  B = D + q I:
+//   zeta  (1-e^2)^2 vol = sum_q cos(q th) (2 e A_q - i s B_q) + sin(q th) (s q A_q + 2 i e I_q)
+//   sigma (1-e^2) R     = - sum_q cos(q th) Re A_q
+// where e = cos th and s = sin th.  As M x M sums per energy the two were bound by
+// the FP64 pipe (6 FMAs per moment and energy): M = 512, 1,024 energies took 4.00 +
+// 0.94 ms in their kernels, 5.62 ms for both calls with the host copies; as series
+// both calls take 0.72 ms, nearly all of it copies and allocations.
+constexpr int kDiagThreads = 128;
+constexpr int kDiagRows = 16;       // rows of mu per CTA: M = 512 gives 256 CTAs
+constexpr int kSeriesThreads = 128; // evaluation: one warp per energy
+
+// Partial sums over kDiagRows rows: thread t takes the antidiagonal n + m = t and
+// the diagonal n - m = t - (M - 1), both read along rows (coalesced).
+// part: per row chunk, planes U, V and (BASTIN) D of 2M - 1 values.
+template <bool BASTIN>
+__global__ void __launch_bounds__(kDiagThreads) diag_sums_kernel(const double2* __restrict__ mu, int32_t M,
+                                                                 double2* __restrict__ part) {
+  const int32_t L = 2 * M - 1;
+  const int32_t t = blockIdx.x * kDiagThreads + threadIdx.x;
+  if (t >= L) return;
+  const int32_t m0 = blockIdx.y * kDiagRows;
+  double2 u = make_double2(0.0, 0.0), v = u, d = u;
+#pragma unroll 8
+  for (int32_t k = 0; k < kDiagRows; ++k) {
+    const int32_t m = m0 + k;
+    if (m >= M) break;
+    const double am = m == 0 ? 0.5 : 1.0;                  // a_m a_n / 2 = 2 with a_0 = 1, a_k = 2
+    const int32_t n = t - m, n2 = t - (M - 1) + m;
+    if (n >= 0 && n < M) {
+      const double2 x = mu[(int64_t)m * M + n];
+      const double f = am * (n == 0 ? 1.0 : 2.0);
+      u.x += f * x.x;
+      if constexpr (BASTIN) {
+        const double g = f * (double)(n - m);
+        u.y += f * x.y;
+        d.x += g * x.x;
+        d.y += g * x.y;
+      }
     }
-    const double qm = am * cm;                                    // a_m T_m
-    const double pr = am * (e * cm + m * s * sm_), pi = am * (-e * sm_ + m * s * cm);   // (e + i m s)(cm - i sm)
-    zr += qm * r1 + (pr * r2 - pi * i2);
-    zi += qm * i1 + (pr * i2 + pi * r2);
+    if (n2 >= 0 && n2 < M) {
+      const double2 x = mu[(int64_t)m * M + n2];
+      const double f = am * (n2 == 0 ? 1.0 : 2.0);
+      v.x += f * x.x;
+      if constexpr (BASTIN) v.y += f * x.y;
+    }
   }
-  __shared__ double red[2][32];
-  for (int o = 16; o > 0; o >>= 1) { zr += __shfl_xor_sync(0xffffffffu, zr, o); zi += __shfl_xor_sync(0xffffffffu, zi, o); }
-  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = zr; red[1][threadIdx.x >> 5] = zi; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += red[0][w]; b += red[1][w]; }
-    const double den = (1.0 - e * e) * (1.0 - e * e) * vol;
-    zeta[blockIdx.x] = make_double2(a / den, b / den);
+  double2* p = part + (int64_t)blockIdx.y * (BASTIN ? 3 : 2) * L;
+  p[t] = u;
+  p[L + t] = v;
+  if constexpr (BASTIN) p[2 * L + t] = d;
+}
+
+// The row chunks summed in order, then the series coefficients A, (BASTIN) B and I.
+template <bool BASTIN>
+__global__ void __launch_bounds__(kDiagThreads) series_coef_kernel(const double2* __restrict__ part, int32_t M,
+                                                                   int32_t chunks, double2* __restrict__ coef) {
+  const int32_t L = 2 * M - 1;
+  const int32_t q = blockIdx.x * kDiagThreads + threadIdx.x;
+  if (q >= L) return;
+  double2 u = make_double2(0.0, 0.0), d = u, vp = u, vm = u;
+#pragma unroll 4
+  for (int32_t c = 0; c < chunks; ++c) {
+    const double2* p = part + (int64_t)c * (BASTIN ? 3 : 2) * L;
+    const double2 a = p[q];
+    u.x += a.x;
+    u.y += a.y;
+    if (q < M) {
+      const double2 b = p[L + (M - 1) + q], e = p[L + (M - 1) - q];
+      vp.x += b.x;
+      vp.y += b.y;
+      vm.x += e.x;
+      vm.y += e.y;
+    }
+    if constexpr (BASTIN) {
+      const double2 g = p[2 * L + q];
+      d.x += g.x;
+      d.y += g.y;
+    }
+  }
+  if (q == 0) vm = make_double2(0.0, 0.0);                 // the main diagonal counts once
+  const double2 i = q == 0 ? vm : make_double2(vp.x - vm.x, vp.y - vm.y);
+  coef[q] = make_double2(u.x + vp.x + vm.x, u.y + vp.y + vm.y);
+  if constexpr (BASTIN) {
+    coef[L + q] = make_double2(d.x + q * i.x, d.y + q * i.y);
+    coef[2 * L + q] = i;
   }
 }
 
-// sigma(e) = -sum_mn Re(mu_mn) a_m a_n T_m(e) T_n(e) / (1 - e^2) / R
-__global__ void greenwood_kernel(const double2* __restrict__ mu, int32_t M, const double* __restrict__ eps, double R,
-                                 double* __restrict__ sigma) {
-  extern __shared__ double2 sm[];
-  double* T = reinterpret_cast<double*>(sm);
-  const double e = eps[blockIdx.x];
-  const double th = acos(e);
-  for (int n = threadIdx.x; n < M; n += blockDim.x) T[n] = (n == 0 ? 1.0 : 2.0) * cos(n * th);
-  __syncthreads();
-  double acc = 0.0;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    double r = 0.0;
-    const double2* row = mu + (int64_t)m * M;
-    for (int n = 0; n < M; ++n) r += row[n].x * T[n];
-    acc += T[m] * r;
+// One warp per energy: lane l takes q = l, l + 32, ..., with (cos, sin)(q th)
+// advanced by the rotation through 32 th.
+template <bool BASTIN>
+__global__ void __launch_bounds__(kSeriesThreads) series_eval_kernel(const double2* __restrict__ coef, int32_t M,
+                                                                     int32_t n_eps, const double* __restrict__ eps,
+                                                                     double norm, double* __restrict__ out) {
+  const int32_t k = blockIdx.x * (kSeriesThreads / 32) + (threadIdx.x >> 5);
+  if (k >= n_eps) return;
+  const int32_t lane = threadIdx.x & 31, L = 2 * M - 1;
+  const double e = eps[k], th = acos(e);
+  double c, s, cr, sr;
+  sincos(lane * th, &s, &c);
+  sincos(32 * th, &sr, &cr);
+  double2 s1 = make_double2(0.0, 0.0), s2 = s1, s3 = s1, s4 = s1;   // A cos, B cos, q A sin, I sin
+  for (int32_t q = lane; q < L; q += 32) {
+    const double2 a = coef[q];
+    s1.x += a.x * c;
+    if constexpr (BASTIN) {
+      const double2 b = coef[L + q], i = coef[2 * L + q];
+      const double qs = q * s;
+      s1.y += a.y * c;
+      s2.x += b.x * c;
+      s2.y += b.y * c;
+      s3.x += a.x * qs;
+      s3.y += a.y * qs;
+      s4.x += i.x * s;
+      s4.y += i.y * s;
+    }
+    const double cn = c * cr - s * sr;
+    s = s * cr + c * sr;
+    c = cn;
   }
-  __shared__ double red[32];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += red[w];
-    sigma[blockIdx.x] = -a / (1.0 - e * e) / R;
+  const double sn = sqrt(1.0 - e * e);
+  double zr, zi = 0.0;
+  if constexpr (BASTIN) {
+    zr = 2.0 * e * s1.x + sn * s2.y + sn * s3.x - 2.0 * e * s4.y;
+    zi = 2.0 * e * s1.y - sn * s2.x + sn * s3.y + 2.0 * e * s4.x;
+  } else {
+    zr = s1.x;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    zr += __shfl_xor_sync(0xffffffffu, zr, o);
+    if constexpr (BASTIN) zi += __shfl_xor_sync(0xffffffffu, zi, o);
+  }
+  if (lane == 0) {
+    if constexpr (BASTIN) {
+      const double den = (1.0 - e * e) * (1.0 - e * e) * norm;
+      out[2 * k] = zr / den;
+      out[2 * k + 1] = zi / den;
+    } else {
+      out[k] = -zr / (1.0 - e * e) / norm;
+    }
   }
 }
 
-
+template <bool BASTIN>
+int moment_series(int32_t M, const double* mu, int32_t n_eps, const double* eps, double norm, double* out,
+                  cudaStream_t st) {
+  const int32_t L = 2 * M - 1, chunks = (M + kDiagRows - 1) / kDiagRows, planes = BASTIN ? 3 : 2;
+  const size_t ob = sizeof(double) * (BASTIN ? 2 : 1) * (size_t)n_eps;
+  DevBuf dm, de, dz, part, coef;
+  TBK_TRY(dm.alloc(sizeof(double2) * (size_t)M * M));
+  TBK_TRY(de.alloc(sizeof(double) * n_eps));
+  TBK_TRY(dz.alloc(ob));
+  TBK_TRY(part.alloc(sizeof(double2) * (size_t)chunks * planes * L));
+  TBK_TRY(coef.alloc(sizeof(double2) * (size_t)planes * L));
+  TBK_CUDA(cudaMemcpyAsync(dm.p, mu, sizeof(double2) * (size_t)M * M, cudaMemcpyHostToDevice, st));
+  TBK_CUDA(cudaMemcpyAsync(de.p, eps, sizeof(double) * n_eps, cudaMemcpyHostToDevice, st));
+  const int32_t qb = (L + kDiagThreads - 1) / kDiagThreads;
+  diag_sums_kernel<BASTIN><<<dim3(qb, chunks), kDiagThreads, 0, st>>>(dm.as<double2>(), M, part.as<double2>());
+  TBK_CHECK_LAUNCH();
+  series_coef_kernel<BASTIN><<<qb, kDiagThreads, 0, st>>>(part.as<double2>(), M, chunks, coef.as<double2>());
+  TBK_CHECK_LAUNCH();
+  constexpr int kPer = kSeriesThreads / 32;
+  series_eval_kernel<BASTIN><<<(n_eps + kPer - 1) / kPer, kSeriesThreads, 0, st>>>(coef.as<double2>(), M, n_eps,
+                                                                                   de.as<double>(), norm,
+                                                                                   dz.as<double>());
+  TBK_CHECK_LAUNCH();
+  TBK_CUDA(cudaMemcpyAsync(out, dz.p, ob, cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaStreamSynchronize(st));
+  return TBK_OK;
+}
 
 // timing of the last tbk_kubo_mu call (CUDA events on the caller's stream)
 struct KuboTiming { double ms_blocks = 0, ms_gemm = 0, gemm_flops = 0, block_bytes = 0; int chunks = 0; };
@@ -793,20 +891,7 @@ int tbk_kubo_bastin_zeta(int32_t M, const double* mu, int32_t n_eps, const doubl
                          void* stream) {
   if (M < 1 || !mu || n_eps < 0 || (n_eps && (!eps || !zeta_out))) return fail(TBK_ERR_INVALID, "tbk_kubo_bastin_zeta: bad argument");
   if (n_eps == 0) return TBK_OK;
-  cudaStream_t st = as_stream(stream);
-  DevBuf dm, de, dz;
-  TBK_TRY(dm.alloc(sizeof(double2) * (size_t)M * M));
-  TBK_TRY(de.alloc(sizeof(double) * n_eps));
-  TBK_TRY(dz.alloc(sizeof(double2) * n_eps));
-  TBK_CUDA(cudaMemcpyAsync(dm.p, mu, sizeof(double2) * (size_t)M * M, cudaMemcpyHostToDevice, st));
-  TBK_CUDA(cudaMemcpyAsync(de.p, eps, sizeof(double) * n_eps, cudaMemcpyHostToDevice, st));
-  const size_t smem = sizeof(double2) * 2 * M;
-  if (smem > 48 * 1024) TBK_CUDA(cudaFuncSetAttribute(bastin_zeta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  bastin_zeta_kernel<<<n_eps, 256, smem, st>>>(dm.as<double2>(), M, de.as<double>(), vol, dz.as<double2>());
-  TBK_CHECK_LAUNCH();
-  TBK_CUDA(cudaMemcpyAsync(zeta_out, dz.p, sizeof(double2) * n_eps, cudaMemcpyDeviceToHost, st));
-  TBK_CUDA(cudaStreamSynchronize(st));
-  return TBK_OK;
+  return moment_series<true>(M, mu, n_eps, eps, vol, zeta_out, as_stream(stream));
 }
 
 int tbk_kubo_greenwood_sigma(int32_t M, const double* mu, int32_t n_eps, const double* eps, double R,
@@ -814,18 +899,7 @@ int tbk_kubo_greenwood_sigma(int32_t M, const double* mu, int32_t n_eps, const d
   if (M < 1 || !mu || n_eps < 0 || (n_eps && (!eps || !sigma_out)) || !(R > 0))
     return fail(TBK_ERR_INVALID, "tbk_kubo_greenwood_sigma: bad argument");
   if (n_eps == 0) return TBK_OK;
-  cudaStream_t st = as_stream(stream);
-  DevBuf dm, de, ds;
-  TBK_TRY(dm.alloc(sizeof(double2) * (size_t)M * M));
-  TBK_TRY(de.alloc(sizeof(double) * n_eps));
-  TBK_TRY(ds.alloc(sizeof(double) * n_eps));
-  TBK_CUDA(cudaMemcpyAsync(dm.p, mu, sizeof(double2) * (size_t)M * M, cudaMemcpyHostToDevice, st));
-  TBK_CUDA(cudaMemcpyAsync(de.p, eps, sizeof(double) * n_eps, cudaMemcpyHostToDevice, st));
-  greenwood_kernel<<<n_eps, 256, sizeof(double2) * M, st>>>(dm.as<double2>(), M, de.as<double>(), R, ds.as<double>());
-  TBK_CHECK_LAUNCH();
-  TBK_CUDA(cudaMemcpyAsync(sigma_out, ds.p, sizeof(double) * n_eps, cudaMemcpyDeviceToHost, st));
-  TBK_CUDA(cudaStreamSynchronize(st));
-  return TBK_OK;
+  return moment_series<false>(M, mu, n_eps, eps, R, sigma_out, as_stream(stream));
 }
 
 // Bastin: drop N/24 nodes at each end, ascending order, cumulative trapezoid from
