@@ -321,10 +321,31 @@ __device__ __forceinline__ void dot_acc(const LaneV<F, VPL>& a, const LaneV<F, V
     if constexpr (is_dd<F>) {
       dd_fma_acc(a.re[q], b.re[q], m);
       dd_fma_acc(a.im[q], b.im[q], m);
+    } else if constexpr (sizeof(F) == 8) {
+      m = fma(a.re[q], b.re[q], m);                        // two FP64 instructions instead of three
+      m = fma(a.im[q], b.im[q], m);
     } else {
       m += a.re[q] * b.re[q] + a.im[q] * b.im[q];
     }
   }
+}
+
+// FP64 sum over the warp, in every lane
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// Two FP64 sums over the warp in the five additions of one: after one exchange the
+// lower half of the lanes carries a, the upper half b.  Lanes 0-15 return the sum of
+// a, lanes 16-31 the sum of b.
+__device__ __forceinline__ double warp_pair_sum(double a, double b) {
+  const bool up = (threadIdx.x & 16) != 0;
+  double v = up ? b : a;
+  v += __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
 // a row sum built by HVal::fma, ready for use: double-float sums are

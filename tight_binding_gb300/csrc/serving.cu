@@ -293,19 +293,10 @@ __global__ void __launch_bounds__(kSrvThreads, sizeof(F) == 4 ? (CLS ? 6 : 5) : 
       if (!dot_only) st_v<F, VPL>(vt->y + me * VPL, out);
     }
     __syncwarp();
-    // slab partial in FP64: a fixed shuffle tree, lane 0 writes (an empty
+    // slab partial in FP64: a fixed shuffle tree, lanes 0 and 16 write (an empty
     // slab of a lane's last tile writes zeros)
-    double d0 = (double)m0, d1 = (double)m1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-      d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-    }
-    if (lane == 0) {
-      double* pp = part + ((int64_t)j * slab_cap + (int64_t)ti * kSrvWarps + warp) * 2;
-      pp[0] = d0;
-      pp[1] = d1;
-    }
+    const double d = warp_pair_sum((double)m0, (double)m1);
+    if ((lane & 15) == 0) part[((int64_t)j * slab_cap + (int64_t)ti * kSrvWarps + warp) * 2 + (lane >> 4)] = d;
   }
 }
 
