@@ -135,6 +135,8 @@ template <> struct C2<double> { using T = double2; };
 template <> struct C2<dd> { using T = dd2; };
 template <typename F> constexpr bool is_dd = false;
 template <> constexpr bool is_dd<dd> = true;
+template <typename F> constexpr bool is_f64 = false;
+template <> constexpr bool is_f64<double> = true;
 
 // Lane slice of a site's R vectors: VPL complex values moved as one access.
 template <typename F, int VPL>
@@ -206,6 +208,28 @@ __device__ __forceinline__ LaneV<F, VPL> ld_smem(const typename C2<F>::T* p) {
   return o;
 }
 
+// 2 x and -x on the integer pipe (the compiler negates a double with an FP64 add, and
+// an FP64 instruction holds its quarter of the SM for 64 clocks)
+__device__ __forceinline__ double times2(double x) {
+  const uint64_t u = (uint64_t)__double_as_longlong(x), sign = u & 0x8000000000000000ull;
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  uint64_t r = u + 0x0010000000000000ull;                            // normal numbers: exponent + 1
+  if (e == 0u) r = sign | (u << 1);                                  // zero, subnormals
+  if (e == 0x7feu) r = sign | 0x7ff0000000000000ull;                 // overflow
+  if (e == 0x7ffu) r = u;                                            // infinities, NaN
+  return __longlong_as_double((long long)r);
+}
+__device__ __forceinline__ double negate(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+
+// FP64 steps after the first start a row's sum at -v_{n-1} and gather with 2 H (exact),
+// so v_{n+1} = 2 H v_n - v_{n-1} is the sum itself, without closing instructions, and
+// skip zero padding entries instead of multiplying with them: the FP64 pipe bounds them
+// (honeycomb 1024x1024, R = 32, braket: 15 FP64 instructions a row and 2,055 us a step;
+// 10 and 1,483 us so).
+template <typename F> constexpr bool kFoldStep = is_f64<F>;
+
 template <typename F, bool CPLX_H>
 struct HVal;
 template <typename F>
@@ -221,6 +245,7 @@ struct HVal<F, false> {
   }
   __device__ __forceinline__ static HVal load_smem(const F* p, int32_t o) { return HVal{p[o]}; }
   __device__ __forceinline__ static HVal zero() { return HVal{F(0)}; }
+  __device__ __forceinline__ HVal twice() const { return HVal{times2(v)}; }   // FP64
   template <int VPL>
   __device__ __forceinline__ void fma(const LaneV<F, VPL>& x, LaneV<F, VPL>& acc) const {
     if constexpr (is_dd<F>) {
@@ -255,6 +280,7 @@ struct HVal<F, true> {
     return HVal{q.x, q.y};
   }
   __device__ __forceinline__ static HVal zero() { return HVal{F(0), F(0)}; }
+  __device__ __forceinline__ HVal twice() const { return HVal{times2(r), times2(i)}; }
   template <int VPL>
   __device__ __forceinline__ void fma(const LaneV<F, VPL>& x, LaneV<F, VPL>& acc) const {
     if constexpr (is_dd<F>) {

@@ -32,6 +32,15 @@ inline size_t class_smem_bytes(const ClassTab& ct) {
   return ne * class_value_bytes<F, CPLX_H>() + ne * 4 + (size_t)ct.n_cls * 4;
 }
 
+// acc += (2) p[o] x for a matrix value in memory
+template <typename F, int VPL, bool CPLX_H, bool FOLD>
+__device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, const LaneV<F, VPL>& xs,
+                                          LaneV<F, VPL>& acc) {
+  const HVal<F, CPLX_H> h = HVal<F, CPLX_H>::load(p, o);
+  if constexpr (FOLD) h.twice().template fma<VPL>(xs, acc);
+  else h.template fma<VPL>(xs, acc);
+}
+
 // One recursion step over all rows, x = v_s, y = v_{s-1} on entry.
 //   FIRST: y = H x                    else: y = 2 H x - y  (v_{s+1} over v_{s-1})
 //   doubling (BRAKET false): part[0] += <x|x>; part[1] += <x|y_in> (= <v_s|v_{s-1}>),
@@ -76,6 +85,7 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % LPR;
   Acc m0 = 0, m1 = 0;
+  constexpr bool FOLD = kFoldStep<F> && !FIRST;
   static_assert(!(CLS && (PIPE || KST == 2)), "class form: no column pipeline, no operator products");
 
   // class form: the table in shared memory (4-byte words: values, offsets, counts)
@@ -89,7 +99,13 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
     const int32_t vw = ne * (class_value_bytes<F, CPLX_H>() / 4);
     uint32_t* sw = reinterpret_cast<uint32_t*>(cls_smem);
     const uint32_t* gv = static_cast<const uint32_t*>(ct.val);
-    for (int32_t q = threadIdx.x; q < vw; q += blockDim.x) sw[q] = gv[q];
+    if constexpr (FOLD) {
+      F* dv = reinterpret_cast<F*>(cls_smem);
+      for (int32_t q = threadIdx.x; q < ne * (CPLX_H ? 2 : 1); q += blockDim.x)
+        dv[q] = times2(static_cast<const F*>(ct.val)[q]);
+    } else {
+      for (int32_t q = threadIdx.x; q < vw; q += blockDim.x) sw[q] = gv[q];
+    }
     for (int32_t q = threadIdx.x; q < ne; q += blockDim.x) sw[vw + q] = (uint32_t)ct.off[q];
     for (int32_t q = threadIdx.x; q < ct.n_cls; q += blockDim.x) sw[vw + ne + q] = (uint32_t)ct.cnt[q];
     s_off = reinterpret_cast<const int32_t*>(sw + vw);
@@ -100,6 +116,12 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
       const int32_t r0 = (reverse ? (n_tiles - 1 - t0) : t0) * ROWS_PER_TILE + warp * RPW + lane / LPR;
       if (r0 < n) c_next = __ldg(ct.cls + r0);
     }
+  }
+
+  HVal<F, true> add_c{F(0), F(0)};         // c_k of a Clenshaw step
+  if constexpr (KST == 3) {
+    const double f = is_dd<F> ? 0.5 : 1.0;
+    add_c = HVal<F, true>{F(f * ks.addc[0]), F(f * ks.addc[1])};
   }
 
   for (int32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -153,7 +175,10 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
     if constexpr (!FIRST) prev = ld_stream<F, VPL>(pv + me * VPL);   // pv == y: in place
     LaneV<F, VPL> acc, vacc;
 #pragma unroll
-    for (int q = 0; q < VPL; ++q) { acc.re[q] = 0; acc.im[q] = 0; }
+    for (int q = 0; q < VPL; ++q) {
+      if constexpr (FOLD) { acc.re[q] = negate(prev.re[q]); acc.im[q] = negate(prev.im[q]); }
+      else { acc.re[q] = 0; acc.im[q] = 0; }
+    }
     // column group of this lane (its VPL columns never straddle two groups)
     const int grp = (KST == 2 && ks.halves == 2 && sub * VPL >= R / 2) ? 1 : 0;
     const F* vval = nullptr;
@@ -167,7 +192,7 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
       for (int q = 0; q < VPL; ++q) { vacc.re[q] = 0; vacc.im[q] = 0; }
     }
     if (gather && CLS) {
-      HVal<F, CPLX_H>::load(diag, r).template fma<VPL>(xs, acc);
+      ell_entry<F, VPL, CPLX_H, FOLD>(diag, r, xs, acc);
       const int32_t cnt = s_cnt[c_cur];
       const int32_t tb = (int32_t)c_cur * ct.w;
       // a class's tail entries up to the table width (a multiple of 4) are
@@ -176,7 +201,24 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
       // instructions and registers); the wider types keep the predicates,
       // whose unconditional form holds more gathers in registers
       constexpr bool WHOLE = sizeof(F) == 4;
-      for (int k = 0; k < cnt; k += 4) {
+      int k0 = 0;
+      if constexpr (is_f64<F>) {
+        // FP64: whole groups, then single entries (a predicated product still
+        // takes its turn on the FP64 pipe)
+        for (; k0 + 4 <= cnt; k0 += 4) {
+          LaneV<F, VPL> xv[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            xv[u] = ld_ro<F, VPL>(x + ((int64_t)min(max(r + s_off[tb + k0 + u], 0), n - 1) * LPR + sub) * VPL);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) HVal<F, CPLX_H>::load_smem(s_val, tb + k0 + u).template fma<VPL>(xv[u], acc);
+        }
+#pragma unroll 1
+        for (; k0 < cnt; ++k0)
+          HVal<F, CPLX_H>::load_smem(s_val, tb + k0).template fma<VPL>(
+              ld_ro<F, VPL>(x + ((int64_t)min(max(r + s_off[tb + k0], 0), n - 1) * LPR + sub) * VPL), acc);
+      }
+      for (int k = k0; k < cnt; k += 4) {
         HVal<F, CPLX_H> h[4];
         LaneV<F, VPL> xv[4];
 #pragma unroll
@@ -192,19 +234,35 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
         for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], acc);
       }
     } else if (gather) {
-      HVal<F, CPLX_H>::load(diag, r).template fma<VPL>(xs, acc);
+      ell_entry<F, VPL, CPLX_H, FOLD>(diag, r, xs, acc);
       if constexpr (KST == 2) HVal<F, CPLX_H>::load(vdiag, r).template fma<VPL>(xs, vacc);
       const int32_t s = r >> 5, l = r & 31;
       const int32_t off = soff[s];
       const int32_t w = (soff[s + 1] - off) >> 5;
       const int32_t* cp = ecol + off + l;
-      // all of a row's gathers in flight together: predicated groups of 4
       int32_t cn[4];
-      if constexpr (PIPE) {
+      if constexpr (PIPE && !(is_f64<F> && KST != 2)) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) cn[u] = u < w ? __ldg(cp + u * 32) : r;
       }
-      for (int k = 0; k < w; k += 4) {
+      int k0 = 0;
+      if constexpr (is_f64<F> && KST != 2) {                        // as in the class form
+        for (; k0 + 4 <= w; k0 += 4) {
+          LaneV<F, VPL> xv[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            xv[u] = ld_ro<F, VPL>(x + ((int64_t)__ldg(cp + (k0 + u) * 32) * LPR + sub) * VPL);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            ell_entry<F, VPL, CPLX_H, FOLD>(eval, off + l + (int64_t)(k0 + u) * 32, xv[u], acc);
+        }
+#pragma unroll 1
+        for (; k0 < w; ++k0)
+          ell_entry<F, VPL, CPLX_H, FOLD>(eval, off + l + (int64_t)k0 * 32,
+                                          ld_ro<F, VPL>(x + ((int64_t)__ldg(cp + k0 * 32) * LPR + sub) * VPL), acc);
+      }
+      // all of a row's gathers in flight together: predicated groups of 4
+      for (int k = k0; k < w; k += 4) {
         int32_t c[4];
         HVal<F, CPLX_H> h[4];
 #pragma unroll
@@ -222,7 +280,13 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
 #pragma unroll
         for (int u = 0; u < 4; ++u) xv[u] = ld_ro<F, VPL>(x + ((int64_t)c[u] * LPR + sub) * VPL);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], acc);
+        for (int u = 0; u < 4; ++u) {
+          if constexpr (FOLD) {
+            h[u].twice().template fma<VPL>(xv[u], acc);
+          } else {
+            h[u].template fma<VPL>(xv[u], acc);
+          }
+        }
         if constexpr (KST == 2) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
@@ -233,19 +297,22 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
         }
       }
     }
+    if constexpr (KST == 3 && sizeof(F) == 8) {
+      // Clenshaw step of a Chebyshev expansion: b_k = 2 H b_{k+1} - b_{k+2} + c_k v, the
+      // last term summed with the row's (add_c = c_k / 2 where the sum is doubled after)
+      add_c.template fma<VPL>(ld_ro<F, VPL>(static_cast<const CT*>(ks.addv) + me * VPL), acc);
+    }
     finish_acc<F, VPL>(acc);
     if constexpr (KST == 2) finish_acc<F, VPL>(vacc);
     LaneV<F, VPL> out;
-    if constexpr (FIRST) out = acc;
+    if constexpr (FIRST || FOLD) out = acc;
     else recur_out<F, VPL>(acc, prev, out);
-    if constexpr (KST == 3) {
-      // Clenshaw step of a Chebyshev expansion: b_k = 2 H b_{k+1} - b_{k+2} + c_k v
+    if constexpr (KST == 3 && sizeof(F) == 4) {
       const LaneV<F, VPL> vv = ld_ro<F, VPL>(static_cast<const CT*>(ks.addv) + me * VPL);
-      const F cr = F(ks.addc[0]), ci = F(ks.addc[1]);
 #pragma unroll
       for (int q = 0; q < VPL; ++q) {
-        out.re[q] = out.re[q] + (cr * vv.re[q] - ci * vv.im[q]);
-        out.im[q] = out.im[q] + (cr * vv.im[q] + ci * vv.re[q]);
+        out.re[q] = out.re[q] + (add_c.r * vv.re[q] - add_c.i * vv.im[q]);
+        out.im[q] = out.im[q] + (add_c.r * vv.im[q] + add_c.i * vv.re[q]);
       }
     }
     // moment partial sums (before the store, from registers only); steps that

@@ -34,7 +34,7 @@ namespace {
 // few against the rows, and the scalars formed by one thread.
 // 1,025,280-site honeycomb, 200 iterations: 21.9 ms with a 38 us product (the step
 // kernel, with a norm it did not need), an 18 us update, a 6 us scaling and two host
-// round trips (48 us) per iteration; 11.5 ms now (27 + 21 us).
+// round trips (48 us) per iteration; 10.7 ms now (22 + 21 us).
 constexpr int kLzThreads = 512;
 constexpr int kLzWarps = kLzThreads / 32;
 
@@ -94,27 +94,31 @@ __global__ void __launch_bounds__(kLzThreads) lanczos_product_kernel(
     HV::load(diag, r).template fma<1>(xs, acc);
     if constexpr (CLS) {
       const int32_t c = __ldg(ct.cls + r), cnt = s_cnt[c], tb = c * ct.w;
-      for (int32_t k = 0; k < cnt; k += 4) {
+      int32_t k = 0;
+      for (; k + 4 <= cnt; k += 4) {
         LaneV<double, 1> xv[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (k + q < cnt) xv[q] = ld_ro<double, 1>(u + min(max(r + s_off[tb + k + q], 0), n - 1));
+        for (int q = 0; q < 4; ++q) xv[q] = ld_ro<double, 1>(u + min(max(r + s_off[tb + k + q], 0), n - 1));
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (k + q < cnt) HV::load_smem(s_val, tb + k + q).template fma<1>(xv[q], acc);
+        for (int q = 0; q < 4; ++q) HV::load_smem(s_val, tb + k + q).template fma<1>(xv[q], acc);
       }
+#pragma unroll 1
+      for (; k < cnt; ++k)
+        HV::load_smem(s_val, tb + k).template fma<1>(ld_ro<double, 1>(u + min(max(r + s_off[tb + k], 0), n - 1)), acc);
     } else {
       const int32_t s = r >> 5, o = soff[s], wd = (soff[s + 1] - o) >> 5;
       const int64_t b = (int64_t)o + (r & 31);
-      for (int32_t k = 0; k < wd; k += 4) {
+      int32_t k = 0;
+      for (; k + 4 <= wd; k += 4) {
         LaneV<double, 1> xv[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (k + q < wd) xv[q] = ld_ro<double, 1>(u + __ldg(ecol + b + (int64_t)(k + q) * 32));
+        for (int q = 0; q < 4; ++q) xv[q] = ld_ro<double, 1>(u + __ldg(ecol + b + (int64_t)(k + q) * 32));
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (k + q < wd) HV::load(eval, b + (int64_t)(k + q) * 32).template fma<1>(xv[q], acc);
+        for (int q = 0; q < 4; ++q) HV::load(eval, b + (int64_t)(k + q) * 32).template fma<1>(xv[q], acc);
       }
+#pragma unroll 1
+      for (; k < wd; ++k)
+        HV::load(eval, b + (int64_t)k * 32).template fma<1>(ld_ro<double, 1>(u + __ldg(ecol + b + (int64_t)k * 32)), acc);
     }
     dot = fma(xs.re[0], acc.re[0], dot);
     dot = fma(xs.im[0], acc.im[0], dot);
