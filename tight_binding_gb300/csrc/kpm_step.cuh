@@ -32,6 +32,42 @@ inline size_t class_smem_bytes(const ClassTab& ct) {
   return ne * class_value_bytes<F, CPLX_H>() + ne * 4 + (size_t)ct.n_cls * 4;
 }
 
+// The moment sums of a step, part[slot][CTA].  FP64 from here on, and an FP64
+// instruction holds its quarter of the SM for 64 clocks: steps without moments do no
+// sums at all, braket steps after the first (kTwo false) sum one value, and two values
+// share one shuffle tree (warp_pair_sum).  Against two full trees per warp and 16
+// serial adds per CTA in every step: square 64x64, R = 8, FP64 braket 4.66 -> 4.06 us a
+// step; honeycomb 301x253, R = 4: complex64 doubling 9.86 -> 6.77 us, FP64 doubling
+// 29.2 -> 23.9 us; square 500x333 with a flux, R = 6, double-float braket 28.0 -> 23.1 us.
+template <typename F, bool kTwo>
+__device__ __forceinline__ void step_sums(F m0, F m1, double* __restrict__ part) {
+  __shared__ double sh[2][kStepWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr (kTwo) {
+    const double d = warp_pair_sum((double)m0, (double)m1);
+    if ((lane & 15) == 0) sh[lane >> 4][warp] = d;
+  } else {
+    const double d = warp_sum((double)m0);
+    if (lane == 0) sh[0][warp] = d;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * kStepWarps) {
+    const int slot = threadIdx.x / kStepWarps;
+    double d = (kTwo || slot == 0) ? sh[slot][threadIdx.x % kStepWarps] : 0.0;
+#pragma unroll
+    for (int o = kStepWarps / 2; o > 0; o >>= 1) d += __shfl_xor_sync((1u << 2 * kStepWarps) - 1u, d, o);
+    if (threadIdx.x % kStepWarps == 0) part[slot * gridDim.x + blockIdx.x] = d;
+  }
+}
+// Complex64 steps call it out of line: inlined, its FP64 registers change how the row
+// loop is scheduled (both 40 registers; honeycomb 701x600 with vacancies, ELL form:
+// R = 32 122.0 -> 108.8 us a step, R = 16 66.1 -> 59.7; honeycomb 1024x1024, class form,
+// R = 32 253.2 -> 248.8).  The wider types run 2-6% faster with it inlined.
+template <bool kTwo>
+__device__ __noinline__ void step_sums_call(float m0, float m1, double* __restrict__ part) {
+  step_sums<float, kTwo>(m0, m1, part);
+}
+
 // acc += (2) p[o] x for a matrix value in memory
 template <typename F, int VPL, bool CPLX_H, bool FOLD>
 __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, const LaneV<F, VPL>& xs,
@@ -68,8 +104,12 @@ __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, co
 //   its value comes from there too, so no column index or value is loaded and
 //   the only index read (the row's class byte) is issued one grid-stride
 //   iteration ahead.  Same entries in the same order as the ELL: the same sums.
+//   Class-form steps of the 8-byte types may take all the registers they like (a stated
+//   minimum of one CTA; unstated, the compiler stops at 64): they are bound by arithmetic,
+//   and fewer warps with more gathers each in flight run faster (honeycomb 1024x1024,
+//   R = 32: FP64 braket 1,483 -> 1,226 us, double-float 795 -> 744-762 us).
 template <typename F, int R, bool CPLX_H, bool FIRST, bool BRAKET, int KST = 0, bool PIPE = false, bool CLS = false>
-__global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
+__global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0) kpm_step_kernel(
     int32_t n, int32_t n_tiles, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
     const F* __restrict__ eval, const F* __restrict__ diag, const typename C2<F>::T* __restrict__ x,
     typename C2<F>::T* y, const typename C2<F>::T* pv, const typename C2<F>::T* __restrict__ bras,
@@ -349,31 +389,9 @@ __global__ void __launch_bounds__(kStepThreads) kpm_step_kernel(
       }
     }
   }
-  // FP64 from here on.  An FP64 instruction holds its quarter of the SM for 64 clocks,
-  // so steps without moments do no sums at all, braket steps after the first sum one
-  // value, and two values share one shuffle tree (warp_pair_sum).  Against two full
-  // trees per warp and 16 serial adds per CTA in every step: square 64x64, R = 8, FP64
-  // braket 4.66 -> 4.06 us a step; honeycomb 301x253, R = 4: complex64 doubling 9.86 ->
-  // 6.77 us, FP64 doubling 29.2 -> 23.9 us; square 500x333 with a flux, R = 6,
-  // double-float braket 28.0 -> 23.1 us.
   if constexpr (KST == 0) {
-    constexpr bool kTwo = !BRAKET || FIRST;
-    __shared__ double sh[2][kStepWarps];
-    if constexpr (kTwo) {
-      const double d = warp_pair_sum((double)m0, (double)m1);
-      if ((lane & 15) == 0) sh[lane >> 4][warp] = d;
-    } else {
-      const double d = warp_sum((double)m0);
-      if (lane == 0) sh[0][warp] = d;
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 * kStepWarps) {
-      const int slot = threadIdx.x / kStepWarps;
-      double d = (kTwo || slot == 0) ? sh[slot][threadIdx.x % kStepWarps] : 0.0;
-#pragma unroll
-      for (int o = kStepWarps / 2; o > 0; o >>= 1) d += __shfl_xor_sync((1u << 2 * kStepWarps) - 1u, d, o);
-      if (threadIdx.x % kStepWarps == 0) part[slot * gridDim.x + blockIdx.x] = d;
-    }
+    if constexpr (sizeof(F) == 4) step_sums_call<!BRAKET || FIRST>(m0, m1, part);
+    else step_sums<F, !BRAKET || FIRST>(m0, m1, part);
   }
 }
 
