@@ -195,10 +195,24 @@ static int tma_setup(int R, bool braket, int smem, int* occ) {
   return fail(TBK_ERR_UNSUPPORTED, "chunk width %d not instantiated", R);
 }
 
+// Width of the chunks that R vectors are processed in, at most cap (even) a chunk: the
+// vectors spread evenly over the fewest chunks, rounded up to a lane's two vectors
+// (complex64, double-float).  A width close to a power of two takes it: those kernels
+// know their width at compile time (honeycomb 701x600, complex64: 20 vectors 80.9 us
+// a step at width 20 against 107.8 at 32; with vacancies 83.5 against 108.8, FP64 braket
+// 334 against 484).
+int step_width(int prec, int R, int cap) {
+  const int chunks = (R + cap - 1) / cap;
+  int w = (R + chunks - 1) / chunks;
+  if (prec != TBK_PREC_FP64 && w > 1) w = (w + 1) & ~1;
+  int p = 1;
+  while (p < w) p <<= 1;
+  return p * 15 <= w * 16 ? p : w;
+}
+
 static int rows_per_tile(int prec, int Rc) {
-  int vpl = (prec == TBK_PREC_MIXED || prec == TBK_PREC_DD) ? (Rc >= 2 ? 2 : 1) : 1;
-  int lpr = Rc / vpl;
-  return (32 / lpr) * kStepWarps;
+  const int vpl = prec != TBK_PREC_FP64 && Rc >= 2 ? 2 : 1;
+  return kStepThreads / (Rc / vpl);
 }
 
 // ---------------------------------------------------------------- internal API
@@ -230,15 +244,22 @@ size_t class_smem(const EllDev& E, int prec) {
   return ne * fb * (E.cplx ? 2 : 1) + ne * 4 + (size_t)E.n_cls * 4;
 }
 
+// CTAs per SM of A's form.  FP64: the smaller of both forms', so that they group their
+// partial sums alike and give the same bits.
+static int step_occupancy(tbk_sparse_s* A, int Rc, int prec, bool sums) {
+  const bool cplx = A->ell.cplx != 0, cls = A->ell.cls_state == 1;
+  const int oc = cls || prec == TBK_PREC_FP64 ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec), sums) : 64;
+  const int oe = !cls || prec == TBK_PREC_FP64 ? occupancy_prec(prec, cplx, Rc, sums) : 64;
+  return std::min(oc, oe);
+}
+
 int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st) {
   TBK_TRY(ensure_ell(A, st));
   if (prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(A, st));
   TBK_TRY(ensure_classes(A, st));
   const int rpt = rows_per_tile(prec, Rc);
   *n_tiles = (A->rows + rpt - 1) / rpt;
-  const bool cplx = A->ell.cplx != 0;
-  const int occ = A->ell.cls_state == 1 ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec))
-                                        : occupancy_prec(prec, cplx, Rc);
+  const int occ = step_occupancy(A, Rc, prec, false);
   *grid = std::max(1, std::min(*n_tiles, sm_count() * occ));
   return TBK_OK;
 }
@@ -324,20 +345,20 @@ static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const St
 int launch_step_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
-int occupancy_f32(bool cplx, int R);
-int occupancy_f64(bool cplx, int R);
-int occupancy_dd(bool cplx, int R);
+int occupancy_f32(bool cplx, int R, bool sums);
+int occupancy_f64(bool cplx, int R, bool sums);
+int occupancy_dd(bool cplx, int R, bool sums);
 int launch_step_cls_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
-int occupancy_cls_f32(bool cplx, int R, size_t smem);
-int occupancy_cls_f64(bool cplx, int R, size_t smem);
-int occupancy_cls_dd(bool cplx, int R, size_t smem);
+int occupancy_cls_f32(bool cplx, int R, size_t smem, bool sums);
+int occupancy_cls_f64(bool cplx, int R, size_t smem, bool sums);
+int occupancy_cls_dd(bool cplx, int R, size_t smem, bool sums);
 
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem) {
-  if (prec == TBK_PREC_FP64) return occupancy_cls_f64(cplx, R, smem);
-  if (prec == TBK_PREC_DD) return occupancy_cls_dd(cplx, R, smem);
-  return occupancy_cls_f32(cplx, R, smem);
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums) {
+  if (prec == TBK_PREC_FP64) return occupancy_cls_f64(cplx, R, smem, sums);
+  if (prec == TBK_PREC_DD) return occupancy_cls_dd(cplx, R, smem, sums);
+  return occupancy_cls_f32(cplx, R, smem, sums);
 }
 
 int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid,
@@ -352,10 +373,10 @@ int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, 
   return launch_step_f32(cplx, R, a, first, braket, grid, st);
 }
 
-int occupancy_prec(int prec, bool cplx, int R) {
-  if (prec == TBK_PREC_FP64) return occupancy_f64(cplx, R);
-  if (prec == TBK_PREC_DD) return occupancy_dd(cplx, R);
-  return occupancy_f32(cplx, R);
+int occupancy_prec(int prec, bool cplx, int R, bool sums) {
+  if (prec == TBK_PREC_FP64) return occupancy_f64(cplx, R, sums);
+  if (prec == TBK_PREC_DD) return occupancy_dd(cplx, R, sums);
+  return occupancy_f32(cplx, R, sums);
 }
 
 int load_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, const double2* src, void* dst,
@@ -966,6 +987,8 @@ int tbk_kpm_create(tbk_kpm* out, tbk_sparse Ht, int32_t R, int32_t flags) {
   const int rmax = prec == TBK_PREC_MIXED ? 64 : 32;
   int rc = 1;
   while (rc < R && rc < rmax) rc <<= 1;
+  // the opt-in forms exist for powers of two only
+  if (!(flags & (TBK_FLAG_STAGED | TBK_FLAG_TWO_STEP | TBK_FLAG_PERSISTENT))) rc = step_width(prec, R, rmax);
   P->Rc = rc;
   P->n_chunks = (R + rc - 1) / rc;
   const int rpt = rows_per_tile(prec, rc);
@@ -980,13 +1003,13 @@ int tbk_kpm_create(tbk_kpm* out, tbk_sparse Ht, int32_t R, int32_t flags) {
     }
   }
   P->use_cls = Ht->ell.cls_state == 1;
-  occ = P->use_cls ? occupancy_cls_prec(prec, cplx, rc, class_smem(Ht->ell, prec)) : occupancy_prec(prec, cplx, rc);
+  occ = step_occupancy(Ht, rc, prec, true);
   P->grid = std::max(1, std::min(P->n_tiles, sm_count() * occ));
   P->grid_max = P->grid;
   if (const char* e = getenv("TBK_PREFETCH")) P->pf_dist = atoi(e);   // tuning override
   P->n_pad = (int64_t)Ht->ell.n_slices * 32;
   // TMA-staged kernel: tiles of whole slices, ~8 KB of vector rows per stream
-  {
+  if (flags & TBK_FLAG_STAGED) {
     const int row_bytes = rc * (int)P->csize;
     int TR = 8192 / row_bytes;
     if (const char* e = getenv("TBK_TMA_ROWS")) TR = atoi(e);   // tuning override (rows per tile)

@@ -77,6 +77,16 @@ __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, co
   else h.template fma<VPL>(xs, acc);
 }
 
+// Steps bound by arithmetic may take more registers than the compiler gives them by
+// itself: fewer warps with more gathers each in flight run faster (honeycomb 1024x1024,
+// R = 32: FP64 braket 1,483 -> 1,364 us, double-float doubling 795 -> 744-762 us).  FP64: 4
+// CTAs per SM in both forms, which then keep one grid and so the same bits (3 would give
+// the class form 1,227 us, the ELL form, R = 32 with vacancies, 577 against 484).  Double-float:
+// any number in the class form's moment steps; not in the ELL form (701x600 with
+// vacancies, R = 20: 200 -> 216 us) nor in its Clenshaw steps.  0: not stated.
+template <typename F, int KST, bool CLS>
+constexpr int kMinCtas = is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
+
 // One recursion step over all rows, x = v_s, y = v_{s-1} on entry.
 //   FIRST: y = H x                    else: y = 2 H x - y  (v_{s+1} over v_{s-1})
 //   doubling (BRAKET false): part[0] += <x|x>; part[1] += <x|y_in> (= <v_s|v_{s-1}>),
@@ -104,26 +114,26 @@ __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, co
 //   its value comes from there too, so no column index or value is loaded and
 //   the only index read (the row's class byte) is issued one grid-stride
 //   iteration ahead.  Same entries in the same order as the ELL: the same sums.
-//   Class-form steps of the 8-byte types may take all the registers they like (a stated
-//   minimum of one CTA; unstated, the compiler stops at 64): they are bound by arithmetic,
-//   and fewer warps with more gathers each in flight run faster (honeycomb 1024x1024,
-//   R = 32: FP64 braket 1,483 -> 1,226 us, double-float 795 -> 744-762 us).
+//   R: vectors per row, a power of two; 0: any other width, LPR lanes per row given
+//   at run time (rows stay whole within a CTA, a few threads at its end idle).
 template <typename F, int R, bool CPLX_H, bool FIRST, bool BRAKET, int KST = 0, bool PIPE = false, bool CLS = false>
-__global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0) kpm_step_kernel(
+__global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_kernel(
     int32_t n, int32_t n_tiles, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
     const F* __restrict__ eval, const F* __restrict__ diag, const typename C2<F>::T* __restrict__ x,
     typename C2<F>::T* y, const typename C2<F>::T* pv, const typename C2<F>::T* __restrict__ bras,
-    double* __restrict__ part, int store, int reverse, int gather, int pf_dist, const KStore ks, const ClassTab ct) {
+    double* __restrict__ part, int store, int reverse, int gather, int pf_dist, const KStore ks, const ClassTab ct, int32_t lpr) {
   using CT = typename C2<F>::T;
-  constexpr int VPL = (R >= VecW<F>::max_vpl) ? VecW<F>::max_vpl : 1;
-  constexpr int LPR = R / VPL;             // lanes per row
-  constexpr int RPW = 32 / LPR;            // rows per warp
-  constexpr int ROWS_PER_TILE = RPW * kStepWarps;
-  static_assert(LPR >= 1 && LPR <= 32 && (32 % LPR) == 0, "R out of range");
+  constexpr int VPL = (R == 0 || R >= VecW<F>::max_vpl) ? VecW<F>::max_vpl : 1;
+  static_assert(R == 0 || (R / VPL >= 1 && R / VPL <= 32 && (32 % (R / VPL)) == 0), "R out of range");
+  const int LPR = R > 0 ? R / VPL : lpr;   // lanes per row
+  const int RW = LPR * VPL;                // vectors per row
+  const int ROWS_PER_TILE = kStepThreads / LPR;
+  const int trow = threadIdx.x / LPR;      // this thread's row in a tile (none: past n)
+  const bool idle = R == 0 && trow >= ROWS_PER_TILE;
   using Acc = F;                           // per-thread sums in the vector precision
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sub = lane % LPR;
+  const int sub = threadIdx.x % LPR;
   Acc m0 = 0, m1 = 0;
   constexpr bool FOLD = kFoldStep<F> && !FIRST;
   static_assert(!(CLS && (PIPE || KST == 2)), "class form: no column pipeline, no operator products");
@@ -153,8 +163,8 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
     __syncthreads();
     const int32_t t0 = blockIdx.x;
     if (t0 < n_tiles) {
-      const int32_t r0 = (reverse ? (n_tiles - 1 - t0) : t0) * ROWS_PER_TILE + warp * RPW + lane / LPR;
-      if (r0 < n) c_next = __ldg(ct.cls + r0);
+      const int32_t r0 = (reverse ? (n_tiles - 1 - t0) : t0) * ROWS_PER_TILE + trow;
+      if (r0 < n && !idle) c_next = __ldg(ct.cls + r0);
     }
   }
 
@@ -170,8 +180,8 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
       const int32_t tn = t + (int32_t)gridDim.x;
       c_next = 0;
       if (tn < n_tiles) {
-        const int32_t rn = (reverse ? (n_tiles - 1 - tn) : tn) * ROWS_PER_TILE + warp * RPW + lane / LPR;
-        if (rn < n) c_next = __ldg(ct.cls + rn);
+        const int32_t rn = (reverse ? (n_tiles - 1 - tn) : tn) * ROWS_PER_TILE + trow;
+        if (rn < n && !idle) c_next = __ldg(ct.cls + rn);
       }
     }
     const int32_t tile = reverse ? (n_tiles - 1 - t) : t;
@@ -184,11 +194,11 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
         const int64_t rf = (int64_t)tilef * ROWS_PER_TILE;
         const int32_t nr = (int32_t)min((int64_t)ROWS_PER_TILE, (int64_t)n - rf);
         if (nr > 0) {
-          const uint32_t vb = (uint32_t)nr * (uint32_t)(R * sizeof(CT));
+          const uint32_t vb = (uint32_t)nr * (uint32_t)(RW * sizeof(CT));
           if ((vb & 15u) == 0) {
-            bulk_prefetch_l2(x + rf * R, vb);
-            if (!FIRST) bulk_prefetch_l2(pv + rf * R, vb);
-            if (BRAKET) bulk_prefetch_l2(bras + rf * R, vb);
+            bulk_prefetch_l2(x + rf * RW, vb);
+            if (!FIRST) bulk_prefetch_l2(pv + rf * RW, vb);
+            if (BRAKET) bulk_prefetch_l2(bras + rf * RW, vb);
           }
           if constexpr (!CLS) {
             if (gather) {
@@ -207,8 +217,8 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
         }
       }
     }
-    const int32_t r = tile * ROWS_PER_TILE + warp * RPW + lane / LPR;
-    if (r >= n) continue;
+    const int32_t r = tile * ROWS_PER_TILE + trow;
+    if (r >= n || idle) continue;
     const int64_t me = (int64_t)r * LPR + sub;
     const LaneV<F, VPL> xs = ld_ro<F, VPL>(x + me * VPL);
     LaneV<F, VPL> prev;
@@ -220,7 +230,7 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
       else { acc.re[q] = 0; acc.im[q] = 0; }
     }
     // column group of this lane (its VPL columns never straddle two groups)
-    const int grp = (KST == 2 && ks.halves == 2 && sub * VPL >= R / 2) ? 1 : 0;
+    const int grp = (KST == 2 && ks.halves == 2 && sub * VPL >= RW / 2) ? 1 : 0;
     const F* vval = nullptr;
     const F* vdiag = nullptr;
     if constexpr (KST == 2) {
@@ -372,13 +382,13 @@ __global__ void __launch_bounds__(kStepThreads, (CLS && sizeof(F) == 8) ? 1 : 0)
       // block km[0] of the K-tiled store: one rounding per value
 #pragma unroll
       for (int q = 0; q < VPL; ++q) {
-        const int64_t k = (int64_t)r * R + sub * VPL + q;
+        const int64_t k = (int64_t)r * RW + sub * VPL + q;
         ks.store[0][((k >> 4) * ks.kM + ks.km[0]) * 16 + (k & 15)] = make_float2(to_f32(out.re[q]), to_f32(out.im[q]));
       }
     } else if constexpr (KST == 2) {
       const int32_t kmg = grp ? ks.km[1] : ks.km[0];
       if (kmg >= 0) {
-        const int32_t Rg = R / ks.halves;
+        const int32_t Rg = RW / ks.halves;
         const LaneV<F, VPL>& sv = (grp ? ks.usev[1] : ks.usev[0]) ? vacc : out;
         float2* dst = grp ? ks.store[1] : ks.store[0];
 #pragma unroll
@@ -416,6 +426,7 @@ struct StepArgs {
   bool pipe = false;           // ELL wider than 4: pipelined column loads
   bool cls = false;            // row classes (ct) instead of the ELL's columns and values
   ClassTab ct;
+  int32_t lpr = 0;             // lanes per row of a width without its own instantiation (R = 0)
 };
 
 template <typename F, int R, bool CPLX_H, bool CLS>
@@ -433,20 +444,21 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
     if constexpr (CLS)                                                                                \
       kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, false, true><<<grid, kStepThreads, smem, st>>>(       \
           a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
-          a.ct);                                                                                      \
+          a.ct, a.lpr);                                                                                      \
     else if (a.pipe)                                                                                  \
       kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, true><<<grid, kStepThreads, 0, st>>>(                 \
           a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
-          a.ct);                                                                                      \
+          a.ct, a.lpr);                                                                                      \
     else                                                                                              \
       kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, false><<<grid, kStepThreads, 0, st>>>(                \
           a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
-          a.ct);                                                                                      \
+          a.ct, a.lpr);                                                                                      \
   } while (0)
   if (a.kst != 0) {
     if (braket) return fail(TBK_ERR_UNSUPPORTED, "K-tiled store with a braket step");
-    constexpr int VPLR = (R >= VecW<F>::max_vpl) ? VecW<F>::max_vpl : 1;
-    if (a.kst == 2 && a.ks.halves == 2 && (R / 2) % VPLR != 0)
+    constexpr int VPLR = (R == 0 || R >= VecW<F>::max_vpl) ? VecW<F>::max_vpl : 1;
+    const int rw = R > 0 ? R : a.lpr * VPLR;
+    if (a.kst == 2 && a.ks.halves == 2 && (rw / 2) % VPLR != 0)
       return fail(TBK_ERR_UNSUPPORTED, "column groups narrower than a lane's vectors");
     if (a.kst == 3) {
       if (first) return fail(TBK_ERR_UNSUPPORTED, "Clenshaw term on a first step");
@@ -478,36 +490,47 @@ inline int launch_step(int R, const StepArgs& a, bool first, bool braket, int gr
       if constexpr (sizeof(F) == 4) return launch_step_r<F, 64, CPLX_H, CLS>(a, first, braket, grid, st);
       break;
   }
+  if (R > 0 && R < 64 && R % VecW<F>::max_vpl == 0) {
+    StepArgs b = a;
+    b.lpr = R / VecW<F>::max_vpl;
+    return launch_step_r<F, 0, CPLX_H, CLS>(b, first, braket, grid, st);
+  }
   return fail(TBK_ERR_UNSUPPORTED, "chunk width %d not instantiated", R);
 }
 
 
 template <typename F, bool CPLX_H, int R, bool CLS = false>
-inline int occupancy_blocks(size_t smem = 0) {
+inline int occupancy_blocks(size_t smem, bool sums) {
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 0, false, CLS>,
-                                                kStepThreads, smem);
+  if (sums)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 0, false, CLS>,
+                                                  kStepThreads, smem);
+  else
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 4, false, CLS>,
+                                                  kStepThreads, smem);
   return nb > 0 ? nb : 1;
 }
 
 template <typename F, bool CLS>
-inline int occupancy_r(bool cplx, int R, size_t smem) {
+inline int occupancy_r(bool cplx, int R, size_t smem, bool sums) {
   switch (R) {
-    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem) : occupancy_blocks<F, false, 1, CLS>(smem);
-    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem) : occupancy_blocks<F, false, 2, CLS>(smem);
-    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem) : occupancy_blocks<F, false, 4, CLS>(smem);
-    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem) : occupancy_blocks<F, false, 8, CLS>(smem);
-    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem) : occupancy_blocks<F, false, 16, CLS>(smem);
-    default: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem) : occupancy_blocks<F, false, 32, CLS>(smem);
+    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem, sums) : occupancy_blocks<F, false, 1, CLS>(smem, sums);
+    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem, sums) : occupancy_blocks<F, false, 2, CLS>(smem, sums);
+    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem, sums) : occupancy_blocks<F, false, 4, CLS>(smem, sums);
+    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem, sums) : occupancy_blocks<F, false, 8, CLS>(smem, sums);
+    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem, sums) : occupancy_blocks<F, false, 16, CLS>(smem, sums);
+    case 32: case 64: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem, sums) : occupancy_blocks<F, false, 32, CLS>(smem, sums);
+    default: return cplx ? occupancy_blocks<F, true, 0, CLS>(smem, sums) : occupancy_blocks<F, false, 0, CLS>(smem, sums);
   }
 }
 
 // per-precision entry points (TBK_PREC_*); a.cls selects the class form
 int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid,
                      cudaStream_t st);
-int occupancy_prec(int prec, bool cplx, int R);
-// CTAs per SM of the class-form kernel with its shared-memory table
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem);
+// CTAs per SM; sums: of the steps that form moment sums
+int occupancy_prec(int prec, bool cplx, int R, bool sums);
+// the same of the class-form kernel with its shared-memory table
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums);
 // the class table of a matrix in a precision (ct.n_cls == 0: no class form)
 ClassTab class_tab(const EllDev& E, int prec);
 size_t class_smem(const EllDev& E, int prec);

@@ -444,10 +444,22 @@ cudaMemPool_t kubo_pool() {
   return pools[dev];
 }
 
-int pick_chunk(int R) {
-  int c = 1;
-  while (c < R && c < 32) c <<= 1;
-  return c;
+// Vectors per chunk: the widest whose two stored sides (per_vector bytes each vector)
+// fit the budget; 1 when none does.  The same in every recursion precision (the GEMM
+// then sums in the same order).  both: a power of two (the widths of the one recursion
+// that carries both sides).
+int pick_chunk(int R, bool both, double per_vector, double budget) {
+  if (both) {
+    int c = 1;
+    while (c < R && c < 32) c <<= 1;
+    while (c > 1 && per_vector * c > budget) c >>= 1;
+    return c;
+  }
+  for (int cap = 32; cap > 1; cap -= 2) {
+    const int w = step_width(TBK_PREC_MIXED, R, cap);
+    if (per_vector * w <= budget) return w;
+  }
+  return 1;
 }
 
 }  // namespace
@@ -476,8 +488,6 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   for (auto* o : ops) if (o) TBK_TRY(ensure_ell(o, st));
   trace.mark("ell");
   const int64_t n_pad = (int64_t)Ht->ell.n_slices * 32;
-  // chunk of random vectors: both stored sides within the budget
-  int Rc = pick_chunk(R);
   // default budget: 60% of the free device memory (more vectors per chunk stream
   // the matrix fewer times)
   double budget = block_budget_gb * 1e9;
@@ -488,7 +498,11 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   }
   const bool f64b = (flags & TBK_MU_FP64_BLOCKS) != 0;   // FP64 reference form: complex128 blocks, FP64 GEMM
   const double sel = f64b ? 16.0 : 8.0;                   // bytes per stored element
-  while (Rc > 1 && 2.0 * M * n_pad * Rc * sel > budget) Rc >>= 1;
+  const int prec = (flags & TBK_MU_MIXED_RECURSION) ? TBK_PREC_MIXED
+                   : (flags & TBK_MU_DD_RECURSION)  ? TBK_PREC_DD
+                                                    : TBK_PREC_FP64;
+  // chunk of random vectors: both stored sides within the budget
+  const int Rc = pick_chunk(R, (flags & TBK_MU_BOTH_SIDES) != 0, 2.0 * M * n_pad * sel, budget);
   if (2.0 * M * n_pad * Rc * sel > budget)
     return fail(TBK_ERR_BUDGET, "stored Chebyshev blocks need %.1f GB > budget %.1f GB", 2.0 * M * n_pad * sel / 1e9,
                 budget / 1e9);
@@ -498,9 +512,6 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // near the band edges, where the Kubo weights 1/(1-e^2)^2 are largest; each
   // stored value is rounded to complex64 exactly once); TBK_MU_MIXED_RECURSION
   // runs them in complex64 with FP32 H~ (HBM-bound instead of FP64-pipe-bound).
-  const int prec = (flags & TBK_MU_MIXED_RECURSION) ? TBK_PREC_MIXED
-                   : (flags & TBK_MU_DD_RECURSION)  ? TBK_PREC_DD
-                                                    : TBK_PREC_FP64;
   const size_t csz = prec == TBK_PREC_MIXED ? sizeof(float2) : sizeof(double2);
   DevBuf Ls, Rs, work, partd, part, macc, gdev, kstage;
   const int64_t blk16 = (blk + 15) / 16 * 16;           // K padded to whole 16-element tiles (zeros)

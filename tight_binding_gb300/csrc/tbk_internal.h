@@ -163,6 +163,7 @@ struct KStore {
 // TBK_PREC_* (complex64, complex128 or double-float vectors): y = H x (first)
 // or y = 2 H x - pv; moment partials into part[2 * grid].  Block loaders:
 // Eigen-layout kets / seeded random phases.
+int step_width(int prec, int R, int cap);   // chunk width of R vectors
 int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st);
 // kstore: optional complex64 K-tiled store that receives the step's output as
 // block km of kM (store_y false: only there)
