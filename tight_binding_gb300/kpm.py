@@ -179,6 +179,13 @@ def kernel_seq(N: int, kernel: Kernel) -> np.ndarray:
 
 
 # -------------------------------------------------------------- Green's function
+def _doubles(precision) -> bool:
+    """Whether moments of equal bras and kets come from half the steps by the product
+    rule.  Not in complex64: mu_2n = 2 <v_n|v_n> - mu_0 carries the single-precision
+    sums' error of mu_0, <b|v_n> only that of the small moment itself."""
+    return _prec(precision) != capi.PREC_MIXED
+
+
 class GreenFunctionImag:
     """Functor e -> <bras| Im G(e) |kets> from Chebyshev moments, TB/lattice.h:600-647."""
 
@@ -188,11 +195,24 @@ class GreenFunctionImag:
         same = bras is kets
         K = _block(kets, n)
         B = K if same else _block(bras, n)
-        solver = KpmSolver(G.scaled_HE, K.shape[1], precision=precision, doubling=False)
-        self.moments = solver.run(G.N, B, K)
+        solver = KpmSolver(G.scaled_HE, K.shape[1], precision=precision, doubling=same and _doubles(precision))
+        self._finish(solver.run(G.N, B, K), kernel)
+
+    @classmethod
+    def of_random_phases(cls, G: "GreenFunction", R: int, seed: int, precision="fp64", kernel: Kernel | None = None):
+        """The functor of R seeded random-phase vectors as bras and kets, drawn on the
+        device: the vectors of bases_of_uniform_ampl_with_random_phases(n, R, seed)."""
+        self = object.__new__(cls)
+        self.G = G
+        solver = KpmSolver(G.scaled_HE, R, precision=precision, doubling=_doubles(precision))
+        self._finish(solver.run_random(G.N, seed), kernel)
+        return self
+
+    def _finish(self, moments: np.ndarray, kernel: Kernel | None) -> None:
+        self.moments = moments
         # the reference hard-codes Lorentz(N, 4) here (TB/lattice.h:613)
         self.kernel = kernel if kernel is not None else Lorentz(4.0)
-        self.g = self.kernel.seq(G.N)
+        self.g = self.kernel.seq(self.G.N)
 
     @staticmethod
     def weight(x: float) -> float:
@@ -363,8 +383,7 @@ def time_evolve(G: "GreenFunction", t: float, kets, precision="dd", tol: float =
 # ------------------------------------------------------------------ DoS entry points
 def density_of_states_function(G: GreenFunction, R: int = 4, seed: int = 0, precision="fp64"):
     """TB/functions.h:5-13: returns E -> -1/(4 pi) f(G.scale(E + 0i, i))."""
-    kets = bases_of_uniform_ampl_with_random_phases(G.scaled_HE.shape[0], R, seed)
-    f = G.imag(kets, kets, precision=precision)
+    f = GreenFunctionImag.of_random_phases(G, R, seed, precision)
 
     def dos(E):
         omega_t = G.scale(np.asarray(E, dtype=np.complex128) + 0j, 1.0j)
@@ -379,8 +398,7 @@ def density_of_states_seq(X: PartialLattice, N: int, E_list, E_min: float, E_max
     E_max+1e-8), R random-phase kets, rho(e) = -f(e)/(R pi) on already rescaled e."""
     H = X.get_Hamiltonian_periodic_extend_bare_sparse([1] * X.dim, scalar)
     G = GreenFunction(N, H, E_min - 1e-8, E_max + 1e-8)
-    kets = bases_of_uniform_ampl_with_random_phases(X.get_total_number(), R, seed)
-    f = G.imag(kets, kets, precision=precision, kernel=kernel)
+    f = GreenFunctionImag.of_random_phases(G, R, seed, precision, kernel)
     e = np.ascontiguousarray(E_list, dtype=np.float64)
     return -1.0 / R / math.pi * f(e)
 
