@@ -303,8 +303,9 @@ int tbk_cheb_braket_complex(int32_t n_rows, int64_t nnz, const int32_t* col_ptr,
                             const int32_t* row_idx, const double* values, int32_t n,
                             const double* bras, const double* kets, int32_t R,
                             int32_t flags, double* mu_out);
-/* Frees the matrix and plans cached by tbk_cheb_braket_* (no counterpart in
- * the reference, which keeps nothing between calls). */
+/* Frees the matrix and plans cached by tbk_cheb_braket_*, and the memory the
+ * library's workspace pool keeps on the current device (at most 256 MB; no
+ * counterpart in the reference, which keeps nothing between calls). */
 void tbk_cheb_braket_release(void);
 /* Polls a bounded device wait of the TMA-staged step kernel (TBK_FLAG_STAGED)
  * makes before it gives up, records an error and lets the call return
@@ -402,8 +403,9 @@ enum {
 int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_sparse BR, int32_t M,
                 int32_t R, uint64_t seed, const double* kets, int32_t kernel_kind, double kp0,
                 double kp1, int32_t flags, double block_budget_gb, double* mu_out, void* stream);
-/* Returns the memory tbk_kubo_mu's pool keeps on the current device (no
- * counterpart in the reference).  Calls in flight keep theirs. */
+/* Returns the memory that tbk_kubo_mu's pool and the library's workspace pool
+ * keep on the current device (no counterpart in the reference).  Calls in
+ * flight keep theirs. */
 int tbk_kubo_release(void);
 /* Device time of the last tbk_kubo_mu call in this process (CUDA events on its
  * stream): building the stored blocks, the mu GEMM (+ split-K reduction), the

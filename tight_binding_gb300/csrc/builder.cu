@@ -966,6 +966,7 @@ static int build_matrix(tbk_sparse* out, tbk_lattice L, int32_t mode, const int3
   *out = nullptr;
   if (mode < 0 || mode > 2) return fail(TBK_ERR_INVALID, "unknown build mode %d", mode);
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const Cell& C = L->cell;
   if (C.hops.empty()) { /* "Warning: no hopping is added!" — an all-zero matrix */ }
   BuildParams P;
@@ -1107,6 +1108,7 @@ int tbk_sparse_from_csc(tbk_sparse* out, int32_t rows, int32_t cols, int64_t nnz
   *out = nullptr;
   if (rows < 0 || cols < 0 || nnz < 0 || nnz > INT32_MAX) return fail(TBK_ERR_INVALID, "tbk_sparse_from_csc: bad sizes");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   tbk_sparse_s* A = nullptr;
   TBK_TRY(new_sparse(&A, rows, cols, nnz, is_complex ? 1 : 0));
   cudaMemcpyKind k = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
@@ -1122,6 +1124,7 @@ int tbk_sparse_from_csc(tbk_sparse* out, int32_t rows, int32_t cols, int64_t nnz
 
 int tbk_sparse_row_classes(tbk_sparse A, int32_t* n_classes, void* stream) {
   if (!A || !n_classes) return fail(TBK_ERR_INVALID, "tbk_sparse_row_classes: null argument");
+  ScratchScope scope(as_stream(stream));
   TBK_TRY(ensure_classes(A, as_stream(stream)));
   *n_classes = A->ell.cls_state == 1 ? A->ell.n_cls : 0;
   return TBK_OK;
@@ -1139,6 +1142,7 @@ int tbk_sparse_info(tbk_sparse A, int32_t* rows, int32_t* cols, int64_t* nnz, in
 int tbk_sparse_download(tbk_sparse A, int32_t* col_ptr, int32_t* row_idx, double* values, void* stream) {
   if (!A) return fail(TBK_ERR_INVALID, "tbk_sparse_download: null matrix");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   if (col_ptr) TBK_CUDA(cudaMemcpyAsync(col_ptr, A->col_ptr.p, sizeof(int32_t) * (A->cols + 1), cudaMemcpyDeviceToHost, st));
   if (row_idx && A->nnz) TBK_CUDA(cudaMemcpyAsync(row_idx, A->row_idx.p, sizeof(int32_t) * A->nnz, cudaMemcpyDeviceToHost, st));
   if (values && A->nnz)
@@ -1158,6 +1162,7 @@ int tbk_sparse_rescale(tbk_sparse* out, tbk_sparse H, double a, double b, void* 
   if (H->rows != H->cols) return fail(TBK_ERR_INVALID, "rescale needs a square matrix");
   if (!(a != 0.0)) return fail(TBK_ERR_INVALID, "rescale: a must be nonzero (got %g)", a);
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int32_t n = H->rows;
   const int T = 256;
   DevBuf cnt, cp;
@@ -1192,6 +1197,7 @@ int tbk_sparse_commutator(tbk_sparse* out, tbk_sparse H, tbk_sparse X, void* str
   if (H->rows != H->cols || X->rows != H->rows || X->cols != H->cols)
     return fail(TBK_ERR_INVALID, "commutator: size mismatch");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int32_t n = H->rows;
   const int T = 256;
   DevBuf x;

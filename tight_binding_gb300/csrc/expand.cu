@@ -132,6 +132,7 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
   if (prec != TBK_PREC_FP64 && prec != TBK_PREC_MIXED && prec != TBK_PREC_DD)
     return fail(TBK_ERR_INVALID, "tbk_cheb_expand: unknown precision %d", prec);
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int32_t n = Ht->rows;
   const int Rc = chunk_width(prec, R);
   int grid = 1, n_tiles = 1;
@@ -190,6 +191,7 @@ int tbk_cheb_view_create(tbk_cheb_view* out, tbk_sparse Ht, int32_t R, const dou
   if (precision != TBK_PREC_FP64 && precision != TBK_PREC_MIXED && precision != TBK_PREC_DD)
     return fail(TBK_ERR_INVALID, "tbk_cheb_view_create: unknown precision %d", precision);
   cudaStream_t st = nullptr;
+  ScratchScope scope(st);
   auto* V = new tbk_cheb_view_s();
   V->H = Ht;
   V->n = Ht->rows;
@@ -229,6 +231,7 @@ int tbk_cheb_view_create(tbk_cheb_view* out, tbk_sparse Ht, int32_t R, const dou
 int tbk_cheb_view_next(tbk_cheb_view V, int32_t* index, double* block, void* stream) {
   if (!V) return fail(TBK_ERR_INVALID, "tbk_cheb_view_next: null view");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int64_t cnt = (int64_t)V->H->ell.n_slices * 32 * V->Rc;
   for (int32_t c = 0; c < V->n_chunks; ++c) {
     if (block) {

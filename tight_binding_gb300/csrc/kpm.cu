@@ -975,6 +975,7 @@ int tbk_kpm_create(tbk_kpm* out, tbk_sparse Ht, int32_t R, int32_t flags) {
   if (prec != TBK_PREC_FP64 && prec != TBK_PREC_MIXED && prec != TBK_PREC_DD)
     return fail(TBK_ERR_INVALID, "unknown precision %d", prec);
   cudaStream_t st = nullptr;
+  ScratchScope scope(st);
   TBK_TRY(ensure_ell(Ht, st));
   if (prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Ht, st));
   auto* P = new tbk_kpm_s();
@@ -1059,6 +1060,10 @@ int tbk_kpm_create(tbk_kpm* out, tbk_sparse Ht, int32_t R, int32_t flags) {
     delete P;
     return s;
   }
+  if (cudaStreamSynchronize(st) != cudaSuccess) {          // the blocks are ready for any stream
+    delete P;
+    return fail(TBK_ERR_CUDA, "tbk_kpm_create: work blocks");
+  }
   *out = P;
   return TBK_OK;
 }
@@ -1079,6 +1084,7 @@ int tbk_kpm_run(tbk_kpm P, int32_t n_mom, const double* bras, const double* kets
                 void* stream) {
   if (!P || !kets || !bras || !mu_out) return fail(TBK_ERR_INVALID, "tbk_kpm_run: null argument");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const bool dev = (P->flags & TBK_FLAG_DEVICE_PTRS) != 0;
   const bool doubling = (P->flags & TBK_FLAG_DOUBLING) != 0;
   if (doubling && bras != kets) return fail(TBK_ERR_INVALID, "TBK_FLAG_DOUBLING needs bras == kets");
@@ -1140,6 +1146,7 @@ int tbk_kpm_run(tbk_kpm P, int32_t n_mom, const double* bras, const double* kets
 int tbk_kpm_run_random(tbk_kpm P, int32_t n_mom, uint64_t seed, double* mu_out, void* stream) {
   if (!P || !mu_out) return fail(TBK_ERR_INVALID, "tbk_kpm_run_random: null argument");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const bool dev = (P->flags & TBK_FLAG_DEVICE_PTRS) != 0;
   const bool mixed = P->prec == TBK_PREC_MIXED;
   const bool doubling = (P->flags & TBK_FLAG_DOUBLING) != 0;
@@ -1227,6 +1234,7 @@ int cheb_braket_cached(int32_t n_rows, int64_t nnz, const int32_t* cp, const int
   DropinCache& C = g_dropin;
   std::lock_guard<std::mutex> lock(C.mu);
   cudaStream_t st = nullptr;                               // synchronous, as the reference
+  ScratchScope scope(st);
   const size_t bcp = sizeof(int32_t) * ((size_t)n_rows + 1), bri = sizeof(int32_t) * (size_t)nnz;
   const size_t bv = sizeof(double) * (cplx ? 2 : 1) * (size_t)nnz;
   const size_t o_ri = align16(bcp), o_v = o_ri + align16(bri), need = o_v + align16(bv);
@@ -1314,6 +1322,7 @@ int tbk_set_wait_limit(int64_t polls) {
 void tbk_cheb_braket_release(void) {
   std::lock_guard<std::mutex> lock(g_dropin.mu);
   g_dropin.drop();
+  scratch_trim();
 }
 
 int tbk_cheb_braket_real(int32_t n_rows, int64_t nnz, const int32_t* cp, const int32_t* ri, const double* v,

@@ -355,6 +355,7 @@ __global__ void __launch_bounds__(kSeriesThreads) series_eval_kernel(const doubl
 template <bool BASTIN>
 int moment_series(int32_t M, const double* mu, int32_t n_eps, const double* eps, double norm, double* out,
                   cudaStream_t st) {
+  ScratchScope scope(st);
   const int32_t L = 2 * M - 1, chunks = (M + kDiagRows - 1) / kDiagRows, planes = BASTIN ? 3 : 2;
   const size_t ob = sizeof(double) * (BASTIN ? 2 : 1) * (size_t)n_eps;
   DevBuf dm, de, dz, part, coef;
@@ -479,6 +480,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   for (auto* o : ops)
     if (o && (o->rows != Ht->rows || o->cols != Ht->cols)) return fail(TBK_ERR_INVALID, "tbk_kubo_mu: operator size mismatch");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   PhaseTrace trace(st);
   // outside a server (which sets its own pool): stores and work blocks that
   // the pool keeps come from kubo_pool (decided below, once their size is known)
@@ -515,7 +517,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   const size_t csz = prec == TBK_PREC_MIXED ? sizeof(float2) : sizeof(double2);
   DevBuf Ls, Rs, work, partd, part, macc, gdev, kstage;
   const int64_t blk16 = (blk + 15) / 16 * 16;           // K padded to whole 16-element tiles (zeros)
-  if (!tl_async_alloc && 2.0 * sel * blk16 * M + 12.0 * csz * blk <= (double)kKuboPoolKeep) {
+  if ((!tl_async_alloc || tl_async_alloc->scratch) && 2.0 * sel * blk16 * M + 12.0 * csz * blk <= (double)kKuboPoolKeep) {
     kctx.pool = kubo_pool();
     kctx.stream = st;
   }
@@ -823,6 +825,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
                        void* stream) {
   if (M < 1 || K < 1 || !L || !Rb || !mu_out) return fail(TBK_ERR_INVALID, "tbk_mu_from_blocks: bad argument");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int64_t K16 = (K + 15) / 16 * 16;
   DevBuf stage, Ld, Rd, acc, part;
   TBK_TRY(stage.alloc(sizeof(double2) * K));
@@ -877,6 +880,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
 }
 
 int tbk_kubo_release(void) {
+  scratch_trim();
   cudaMemPool_t pl = kubo_pool();
   if (!pl) return TBK_OK;
   TBK_CUDA(cudaDeviceSynchronize());

@@ -240,6 +240,7 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
   if (A->rows != A->cols) return fail(TBK_ERR_INVALID, "tbk_spectral_range: matrix must be square");
   if (iters < 2) return fail(TBK_ERR_INVALID, "tbk_spectral_range: iters must be >= 2");
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int32_t n = A->rows;
   TBK_TRY(ensure_classes(A, st));
   const EllDev& E = A->ell;

@@ -129,6 +129,7 @@ int tbk_expn_coef_alpha_seq(double z_re, double z_im, int32_t n, double* alpha) 
 int tbk_kernel_seq(int32_t kind, int32_t N, double p0, double p1, double* g_out) {
   if (N < 1 || !g_out) return fail(TBK_ERR_INVALID, "tbk_kernel_seq: bad argument");
   if (kind < 0 || kind > 5) return fail(TBK_ERR_INVALID, "unknown kernel %d", kind);
+  ScratchScope scope(nullptr);
   DevBuf g;
   TBK_TRY(g.alloc(sizeof(double) * N));
   kernel_seq_kernel<<<(N + 255) / 256, 256>>>(kind, N, p0, p1, g.as<double>());
@@ -142,6 +143,7 @@ int tbk_green_imag_eval(int32_t n, const double* g, const double* mu, int32_t n_
   if (n < 1 || n_z < 0 || !g || !mu || (n_z && (!z || !out))) return fail(TBK_ERR_INVALID, "tbk_green_imag_eval: bad argument");
   if (n_z == 0) return TBK_OK;
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   DevBuf dg, dm, dz, dout;
   TBK_TRY(upload(dg, g, n, st));
   TBK_TRY(upload(dm, mu, n, st));
@@ -160,6 +162,7 @@ int tbk_green_imag_fft(int32_t n, const double* g, const double* mu, int32_t ups
   if (n < 1 || !g || !mu || !E_out || !val_out) return fail(TBK_ERR_INVALID, "tbk_green_imag_fft: bad argument");
   if (upsample < 1) upsample = 1;
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   const int32_t N = n * upsample;
   DevBuf dg, dm, dE, dv;
   TBK_TRY(upload(dg, g, n, st));
@@ -182,6 +185,7 @@ int tbk_dos_from_moments(int32_t n, const double* mu, int32_t kind, double p0, d
   if (kind < 0 || kind > 5) return fail(TBK_ERR_INVALID, "unknown kernel %d", kind);
   if (n_e == 0) return TBK_OK;
   cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
   DevBuf dg, dm, dz, dout;
   TBK_TRY(dg.alloc(sizeof(double) * n));
   kernel_seq_kernel<<<(n + 255) / 256, 256, 0, st>>>(kind, n, p0, p1, dg.as<double>());

@@ -36,43 +36,85 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 struct AsyncAllocCtx {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  bool scratch = false;      // the library's own pool (ScratchScope)
 };
 extern thread_local const AsyncAllocCtx* tl_async_alloc;
+
+// The library's pool (scratch.cpp): buffers of up to kScratchMax bytes, of which it
+// keeps kScratchKeep between calls (a cudaMalloc and cudaFree pair costs 60-70 us, a
+// small solve makes sixty).  tbk_cheb_braket_release and tbk_kubo_release give the rest
+// back; so does an allocation that would fail otherwise.
+constexpr size_t kScratchMax = size_t(64) << 20;
+constexpr uint64_t kScratchKeep = uint64_t(256) << 20;
+cudaMemPool_t scratch_pool();
+void scratch_trim();
+// Installed by an entry point for its own stream: buffers it allocates and drops are
+// ordered on that stream.  Buffers that outlive the call are used elsewhere only after
+// the call has synchronised the stream, and freed after cudaDeviceSynchronize or inside
+// a later call.  A server's own context stays in place.
+struct ScratchScope {
+  AsyncAllocCtx ctx;
+  const AsyncAllocCtx* outer;
+  explicit ScratchScope(cudaStream_t st) : outer(tl_async_alloc) {
+    if (outer && !outer->scratch) return;
+    ctx.pool = scratch_pool();
+    ctx.stream = st;
+    ctx.scratch = true;
+    tl_async_alloc = ctx.pool ? &ctx : nullptr;
+  }
+  ~ScratchScope() { tl_async_alloc = outer; }
+  ScratchScope(const ScratchScope&) = delete;
+  ScratchScope& operator=(const ScratchScope&) = delete;
+};
 
 // ---- device buffer (RAII, cudaMalloc or the thread's stream-ordered pool)
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   const AsyncAllocCtx* ctx = nullptr;
+  bool scratch = false;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), ctx(o.ctx) { o.p = nullptr; o.bytes = 0; o.ctx = nullptr; }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), ctx(o.ctx), scratch(o.scratch) { o.forget(); }
   DevBuf& operator=(DevBuf&& o) noexcept {
     if (this != &o) {
       release();
-      p = o.p; bytes = o.bytes; ctx = o.ctx;
-      o.p = nullptr; o.bytes = 0; o.ctx = nullptr;
+      p = o.p; bytes = o.bytes; ctx = o.ctx; scratch = o.scratch;
+      o.forget();
     }
     return *this;
   }
   ~DevBuf() { release(); }
+  void forget() { p = nullptr; bytes = 0; ctx = nullptr; scratch = false; }
   void release() {
     if (p) {
-      if (ctx) cudaFreeAsync(p, ctx->stream);
+      if (scratch) cudaFreeAsync(p, tl_async_alloc && tl_async_alloc->scratch ? tl_async_alloc->stream : nullptr);
+      else if (ctx) cudaFreeAsync(p, ctx->stream);
       else cudaFree(p);
     }
-    p = nullptr; bytes = 0; ctx = nullptr;
+    forget();
   }
   int alloc(size_t n) {
     release();
     if (n == 0) n = 16;
-    cudaError_t e;
-    if (tl_async_alloc) {
-      e = cudaMallocFromPoolAsync(&p, n, tl_async_alloc->pool, tl_async_alloc->stream);
-      if (e == cudaSuccess) ctx = tl_async_alloc;
-    } else {
+    cudaError_t e = cudaErrorMemoryAllocation;
+    const AsyncAllocCtx* c = tl_async_alloc;
+    if (c && (!c->scratch || n <= kScratchMax)) {
+      e = cudaMallocFromPoolAsync(&p, n, c->pool, c->stream);
+      if (e == cudaSuccess) {
+        if (c->scratch) scratch = true;
+        else ctx = c;
+      }
+    }
+    if (e != cudaSuccess && (!c || c->scratch)) {
+      cudaGetLastError();
       e = cudaMalloc(&p, n);
+      if (e == cudaErrorMemoryAllocation) {        // what the pool keeps may be what is missing
+        cudaGetLastError();
+        scratch_trim();
+        e = cudaMalloc(&p, n);
+      }
     }
     if (e != cudaSuccess) { p = nullptr; return fail(TBK_ERR_NOMEM, "device allocation of %zu bytes: %s", n, cudaGetErrorString(e)); }
     bytes = n;
