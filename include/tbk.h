@@ -370,7 +370,9 @@ int tbk_dos_from_moments(int32_t n, const double* mu, int32_t kernel_kind, doubl
  * ========================================================================= */
 enum {
   TBK_MU_CUDA_CORE = 0,             /* mu_nm GEMM on CUDA cores (FP32 chunks, FP64 sums) */
-  TBK_MU_TENSOR = 1,                /* mu_nm GEMM on tcgen05 (split TF32)               */
+  TBK_MU_TENSOR = 1,                /* mu_nm GEMM on tcgen05 (FP16-pair stores; complex64
+                                       stores and CUDA cores where values leave FP16's
+                                       range)                                          */
   TBK_MU_MIXED_RECURSION = 2,       /* complex64 recursion for the stored blocks (FP32
                                        H~); default: complex128 recursion, FP64 H~      */
   TBK_MU_DD_RECURSION = 4,          /* double-float recursion for the stored blocks     */
@@ -391,7 +393,8 @@ enum {
  * aR_n = g_n AR T_n(H~) BR |r> (NULL operator = identity), m, n < M: the stored
  * Chebyshev blocks of TB/numerical.h:333-344 contracted as in TB/snippets.h:
  * 337-342 (Bastin: AL=BL=1, AR=v_x, BR=v_y), :225-260 (Greenwood: AL=BL=v_x)
- * and :491-518 (generate_V_moments).  Blocks are complex64 in HBM; R vectors
+ * and :491-518 (generate_V_moments).  Blocks are complex64 in HBM (TBK_MU_TENSOR: FP16 (hi, lo) pairs
+ * of the same size and 22 significant bits); R vectors
  * are processed in chunks so both sides fit block_budget_gb (<= 0: 60% of the
  * free device memory).
  * kets: host N x R column-major complex128, or NULL for seeded random phases.
@@ -409,7 +412,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
 int tbk_kubo_release(void);
 /* Device time of the last tbk_kubo_mu call in this process (CUDA events on its
  * stream): building the stored blocks, the mu GEMM (+ split-K reduction), the
- * real flops of the GEMM products issued (3 split-TF32 terms on the tensor
+ * real flops of the GEMM products issued (3 split-FP16 terms on the tensor
  * path), the algorithmic DRAM bytes of the block phase (work vectors read and
  * written, matrix per pass, complex64 stores), and the number of vector chunks. */
 int tbk_kubo_last_timing(double* ms_blocks, double* ms_gemm, double* gemm_flops, double* block_bytes,
@@ -417,7 +420,7 @@ int tbk_kubo_last_timing(double* ms_blocks, double* ms_gemm, double* gemm_flops,
 /* mu_mn = sum_k conj(L_m[k]) R_n[k] for given blocks (host, M x K complex128
  * row-major each, rounded to complex64 on the device): the contraction of
  * TB/snippets.h:337-342 on caller-supplied Chebyshev blocks.  flags: TBK_MU_*
- * (TBK_MU_TENSOR: tcgen05 split-TF32 GEMM).  mu_out: host M x M complex128. */
+ * (TBK_MU_TENSOR: tcgen05 split-FP16 GEMM, every block with its own scale).  mu_out: host M x M complex128. */
 int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, int32_t flags,
                        double* mu_out, void* stream);
 /* zeta(e) = sum_mn mu_mn Gamma_mn(e) / (1-e^2)^2 / vol (FP64 on the device),

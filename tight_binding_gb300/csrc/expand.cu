@@ -220,7 +220,7 @@ int tbk_cheb_view_create(tbk_cheb_view* out, tbk_sparse Ht, int32_t R, const dou
     // v_0 = v, v_1 = x v (the view's constructor)
     if ((rc = load_block_any(precision, V->n, R, c * V->Rc, V->Rc, src.as<double2>(), V->cur[c].p, st)) != TBK_OK ||
         (rc = step_any(Ht, V->Rc, precision, V->cur[c].p, V->nxt[c].p, nullptr, true, V->part.as<double>(), V->grid,
-                       V->n_tiles, st, nullptr, 0, 0, true, nullptr, false)) != TBK_OK)
+                       V->n_tiles, st, nullptr, true, nullptr, false)) != TBK_OK)
       return bail(rc);
   }
   if (cudaStreamSynchronize(st) != cudaSuccess) return bail(fail(TBK_ERR_CUDA, "tbk_cheb_view_create: sync failed"));
@@ -245,7 +245,7 @@ int tbk_cheb_view_next(tbk_cheb_view V, int32_t* index, double* block, void* str
     }
     // T_{i+2} = 2 x T_{i+1} - T_i, written over T_i; then cur <-> nxt
     TBK_TRY(step_any(V->H, V->Rc, V->prec, V->nxt[c].p, V->cur[c].p, V->cur[c].p, false, V->part.as<double>(),
-                     V->grid, V->n_tiles, st, nullptr, 0, 0, true, nullptr, false));
+                     V->grid, V->n_tiles, st, nullptr, true, nullptr, false));
     std::swap(V->cur[c], V->nxt[c]);
   }
   if (block)

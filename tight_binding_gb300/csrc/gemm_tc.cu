@@ -1,36 +1,41 @@
 // gemm_tc.cu — the Kubo moment matrix mu_mn on the 5th-generation tensor cores.
 //
-// mu_mn = sum_k conj(L_m[k]) R_n[k] over stored complex64 Chebyshev blocks, as a
-// real GEMM over interleaved (re, im) pairs:
-//   Re mu = A . B^T,  Im mu = A . B'^T,  A = L, B = R, B' = per pair (im, -re),
-// computed in split precision (3 x TF32): x = hi + lo with hi = rna_tf32(x) and
-// lo = rna_tf32(x - hi) (|lo| <= 2^-11 |x|, and the omitted lo.lo term has no
-// sign bias), and
-//   A.B ~ A_hi B_hi + A_hi B_lo + A_lo B_hi           (FP32 accumulation).
+// mu_mn = sum_k conj(L_m[k]) R_n[k] over stored Chebyshev blocks in split precision
+// (3 x FP16): the stores hold s x = hi + lo per real number, hi = half(s x) and lo =
+// half(s x - hi) (|lo| <= 2^-11 |s x|, 22 significant bits), with a power of two s per
+// block row that keeps the values inside FP16's range (split_store.cuh).  An FP16 and a
+// TF32 number have the same 11 significant bits, and kind::f16 runs at twice the rate of
+// kind::tf32.  With the real and imaginary parts in rows of their own,
+//   Re mu = Lr Rr + Li Ri,  Im mu = Lr Ri - Li Rr,
+//   A B ~ A_hi B_hi + A_hi B_lo + A_lo B_hi           (FP32 accumulation).
 //
-// One CTA: a 128 (m) x 64 (n, complex) output tile over a K range (split-K).
-// The MMA is tcgen05.mma.cta_group::1.kind::tf32 M=128 N=128 K=8 with
-// D = [Re | Im] (128 x 128 FP32) in tensor memory.  The stored blocks are
-// K-tiled (16 complex = 32 floats of K per block row, 128 B), so one K tile of
-// 128 consecutive blocks is a 128-row x 128-B box: TMA loads it with the
-// 128-byte swizzle straight into the UMMA K-major SWIZZLE_128B layout.  Two
-// CTAs of a cluster share an m tile (adjacent n tiles): each loads half of the
-// A box and multicasts it to both, and a stage is reused only when both CTAs'
-// MMAs have released it (their commits arrive on both CTAs' barriers).  A
-// (hi and lo) then lives in tensor memory, B (hi, lo, and B' of each) in
-// shared memory, so the MMAs read only B through the shared-memory port.
+// One CTA: a 128 (m) x 128 (n) complex output tile over a K range (split-K).  A stage
+// is one K tile of the stores (32 values of k: 128-byte rows of hi and lo halves, re and
+// im, for A and for B, 64 KB), loaded by TMA with the 128-byte swizzle straight into the
+// UMMA K-major SWIZZLE_128B layout, three stages deep; nothing converts.  Per 16 k and
+// product the issuing thread runs D[Re|Im] += A_re x [B_re|B_im] (N = 256, the parts lie one
+// after the other), D[Re] += A_im x B_im and D[Im] += (-A_im) x B_re (N = 128, A negated by the
+// instruction).  Two CTAs of a cluster share an m tile (adjacent n tiles): each loads
+// half of the A boxes and multicasts them to both, and a stage is reused only when both
+// CTAs' MMAs have released it (their commits arrive on both CTAs' barriers).
 // Roles:
-//   warp 21    TMA producer: one thread issues the A and B boxes of each stage;
-//   warps 16-19 converters: each thread takes one A row (its TMEM lane), splits
-//              it into hi / lo and stores both with tcgen05.st; B is split in
-//              place per 16-byte chunk with B' hi, B lo, B' lo beside it
-//              (elementwise, so the swizzle is irrelevant);
-//   warp 20    TMEM allocation and, lane 0, MMA issue + tcgen05.commit;
-//   warps 0-15 epilogue (32 columns each): every 256 K-floats read the
-//              accumulator with tcgen05.ld and add it into float-float (hi, lo)
-//              pairs by TwoSum (long FP32 sums lose the accuracy the Kubo
-//              weights need; FP64 adds would saturate GB300's FP64 pipe),
-//              double-buffered in TMEM; FP64 once at the end.
+//   warp 17    TMA producer: one thread issues the boxes of each stage;
+//   warp 16    TMEM allocation and, lane 0, MMA issue + tcgen05.commit;
+//   warps 0-15 epilogue (64 columns each): every kChunk tiles read the accumulator with
+//              tcgen05.ld (double-buffered in TMEM, all 512 columns) and add it into FP32
+//              registers, every kFlush chunks add those into the CTA's FP64 partial tile
+//              in global memory (column after column, so that a warp's 32 rows are one
+//              256-byte access; L2 holds it): long FP32 sums lose the accuracy the Kubo weights
+//              need, and 128 x 128 complex float-float pairs would fill the register file.
+// What bounds it: shared memory, and the power cap on long runs.  The MMAs of 16 k read 3
+// x (12 + 16) KB and the TMA writes 32 KB in the 768 clocks of the 12 products at full
+// rate, 151 bytes a clock against 128.  FCC 128^3, M = 1024, R = 8: 286 ms, 1,478 TFLOP/s of
+// issued products, 76% of cuBLAS' bf16 burst rate and 86% of its sustained rate (641 ms
+// with complex64 stores split into TF32 pairs by converter warps, 70% of the TF32 rate;
+// 410 ms with a row-major partial tile, whose flush held the accumulators up); square
+// 256^2, M = 512, R = 16: 10.0 -> 3.9 ms.  Error against 64 bits of the latter's mu_nm
+// 1.2e-6 (2-norm; 2.0e-6 before: FP16 products take 16 k at a time, so a chunk of 128 k is
+// half as many FP32 accumulations).
 // Every mbarrier wait is bounded; on timeout the CTA records an error, waits
 // (bounded) for its copies and MMAs in flight and frees its tensor memory.
 #include <cuda.h>
@@ -40,42 +45,35 @@
 #include <mutex>
 #include <vector>
 
+#include "split_store.cuh"
 #include "tbk_internal.h"
 
 namespace tbk {
 namespace {
 
 constexpr int kTM = 128;            // MMA M (output rows m per CTA)
-constexpr int kTNc = 64;            // complex output columns n per CTA
-constexpr int kTN = 2 * kTNc;       // MMA N (Re | Im)
-constexpr int kKS = 32;             // floats per stage: one K tile (4 MMA k-steps of 8)
-constexpr int kKC = 256;            // floats per FP32 accumulation chunk
-constexpr int kStages = 4;
-constexpr int kEpiWarps = 16, kCvtWarps = 4;
-constexpr int kMmaWarp = kEpiWarps + kCvtWarps;
+constexpr int kTN = 128;            // complex output columns n per CTA
+constexpr int kKS = kSplitTile;     // k per stage: one K tile of the stores (2 MMA k-steps of 16)
+constexpr int kChunk = 4;           // stages per FP32 accumulation in tensor memory (128 k)
+constexpr int kFlush = 32;          // chunks per FP32 register sum
+constexpr int kStages = 3;
+constexpr int kEpiWarps = 16;
+constexpr int kMmaWarp = kEpiWarps;
 constexpr int kTmaWarp = kMmaWarp + 1;
 constexpr int kThreads = 32 * (kTmaWarp + 1);
-// tensor memory columns: two accumulators, then per stage A hi (32) | A lo (32)
-constexpr uint32_t kAccCols = 2 * kTN;
-constexpr uint32_t kACols = 2 * kKS;
-constexpr uint32_t kTmemCols = 512;
-static_assert(kAccCols + kStages * kACols <= kTmemCols, "tensor memory budget");
+constexpr uint32_t kAccCols = 2 * kTN;          // one accumulator: Re | Im
+constexpr uint32_t kTmemCols = 2 * kAccCols;    // double-buffered: all of tensor memory
+static_assert(kTmemCols == 512, "tensor memory");
 constexpr uint32_t kWait = 1u << 24;
 
-// stage layout (every region 1024-byte aligned, so that derived planes carry
-// the raw planes' swizzle): A raw | B raw/hi | B' hi | B lo | B' lo.
-// B hi and B' hi form one 128-row operand, B lo and B' lo another.
-constexpr int kAPlane = kTM * kKS * 4;    // 16 KB
-constexpr int kBPlane = kTNc * kKS * 4;   // 8 KB (64 rows)
-constexpr int kOffAraw = 0;
-constexpr int kOffBhi = kOffAraw + kAPlane;
-constexpr int kOffBphi = kOffBhi + kBPlane;
-constexpr int kOffBlo = kOffBphi + kBPlane;
-constexpr int kOffBplo = kOffBlo + kBPlane;
-constexpr int kStageBytes = kOffBplo + kBPlane;   // 48 KB
+// stage layout: A re | A im | B re | B im; 128 rows of 128 bytes (32 hi, 32 lo) each
+constexpr int kPart = kTM * kKS * 4;            // 16 KB
+constexpr int kOffB = 2 * kPart;
+constexpr int kStageBytes = 4 * kPart;          // 64 KB
 constexpr int kSmemBytes = kStages * kStageBytes + 1024;   // + alignment slack
-constexpr uint32_t kTxBytes = kAPlane + kBPlane;           // raw bytes per stage
+constexpr uint32_t kTxBytes = kStageBytes;
 constexpr uint32_t kSBO = 1024;                 // 8 rows x 128 B swizzle atom
+constexpr uint32_t kLo = kKS * 2;               // bytes from a row's hi halves to its lo halves
 
 enum : int { kErrFull = 1, kErrEmpty = 2, kErrAcc = 4, kErrAccEmpty = 8, kErrDrain = 16, kErrRaw = 32 };
 
@@ -148,42 +146,18 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-// Instruction descriptor, kind::tf32: D F32, A/B TF32, both K-major, N, M.
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kTN >> 3) << 17) |
-                            ((uint32_t)(kTM >> 4) << 24);
-// D (tmem) += A (tmem: lane = row, column = k) . B (shared-memory descriptor)
-__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t accumulate) {
+// Instruction descriptors, kind::f16: D F32, A/B FP16, both K-major, N, M; A negated.
+constexpr uint32_t idesc(int n, bool neg_a) {
+  return (1u << 4) | (neg_a ? 1u << 13 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
+}
+// D (tmem) += A . B (shared-memory descriptors)
+template <int N, bool NEG>
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b), "r"(kIdesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc(N, NEG)), "r"(accumulate)
       : "memory");
-}
-// 16 consecutive columns of this warp's 32 tensor-memory lanes from registers
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-          taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-// TF32 value of x, rounded to nearest with ties away from zero (the rounding
-// of cvt.rna.tf32.f32), on the integer pipe: TF32 keeps 10 of FP32's 23
-// mantissa bits, so adding half a unit of the 13 dropped bits (0x1000) to the
-// sign-magnitude pattern and clearing them rounds the magnitude half-up
-// (a carry into the exponent is the correct rounding to the next binade).
-// Finite inputs only (the stored blocks are finite).
-__device__ __forceinline__ float to_tf32_rna(float x) {
-  return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
-}
-// (hi, lo) += v with TwoSum (Knuth): hi + lo carries the sum to ~2^-48.
-__device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float v) {
-  const float s = hi + v;
-  const float bp = s - hi;
-  const float e = (hi - (s - bp)) + (v - bp);
-  hi = s;
-  lo += e;
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
@@ -196,38 +170,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-// L, Rb: M blocks in the K-tiled layout (element k of block m at
-// ((k/16)*M + m)*16 + k%16, K padded with zeros to whole 16-element tiles),
-// seen by the tensor maps as rows of 32 floats: row (k/16)*M + m.  The CTA
-// covers rows m0.., n0.. and floats [kf0, kf1) (kf0 a multiple of kKC).
-// Writes FP64 partial tiles.
+// L, Rb: split stores of M blocks (split_store.cuh), seen by the tensor maps as rows of
+// 64 halves: row (k tile * 2 + part) * M + m.  The CTA covers rows m0.., n0.. and K
+// tiles [t0, t1).  Writes FP64 partial tiles (of s_m s_n mu).
 __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constant__ CUtensorMap map_l,
                                                             const __grid_constant__ CUtensorMap map_r, int32_t M,
-                                                            int64_t K, int64_t kf_split,
-                                                            double* __restrict__ part_re, double* __restrict__ part_im,
-                                                            int* __restrict__ err) {
+                                                            int32_t n_tiles_k, int32_t tiles_split,
+                                                            double* __restrict__ part, int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t raw_bar[kStages], full_bar[kStages], empty_bar[kStages], acc_full[2], acc_empty[2], drain_bar;
+  __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[2], acc_empty[2], drain_bar;
   __shared__ uint32_t tmem_base_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // blockIdx.x = m_tile * n_tiles_p + n_tile (n_tiles_p even): cluster pairs
   // share the m tile
-  const int n_tiles_p = ((M + kTNc - 1) / kTNc + 1) & ~1;
+  const int n_tiles_p = ((M + kTN - 1) / kTN + 1) & ~1;
   const int32_t m0 = (int32_t)(blockIdx.x / n_tiles_p) * kTM;
-  const int32_t n0 = (int32_t)(blockIdx.x % n_tiles_p) * kTNc;
+  const int32_t n0 = (int32_t)(blockIdx.x % n_tiles_p) * kTN;
   const uint32_t crank = cluster_rank();
-  const int64_t KF = 2 * K;                                   // floats
-  const int64_t kf0 = (int64_t)blockIdx.y * kf_split;
-  const int64_t kf1 = min(KF, kf0 + kf_split);
-  const int32_t n_slabs = kf1 > kf0 ? (int32_t)((kf1 - kf0 + kKS - 1) / kKS) : 0;
-  const int32_t slabs_per_chunk = kKC / kKS;
-  const int32_t n_chunks = (n_slabs + slabs_per_chunk - 1) / slabs_per_chunk;
-  const int32_t tile0 = (int32_t)(kf0 / kKS);
+  const int32_t t0 = (int32_t)blockIdx.y * tiles_split;
+  const int32_t n_slabs = max(0, min(n_tiles_k - t0, tiles_split));
+  const int32_t n_chunks = (n_slabs + kChunk - 1) / kChunk;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { bar_init(&raw_bar[s], 1); bar_init(&full_bar[s], kCvtWarps); bar_init(&empty_bar[s], 2); }
+    for (int s = 0; s < kStages; ++s) { bar_init(&full_bar[s], 1); bar_init(&empty_bar[s], 2); }
     for (int b = 0; b < 2; ++b) { bar_init(&acc_full[b], 1); bar_init(&acc_empty[b], kEpiWarps); }
     bar_init(&drain_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -255,75 +222,22 @@ __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constan
         const uint32_t ph = (uint32_t)(s / kStages) & 1u;
         if (!bar_wait(&empty_bar[st], ph ^ 1u)) { atomicOr(err, kErrEmpty); break; }
         unsigned char* sb = smem + (size_t)st * kStageBytes;
-        const int32_t row = (tile0 + s) * M;
-        bar_arrive_tx(&raw_bar[st], kTxBytes);
-        // this CTA's half of the A box, to both CTAs of the pair
-        tma_load_2d_mc(sb + kOffAraw + crank * (kAPlane / 2), &map_l, 0, row + m0 + (int32_t)crank * (kTM / 2),
-                       &raw_bar[st], (uint16_t)0x3);
-        tma_load_2d(sb + kOffBhi, &map_r, 0, row + n0, &raw_bar[st]);
+        bar_arrive_tx(&full_bar[st], kTxBytes);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const int32_t row = ((t0 + s) * 2 + p) * M;
+          // this CTA's half of the A box, to both CTAs of the pair
+          tma_load_2d_mc(sb + p * kPart + crank * (kPart / 2), &map_l, 0, row + m0 + (int32_t)crank * (kTM / 2),
+                         &full_bar[st], (uint16_t)0x3);
+          tma_load_2d(sb + kOffB + p * kPart, &map_r, 0, row + n0, &full_bar[st]);
+        }
         issued = s + 1;
       }
       // copies in flight complete before the CTA may leave (bounded)
       for (int32_t s = max(0, issued - kStages); s < issued; ++s)
-        if (!bar_wait(&raw_bar[s % kStages], (uint32_t)(s / kStages) & 1u)) { atomicOr(err, kErrRaw); break; }
+        if (!bar_wait(&full_bar[s % kStages], (uint32_t)(s / kStages) & 1u)) { atomicOr(err, kErrRaw); break; }
     }
     __syncwarp();
-  } else if (warp >= kEpiWarps && warp < kMmaWarp) {
-    // ------------------------------------------------------------ converters
-    const int t = threadIdx.x - 32 * kEpiWarps;     // 0..127
-    for (int32_t s = 0; s < n_slabs; ++s) {
-      const int st = s % kStages;
-      const uint32_t ph = (uint32_t)(s / kStages) & 1u;
-      if (!bar_wait(&raw_bar[st], ph)) { atomicOr(err, kErrFull); break; }
-      unsigned char* sb = smem + (size_t)st * kStageBytes;
-      // A row r (this warp's TMEM lane quarter): its 8 swizzled 16-byte chunks
-      // (chunk c of row r sits at chunk c ^ (r & 7) of the 128-byte row)
-      const int r = 32 * (warp & 3) + lane;
-      const unsigned char* arow = sb + kOffAraw + r * 128;
-      const uint32_t acol = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kAccCols + (uint32_t)st * kACols;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {     // 16 floats at a time (registers)
-        uint32_t hi[16], lo[16];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = 4 * half + u;
-          const float4 v = *reinterpret_cast<const float4*>(arow + ((c ^ (r & 7)) << 4));
-          const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float h = to_tf32_rna(x[e]);
-            hi[4 * u + e] = __float_as_uint(h);
-            lo[4 * u + e] = __float_as_uint(to_tf32_rna(x[e] - h));
-          }
-        }
-        tmem_st16(acol + 16u * half, hi);
-        tmem_st16(acol + kKS + 16u * half, lo);
-      }
-      // B: 512 chunks, 4 per thread; B' = per (re, im) pair (im, -re)
-      constexpr int kQB = kBPlane / 16 / 128;
-      float4* bhp = reinterpret_cast<float4*>(sb + kOffBhi);
-      float4 vb[kQB];
-#pragma unroll
-      for (int q = 0; q < kQB; ++q) vb[q] = bhp[q * 128 + t];
-#pragma unroll
-      for (int q = 0; q < kQB; ++q) {
-        const int c = q * 128 + t;
-        const float4 v = vb[q];
-        const float4 h = make_float4(to_tf32_rna(v.x), to_tf32_rna(v.y), to_tf32_rna(v.z), to_tf32_rna(v.w));
-        const float4 l = make_float4(to_tf32_rna(v.x - h.x), to_tf32_rna(v.y - h.y), to_tf32_rna(v.z - h.z),
-                                     to_tf32_rna(v.w - h.w));
-        bhp[c] = h;
-        reinterpret_cast<float4*>(sb + kOffBphi)[c] = make_float4(h.y, -h.x, h.w, -h.z);
-        reinterpret_cast<float4*>(sb + kOffBlo)[c] = l;
-        reinterpret_cast<float4*>(sb + kOffBplo)[c] = make_float4(l.y, -l.x, l.w, -l.z);
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      // make the generic-proxy writes visible to the tensor cores, then signal
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) bar_arrive(&full_bar[st]);
-    }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issue
     if (lane == 0) {
@@ -331,27 +245,31 @@ __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constan
       int32_t s = 0;
       for (int32_t c = 0; c < n_chunks && ok; ++c) {
         const int b = c & 1;
-        const uint32_t acc = tmem + (uint32_t)(b * kTN);
+        const uint32_t acc = tmem + (uint32_t)b * kAccCols;
         if (c >= 2) {
           if (!bar_wait(&acc_empty[b], (uint32_t)((c - 2) >> 1) & 1u)) { atomicOr(err, kErrAccEmpty); ok = false; break; }
           tc_fence_after();
         }
-        const int32_t s_end = min(n_slabs, (c + 1) * slabs_per_chunk);
-        bool first = true;
+        const int32_t s_end = min(n_slabs, (c + 1) * kChunk);
+        uint32_t accumulate = 0;
         for (; s < s_end; ++s) {
           const int st = s % kStages;
           if (!bar_wait(&full_bar[st], (uint32_t)(s / kStages) & 1u)) { atomicOr(err, kErrFull); ok = false; break; }
           tc_fence_after();
           const uint32_t sb = s_u32(smem + (size_t)st * kStageBytes);
-          const uint32_t a_hi = tmem + kAccCols + (uint32_t)st * kACols, a_lo = a_hi + kKS;
 #pragma unroll
-          for (int j = 0; j < kKS / 8; ++j) {
-            const uint32_t kb = (uint32_t)j * 32u;     // 8 tf32 = 32 B along the 128-B swizzled row
-            const uint64_t bh = smem_desc_sw128(sb + kOffBhi + kb), bl = smem_desc_sw128(sb + kOffBlo + kb);
-            mma_tf32_ts(acc, a_hi + 8u * j, bh, first ? 0u : 1u);
-            mma_tf32_ts(acc, a_hi + 8u * j, bl, 1u);
-            mma_tf32_ts(acc, a_lo + 8u * j, bh, 1u);
-            first = false;
+          for (int j = 0; j < kKS / 16; ++j) {
+            // part 0 re, 1 im; 16 halves = 32 B along the swizzled row
+            auto A = [&](int p, uint32_t lo) { return smem_desc_sw128(sb + (uint32_t)(p * kPart + j * 32) + lo); };
+            auto B = [&](int p, uint32_t lo) { return smem_desc_sw128(sb + (uint32_t)(kOffB + p * kPart + j * 32) + lo); };
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+              const uint32_t la = q == 2 ? kLo : 0, lb = q == 1 ? kLo : 0;     // hi hi, hi lo, lo hi
+              mma_f16<2 * kTN, false>(acc, A(0, la), B(0, lb), accumulate);
+              accumulate = 1;
+              mma_f16<kTN, false>(acc, A(1, la), B(1, lb), 1u);
+              mma_f16<kTN, true>(acc + kTN, A(1, la), B(0, lb), 1u);
+            }
           }
           tc_commit_mc(&empty_bar[st], (uint16_t)0x3);   // frees the stage (in both CTAs) when these MMAs finish
         }
@@ -365,33 +283,42 @@ __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constan
   } else {
     // ------------------------------------------------------------ epilogue
     const int grp = warp & 3;           // TMEM lanes 32*grp .. 32*grp+31
-    const int colq = warp >> 2;         // columns 32*colq ..: 0, 1 Re; 2, 3 Im
-    float acc_hi[32], acc_lo[32];
+    const int colq = warp >> 2;         // columns 64*colq ..: 0, 1 Re; 2, 3 Im
+    float acc[64];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) { acc_hi[j] = 0.f; acc_lo[j] = 0.f; }
+    for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+    double* dst = part + (((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kAccCols + colq * 64) * kTM + 32 * grp + lane;
+    bool fresh = true;                  // the partial tile has not been written yet
     for (int32_t c = 0; c < n_chunks; ++c) {
       const int b = c & 1;
       if (!bar_wait(&acc_full[b], (uint32_t)(c >> 1) & 1u)) { atomicOr(err, kErrAcc); break; }
       tc_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(32 * grp) << 16) + (uint32_t)(b * kTN + colq * 32);
+      const uint32_t taddr = tmem + ((uint32_t)(32 * grp) << 16) + (uint32_t)b * kAccCols + (uint32_t)(colq * 64);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < 4; ++h) {
         float v[16];
         tmem_ld16(taddr + 16u * h, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) two_sum_acc(acc_hi[16 * h + j], acc_lo[16 * h + j], v[j]);
+        for (int j = 0; j < 16; ++j) acc[16 * h + j] += v[j];
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) bar_arrive(&acc_empty[b]);
-    }
-    const int32_t m = m0 + 32 * grp + lane;
-    const int32_t nb = n0 + 32 * (colq & 1);
-    if (m < M) {
-      double* dst = (colq >= 2 ? part_im : part_re) + ((int64_t)blockIdx.y * M + m) * M;
+      if ((c + 1) % kFlush == 0 || c + 1 == n_chunks) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (nb + j < M) dst[nb + j] = (double)acc_hi[j] + (double)acc_lo[j];
+        for (int h = 0; h < 8; ++h) {                    // 8 values in flight: the sums fill the registers
+          double o[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = fresh ? 0.0 : __ldcg(dst + (8 * h + j) * kTM);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            __stcg(dst + (8 * h + j) * kTM, o[j] + (double)acc[8 * h + j]);
+            acc[8 * h + j] = 0.f;
+          }
+          asm volatile("" ::: "memory");
+        }
+        fresh = false;
+      }
     }
   }
   tc_fence_before();
@@ -403,14 +330,24 @@ __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constan
   cluster_sync();        // no multicast or remote arrive targets a CTA that has left
 }
 
-__global__ void mu_tc_reduce_kernel(const double* __restrict__ pr, const double* __restrict__ pi, int32_t M,
-                                    int32_t nsplit, double2* __restrict__ acc) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (int64_t)M * M) return;
+// acc += (split-K partials summed in order) / (s_m s_n), one CTA row of tile rows per
+// output column; nothing where the stores are marked unusable (the caller then forms the
+// chunk from complex64 stores).
+__global__ void __launch_bounds__(kTM) mu_tc_reduce_kernel(const double* __restrict__ part, int32_t M, int32_t n_tiles_p,
+                                                           int32_t tiles, int32_t nsplit, const float* __restrict__ sl,
+                                                           int32_t sl_stride, const float* __restrict__ sr,
+                                                           int32_t sr_stride, const int* __restrict__ bad,
+                                                           double2* __restrict__ acc) {
+  const int32_t n = blockIdx.x, mt = blockIdx.y, m = mt * kTM + threadIdx.x;
+  if (m >= M || *bad) return;
+  const int64_t tile = (int64_t)mt * n_tiles_p + n / kTN, step = (int64_t)tiles * kAccCols * kTM;
+  const double* p = part + (tile * kAccCols + n % kTN) * kTM + threadIdx.x;
   double r = 0.0, i = 0.0;
-  for (int32_t s = 0; s < nsplit; ++s) { r += pr[(int64_t)s * M * M + q]; i += pi[(int64_t)s * M * M + q]; }
-  acc[q].x += r;
-  acc[q].y += i;
+#pragma unroll 4
+  for (int32_t s = 0; s < nsplit; ++s) { r += p[s * step]; i += p[s * step + kTN * kTM]; }
+  const double f = 1.0 / ((double)sl[m * sl_stride] * (double)sr[n * sr_stride]);   // a power of two
+  acc[(int64_t)m * M + n].x += f * r;
+  acc[(int64_t)m * M + n].y += f * i;
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -430,17 +367,16 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// Tensor map over a K-tiled block store: rows of 32 floats (128 B), `rows`
-// rows, boxes of 32 floats x box_rows rows, 128-byte swizzle, zero fill past
-// the end.
-int block_map(CUtensorMap* map, const float2* base, int64_t rows, uint32_t box_rows) {
+// Tensor map over a split store: rows of 64 halves (128 B), `rows` rows, boxes of
+// 64 halves x box_rows rows, 128-byte swizzle, zero fill past the end.
+int block_map(CUtensorMap* map, const void* base, int64_t rows, uint32_t box_rows) {
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return fail(TBK_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  const cuuint64_t dims[2] = {32, (cuuint64_t)rows};
+  const cuuint64_t dims[2] = {64, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {128};
-  const cuuint32_t box[2] = {32, box_rows};
+  const cuuint32_t box[2] = {64, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float2*>(base), dims, strides, box, estr,
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TBK_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -449,26 +385,27 @@ int block_map(CUtensorMap* map, const float2* base, int64_t rows, uint32_t box_r
 
 }  // namespace
 
-int mu_gemm_tc(const float2* L, const float2* Rb, int32_t M, int64_t K, double* mu_acc, cudaStream_t st) {
+int mu_gemm_tc(const SplitStore& L, const SplitStore& Rb, int32_t M, int64_t K, double* mu_acc, bool* usable,
+               cudaStream_t st) {
   if (M < 1 || K < 1) return fail(TBK_ERR_INVALID, "mu_gemm_tc: empty problem");
-  if (((uintptr_t)L | (uintptr_t)Rb) & 15) return fail(TBK_ERR_INVALID, "mu_gemm_tc: blocks must be 16-byte aligned");
-  static bool configured = false;
-  if (!configured) {
-    TBK_CUDA(cudaFuncSetAttribute(mu_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    configured = true;
-  }
-  const int64_t tiles16 = (K + 15) / 16;                 // K tiles of the store (zero padded)
-  if (tiles16 * (int64_t)M > INT32_MAX) return fail(TBK_ERR_UNSUPPORTED, "mu_gemm_tc: store too large for TMA rows");
+  if (((uintptr_t)L.data | (uintptr_t)Rb.data) & 15) return fail(TBK_ERR_INVALID, "mu_gemm_tc: blocks must be 16-byte aligned");
+  static std::once_flag once;
+  static cudaError_t configured = cudaSuccess;
+  std::call_once(once, [] {
+    configured = cudaFuncSetAttribute(mu_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  });
+  TBK_CUDA(configured);
+  const int64_t tiles_k = (K + kKS - 1) / kKS;           // K tiles of the store (zero padded)
+  if (tiles_k * 2 * (int64_t)M > INT32_MAX) return fail(TBK_ERR_UNSUPPORTED, "mu_gemm_tc: store too large for TMA rows");
   CUtensorMap map_l, map_r;
-  TBK_TRY(block_map(&map_l, L, tiles16 * M, kTM / 2));
-  TBK_TRY(block_map(&map_r, Rb, tiles16 * M, kTNc));
-  const int m_tiles = (M + kTM - 1) / kTM, n_tiles = ((M + kTNc - 1) / kTNc + 1) & ~1;   // pairs
+  TBK_TRY(block_map(&map_l, L.data, tiles_k * 2 * M, kTM / 2));
+  TBK_TRY(block_map(&map_r, Rb.data, tiles_k * 2 * M, kTN));
+  const int m_tiles = (M + kTM - 1) / kTM, n_tiles = ((M + kTN - 1) / kTN + 1) & ~1;   // pairs
   const int tiles = m_tiles * n_tiles;
   // split K (whole accumulation chunks per split) so that the CTAs fill whole
   // waves of one CTA per SM: the fewest splits whose last wave is >= 95% full
-  const int64_t KF = 2 * K;
   const int sms = sm_count();
-  const int64_t chunks = (KF + kKC - 1) / kKC;
+  const int64_t chunks = (tiles_k + kChunk - 1) / kChunk;
   int nsplit = 1;
   double best = 0.0;
   for (int ns = 1; ns <= 256 && ns <= chunks; ++ns) {
@@ -478,11 +415,10 @@ int mu_gemm_tc(const float2* L, const float2* Rb, int32_t M, int64_t K, double* 
     if (eff > best + 1e-9) { best = eff; nsplit = ns; }
     if (eff >= 0.95 && units >= sms) { nsplit = ns; break; }
   }
-  int64_t kf_split = (chunks + nsplit - 1) / nsplit * kKC;
-  nsplit = (int)((KF + kf_split - 1) / kf_split);
-  DevBuf pr, pi, errb;
-  TBK_TRY(pr.alloc(sizeof(double) * (size_t)nsplit * M * M));
-  TBK_TRY(pi.alloc(sizeof(double) * (size_t)nsplit * M * M));
+  const int64_t tiles_split = (chunks + nsplit - 1) / nsplit * kChunk;
+  nsplit = (int)((tiles_k + tiles_split - 1) / tiles_split);
+  DevBuf part, errb;
+  TBK_TRY(part.alloc(sizeof(double) * (size_t)nsplit * tiles * kAccCols * kTM));
   TBK_TRY(errb.alloc(sizeof(int)));
   TBK_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
   cudaLaunchConfig_t cfg = {};
@@ -497,15 +433,18 @@ int mu_gemm_tc(const float2* L, const float2* Rb, int32_t M, int64_t K, double* 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  TBK_CUDA(cudaLaunchKernelEx(&cfg, mu_tc_kernel, map_l, map_r, M, K, kf_split, pr.as<double>(), pi.as<double>(),
-                              errb.as<int>()));
-  mu_tc_reduce_kernel<<<(unsigned)(((int64_t)M * M + 255) / 256), 256, 0, st>>>(pr.as<double>(), pi.as<double>(), M,
-                                                                               nsplit, reinterpret_cast<double2*>(mu_acc));
+  TBK_CUDA(cudaLaunchKernelEx(&cfg, mu_tc_kernel, map_l, map_r, M, (int32_t)tiles_k, (int32_t)tiles_split,
+                              part.as<double>(), errb.as<int>()));
+  mu_tc_reduce_kernel<<<dim3(M, m_tiles), kTM, 0, st>>>(part.as<double>(), M, n_tiles, tiles, nsplit, L.scale,
+                                                        L.scale_stride, Rb.scale, Rb.scale_stride, L.bad,
+                                                        reinterpret_cast<double2*>(mu_acc));
   TBK_CHECK_LAUNCH();
-  int herr = 0;
-  TBK_CUDA(cudaMemcpyAsync(&herr, errb.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int h[2] = {0, 0};
+  TBK_CUDA(cudaMemcpyAsync(&h[0], errb.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(&h[1], L.bad, sizeof(int), cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
-  if (herr) return fail(TBK_ERR_TIMEOUT, "tensor-core mu_nm kernel gave up waiting (code %d)", herr);
+  if (h[0]) return fail(TBK_ERR_TIMEOUT, "tensor-core mu_nm kernel gave up waiting (code %d)", h[0]);
+  *usable = h[1] == 0;
   return TBK_OK;
 }
 

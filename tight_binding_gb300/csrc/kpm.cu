@@ -267,8 +267,7 @@ int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cuda
 static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const StepArgs& a, int grid, cudaStream_t st);
 
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-             int grid, int n_tiles, cudaStream_t st, float2* kstore, int32_t kM, int32_t km, bool store_y,
-             tbk_sparse_s* vop, bool dots) {
+             int grid, int n_tiles, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots) {
   StepArgs a;
   a.n = A->rows;
   a.n_tiles = n_tiles;
@@ -288,11 +287,9 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
   a.gather = 1;
   a.pf_dist = 1;
   a.pipe = A->ell.max_width > 4;
-  if (kstore) {
-    a.ks.store[0] = kstore;
-    a.ks.kM = kM;
-    a.ks.km[0] = km;
-    a.kst = 1;
+  if (ks) {
+    a.ks = *ks;
+    a.kst = ks->split ? 5 : 1;
     if (vop) {
       a.ks.vval[0] = ell_vals(vop->ell, prec);
       a.ks.vdiag[0] = ell_diag(vop->ell, prec);

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "kpm_device.cuh"
+#include "split_store.cuh"
 #include "tbk_internal.h"
 
 namespace tbk {
@@ -68,6 +69,26 @@ __device__ __noinline__ void step_sums_call(float m0, float m1, double* __restri
   step_sums<float, kTwo>(m0, m1, part);
 }
 
+// the lane's values k .. into block m of a complex64 or an FP16-pair K-tiled store
+template <typename F, int VPL>
+__device__ __forceinline__ void store_c64(float2* __restrict__ dst, int32_t M, int32_t m, int64_t k0,
+                                          const LaneV<F, VPL>& v) {
+#pragma unroll
+  for (int q = 0; q < VPL; ++q) {
+    const int64_t k = k0 + q;
+    dst[((k >> 4) * M + m) * 16 + (k & 15)] = make_float2(to_f32(v.re[q]), to_f32(v.im[q]));
+  }
+}
+template <typename F, int VPL>
+__device__ __forceinline__ void store_split(float2* __restrict__ dst, int32_t M, int32_t m, int64_t k,
+                                            const LaneV<F, VPL>& v, float s, int* __restrict__ bad) {
+  __half* d = reinterpret_cast<__half*>(dst);
+  if constexpr (VPL == 2)
+    split_put2(d, M, m, k, to_f32(v.re[0]), to_f32(v.im[0]), to_f32(v.re[1]), to_f32(v.im[1]), s, bad);
+  else
+    split_put(d, M, m, k, to_f32(v.re[0]), to_f32(v.im[0]), s, bad);
+}
+
 // acc += (2) p[o] x for a matrix value in memory
 template <typename F, int VPL, bool CPLX_H, bool FOLD>
 __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, const LaneV<F, VPL>& xs,
@@ -102,6 +123,7 @@ constexpr int kMinCtas = is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
 //   two sides of a Kubo pair can run as one recursion of twice the width.  A
 //   template parameter because even an untaken runtime branch there costs the
 //   moments recursion ~8% of its bandwidth.
+//   KST = 5: as 1, into an FP16-pair store (ks.split; KST = 2 looks at it itself).
 //   KST = 4: a plain step whose moments nothing reads (the Kubo recursion
 //   ahead of an operator product).  Only KST = 0 forms the moment sums.
 //   PIPE: rows wider than one group of 4 gathers (ELL width > 4, e.g. FCC's
@@ -168,6 +190,13 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
     }
   }
 
+  float scale0 = 1.f, scale1 = 1.f;        // of FP16-pair stores
+  if constexpr (KST == 5 || KST == 2) {
+    if (ks.split) {
+      scale0 = __ldg(ks.scale[0]);
+      if (KST == 2 && ks.halves == 2) scale1 = __ldg(ks.scale[1]);
+    }
+  }
   HVal<F, true> add_c{F(0), F(0)};         // c_k of a Clenshaw step
   if constexpr (KST == 3) {
     const double f = is_dd<F> ? 0.5 : 1.0;
@@ -380,22 +409,18 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
     if (store) st_v<F, VPL>(y + me * VPL, out);
     if constexpr (KST == 1) {
       // block km[0] of the K-tiled store: one rounding per value
-#pragma unroll
-      for (int q = 0; q < VPL; ++q) {
-        const int64_t k = (int64_t)r * RW + sub * VPL + q;
-        ks.store[0][((k >> 4) * ks.kM + ks.km[0]) * 16 + (k & 15)] = make_float2(to_f32(out.re[q]), to_f32(out.im[q]));
-      }
+      store_c64<F, VPL>(ks.store[0], ks.kM, ks.km[0], (int64_t)r * RW + sub * VPL, out);
+    } else if constexpr (KST == 5) {
+      store_split<F, VPL>(ks.store[0], ks.kM, ks.km[0], (int64_t)r * RW + sub * VPL, out, scale0, ks.bad);
     } else if constexpr (KST == 2) {
       const int32_t kmg = grp ? ks.km[1] : ks.km[0];
       if (kmg >= 0) {
         const int32_t Rg = RW / ks.halves;
         const LaneV<F, VPL>& sv = (grp ? ks.usev[1] : ks.usev[0]) ? vacc : out;
         float2* dst = grp ? ks.store[1] : ks.store[0];
-#pragma unroll
-        for (int q = 0; q < VPL; ++q) {
-          const int64_t k = (int64_t)r * Rg + sub * VPL + q - grp * Rg;
-          dst[((k >> 4) * ks.kM + kmg) * 16 + (k & 15)] = make_float2(to_f32(sv.re[q]), to_f32(sv.im[q]));
-        }
+        const int64_t k = (int64_t)r * Rg + sub * VPL - grp * Rg;
+        if (ks.split) store_split<F, VPL>(dst, ks.kM, kmg, k, sv, grp ? scale1 : scale0, ks.bad);
+        else store_c64<F, VPL>(dst, ks.kM, kmg, k, sv);
       }
     }
   }
@@ -422,7 +447,7 @@ struct StepArgs {
   int store, reverse, gather, pf_dist;
   KStore ks;                   // optional complex64 K-tiled stores (Kubo blocks)
   int kst = 0;                 // 0 moments, 1 output into ks.store[0], 2 per-group output / V x,
-                               // 3 Clenshaw term, 4 plain step without moment sums
+                               // 3 Clenshaw term, 4 plain step without moment sums, 5 as 1 in FP16 pairs
   bool pipe = false;           // ELL wider than 4: pipelined column loads
   bool cls = false;            // row classes (ct) instead of the ELL's columns and values
   ClassTab ct;
@@ -465,6 +490,8 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
       TBK_STEP(false, false, 3);
     } else if (a.kst == 4) {
       if (first) TBK_STEP(true, false, 4); else TBK_STEP(false, false, 4);
+    } else if (a.kst == 5) {
+      if (first) TBK_STEP(true, false, 5); else TBK_STEP(false, false, 5);
     } else if (a.kst == 2) {
       if constexpr (CLS) return fail(TBK_ERR_UNSUPPORTED, "operator products in the class form");
       else { if (first) TBK_STEP(true, false, 2); else TBK_STEP(false, false, 2); }

@@ -10,9 +10,10 @@
 // complex64 in HBM in a K-tiled layout: element k of block m lives at
 // ((k / 16) * M + m) * 16 + k % 16, so the 16-element K slab of any run of
 // consecutive blocks is contiguous (one coalesced 128-byte row per block) for
-// the mu GEMM.  They are produced by the fused recursion
-// step of kpm.cu running in complex128 on a three-block ring (the outer operator
-// AL/AR applied after each step), each stored value rounded to complex64 once.
+// the mu GEMM.  For the tensor-core GEMM they are FP16 (hi, lo) pairs of the same
+// size (split_store.cuh).  They are produced by the fused recursion
+// step of kpm.cu on a three-block ring (the outer operator AL/AR applied after
+// each step), each stored value rounded once.
 // Random vectors are processed in chunks so that both sides fit the block
 // budget; mu accumulates over chunks in FP64 on the device.  The Gamma
 // contractions (FP64) and the Bastin integration follow TB/snippets.h:343-449.
@@ -24,15 +25,14 @@
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "kpm_device.cuh"
+#include "split_store.cuh"
 #include "tbk_internal.h"
 
 namespace tbk {
-
-int mu_gemm_tc(const float2* L, const float2* Rb, int32_t M, int64_t K, double* mu_acc,
-               cudaStream_t st);   // gemm_tc.cu (tensor cores, split TF32, K-tiled blocks)
 
 namespace {
 
@@ -191,6 +191,88 @@ __global__ void round_cols_kernel(int64_t n_pad, int32_t Rc, int32_t c0, const C
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t row = q / Rc;
     store[((q >> 4) * M + m) * 16 + (q & 15)] = to_c64(src[row * 2 * Rc + c0 + (q - row * Rc)]);
+  }
+}
+
+// The scale of an FP16-pair store (split_store.cuh) from n values: a power of two that
+// takes their root mean square to 2^6, or their maximum to 2^13 where that is less.  The
+// last CTA to finish sums the others' partials in a fixed order.
+constexpr int kStatThreads = 256;
+template <typename CT>
+__global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __restrict__ src, int64_t n,
+                                                                   double* __restrict__ part,
+                                                                   unsigned int* __restrict__ count,
+                                                                   float* __restrict__ scale, int* __restrict__ bad) {
+  float big = 0.f;
+  double sum = 0.0;
+  for (int64_t q = (int64_t)blockIdx.x * kStatThreads + threadIdx.x; q < n; q += (int64_t)gridDim.x * kStatThreads) {
+    const float2 v = to_c64(src[q]);
+    const float m = fmaxf(fabsf(v.x), fabsf(v.y));
+    big = (v.x != v.x || v.y != v.y) ? INFINITY : fmaxf(big, m);
+    sum += (double)v.x * v.x + (double)v.y * v.y;
+  }
+  __shared__ double s_sum[kStatThreads], s_big[kStatThreads];
+  __shared__ bool last;
+  auto block_reduce = [&]() {
+    __syncthreads();
+    for (int o = kStatThreads / 2; o > 0; o >>= 1) {
+      if (threadIdx.x < o) {
+        s_sum[threadIdx.x] += s_sum[threadIdx.x + o];
+        s_big[threadIdx.x] = fmax(s_big[threadIdx.x], s_big[threadIdx.x + o]);
+      }
+      __syncthreads();
+    }
+  };
+  s_sum[threadIdx.x] = sum;
+  s_big[threadIdx.x] = big;
+  block_reduce();
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = s_sum[0];
+    part[2 * blockIdx.x + 1] = s_big[0];
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s_sum[threadIdx.x] = 0.0;
+  s_big[threadIdx.x] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kStatThreads) {
+    s_sum[threadIdx.x] += __ldcg(part + 2 * b);
+    s_big[threadIdx.x] = fmax(s_big[threadIdx.x], __ldcg(part + 2 * b + 1));
+  }
+  block_reduce();
+  if (threadIdx.x == 0) {
+    const double mx = s_big[0], rms = sqrt(s_sum[0] / (2.0 * (double)n));
+    float s = 1.f;
+    if (!(mx < (double)INFINITY)) *bad = 1;
+    else if (mx > 0.0) s = ldexpf(1.f, max(-120, min(120, min(12 - ilogb(mx), 6 - ilogb(rms)))));
+    *scale = s;
+    *count = 0;
+  }
+}
+
+// work block -> block m of an FP16-pair store
+template <typename CT>
+__global__ void split_block_kernel(const CT* __restrict__ src, __half* __restrict__ store, int32_t m, int32_t M,
+                                   int64_t n, const float* __restrict__ scale, int* __restrict__ bad) {
+  const float s = __ldg(scale);
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+    const float2 v = to_c64(src[q]);
+    split_put(store, M, m, q, v.x, v.y, s, bad);
+  }
+}
+// the same from columns [c0, c0 + Rc) of a 2 Rc-wide block
+template <typename CT>
+__global__ void split_cols_kernel(int64_t n_pad, int32_t Rc, int32_t c0, const CT* __restrict__ src,
+                                  __half* __restrict__ store, int32_t m, int32_t M, const float* __restrict__ scale,
+                                  int* __restrict__ bad) {
+  const float s = __ldg(scale);
+  const int64_t tot = n_pad * Rc;
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t row = q / Rc;
+    const float2 v = to_c64(src[row * 2 * Rc + c0 + (q - row * Rc)]);
+    split_put(store, M, m, q, v.x, v.y, s, bad);
   }
 }
 
@@ -445,6 +527,36 @@ cudaMemPool_t kubo_pool() {
   return pools[dev];
 }
 
+// f(block as its element type) for a work block in a recursion precision
+template <typename Fn>
+int with_block(int prec, const void* p, Fn&& f) {
+  if (prec == TBK_PREC_FP64) f(static_cast<const double2*>(p));
+  else if (prec == TBK_PREC_DD) f(static_cast<const dd2*>(p));
+  else f(static_cast<const float2*>(p));
+  TBK_CHECK_LAUNCH();
+  return TBK_OK;
+}
+
+// Scratch of split_scale_kernel, the two sides' scales and the flag of values that do
+// not fit.
+struct SplitScales {
+  DevBuf part, words;          // words: scale of the left, of the right side; bad; count
+  int alloc(cudaStream_t st) {
+    TBK_TRY(part.alloc(sizeof(double) * 4 * sm_count()));
+    TBK_TRY(words.alloc(4 * sizeof(int)));
+    TBK_CUDA(cudaMemsetAsync(words.p, 0, words.bytes, st));
+    return TBK_OK;
+  }
+  float* scale(int h) const { return words.as<float>() + h; }
+  int* bad() const { return words.as<int>() + 2; }
+  unsigned int* count() const { return words.as<unsigned int>() + 3; }
+  template <typename CT>
+  void find(const CT* src, int64_t n, float* out, cudaStream_t st) const {
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + kStatThreads - 1) / kStatThreads, 2 * sm_count()));
+    split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, part.as<double>(), count(), out, bad());
+  }
+};
+
 // Vectors per chunk: the widest whose two stored sides (per_vector bytes each vector)
 // fit the budget; 1 when none does.  The same in every recursion precision (the GEMM
 // then sums in the same order).  both: a power of two (the widths of the one recursion
@@ -516,7 +628,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // runs them in complex64 with FP32 H~ (HBM-bound instead of FP64-pipe-bound).
   const size_t csz = prec == TBK_PREC_MIXED ? sizeof(float2) : sizeof(double2);
   DevBuf Ls, Rs, work, partd, part, macc, gdev, kstage;
-  const int64_t blk16 = (blk + 15) / 16 * 16;           // K padded to whole 16-element tiles (zeros)
+  bool use_tc = !f64b && (flags & TBK_MU_TENSOR) != 0;   // FP16-pair stores and the tensor-core GEMM
+  const int64_t blk16 = (blk + 31) / 32 * 32;           // K padded to whole tiles of either store (zeros)
   if ((!tl_async_alloc || tl_async_alloc->scratch) && 2.0 * sel * blk16 * M + 12.0 * csz * blk <= (double)kKuboPoolKeep) {
     kctx.pool = kubo_pool();
     kctx.stream = st;
@@ -546,19 +659,23 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     tl_async_alloc = outer;
     TBK_TRY(a);
   }
-  {
-    // the stores write every k < n Rc of every block; the entries of padded
-    // rows (n <= row < n_pad) and of the K tail up to whole 16-element tiles
-    // must read as zero.  In the K-tiled layout, element ((k/16) M + m) 16 +
-    // k%16, they all lie in the K tiles from floor(n Rc / 16) on: one
-    // contiguous region (the stores overwrite its written part afterwards)
-    const int64_t kt0 = (int64_t)n * Rc / 16, kt1 = blk16 / 16;
-    const size_t tile = (size_t)sel * 16 * M;           // bytes of one K tile of all M blocks
+  // the stores write every k < n Rc of every block; the entries of padded
+  // rows (n <= row < n_pad) and of the K tail up to whole tiles must read as
+  // zero.  In the K-tiled layouts (16 k a tile; FP16 pairs: 32) they all lie
+  // in the K tiles from floor(n Rc / tile) on: one contiguous region (the
+  // stores overwrite its written part afterwards)
+  auto zero_tail = [&]() -> int {
+    const int64_t kt = use_tc ? kSplitTile : 16, kt0 = (int64_t)n * Rc / kt, kt1 = (blk + kt - 1) / kt;
+    const size_t tile = (size_t)sel * kt * M;           // bytes of one K tile of all M blocks
     if (kt1 > kt0) {
       TBK_CUDA(cudaMemsetAsync(Ls.as<char>() + kt0 * tile, 0, (size_t)(kt1 - kt0) * tile, st));
       TBK_CUDA(cudaMemsetAsync(Rs.as<char>() + kt0 * tile, 0, (size_t)(kt1 - kt0) * tile, st));
     }
-  }
+    return TBK_OK;
+  };
+  TBK_TRY(zero_tail());
+  SplitScales sc;
+  if (use_tc) TBK_TRY(sc.alloc(st));
   TBK_CUDA(cudaMemsetAsync(work.p, 0, work.bytes, st));
   TBK_TRY(macc.alloc(sizeof(double2) * (size_t)M * M));
   TBK_CUDA(cudaMemsetAsync(macc.p, 0, macc.bytes, st));
@@ -598,17 +715,20 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     rec_bytes += 2 * vecb + ell_bytes(A, true);
     int g, t;
     TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
-    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, t, st, nullptr, 0, 0, true, nullptr,
-                    false);
+    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, t, st, nullptr, true, nullptr, false);
   };
-  auto round_to = [&](const void* src, float2* store, int32_t m) -> int {
+  const unsigned gblk = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
+  auto round_to = [&](const void* src, const KStore& ks, int32_t m) -> int {
     rec_bytes += vecb + stb;
-    const unsigned g = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
-    if (prec == TBK_PREC_FP64) round_block_kernel<double2><<<g, 256, 0, st>>>(static_cast<const double2*>(src), store, m, M, blk);
-    else if (prec == TBK_PREC_DD) round_block_kernel<dd2><<<g, 256, 0, st>>>(static_cast<const dd2*>(src), store, m, M, blk);
-    else round_block_kernel<float2><<<g, 256, 0, st>>>(static_cast<const float2*>(src), store, m, M, blk);
-    TBK_CHECK_LAUNCH();
-    return TBK_OK;
+    return with_block(prec, src, [&](auto p) {
+      if (ks.split)
+        split_block_kernel<<<gblk, 256, 0, st>>>(p, reinterpret_cast<__half*>(ks.store[0]), m, M, blk, ks.scale[0], ks.bad);
+      else
+        round_block_kernel<<<gblk, 256, 0, st>>>(p, ks.store[0], m, M, blk);
+    });
+  };
+  auto find_scale = [&](const void* src, int h) -> int {
+    return with_block(prec, src, [&](auto p) { sc.find(p, blk, sc.scale(h), st); });
   };
   // FP64 reference form: block m of the complex128 store from a work block
   auto store64 = [&](const void* src, void* store, int32_t m) -> int {
@@ -622,11 +742,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     return TBK_OK;
   };
   // block m of `store` = A x, written by the product itself (no work block)
-  auto apply_to_store = [&](tbk_sparse_s* A, const void* x, void* scratch, float2* store, int32_t m) -> int {
+  auto apply_to_store = [&](tbk_sparse_s* A, const void* x, void* scratch, KStore ks, int32_t m) -> int {
     rec_bytes += vecb + ell_bytes(A, true) + stb;
     int g, t;
     TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
-    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, st, store, M, m, false);
+    ks.km[0] = m;
+    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, st, &ks, false);
   };
   // one side: store[m] = Aout T_m(H~) (Bin v0), m < M; each step writes its
   // complex64 block (Aout absent) or feeds the product that does
@@ -634,9 +755,15 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // (a commutator [X, H~] does), step m also forms Aout T_{m-1} from the x it
   // gathers and writes block m-1: one pass over the matrix and the vectors per
   // block instead of two.  The stored values are the same bits either way.
-  auto side = [&](tbk_sparse_s* Aout, tbk_sparse_s* Bin, float2* store) -> int {
+  auto side = [&](tbk_sparse_s* Aout, tbk_sparse_s* Bin, float2* store, int h) -> int {
     void* r[3] = {wblk(0), wblk(1), wblk(2)};
     void* tmpA = wblk(3);
+    KStore ks;
+    ks.store[0] = store;
+    ks.kM = M;
+    ks.split = use_tc;
+    ks.scale[0] = sc.scale(h);
+    ks.bad = sc.bad();
     if (f64b) {                                           // recursion, operator, complex128 store
       if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
       else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
@@ -645,7 +772,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         if (m >= 1) {
           rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true);
           TBK_TRY(step_any(Ht, Rc, prec, r[(m - 1) % 3], y, m >= 2 ? r[(m - 2) % 3] : nullptr, m == 1,
-                           partd.as<double>(), grid, n_tiles, st, nullptr, 0, 0, true, nullptr, false));
+                           partd.as<double>(), grid, n_tiles, st, nullptr, true, nullptr, false));
         }
         if (Aout) {
           TBK_TRY(apply(Aout, y, tmpA));
@@ -663,24 +790,24 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     }
     if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
     else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
-    for (int32_t m = 0; m < M; ++m) {
+    // block 0; its values set the scale of an FP16-pair store
+    if (use_tc && Aout) TBK_TRY(apply(Aout, r[0], tmpA));
+    if (use_tc) TBK_TRY(find_scale(Aout ? tmpA : r[0], h));
+    if (!Aout) TBK_TRY(round_to(r[0], ks, 0));
+    else if (!fuse && use_tc) TBK_TRY(round_to(tmpA, ks, 0));
+    else if (!fuse) TBK_TRY(apply_to_store(Aout, r[0], tmpA, ks, 0));
+    for (int32_t m = 1; m < M; ++m) {
       void* y = r[m % 3];
-      if (m >= 1) {
-        const void* x = r[(m - 1) % 3];
-        const void* pv = m >= 2 ? r[(m - 2) % 3] : nullptr;
-        rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
-                     (fuse ? ell_bytes(Aout, false) : 0.0);
-        if (fuse)
-          TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, st, store, M, m - 1,
-                           true, Aout));
-        else
-          TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, st,
-                           Aout ? nullptr : store, M, m, true, nullptr, false));
-      }
-      if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, store, m));
-      else if (!Aout && m == 0) TBK_TRY(round_to(y, store, 0));
+      const void* x = r[(m - 1) % 3];
+      const void* pv = m >= 2 ? r[(m - 2) % 3] : nullptr;
+      rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
+                   (fuse ? ell_bytes(Aout, false) : 0.0);
+      ks.km[0] = fuse ? m - 1 : m;
+      TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, st,
+                       fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false));
+      if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
     }
-    if (fuse) TBK_TRY(apply_to_store(Aout, r[(M - 1) % 3], tmpA, store, M - 1));
+    if (fuse) TBK_TRY(apply_to_store(Aout, r[(M - 1) % 3], tmpA, ks, M - 1));
     return TBK_OK;
   };
   // both sides at once: columns [0, Rc) carry the left side (BL v0), [Rc, 2 Rc)
@@ -694,40 +821,37 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     tbk_sparse_s* Bin[2] = {BL, BR};
     tbk_sparse_s* Aout[2] = {AL, AR};
     float2* stores[2] = {Ls.as<float2>(), Rs.as<float2>()};
-    const unsigned gp = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
-    for (int h = 0; h < 2; ++h) {
-      if (Bin[h]) TBK_TRY(apply(Bin[h], v0, half[h]));
-      else TBK_CUDA(cudaMemcpyAsync(half[h], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
-      if (prec == TBK_PREC_FP64)
-        pack_cols_kernel<double2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const double2*>(half[h]),
-                                                      static_cast<double2*>(r[0]));
-      else if (prec == TBK_PREC_DD)
-        pack_cols_kernel<dd2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const dd2*>(half[h]),
-                                                  static_cast<dd2*>(r[0]));
-      else
-        pack_cols_kernel<float2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const float2*>(half[h]),
-                                                     static_cast<float2*>(r[0]));
-      TBK_CHECK_LAUNCH();
-      if (!Aout[h]) {
-        if (prec == TBK_PREC_FP64)
-          round_cols_kernel<double2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const double2*>(r[0]),
-                                                         stores[h], 0, M);
-        else if (prec == TBK_PREC_DD)
-          round_cols_kernel<dd2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const dd2*>(r[0]), stores[h], 0, M);
-        else
-          round_cols_kernel<float2><<<gp, 256, 0, st>>>(n_pad, Rc, h * Rc, static_cast<const float2*>(r[0]),
-                                                        stores[h], 0, M);
-        TBK_CHECK_LAUNCH();
-      }
-    }
     KStore ks;
     ks.halves = 2;
     ks.kM = M;
+    ks.split = use_tc;
+    ks.bad = sc.bad();
     for (int h = 0; h < 2; ++h) {
       ks.store[h] = stores[h];
       ks.usev[h] = Aout[h] ? 1 : 0;
       ks.vval[h] = Aout[h] ? ell_vals(Aout[h]->ell, prec) : nullptr;
       ks.vdiag[h] = Aout[h] ? ell_diag(Aout[h]->ell, prec) : nullptr;
+      ks.scale[h] = sc.scale(h);
+    }
+    for (int h = 0; h < 2; ++h) {
+      if (Bin[h]) TBK_TRY(apply(Bin[h], v0, half[h]));
+      else TBK_CUDA(cudaMemcpyAsync(half[h], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
+      if (use_tc) {
+        if (Aout[h]) TBK_TRY(apply(Aout[h], half[h], wblk(3)));
+        TBK_TRY(find_scale(Aout[h] ? wblk(3) : half[h], h));
+      }
+      TBK_TRY(with_block(prec, half[h], [&](auto p) {
+        using CT = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
+        pack_cols_kernel<CT><<<gblk, 256, 0, st>>>(n_pad, Rc, h * Rc, p, static_cast<CT*>(r[0]));
+      }));
+      if (!Aout[h])
+        TBK_TRY(with_block(prec, r[0], [&](auto p) {
+          if (use_tc)
+            split_cols_kernel<<<gblk, 256, 0, st>>>(n_pad, Rc, h * Rc, p, reinterpret_cast<__half*>(stores[h]), 0, M,
+                                                    ks.scale[h], ks.bad);
+          else
+            round_cols_kernel<<<gblk, 256, 0, st>>>(n_pad, Rc, h * Rc, p, stores[h], 0, M);
+        }));
     }
     rec_bytes += 2 * (vecb + 2 * vecb);                  // start halves packed into the wide block
     for (int h = 0; h < 2; ++h) rec_bytes += Aout[h] ? 0.0 : 2 * vecb + stb;
@@ -745,7 +869,6 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     }
     return TBK_OK;
   };
-  const bool use_tc = !f64b && (flags & TBK_MU_TENSOR) != 0;
   // split-K: at least 16,384 K values per CTA, at most 64 partial M x M blocks
   const int64_t ksplit = std::max<int64_t>(16384, (blk + 63) / 64);
   const int32_t nsplit = (int32_t)((blk + ksplit - 1) / ksplit);
@@ -757,12 +880,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     TBK_CUDA(cudaEventRecord(ev[0], st));
     if (kets) TBK_TRY(load_block_any(prec, n, R, r0, Rc, kstage.as<double2>(), v0, st));
     else TBK_TRY(random_block_any(prec, n, R, r0, Rc, seed, v0, st));
-    if (both) {
-      TBK_TRY(both_sides());
-    } else {
-      TBK_TRY(side(AL, BL, Ls.as<float2>()));
-      TBK_TRY(side(AR, BR, Rs.as<float2>()));
-    }
+    auto blocks = [&]() -> int {
+      if (both) return both_sides();
+      TBK_TRY(side(AL, BL, Ls.as<float2>(), 0));
+      return side(AR, BR, Rs.as<float2>(), 1);
+    };
+    TBK_TRY(blocks());
     TBK_CUDA(cudaEventRecord(ev[1], st));
     trace.mark("blocks");
     if (f64b) {
@@ -772,9 +895,19 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       mu_split_reduce_kernel<<<(unsigned)(((int64_t)M * M + 255) / 256), 256, 0, st>>>(part.as<double2>(), M, nsplit,
                                                                                        macc.as<double2>());
       TBK_CHECK_LAUNCH();
-    } else if (use_tc) {
-      TBK_TRY(mu_gemm_tc(Ls.as<float2>(), Rs.as<float2>(), M, blk, macc.as<double>(), st));
-    } else {
+    }
+    if (use_tc) {
+      const SplitStore L{Ls.as<__half>(), sc.scale(0), 0, sc.bad()}, R_{Rs.as<__half>(), sc.scale(1), 0, sc.bad()};
+      bool usable = false;
+      TBK_TRY(mu_gemm_tc(L, R_, M, blk, macc.as<double>(), &usable, st));
+      if (!usable) {                                     // values past FP16's range: complex64 stores from here on
+        use_tc = false;
+        TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
+        TBK_TRY(zero_tail());
+        TBK_TRY(blocks());
+      }
+    }
+    if (!use_tc && !f64b) {
       dim3 g((M + kGT - 1) / kGT, (M + kGT - 1) / kGT, nsplit);
       mu_gemm_cc_kernel<<<g, 256, 0, st>>>(Ls.as<float2>(), Rs.as<float2>(), M, blk, blk, ksplit, part.as<double2>());
       TBK_CHECK_LAUNCH();
@@ -826,8 +959,10 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   if (M < 1 || K < 1 || !L || !Rb || !mu_out) return fail(TBK_ERR_INVALID, "tbk_mu_from_blocks: bad argument");
   cudaStream_t st = as_stream(stream);
   ScratchScope scope(st);
-  const int64_t K16 = (K + 15) / 16 * 16;
-  DevBuf stage, Ld, Rd, acc, part;
+  const bool tensor = (flags & TBK_MU_TENSOR) != 0;
+  const int64_t K16 = (K + 31) / 32 * 32;                // whole tiles of either store
+  DevBuf stage, Ld, Rd, acc, part, scales;
+  SplitScales sc;
   TBK_TRY(stage.alloc(sizeof(double2) * K));
   TBK_TRY(Ld.alloc(sizeof(float2) * M * K16));
   TBK_TRY(Rd.alloc(sizeof(float2) * M * K16));
@@ -835,22 +970,45 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
   TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
   TBK_CUDA(cudaMemsetAsync(acc.p, 0, acc.bytes, st));
-  for (int side = 0; side < 2; ++side) {
-    float2* dst = side ? Rd.as<float2>() : Ld.as<float2>();
-    const double* src = side ? Rb : L;
-    for (int32_t m = 0; m < M; ++m) {
-      TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K, cudaMemcpyHostToDevice, st));
-      round_block_kernel<double2><<<(unsigned)std::min<int64_t>((K + 255) / 256, 4096), 256, 0, st>>>(stage.as<double2>(), dst, m,
-                                                                                          M, K);
-      TBK_CHECK_LAUNCH();
-    }
+  if (tensor) {
+    TBK_TRY(sc.alloc(st));
+    TBK_TRY(scales.alloc(sizeof(float) * 2 * M));        // a scale for every block
   }
+  const unsigned gk = (unsigned)std::min<int64_t>((K + 255) / 256, 4096);
+  auto upload = [&](bool split) -> int {
+    for (int side = 0; side < 2; ++side) {
+      DevBuf& dst = side ? Rd : Ld;
+      const double* src = side ? Rb : L;
+      for (int32_t m = 0; m < M; ++m) {
+        TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K, cudaMemcpyHostToDevice, st));
+        if (split) {
+          float* s = scales.as<float>() + side * M + m;
+          sc.find(stage.as<const double2>(), K, s, st);
+          split_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<__half>(), m, M, K, s, sc.bad());
+        } else {
+          round_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<float2>(), m, M, K);
+        }
+        TBK_CHECK_LAUNCH();
+      }
+    }
+    return TBK_OK;
+  };
+  TBK_TRY(upload(tensor));
   cudaEvent_t ev[2];
   for (auto& e : ev) TBK_CUDA(cudaEventCreate(&e));
   TBK_CUDA(cudaEventRecord(ev[0], st));
-  if (flags & TBK_MU_TENSOR) {
-    TBK_TRY(mu_gemm_tc(Ld.as<float2>(), Rd.as<float2>(), M, K, acc.as<double>(), st));
-  } else {
+  bool formed = false;
+  if (tensor) {
+    const SplitStore ls{Ld.as<__half>(), scales.as<float>(), 1, sc.bad()};
+    const SplitStore rs{Rd.as<__half>(), scales.as<float>() + M, 1, sc.bad()};
+    TBK_TRY(mu_gemm_tc(ls, rs, M, K, acc.as<double>(), &formed, st));
+    if (!formed) {                                       // infinities or NaN: complex64 blocks
+      TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
+      TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
+      TBK_TRY(upload(false));
+    }
+  }
+  if (!formed) {
     const int64_t ksplit = 16384;
     const int32_t nsplit = (int32_t)((K + ksplit - 1) / ksplit);
     TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));

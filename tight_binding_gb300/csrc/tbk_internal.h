@@ -197,6 +197,10 @@ struct KStore {
   int32_t usev[2] = {0, 0};
   int32_t kM = 0;
   int32_t halves = 1;
+  // split: the stores are FP16 pairs (split_store.cuh), scaled by *scale[h]
+  int32_t split = 0;
+  const float* scale[2] = {nullptr, nullptr};
+  int* bad = nullptr;
   const void* addv = nullptr;      // Clenshaw steps: output += (addc[0] + i addc[1]) addv
   double addc[2] = {0.0, 0.0};
 };
@@ -207,14 +211,14 @@ struct KStore {
 // Eigen-layout kets / seeded random phases.
 int step_width(int prec, int R, int cap);   // chunk width of R vectors
 int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st);
-// kstore: optional complex64 K-tiled store that receives the step's output as
-// block km of kM (store_y false: only there)
-// vop: with kstore, store vop x instead of the output; vop must share A's ELL
+// ks: optional K-tiled store that receives the step's output as block km[0]
+// (store_y false: only there)
+// vop: with ks, store vop x instead of the output; vop must share A's ELL
 // structure (same_ell_structure) and precision arrays
 // dots: form the moment partial sums (false: the step only feeds other work)
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-             int grid, int n_tiles, cudaStream_t st, float2* kstore = nullptr, int32_t kM = 0, int32_t km = 0,
-             bool store_y = true, tbk_sparse_s* vop = nullptr, bool dots = true);
+             int grid, int n_tiles, cudaStream_t st, const KStore* ks = nullptr, bool store_y = true,
+             tbk_sparse_s* vop = nullptr, bool dots = true);
 // ELL value / diagonal arrays of a precision (FP32, FP64 or double-float pairs)
 const void* ell_vals(const EllDev& E, int prec);
 const void* ell_diag(const EllDev& E, int prec);
