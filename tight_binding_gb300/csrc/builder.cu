@@ -931,6 +931,182 @@ int ensure_classes(tbk_sparse_s* A, cudaStream_t st) {
   return TBK_OK;
 }
 
+// ---- the same for FP32 values, of one matrix (v2 null) or of two with the same columns
+// (vw 4-byte words per entry and matrix).
+__global__ void class_hash32_kernel(int32_t n, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
+                                    const uint32_t* __restrict__ v1, const uint32_t* __restrict__ v2, int vw,
+                                    uint64_t* __restrict__ hash) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t s = i >> 5, l = i & 31;
+  const int64_t base = soff[s];
+  const int32_t w = (soff[s + 1] - soff[s]) >> 5;
+  uint64_t h = 0x9e3779b97f4a7c15ull;
+  int32_t cnt = 0;
+  for (int32_t k = 0; k < w; ++k) {
+    const int64_t o = base + (int64_t)k * 32 + l;
+    const int32_t c = ecol[o];
+    if (c == i) continue;                                  // padding
+    ++cnt;
+    h = cls_mix(h ^ (uint64_t)(uint32_t)(c - i));
+    for (int q = 0; q < vw; ++q)
+      h = cls_mix(h ^ ((uint64_t)v1[vw * o + q] << 32 | (v2 ? v2[vw * o + q] : 0u)));
+  }
+  h = cls_mix(h ^ (uint64_t)cnt);
+  hash[i] = h ? h : 1ull;
+}
+
+__global__ void class_verify32_kernel(int32_t n, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
+                                      const uint32_t* __restrict__ v1, const uint32_t* __restrict__ v2, int vw,
+                                      const uint8_t* __restrict__ cls, const int32_t* __restrict__ rep_of,
+                                      int* __restrict__ bad) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t j = rep_of[cls[i]];
+  const int32_t si = i >> 5, li = i & 31, sj = j >> 5, lj = j & 31;
+  const int32_t wi = (soff[si + 1] - soff[si]) >> 5, wj = (soff[sj + 1] - soff[sj]) >> 5;
+  int32_t ki = 0, kj = 0;
+  while (true) {
+    while (ki < wi && ecol[soff[si] + (int64_t)ki * 32 + li] == i) ++ki;
+    while (kj < wj && ecol[soff[sj] + (int64_t)kj * 32 + lj] == j) ++kj;
+    if (ki >= wi || kj >= wj) break;
+    const int64_t oi = soff[si] + (int64_t)ki * 32 + li, oj = soff[sj] + (int64_t)kj * 32 + lj;
+    bool same = (ecol[oi] - i) == (ecol[oj] - j);
+    for (int q = 0; q < vw; ++q)
+      same = same && v1[vw * oi + q] == v1[vw * oj + q] && (!v2 || v2[vw * oi + q] == v2[vw * oj + q]);
+    if (!same) {
+      atomicOr(bad, 1);
+      return;
+    }
+    ++ki;
+    ++kj;
+  }
+  if (ki < wi || kj < wj) atomicOr(bad, 1);                // different entry counts
+}
+
+__global__ void class_table32_kernel(int32_t n_cls, int32_t W, const int32_t* __restrict__ rep_of,
+                                     const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
+                                     const uint32_t* __restrict__ v1, const uint32_t* __restrict__ v2, int vw,
+                                     int32_t* __restrict__ cnt, int32_t* __restrict__ off, uint32_t* __restrict__ t1,
+                                     uint32_t* __restrict__ t2) {
+  const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n_cls) return;
+  const int32_t j = rep_of[c], s = j >> 5, l = j & 31;
+  const int32_t w = (soff[s + 1] - soff[s]) >> 5;
+  int32_t k = 0;
+  for (int32_t e = 0; e < w; ++e) {
+    const int64_t o = soff[s] + (int64_t)e * 32 + l;
+    if (ecol[o] == j) continue;
+    const int64_t t = (int64_t)c * W + k;
+    off[t] = ecol[o] - j;
+    for (int q = 0; q < vw; ++q) {
+      t1[vw * t + q] = v1[vw * o + q];
+      if (v2) t2[vw * t + q] = v2[vw * o + q];
+    }
+    ++k;
+  }
+  cnt[c] = k;
+  for (int32_t e = k; e < W; ++e) {
+    const int64_t t = (int64_t)c * W + e;
+    off[t] = 0;
+    for (int q = 0; q < vw; ++q) {
+      t1[vw * t + q] = 0u;
+      if (v2) t2[vw * t + q] = 0u;
+    }
+  }
+}
+
+// Every CTA of a step copies the table: square 256x256 with flux 1/64 (some 190 classes,
+// 9 KB) takes 8.2 us a step with it against 6.7 in the ELL form; FCC's 27 classes with an
+// operator's values are 4 KB.
+constexpr int64_t kMaxTable32 = 6144;
+
+static int class_set32(const EllDev& E, const float* f1, const float* f2, ClassSet32* out, cudaStream_t st) {
+  out->n_cls = 0;
+  if (const char* e = getenv("TBK_NO_CLASSES"))
+    if (atoi(e) != 0) return TBK_OK;
+  const int32_t n = E.n_rows, W = E.max_width;
+  if (n < 1 || !f1 || !E.col.p || W > kMaxClassEntries) return TBK_OK;
+  const uint32_t* v1 = reinterpret_cast<const uint32_t*>(f1);
+  const uint32_t* v2 = reinterpret_cast<const uint32_t*>(f2);
+  const int vw = E.cplx ? 2 : 1;
+  constexpr int32_t cap = 1024;
+  DevBuf hash, keys, rep, flags, slot_id, rep_of;
+  TBK_TRY(hash.alloc(sizeof(uint64_t) * n));
+  TBK_TRY(keys.alloc(sizeof(unsigned long long) * cap));
+  TBK_TRY(rep.alloc(sizeof(int32_t) * cap));
+  TBK_TRY(flags.alloc(2 * sizeof(int)));
+  TBK_CUDA(cudaMemsetAsync(keys.p, 0, keys.bytes, st));
+  TBK_CUDA(cudaMemsetAsync(rep.p, 0x7f, rep.bytes, st));
+  TBK_CUDA(cudaMemsetAsync(flags.p, 0, flags.bytes, st));
+  const int T = 256;
+  const unsigned g = (unsigned)((n + T - 1) / T);
+  const int32_t* soff = E.slice_off.as<int32_t>();
+  const int32_t* ecol = E.col.as<int32_t>();
+  class_hash32_kernel<<<g, T, 0, st>>>(n, soff, ecol, v1, v2, vw, hash.as<uint64_t>());
+  TBK_CHECK_LAUNCH();
+  class_insert_kernel<<<g, T, 0, st>>>(n, hash.as<uint64_t>(), keys.as<unsigned long long>(), rep.as<int32_t>(), cap,
+                                       flags.as<int>());
+  TBK_CHECK_LAUNCH();
+  std::vector<unsigned long long> hk(cap);
+  std::vector<int32_t> hr(cap);
+  int hf[2] = {0, 0};
+  TBK_CUDA(cudaMemcpyAsync(hk.data(), keys.p, keys.bytes, cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(hr.data(), rep.p, rep.bytes, cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(hf, flags.p, sizeof(hf), cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaStreamSynchronize(st));
+  if (hf[0]) return TBK_OK;                                // more keys than slots
+  std::vector<int32_t> sid(cap, -1), rof;
+  for (int32_t q = 0; q < cap; ++q)
+    if (hk[q]) {
+      sid[q] = (int32_t)rof.size();
+      rof.push_back(hr[q]);
+    }
+  const int32_t C = (int32_t)rof.size(), Wt = (std::max(W, 1) + 3) / 4 * 4;
+  if (C < 1 || C > kMaxClasses || (int64_t)C * Wt * (4 * vw * (v2 ? 2 : 1) + 4) > kMaxTable32) return TBK_OK;
+  ClassSet32 s;
+  TBK_TRY(slot_id.alloc(sizeof(int32_t) * cap));
+  TBK_TRY(rep_of.alloc(sizeof(int32_t) * C));
+  TBK_TRY(s.cls.alloc((size_t)E.n_slices * 32));
+  TBK_TRY(s.cnt.alloc(sizeof(int32_t) * C));
+  TBK_TRY(s.off.alloc(sizeof(int32_t) * C * Wt));
+  for (int h = 0; h < (v2 ? 2 : 1); ++h) TBK_TRY(s.val[h].alloc(sizeof(float) * vw * C * Wt));
+  TBK_CUDA(cudaMemcpyAsync(slot_id.p, sid.data(), sizeof(int32_t) * cap, cudaMemcpyHostToDevice, st));
+  TBK_CUDA(cudaMemcpyAsync(rep_of.p, rof.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice, st));
+  TBK_CUDA(cudaMemsetAsync(s.cls.p, 0, s.cls.bytes, st));
+  class_assign_kernel<<<g, T, 0, st>>>(n, hash.as<uint64_t>(), keys.as<unsigned long long>(), slot_id.as<int32_t>(),
+                                       cap, s.cls.as<uint8_t>(), flags.as<int>() + 1);
+  TBK_CHECK_LAUNCH();
+  class_verify32_kernel<<<g, T, 0, st>>>(n, soff, ecol, v1, v2, vw, s.cls.as<uint8_t>(), rep_of.as<int32_t>(),
+                                         flags.as<int>() + 1);
+  TBK_CHECK_LAUNCH();
+  class_table32_kernel<<<(C + 63) / 64, 64, 0, st>>>(C, Wt, rep_of.as<int32_t>(), soff, ecol, v1, v2, vw,
+                                                     s.cnt.as<int32_t>(), s.off.as<int32_t>(),
+                                                     s.val[0].as<uint32_t>(), s.val[1].as<uint32_t>());
+  TBK_CHECK_LAUNCH();
+  TBK_CUDA(cudaMemcpyAsync(hf, flags.p, sizeof(hf), cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaStreamSynchronize(st));
+  if (hf[1]) return TBK_OK;                                // a row differs from its class (hash collision)
+  s.n_cls = C;
+  s.w = Wt;
+  *out = std::move(s);
+  return TBK_OK;
+}
+
+int ensure_classes32(tbk_sparse_s* A, cudaStream_t st) {
+  TBK_TRY(ensure_classes(A, st));
+  EllDev& E = A->ell;
+  if (E.cls_state == 1 || E.cls32_state != 0) return TBK_OK;
+  E.cls32_state = -1;
+  TBK_TRY(class_set32(E, E.val32.as<float>(), nullptr, &E.c32, st));
+  if (E.c32.n_cls > 0) E.cls32_state = 1;
+  return TBK_OK;
+}
+
+int pair_classes32(tbk_sparse_s* A, tbk_sparse_s* B, ClassSet32* out, cudaStream_t st) {
+  return class_set32(A->ell, A->ell.val32.as<float>(), B->ell.val32.as<float>(), out, st);
+}
+
 }  // namespace tbk
 
 using namespace tbk;

@@ -210,9 +210,9 @@ int step_width(int prec, int R, int cap) {
   return p * 15 <= w * 16 ? p : w;
 }
 
-static int rows_per_tile(int prec, int Rc) {
+static int rows_per_tile(int prec, int Rc, int threads = kStepThreads) {
   const int vpl = prec != TBK_PREC_FP64 && Rc >= 2 ? 2 : 1;
-  return kStepThreads / (Rc / vpl);
+  return threads / (Rc / vpl);
 }
 
 // ---------------------------------------------------------------- internal API
@@ -225,9 +225,26 @@ const void* ell_diag(const EllDev& E, int prec) {
   return prec == TBK_PREC_MIXED ? E.diag32.p : prec == TBK_PREC_DD ? E.diagdd.p : E.diag64.p;
 }
 
+bool has_classes(const EllDev& E, int prec) {
+  return E.cls_state == 1 || (prec == TBK_PREC_MIXED && E.cls32_state == 1);
+}
+
+static ClassTab class_tab32(const ClassSet32& c) {
+  ClassTab t;
+  t.cls = c.cls.as<uint8_t>();
+  t.cnt = c.cnt.as<int32_t>();
+  t.off = c.off.as<int32_t>();
+  t.val = c.val[0].p;
+  t.val2 = c.val[1].p;
+  t.n_cls = c.n_cls;
+  t.w = c.w;
+  return t;
+}
+
 ClassTab class_tab(const EllDev& E, int prec) {
   ClassTab t;
-  if (E.cls_state != 1) return t;
+  if (!has_classes(E, prec)) return t;
+  if (E.cls_state != 1) return class_tab32(E.c32);
   t.cls = E.cls.as<uint8_t>();
   t.cnt = E.cls_cnt.as<int32_t>();
   t.off = E.cls_off.as<int32_t>();
@@ -238,36 +255,62 @@ ClassTab class_tab(const EllDev& E, int prec) {
 }
 
 size_t class_smem(const EllDev& E, int prec) {
-  if (E.cls_state != 1) return 0;
-  const size_t ne = (size_t)E.n_cls * E.cls_w;
+  const ClassTab t = class_tab(E, prec);
+  const size_t ne = (size_t)t.n_cls * t.w;
   const size_t fb = prec == TBK_PREC_MIXED ? 4 : 8;         // float, double, double-float pair
-  return ne * fb * (E.cplx ? 2 : 1) + ne * 4 + (size_t)E.n_cls * 4;
+  return ne * fb * (E.cplx ? 2 : 1) + ne * 4 + (size_t)t.n_cls * 4;
+}
+
+// Threads per CTA of the steps without sums: wide ones where every SM gets two waves of
+// them (below that the smaller CTAs spread better).
+static int step_threads(tbk_sparse_s* A, int Rc, int prec, int wide) {
+  if (prec != TBK_PREC_MIXED || !has_classes(A->ell, prec)) return kStepThreads;
+  const int64_t lanes = (int64_t)A->rows * (Rc >= 2 ? Rc / 2 : 1);
+  return lanes >= (int64_t)wide * 2 * 2 * sm_count() ? wide : kStepThreads;
 }
 
 // CTAs per SM of A's form.  FP64: the smaller of both forms', so that they group their
 // partial sums alike and give the same bits.
-static int step_occupancy(tbk_sparse_s* A, int Rc, int prec, bool sums) {
-  const bool cplx = A->ell.cplx != 0, cls = A->ell.cls_state == 1;
-  const int oc = cls || prec == TBK_PREC_FP64 ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec), sums) : 64;
+static int step_occupancy(tbk_sparse_s* A, int Rc, int prec, bool sums, int threads = kStepThreads) {
+  const bool cplx = A->ell.cplx != 0, cls = has_classes(A->ell, prec);
+  const int oc = cls || prec == TBK_PREC_FP64
+                     ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec), sums, threads) : 64;
   const int oe = !cls || prec == TBK_PREC_FP64 ? occupancy_prec(prec, cplx, Rc, sums) : 64;
   return std::min(oc, oe);
 }
 
+// grid and tiles of the steps without sums (step_any, step_ks)
 int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st) {
   TBK_TRY(ensure_ell(A, st));
   if (prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(A, st));
-  TBK_TRY(ensure_classes(A, st));
-  const int rpt = rows_per_tile(prec, Rc);
+  if (prec == TBK_PREC_MIXED) TBK_TRY(ensure_classes32(A, st));
+  else TBK_TRY(ensure_classes(A, st));
+  const int threads = step_threads(A, Rc, prec, kWideThreads<4>);
+  const int rpt = rows_per_tile(prec, Rc, threads);
   *n_tiles = (A->rows + rpt - 1) / rpt;
-  const int occ = step_occupancy(A, Rc, prec, false);
-  *grid = std::max(1, std::min(*n_tiles, sm_count() * occ));
+  *grid = std::max(1, std::min(*n_tiles, sm_count() * step_occupancy(A, Rc, prec, false, threads)));
   return TBK_OK;
 }
 
 static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const StepArgs& a, int grid, cudaStream_t st);
 
+static int pair_threads(tbk_sparse_s* A, int Rc) {
+  const int64_t lanes = (int64_t)A->rows * (Rc >= 2 ? Rc / 2 : 1);
+  return lanes >= (int64_t)kWideThreads<2> * 2 * 2 * sm_count() ? kWideThreads<2> : kStepThreads;
+}
+
+int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles) {
+  const int threads = pair_threads(A, Rc), rpt = rows_per_tile(TBK_PREC_MIXED, Rc, threads);
+  *n_tiles = (A->rows + rpt - 1) / rpt;
+  // launch bounds: two CTAs of the wide size per SM
+  const int per_sm = 2 * kWideThreads<2> / threads;
+  *grid = std::max(1, std::min(*n_tiles, sm_count() * per_sm));
+  return TBK_OK;
+}
+
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-             int grid, int n_tiles, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots) {
+             int grid, int n_tiles, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots,
+             const ClassSet32* pair) {
   StepArgs a;
   a.n = A->rows;
   a.n_tiles = n_tiles;
@@ -295,6 +338,10 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
       a.ks.vdiag[0] = ell_diag(vop->ell, prec);
       a.ks.usev[0] = 1;
       a.kst = 2;
+      if (pair) {
+        a.ct = class_tab32(*pair);
+        a.threads = pair_threads(A, Rc);
+      }
     }
   } else if (vop) {
     return fail(TBK_ERR_INVALID, "operator product without a store");
@@ -332,9 +379,12 @@ int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const voi
 
 static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const StepArgs& a0, int grid, cudaStream_t st) {
   StepArgs a = a0;
-  if (A->ell.cls_state == 1 && a.kst != 2) {                // the class form where it applies
+  if (a.ct.val2) {                                          // joint classes with the operator
+    a.cls = true;
+  } else if (has_classes(A->ell, prec) && a.kst != 2) {     // the class form where it applies
     a.cls = true;
     a.ct = class_tab(A->ell, prec);
+    a.threads = step_threads(A, Rc, prec, kWideThreads<4>);
   }
   return launch_step_prec(prec, A->ell.cplx != 0, Rc, a, first, false, grid, st);
 }
@@ -348,14 +398,14 @@ int occupancy_dd(bool cplx, int R, bool sums);
 int launch_step_cls_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
-int occupancy_cls_f32(bool cplx, int R, size_t smem, bool sums);
+int occupancy_cls_f32(bool cplx, int R, size_t smem, bool sums, int threads);
 int occupancy_cls_f64(bool cplx, int R, size_t smem, bool sums);
 int occupancy_cls_dd(bool cplx, int R, size_t smem, bool sums);
 
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums) {
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums, int threads) {
   if (prec == TBK_PREC_FP64) return occupancy_cls_f64(cplx, R, smem, sums);
   if (prec == TBK_PREC_DD) return occupancy_cls_dd(cplx, R, smem, sums);
-  return occupancy_cls_f32(cplx, R, smem, sums);
+  return occupancy_cls_f32(cplx, R, smem, sums, threads);
 }
 
 int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid,
@@ -630,8 +680,9 @@ static int plan_small(tbk_kpm_s* P, bool tma) {
   if (P->use_cls && P->prec == TBK_PREC_MIXED) {
     CtaLayout C;
     C.n = n;
-    C.n_cls = E.n_cls;
-    C.w = E.cls_w;
+    const ClassTab ct = class_tab(E, P->prec);
+    C.n_cls = ct.n_cls;
+    C.w = ct.w;
     C.csz = (int32_t)P->csize;
     C.vb = (P->prec == TBK_PREC_MIXED ? 4 : 8) * (E.cplx ? 2 : 1);
     if ((int64_t)C.bytes() <= kSmallSmemBytes) {
@@ -994,13 +1045,13 @@ int tbk_kpm_create(tbk_kpm* out, tbk_sparse Ht, int32_t R, int32_t flags) {
   int occ = 1;
   const bool cplx = Ht->ell.cplx != 0;
   {
-    const int s0 = ensure_classes(Ht, st);
+    const int s0 = prec == TBK_PREC_MIXED ? ensure_classes32(Ht, st) : ensure_classes(Ht, st);
     if (s0 != TBK_OK) {
       delete P;
       return s0;
     }
   }
-  P->use_cls = Ht->ell.cls_state == 1;
+  P->use_cls = has_classes(Ht->ell, prec);
   occ = step_occupancy(Ht, rc, prec, true);
   P->grid = std::max(1, std::min(P->n_tiles, sm_count() * occ));
   P->grid_max = P->grid;

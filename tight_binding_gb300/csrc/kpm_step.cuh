@@ -22,6 +22,7 @@ struct ClassTab {
   const int32_t* cnt = nullptr;
   const int32_t* off = nullptr;
   const void* val = nullptr;
+  const void* val2 = nullptr;   // values of a second matrix with the same columns (KST = 2)
   int32_t n_cls = 0, w = 0;
 };
 // shared-memory table of the class form: values, offsets, counts
@@ -30,7 +31,7 @@ constexpr int class_value_bytes() { return (CPLX_H ? 2 : 1) * (int)sizeof(F); }
 template <typename F, bool CPLX_H>
 inline size_t class_smem_bytes(const ClassTab& ct) {
   const size_t ne = (size_t)ct.n_cls * ct.w;
-  return ne * class_value_bytes<F, CPLX_H>() + ne * 4 + (size_t)ct.n_cls * 4;
+  return ne * class_value_bytes<F, CPLX_H>() * (ct.val2 ? 2 : 1) + ne * 4 + (size_t)ct.n_cls * 4;
 }
 
 // The moment sums of a step, part[slot][CTA].  FP64 from here on, and an FP64
@@ -98,6 +99,16 @@ __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, co
   else h.template fma<VPL>(xs, acc);
 }
 
+// Class-form complex64 steps that feed stores or an operator product may run with up to
+// kWideThreads threads per CTA.  On 3D lattices the neighbours' rows come from L2, and a
+// CTA of consecutive rows shares their lines in L1: FCC 128^3 with 4 vectors has 128 rows
+// to a lattice line, so that 256 threads hold one line, 768 three: a step with an FP16-pair
+// store 71.6 -> 61.0 us.
+template <typename F, int KST, bool CLS>
+constexpr bool kWideSteps = CLS && sizeof(F) == 4 && KST != 0 && KST != 3;
+template <int KST>
+constexpr int kWideThreads = KST == 2 ? 512 : 768;
+
 // Steps bound by arithmetic may take more registers than the compiler gives them by
 // itself: fewer warps with more gathers each in flight run faster (honeycomb 1024x1024,
 // R = 32: FP64 braket 1,483 -> 1,364 us, double-float doubling 795 -> 744-762 us).  FP64: 4
@@ -106,7 +117,7 @@ __device__ __forceinline__ void ell_entry(const F* __restrict__ p, int64_t o, co
 // any number in the class form's moment steps; not in the ELL form (701x600 with
 // vacancies, R = 20: 200 -> 216 us) nor in its Clenshaw steps.  0: not stated.
 template <typename F, int KST, bool CLS>
-constexpr int kMinCtas = is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
+constexpr int kMinCtas = kWideSteps<F, KST, CLS> ? 2 : is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
 
 // One recursion step over all rows, x = v_s, y = v_{s-1} on entry.
 //   FIRST: y = H x                    else: y = 2 H x - y  (v_{s+1} over v_{s-1})
@@ -139,7 +150,8 @@ constexpr int kMinCtas = is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
 //   R: vectors per row, a power of two; 0: any other width, LPR lanes per row given
 //   at run time (rows stay whole within a CTA, a few threads at its end idle).
 template <typename F, int R, bool CPLX_H, bool FIRST, bool BRAKET, int KST = 0, bool PIPE = false, bool CLS = false>
-__global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_kernel(
+__global__ void __launch_bounds__(kWideSteps<F, KST, CLS> ? kWideThreads<KST> : kStepThreads, kMinCtas<F, KST, CLS>)
+kpm_step_kernel(
     int32_t n, int32_t n_tiles, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
     const F* __restrict__ eval, const F* __restrict__ diag, const typename C2<F>::T* __restrict__ x,
     typename C2<F>::T* y, const typename C2<F>::T* pv, const typename C2<F>::T* __restrict__ bras,
@@ -149,7 +161,7 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
   static_assert(R == 0 || (R / VPL >= 1 && R / VPL <= 32 && (32 % (R / VPL)) == 0), "R out of range");
   const int LPR = R > 0 ? R / VPL : lpr;   // lanes per row
   const int RW = LPR * VPL;                // vectors per row
-  const int ROWS_PER_TILE = kStepThreads / LPR;
+  const int ROWS_PER_TILE = (kWideSteps<F, KST, CLS> ? (int)blockDim.x : kStepThreads) / LPR;
   const int trow = threadIdx.x / LPR;      // this thread's row in a tile (none: past n)
   const bool idle = R == 0 && trow >= ROWS_PER_TILE;
   using Acc = F;                           // per-thread sums in the vector precision
@@ -158,17 +170,18 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
   const int sub = threadIdx.x % LPR;
   Acc m0 = 0, m1 = 0;
   constexpr bool FOLD = kFoldStep<F> && !FIRST;
-  static_assert(!(CLS && (PIPE || KST == 2)), "class form: no column pipeline, no operator products");
+  static_assert(!(CLS && PIPE), "class form: no column pipeline");
 
   // class form: the table in shared memory (4-byte words: values, offsets, counts)
   extern __shared__ __align__(16) unsigned char cls_smem[];
   const F* s_val = reinterpret_cast<const F*>(cls_smem);
+  const F* s_val2 = nullptr;               // the operator's values (KST = 2)
   const int32_t* s_off = nullptr;
   const int32_t* s_cnt = nullptr;
   uint32_t c_next = 0;                     // class of this thread's row in the next iteration
   if constexpr (CLS) {
     const int32_t ne = ct.n_cls * ct.w;
-    const int32_t vw = ne * (class_value_bytes<F, CPLX_H>() / 4);
+    const int32_t v1 = ne * (class_value_bytes<F, CPLX_H>() / 4), vw = KST == 2 ? 2 * v1 : v1;
     uint32_t* sw = reinterpret_cast<uint32_t*>(cls_smem);
     const uint32_t* gv = static_cast<const uint32_t*>(ct.val);
     if constexpr (FOLD) {
@@ -176,7 +189,12 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
       for (int32_t q = threadIdx.x; q < ne * (CPLX_H ? 2 : 1); q += blockDim.x)
         dv[q] = times2(static_cast<const F*>(ct.val)[q]);
     } else {
-      for (int32_t q = threadIdx.x; q < vw; q += blockDim.x) sw[q] = gv[q];
+      for (int32_t q = threadIdx.x; q < v1; q += blockDim.x) sw[q] = gv[q];
+    }
+    if constexpr (KST == 2) {
+      const uint32_t* gw = static_cast<const uint32_t*>(ct.val2);
+      for (int32_t q = threadIdx.x; q < v1; q += blockDim.x) sw[v1 + q] = gw[q];
+      s_val2 = reinterpret_cast<const F*>(sw + v1);
     }
     for (int32_t q = threadIdx.x; q < ne; q += blockDim.x) sw[vw + q] = (uint32_t)ct.off[q];
     for (int32_t q = threadIdx.x; q < ct.n_cls; q += blockDim.x) sw[vw + ne + q] = (uint32_t)ct.cnt[q];
@@ -272,6 +290,7 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
     }
     if (gather && CLS) {
       ell_entry<F, VPL, CPLX_H, FOLD>(diag, r, xs, acc);
+      if constexpr (KST == 2) HVal<F, CPLX_H>::load(vdiag, r).template fma<VPL>(xs, vacc);
       const int32_t cnt = s_cnt[c_cur];
       const int32_t tb = (int32_t)c_cur * ct.w;
       // a class's tail entries up to the table width (a multiple of 4) are
@@ -281,7 +300,7 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
       // whose unconditional form holds more gathers in registers
       constexpr bool WHOLE = sizeof(F) == 4;
       int k0 = 0;
-      if constexpr (is_f64<F>) {
+      if constexpr (is_f64<F> && KST != 2) {
         // FP64: whole groups, then single entries (a predicated product still
         // takes its turn on the FP64 pipe)
         for (; k0 + 4 <= cnt; k0 += 4) {
@@ -311,6 +330,11 @@ __global__ void __launch_bounds__(kStepThreads, kMinCtas<F, KST, CLS>) kpm_step_
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], acc);
+        if constexpr (KST == 2) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (WHOLE || k + u < cnt) HVal<F, CPLX_H>::load_smem(s_val2, tb + k + u).template fma<VPL>(xv[u], vacc);
+        }
       }
     } else if (gather) {
       ell_entry<F, VPL, CPLX_H, FOLD>(diag, r, xs, acc);
@@ -451,6 +475,7 @@ struct StepArgs {
   bool pipe = false;           // ELL wider than 4: pipelined column loads
   bool cls = false;            // row classes (ct) instead of the ELL's columns and values
   ClassTab ct;
+  int32_t threads = kStepThreads;   // per CTA (class-form complex64 steps without sums)
   int32_t lpr = 0;             // lanes per row of a width without its own instantiation (R = 0)
 };
 
@@ -467,7 +492,7 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
 #define TBK_STEP(FI, BR, KS)                                                                          \
   do {                                                                                                \
     if constexpr (CLS)                                                                                \
-      kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, false, true><<<grid, kStepThreads, smem, st>>>(       \
+      kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, false, true><<<grid, kWideSteps<F, KS, true> ? a.threads : kStepThreads, smem, st>>>( \
           a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
           a.ct, a.lpr);                                                                                      \
     else if (a.pipe)                                                                                  \
@@ -493,8 +518,8 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
     } else if (a.kst == 5) {
       if (first) TBK_STEP(true, false, 5); else TBK_STEP(false, false, 5);
     } else if (a.kst == 2) {
-      if constexpr (CLS) return fail(TBK_ERR_UNSUPPORTED, "operator products in the class form");
-      else { if (first) TBK_STEP(true, false, 2); else TBK_STEP(false, false, 2); }
+      if (CLS && !a.ct.val2) return fail(TBK_ERR_UNSUPPORTED, "operator product without its class values");
+      if (first) TBK_STEP(true, false, 2); else TBK_STEP(false, false, 2);
     }
     else { if (first) TBK_STEP(true, false, 1); else TBK_STEP(false, false, 1); }
   } else if (first) { if (braket) TBK_STEP(true, true, 0); else TBK_STEP(true, false, 0); }
@@ -526,28 +551,29 @@ inline int launch_step(int R, const StepArgs& a, bool first, bool braket, int gr
 }
 
 
+// threads: of a wide step (kWideSteps)
 template <typename F, bool CPLX_H, int R, bool CLS = false>
-inline int occupancy_blocks(size_t smem, bool sums) {
+inline int occupancy_blocks(size_t smem, bool sums, int threads = kStepThreads) {
   int nb = 0;
   if (sums)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 0, false, CLS>,
                                                   kStepThreads, smem);
   else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 4, false, CLS>,
-                                                  kStepThreads, smem);
+                                                  threads, smem);
   return nb > 0 ? nb : 1;
 }
 
 template <typename F, bool CLS>
-inline int occupancy_r(bool cplx, int R, size_t smem, bool sums) {
+inline int occupancy_r(bool cplx, int R, size_t smem, bool sums, int threads = kStepThreads) {
   switch (R) {
-    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem, sums) : occupancy_blocks<F, false, 1, CLS>(smem, sums);
-    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem, sums) : occupancy_blocks<F, false, 2, CLS>(smem, sums);
-    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem, sums) : occupancy_blocks<F, false, 4, CLS>(smem, sums);
-    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem, sums) : occupancy_blocks<F, false, 8, CLS>(smem, sums);
-    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem, sums) : occupancy_blocks<F, false, 16, CLS>(smem, sums);
-    case 32: case 64: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem, sums) : occupancy_blocks<F, false, 32, CLS>(smem, sums);
-    default: return cplx ? occupancy_blocks<F, true, 0, CLS>(smem, sums) : occupancy_blocks<F, false, 0, CLS>(smem, sums);
+    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 1, CLS>(smem, sums, threads);
+    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 2, CLS>(smem, sums, threads);
+    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 4, CLS>(smem, sums, threads);
+    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 8, CLS>(smem, sums, threads);
+    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 16, CLS>(smem, sums, threads);
+    case 32: case 64: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 32, CLS>(smem, sums, threads);
+    default: return cplx ? occupancy_blocks<F, true, 0, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 0, CLS>(smem, sums, threads);
   }
 }
 
@@ -557,7 +583,9 @@ int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, 
 // CTAs per SM; sums: of the steps that form moment sums
 int occupancy_prec(int prec, bool cplx, int R, bool sums);
 // the same of the class-form kernel with its shared-memory table
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums);
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums, int threads = kStepThreads);
+// whether a matrix runs in the class form in a precision
+bool has_classes(const EllDev& E, int prec);
 // the class table of a matrix in a precision (ct.n_cls == 0: no class form)
 ClassTab class_tab(const EllDev& E, int prec);
 size_t class_smem(const EllDev& E, int prec);

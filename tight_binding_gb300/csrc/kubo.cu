@@ -708,7 +708,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // class form (row classes): the row's class byte and diagonal; the table is in shared memory
   auto ell_bytes = [&](tbk_sparse_s* A, bool cols) {
     const double hv = (double)vsz * (A->ell.cplx ? 2 : 1);
-    if (cols && A->ell.cls_state == 1) return (double)A->rows * (1.0 + hv);
+    if (cols && (A->ell.cls_state == 1 || (prec == TBK_PREC_MIXED && A->ell.cls32_state == 1))) return (double)A->rows * (1.0 + hv);
     return (double)A->ell.n_entries * ((cols ? 4.0 : 0.0) + hv) + (double)A->rows * hv;
   };
   auto apply = [&](tbk_sparse_s* A, const void* x, void* y) -> int {   // y = A x
@@ -783,10 +783,18 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       }
       return TBK_OK;
     }
+    // complex64 recursions take the operator's products inside the step wherever H~ and
+    // the operator have joint row classes: one pass over the vectors' neighbours per block
+    // instead of two (FCC 128^3, 4 vectors: 77.9 us against 56.5 + 83.7)
     bool fuse = false;
-    if (Aout && (flags & TBK_MU_FUSED_OPS)) {
+    ClassSet32 pair;
+    int pgrid = grid, ptiles = n_tiles;
+    if (Aout && ((flags & TBK_MU_FUSED_OPS) || prec == TBK_PREC_MIXED)) {
       TBK_TRY(same_ell_structure(Ht, Aout, &fuse, st));
       if (fuse && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
+      if (fuse && prec == TBK_PREC_MIXED) TBK_TRY(pair_classes32(Ht, Aout, &pair, st));
+      if (pair.n_cls > 0) TBK_TRY(pair_config(Ht, Rc, pair, &pgrid, &ptiles));
+      else fuse = fuse && (flags & TBK_MU_FUSED_OPS);
     }
     if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
     else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
@@ -803,8 +811,9 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
                    (fuse ? ell_bytes(Aout, false) : 0.0);
       ks.km[0] = fuse ? m - 1 : m;
-      TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, st,
-                       fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false));
+      TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), pgrid, ptiles, st,
+                       fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false,
+                       pair.n_cls > 0 ? &pair : nullptr));
       if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
     }
     if (fuse) TBK_TRY(apply_to_store(Aout, r[(M - 1) % 3], tmpA, ks, M - 1));

@@ -128,6 +128,10 @@ struct DevBuf {
 // slice (entry k of row 32*s + l at off[s] + 32*k + l).  The diagonal is kept
 // apart so that every row owns its v_n element.  Padding entries point at the
 // row itself with value 0.
+struct ClassSet32 {        // row classes of FP32 values: one matrix, or two with the same columns
+  int32_t n_cls = 0, w = 0;
+  DevBuf cls, cnt, off, val[2];
+};
 struct EllDev {
   int32_t n_rows = 0, n_slices = 0;
   int64_t n_entries = 0;
@@ -156,6 +160,11 @@ struct EllDev {
   DevBuf cls_v64;          // double / double2 [n_cls * cls_w]
   DevBuf cls_v32;          // float / float2
   DevBuf cls_vdd;          // double-float pairs (real: float2, complex: float4)
+  // The same of the FP32 values alone, for complex64 vectors where the FP64 values do not
+  // repeat (ensure_classes32): a commutator [X, H~] or a rational flux whose entries
+  // differ in FP64's last bits from row to row.
+  int32_t cls32_state = 0;
+  ClassSet32 c32;
 };
 constexpr int32_t kMaxClasses = 255;
 constexpr int32_t kMaxClassEntries = 1024;   // n_cls * cls_w (shared-memory table of the step kernel)
@@ -180,6 +189,9 @@ namespace tbk {
 int ensure_ell(tbk_sparse_s* A, cudaStream_t st);
 int ensure_ell_dd(tbk_sparse_s* A, cudaStream_t st);   // double-float copy of the FP64 values
 int ensure_classes(tbk_sparse_s* A, cudaStream_t st);  // row classes of the ELL (cls_state 1 or -1)
+int ensure_classes32(tbk_sparse_s* A, cudaStream_t st);   // FP32 classes where A has none in FP64 (cls32_state)
+// joint classes of A's and B's FP32 values; B must share A's ELL structure.  n_cls 0: none
+int pair_classes32(tbk_sparse_s* A, tbk_sparse_s* B, ClassSet32* out, cudaStream_t st);
 int exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStream_t st, int32_t* total_host);
 int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t st, int64_t* total_host);
 int sm_count();
@@ -214,11 +226,14 @@ int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cuda
 // ks: optional K-tiled store that receives the step's output as block km[0]
 // (store_y false: only there)
 // vop: with ks, store vop x instead of the output; vop must share A's ELL
-// structure (same_ell_structure) and precision arrays
+// structure (same_ell_structure) and precision arrays; pair: their joint classes
 // dots: form the moment partial sums (false: the step only feeds other work)
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
              int grid, int n_tiles, cudaStream_t st, const KStore* ks = nullptr, bool store_y = true,
-             tbk_sparse_s* vop = nullptr, bool dots = true);
+             tbk_sparse_s* vop = nullptr, bool dots = true, const ClassSet32* pair = nullptr);
+// grid and tiles of a step with an operator product in the joint class form (complex64;
+// pair: pair_classes32 of A and the operator)
+int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles);
 // ELL value / diagonal arrays of a precision (FP32, FP64 or double-float pairs)
 const void* ell_vals(const EllDev& E, int prec);
 const void* ell_diag(const EllDev& E, int prec);
