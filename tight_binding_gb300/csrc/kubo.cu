@@ -37,38 +37,72 @@ namespace tbk {
 namespace {
 
 // ------------------------------------------------------------------ CUDA-core GEMM
-// C[m][n] += sum_k conj(L[m][k]) R[n][k] for a K range per CTA (split-K), blocks
-// in the K-tiled layout;
-// FP32 products, FP32 sums over 32 terms promoted to FP64, FP64 partial tiles.
-constexpr int kGT = 32;      // output tile (complex) per CTA side
-constexpr int kGK = 32;      // K chunk staged in shared memory
+// C[m][n] += sum_k conj(L[m][k]) R[n][k] for a K range per CTA (split-K), blocks in the
+// K-tiled layout; FP32 products, FP32 sums over 32 terms added into float-float pairs by
+// TwoSum (48 bits, on the FP32 pipe: FP64 sums of the chunks took twice the time of the
+// products), FP64 partial tiles.  64 x 32 complex outputs per CTA, 4 x 2 per thread: 6
+// shared-memory reads for 32 FMAs, each one wavefront (rows 17 values apart), so the FMAs
+// bound it; the K tiles arrive by cp.async, three deep.  M = 200, K = 56,064: 2.20 ms with
+// 2 x 2 outputs per thread and FP64 sums, 0.86 ms so.
+constexpr int kGT = 32;      // output tile (complex) per CTA side of the FP64 form, and n here
+constexpr int kGM = 64;      // m
+constexpr int kGStages = 3;
+constexpr int kGPitch = 17;  // a K tile's 16 values and one of padding
 
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(real ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void ff_add(float& hi, float& lo, float v) {      // TwoSum (Knuth)
+  const float s = __fadd_rn(hi, v), b = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(v, b)));
+  hi = s;
+}
+
+// K tiles [t0, t1) of blockIdx.z; M blocks per K tile in both stores
 __global__ void __launch_bounds__(256) mu_gemm_cc_kernel(const float2* __restrict__ L, const float2* __restrict__ Rb,
-                                                         int32_t M, int64_t K, int64_t ld, int64_t ksplit,
+                                                         int32_t M, int64_t tiles, int64_t tiles_split,
                                                          double2* __restrict__ part) {
-  __shared__ float2 Ls[kGT][kGK + 1], Rs[kGT][kGK + 1];
+  __shared__ float2 sm[kGStages][kGM + kGT][kGPitch];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int32_t m0 = blockIdx.y * kGT, n0 = blockIdx.x * kGT;
-  const int64_t k0 = (int64_t)blockIdx.z * ksplit;
-  const int64_t k1 = min(K, k0 + ksplit);
-  float ar[2][2] = {{0, 0}, {0, 0}}, ai[2][2] = {{0, 0}, {0, 0}};
-  double dr[2][2] = {{0, 0}, {0, 0}}, di[2][2] = {{0, 0}, {0, 0}};
-  for (int64_t kb = k0; kb < k1; kb += kGK) {
-    for (int q = threadIdx.x; q < kGT * kGK; q += 256) {
-      const int row = q / kGK, kk = q % kGK;
-      const int64_t k = kb + kk;
-      float2 z = make_float2(0.f, 0.f);
-      Ls[row][kk] = (m0 + row < M && k < k1) ? L[((k >> 4) * M + (m0 + row)) * 16 + (k & 15)] : z;
-      Rs[row][kk] = (n0 + row < M && k < k1) ? Rb[((k >> 4) * M + (n0 + row)) * 16 + (k & 15)] : z;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < kGK; ++kk) {
-      const float2 a0 = Ls[ty * 2][kk], a1 = Ls[ty * 2 + 1][kk];
-      const float2 b0 = Rs[tx * 2][kk], b1 = Rs[tx * 2 + 1][kk];
-      const float2 a[2] = {a0, a1}, b[2] = {b0, b1};
+  const int32_t m0 = blockIdx.y * kGM, n0 = blockIdx.x * kGT;
+  const int64_t t0 = (int64_t)blockIdx.z * tiles_split, t1 = min(tiles, t0 + tiles_split);
+  // 6 values of a stage per thread: value tx of rows ty, ty + 16, ...; rows past M read as zero
+  auto load = [&](int64_t t) {
+    if (t < t1) {
+      float2(*st)[kGPitch] = sm[(t - t0) % kGStages];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int q = 0; q < (kGM + kGT) / 16; ++q) {
+        const int row = ty + 16 * q;
+        const bool left = row < kGM;
+        const int32_t b = left ? m0 + row : n0 + row - kGM;
+        const float2* src = (left ? L : Rb) + (t * M + min(b, M - 1)) * 16 + tx;
+        cp_async8(&st[row][tx], src, b < M);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float hr[4][2], lr[4][2], hi[4][2], li[4][2], ar[4][2], ai[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) hr[i][j] = lr[i][j] = hi[i][j] = li[i][j] = ar[i][j] = ai[i][j] = 0.f;
+  load(t0);
+  load(t0 + 1);
+  for (int64_t t = t0; t < t1; ++t) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const float2(*st)[kGPitch] = sm[(t - t0) % kGStages];
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+      float2 a[4], b[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = st[ty + 16 * i][kk];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) b[j] = st[kGM + tx + 16 * j][kk];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           // conj(a) * b
@@ -76,20 +110,29 @@ __global__ void __launch_bounds__(256) mu_gemm_cc_kernel(const float2* __restric
           ai[i][j] += a[i].x * b[j].y - a[i].y * b[j].x;
         }
     }
-    __syncthreads();
-    // FP32 sums cover one 32-term chunk only: long FP32 accumulations lose
-    // accuracy where the sum is much smaller than its terms (mu_nm at large m, n)
+    load(t + 2);                 // over the stage that every thread left before this barrier
+    // FP32 sums cover two K tiles (32 terms) only: long FP32 accumulations lose accuracy
+    // where the sum is much smaller than its terms (mu_nm at large m, n)
+    if (((t - t0) & 1) || t + 1 == t1) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) { dr[i][j] += ar[i][j]; di[i][j] += ai[i][j]; ar[i][j] = 0; ai[i][j] = 0; }
+        for (int j = 0; j < 2; ++j) {
+          ff_add(hr[i][j], lr[i][j], ar[i][j]);
+          ff_add(hi[i][j], li[i][j], ai[i][j]);
+          ar[i][j] = ai[i][j] = 0.f;
+        }
+    }
   }
-  for (int i = 0; i < 2; ++i)
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
     for (int j = 0; j < 2; ++j) {
-      dr[i][j] += ar[i][j];
-      di[i][j] += ai[i][j];
-      const int32_t m = m0 + ty * 2 + i, n = n0 + tx * 2 + j;
-      if (m < M && n < M) part[((int64_t)blockIdx.z * M + m) * M + n] = make_double2(dr[i][j], di[i][j]);
+      const int32_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      if (m < M && n < M)
+        part[((int64_t)blockIdx.z * M + m) * M + n] = make_double2((double)hr[i][j] + (double)lr[i][j],
+                                                                   (double)hi[i][j] + (double)li[i][j]);
     }
 }
 
@@ -101,6 +144,25 @@ __global__ void mu_split_reduce_kernel(const double2* __restrict__ part, int32_t
   for (int32_t s = 0; s < nsplit; ++s) { const double2 v = part[(int64_t)s * M * M + q]; r += v.x; i += v.y; }
   acc[q].x += r;
   acc[q].y += i;
+}
+
+// acc += L^H R of complex64 K-tiled stores.  K is split until the CTAs fill the SMs twice
+// over (three CTAs each), into at most 64 partial M x M blocks of 1,024 values of k or
+// more, and at least into those of 16,384 or K / 64.
+int mu_gemm_cc(const float2* L, const float2* Rb, int32_t M, int64_t K, DevBuf* part, double2* acc, cudaStream_t st) {
+  const int64_t tiles = (K + 15) / 16;
+  const dim3 out((M + kGT - 1) / kGT, (M + kGM - 1) / kGM);
+  const int64_t want = (6LL * sm_count() + (int64_t)out.x * out.y - 1) / ((int64_t)out.x * out.y);
+  int64_t split = std::max<int64_t>(64, (tiles + std::min<int64_t>(want, 64) - 1) / std::min<int64_t>(want, 64));
+  split = std::min(split, std::max<int64_t>(1024, (tiles + 63) / 64));
+  const int32_t nsplit = (int32_t)((tiles + split - 1) / split);
+  const size_t need = sizeof(double2) * (size_t)nsplit * M * M;
+  if (part->bytes < need) TBK_TRY(part->alloc(need));
+  mu_gemm_cc_kernel<<<dim3(out.x, out.y, nsplit), 256, 0, st>>>(L, Rb, M, tiles, split, part->as<double2>());
+  TBK_CHECK_LAUNCH();
+  mu_split_reduce_kernel<<<(unsigned)(((int64_t)M * M + 255) / 256), 256, 0, st>>>(part->as<double2>(), M, nsplit, acc);
+  TBK_CHECK_LAUNCH();
+  return TBK_OK;
 }
 
 // FP64 reference GEMM on complex128 K-tiled blocks: C[m][n] += sum_k
@@ -878,10 +940,10 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     }
     return TBK_OK;
   };
-  // split-K: at least 16,384 K values per CTA, at most 64 partial M x M blocks
+  // split-K of the FP64 form: at least 16,384 K values per CTA, at most 64 partial M x M blocks
   const int64_t ksplit = std::max<int64_t>(16384, (blk + 63) / 64);
   const int32_t nsplit = (int32_t)((blk + ksplit - 1) / ksplit);
-  if (!use_tc) TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
+  if (f64b) TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
   cudaEvent_t ev[3];
   for (auto& e : ev) TBK_CUDA(cudaEventCreate(&e));
   KuboTiming tm;
@@ -911,19 +973,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       TBK_TRY(mu_gemm_tc(L, R_, M, blk, macc.as<double>(), &usable, st));
       if (!usable) {                                     // values past FP16's range: complex64 stores from here on
         use_tc = false;
-        TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
         TBK_TRY(zero_tail());
         TBK_TRY(blocks());
       }
     }
-    if (!use_tc && !f64b) {
-      dim3 g((M + kGT - 1) / kGT, (M + kGT - 1) / kGT, nsplit);
-      mu_gemm_cc_kernel<<<g, 256, 0, st>>>(Ls.as<float2>(), Rs.as<float2>(), M, blk, blk, ksplit, part.as<double2>());
-      TBK_CHECK_LAUNCH();
-      mu_split_reduce_kernel<<<(unsigned)(((int64_t)M * M + 255) / 256), 256, 0, st>>>(part.as<double2>(), M, nsplit,
-                                                                                       macc.as<double2>());
-      TBK_CHECK_LAUNCH();
-    }
+    if (!use_tc && !f64b)
+      TBK_TRY(mu_gemm_cc(Ls.as<float2>(), Rs.as<float2>(), M, blk, &part, macc.as<double2>(), st));
     TBK_CUDA(cudaEventRecord(ev[2], st));
     TBK_CUDA(cudaEventSynchronize(ev[2]));
     trace.mark("gemm");
@@ -1017,17 +1072,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
       TBK_TRY(upload(false));
     }
   }
-  if (!formed) {
-    const int64_t ksplit = 16384;
-    const int32_t nsplit = (int32_t)((K + ksplit - 1) / ksplit);
-    TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
-    dim3 g((M + kGT - 1) / kGT, (M + kGT - 1) / kGT, nsplit);
-    mu_gemm_cc_kernel<<<g, 256, 0, st>>>(Ld.as<float2>(), Rd.as<float2>(), M, K, 0, ksplit, part.as<double2>());
-    TBK_CHECK_LAUNCH();
-    mu_split_reduce_kernel<<<(unsigned)(((int64_t)M * M + 255) / 256), 256, 0, st>>>(part.as<double2>(), M, nsplit,
-                                                                                     acc.as<double2>());
-    TBK_CHECK_LAUNCH();
-  }
+  if (!formed) TBK_TRY(mu_gemm_cc(Ld.as<float2>(), Rd.as<float2>(), M, K, &part, acc.as<double2>(), st));
   TBK_CUDA(cudaEventRecord(ev[1], st));
   TBK_CUDA(cudaMemcpyAsync(mu_out, acc.p, sizeof(double2) * (size_t)M * M, cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
