@@ -123,13 +123,15 @@ __global__ void diff_i32_kernel(int64_t n, const int32_t* __restrict__ a, const 
     if (a[i] != b[i]) *flag = 1;
 }
 
-int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st) {
+int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st, bool* b_real) {
   *same = false;
   TBK_TRY(ensure_ell(A, st));
   TBK_TRY(ensure_ell(B, st));
   const EllDev& a = A->ell;
   const EllDev& b = B->ell;
-  if (a.n_rows != b.n_rows || a.n_slices != b.n_slices || a.n_entries != b.n_entries || a.cplx != b.cplx)
+  if (b_real) *b_real = a.cplx && !b.cplx;
+  if (a.n_rows != b.n_rows || a.n_slices != b.n_slices || a.n_entries != b.n_entries ||
+      (a.cplx != b.cplx && !(b_real && *b_real)))
     return TBK_OK;
   DevBuf flag;
   TBK_TRY(flag.alloc(sizeof(int)));

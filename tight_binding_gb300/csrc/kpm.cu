@@ -229,6 +229,8 @@ bool has_classes(const EllDev& E, int prec) {
   return E.cls_state == 1 || (prec == TBK_PREC_MIXED && E.cls32_state == 1);
 }
 
+bool has_row_classes(tbk_sparse_s* A, int prec) { return has_classes(A->ell, prec); }
+
 static ClassTab class_tab32(const ClassSet32& c) {
   ClassTab t;
   t.cls = c.cls.as<uint8_t>();
@@ -337,6 +339,7 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
       a.ks.vval[0] = ell_vals(vop->ell, prec);
       a.ks.vdiag[0] = ell_diag(vop->ell, prec);
       a.ks.usev[0] = 1;
+      a.ks.vreal[0] = A->ell.cplx && !vop->ell.cplx;
       a.kst = 2;
       if (pair) {
         a.ct = class_tab32(*pair);

@@ -70,6 +70,15 @@ __device__ __noinline__ void step_sums_call(float m0, float m1, double* __restri
   step_sums<float, kTwo>(m0, m1, part);
 }
 
+// operator value o, real (vreal) or of H's type
+template <typename F, bool CPLX_H>
+__device__ __forceinline__ HVal<F, CPLX_H> op_value(const F* __restrict__ p, int64_t o, bool vreal) {
+  if constexpr (CPLX_H) {
+    if (vreal) return HVal<F, true>{HVal<F, false>::load(p, o).v, F(0)};
+  }
+  return HVal<F, CPLX_H>::load(p, o);
+}
+
 // the lane's values k .. into block m of a complex64 or an FP16-pair K-tiled store
 template <typename F, int VPL>
 __device__ __forceinline__ void store_c64(float2* __restrict__ dst, int32_t M, int32_t m, int64_t k0,
@@ -280,7 +289,9 @@ kpm_step_kernel(
     const int grp = (KST == 2 && ks.halves == 2 && sub * VPL >= RW / 2) ? 1 : 0;
     const F* vval = nullptr;
     const F* vdiag = nullptr;
+    bool vreal = false;
     if constexpr (KST == 2) {
+      vreal = CPLX_H && (grp ? ks.vreal[1] : ks.vreal[0]) != 0;
       const void* vv = grp ? ks.vval[1] : ks.vval[0];      // selects, not an indexed parameter array
       const void* vd = grp ? ks.vdiag[1] : ks.vdiag[0];
       vval = vv ? static_cast<const F*>(vv) : eval;
@@ -338,7 +349,7 @@ kpm_step_kernel(
       }
     } else if (gather) {
       ell_entry<F, VPL, CPLX_H, FOLD>(diag, r, xs, acc);
-      if constexpr (KST == 2) HVal<F, CPLX_H>::load(vdiag, r).template fma<VPL>(xs, vacc);
+      if constexpr (KST == 2) op_value<F, CPLX_H>(vdiag, r, vreal).template fma<VPL>(xs, vacc);
       const int32_t s = r >> 5, l = r & 31;
       const int32_t off = soff[s];
       const int32_t w = (soff[s + 1] - off) >> 5;
@@ -393,7 +404,7 @@ kpm_step_kernel(
         if constexpr (KST == 2) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const HVal<F, CPLX_H> hv = k + u < w ? HVal<F, CPLX_H>::load(vval, off + l + (int64_t)(k + u) * 32)
+            const HVal<F, CPLX_H> hv = k + u < w ? op_value<F, CPLX_H>(vval, off + l + (int64_t)(k + u) * 32, vreal)
                                                  : HVal<F, CPLX_H>::zero();
             hv.template fma<VPL>(xv[u], vacc);
           }

@@ -602,20 +602,49 @@ int with_block(int prec, const void* p, Fn&& f) {
 // Scratch of split_scale_kernel, the two sides' scales and the flag of values that do
 // not fit.
 struct SplitScales {
-  DevBuf part, words;          // words: scale of the left, of the right side; bad; count
+  DevBuf part, words;          // words: scale of the left, of the right side; bad; count of each side
   int alloc(cudaStream_t st) {
-    TBK_TRY(part.alloc(sizeof(double) * 4 * sm_count()));
-    TBK_TRY(words.alloc(4 * sizeof(int)));
+    TBK_TRY(part.alloc(sizeof(double) * 8 * sm_count()));
+    TBK_TRY(words.alloc(5 * sizeof(int)));
     TBK_CUDA(cudaMemsetAsync(words.p, 0, words.bytes, st));
     return TBK_OK;
   }
   float* scale(int h) const { return words.as<float>() + h; }
   int* bad() const { return words.as<int>() + 2; }
-  unsigned int* count() const { return words.as<unsigned int>() + 3; }
+  // h: the side, each with scratch of its own
   template <typename CT>
-  void find(const CT* src, int64_t n, float* out, cudaStream_t st) const {
+  void find(const CT* src, int64_t n, float* out, int h, cudaStream_t st) const {
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + kStatThreads - 1) / kStatThreads, 2 * sm_count()));
-    split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, part.as<double>(), count(), out, bad());
+    split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, part.as<double>() + 4 * h * sm_count(),
+                                                       words.as<unsigned int>() + 3 + h, out, bad());
+  }
+};
+
+// Blocks of up to this size leave much of the GPU idle in one recursion: both sides of
+// square 256x256 with a flux, M = 512, 16 vectors (8 MB a block), took 9.8 ms one after the
+// other, the operator's products in a pass of their own, and take 7.9 ms on two streams;
+// honeycomb 91x77, M = 200, 3 vectors, 1.25 and 0.75 ms.
+constexpr double kDualBlock = 16e6;
+
+// A stream beside the caller's, of its priority, for the length of a call
+struct SecondStream {
+  cudaStream_t st = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int create(cudaStream_t beside) {
+    int prio = 0;
+    TBK_CUDA(cudaStreamGetPriority(beside, &prio));
+    TBK_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, prio));
+    TBK_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    TBK_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    return TBK_OK;
+  }
+  ~SecondStream() {
+    if (st) {
+      cudaStreamSynchronize(st);
+      cudaStreamDestroy(st);
+    }
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
   }
 };
 
@@ -714,10 +743,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     TBK_TRY(same_ell_structure(Ht, o, &same, st));
     both = same;
   }
+  // small blocks: the two sides' recursions run side by side on two streams
+  const bool dual = !both && !f64b && (double)csz * blk <= kDualBlock;
   {
     const AsyncAllocCtx* outer = tl_async_alloc;
     if (kctx.pool) tl_async_alloc = &kctx;
-    const int a = work.alloc(csz * blk * (both ? 12 : 6));
+    const int a = work.alloc(csz * blk * (both ? 12 : dual ? 11 : 6));
     tl_async_alloc = outer;
     TBK_TRY(a);
   }
@@ -773,33 +804,57 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     if (cols && (A->ell.cls_state == 1 || (prec == TBK_PREC_MIXED && A->ell.cls32_state == 1))) return (double)A->rows * (1.0 + hv);
     return (double)A->ell.n_entries * ((cols ? 4.0 : 0.0) + hv) + (double)A->rows * hv;
   };
+  // Complex64 recursions take the operator's products inside the step wherever H~ and the
+  // operator have joint row classes: one pass over the vectors' neighbours per block
+  // instead of two (FCC 128^3, 4 vectors: 77.9 us against 56.5 + 83.7); and where H~ runs in
+  // the ELL form anyway, whose columns they then load once (a flux).
+  struct Fused {
+    bool on = false;
+    ClassSet32 pair;
+    int grid = 1, tiles = 1;
+  } fused[2];
+  for (int h = 0; h < 2 && !both && !f64b; ++h) {
+    tbk_sparse_s* Aout = h ? AR : AL;
+    Fused& F = fused[h];
+    F.grid = grid;
+    F.tiles = n_tiles;
+    const bool mixed = prec == TBK_PREC_MIXED;
+    if (!Aout || !((flags & TBK_MU_FUSED_OPS) || mixed)) continue;
+    bool v_real = false;
+    TBK_TRY(same_ell_structure(Ht, Aout, &F.on, st, mixed ? &v_real : nullptr));
+    if (F.on && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
+    if (F.on && mixed && !v_real) TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
+    if (F.pair.n_cls > 0) TBK_TRY(pair_config(Ht, Rc, F.pair, &F.grid, &F.tiles));
+    else F.on = F.on && ((flags & TBK_MU_FUSED_OPS) || !has_row_classes(Ht, prec));
+  }
+  cudaStream_t q = st;                                   // the stream the side being issued runs on
   auto apply = [&](tbk_sparse_s* A, const void* x, void* y) -> int {   // y = A x
     rec_bytes += 2 * vecb + ell_bytes(A, true);
     int g, t;
     TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
-    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, t, st, nullptr, true, nullptr, false);
+    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, t, q, nullptr, true, nullptr, false);
   };
   const unsigned gblk = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
   auto round_to = [&](const void* src, const KStore& ks, int32_t m) -> int {
     rec_bytes += vecb + stb;
     return with_block(prec, src, [&](auto p) {
       if (ks.split)
-        split_block_kernel<<<gblk, 256, 0, st>>>(p, reinterpret_cast<__half*>(ks.store[0]), m, M, blk, ks.scale[0], ks.bad);
+        split_block_kernel<<<gblk, 256, 0, q>>>(p, reinterpret_cast<__half*>(ks.store[0]), m, M, blk, ks.scale[0], ks.bad);
       else
-        round_block_kernel<<<gblk, 256, 0, st>>>(p, ks.store[0], m, M, blk);
+        round_block_kernel<<<gblk, 256, 0, q>>>(p, ks.store[0], m, M, blk);
     });
   };
   auto find_scale = [&](const void* src, int h) -> int {
-    return with_block(prec, src, [&](auto p) { sc.find(p, blk, sc.scale(h), st); });
+    return with_block(prec, src, [&](auto p) { sc.find(p, blk, sc.scale(h), h, q); });
   };
   // FP64 reference form: block m of the complex128 store from a work block
   auto store64 = [&](const void* src, void* store, int32_t m) -> int {
     rec_bytes += vecb + 2 * stb;
     const unsigned g = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
     double2* d = static_cast<double2*>(store);
-    if (prec == TBK_PREC_FP64) store_block64_kernel<double2><<<g, 256, 0, st>>>(static_cast<const double2*>(src), d, m, M, blk);
-    else if (prec == TBK_PREC_DD) store_block64_kernel<dd2><<<g, 256, 0, st>>>(static_cast<const dd2*>(src), d, m, M, blk);
-    else store_block64_kernel<float2><<<g, 256, 0, st>>>(static_cast<const float2*>(src), d, m, M, blk);
+    if (prec == TBK_PREC_FP64) store_block64_kernel<double2><<<g, 256, 0, q>>>(static_cast<const double2*>(src), d, m, M, blk);
+    else if (prec == TBK_PREC_DD) store_block64_kernel<dd2><<<g, 256, 0, q>>>(static_cast<const dd2*>(src), d, m, M, blk);
+    else store_block64_kernel<float2><<<g, 256, 0, q>>>(static_cast<const float2*>(src), d, m, M, blk);
     TBK_CHECK_LAUNCH();
     return TBK_OK;
   };
@@ -809,7 +864,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     int g, t;
     TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
     ks.km[0] = m;
-    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, st, &ks, false);
+    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, q, &ks, false);
   };
   // one side: store[m] = Aout T_m(H~) (Bin v0), m < M; each step writes its
   // complex64 block (Aout absent) or feeds the product that does
@@ -817,68 +872,57 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // (a commutator [X, H~] does), step m also forms Aout T_{m-1} from the x it
   // gathers and writes block m-1: one pass over the matrix and the vectors per
   // block instead of two.  The stored values are the same bits either way.
-  auto side = [&](tbk_sparse_s* Aout, tbk_sparse_s* Bin, float2* store, int h) -> int {
-    void* r[3] = {wblk(0), wblk(1), wblk(2)};
-    void* tmpA = wblk(3);
+  // steps m_begin <= m < m_end of side h on stream q; the side ends with step M
+  auto side = [&](int h, int32_t m_begin, int32_t m_end) -> int {
+    tbk_sparse_s* Aout = h ? AR : AL;
+    tbk_sparse_s* Bin = h ? BR : BL;
+    const int w0 = dual && h ? 6 : 0;                     // this side's work blocks
+    void* r[3] = {wblk(w0), wblk(w0 + 1), wblk(w0 + 2)};
+    void* tmpA = wblk(w0 + 3);
+    const Fused& F = fused[h];
+    const bool fuse = F.on;
     KStore ks;
-    ks.store[0] = store;
+    ks.store[0] = (h ? Rs : Ls).as<float2>();
     ks.kM = M;
     ks.split = use_tc;
     ks.scale[0] = sc.scale(h);
     ks.bad = sc.bad();
-    if (f64b) {                                           // recursion, operator, complex128 store
-      if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
-      else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
-      for (int32_t m = 0; m < M; ++m) {
-        void* y = r[m % 3];
+    for (int32_t m = m_begin; m < m_end; ++m) {
+      if (m == 0) {
+        if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
+        else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, q));
+      }
+      void* y = r[m % 3];
+      const void* x = m >= 1 ? r[(m - 1) % 3] : nullptr;
+      const void* pv = m >= 2 ? r[(m - 2) % 3] : nullptr;
+      if (f64b) {                                         // recursion, operator, complex128 store
+        if (m == M) break;
         if (m >= 1) {
           rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true);
-          TBK_TRY(step_any(Ht, Rc, prec, r[(m - 1) % 3], y, m >= 2 ? r[(m - 2) % 3] : nullptr, m == 1,
-                           partd.as<double>(), grid, n_tiles, st, nullptr, true, nullptr, false));
+          TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, q, nullptr, true, nullptr,
+                           false));
         }
-        if (Aout) {
-          TBK_TRY(apply(Aout, y, tmpA));
-          TBK_TRY(store64(tmpA, store, m));
-        } else {
-          TBK_TRY(store64(y, store, m));
-        }
+        if (Aout) TBK_TRY(apply(Aout, y, tmpA));
+        TBK_TRY(store64(Aout ? tmpA : y, ks.store[0], m));
+      } else if (m == 0) {
+        // block 0; its values set the scale of an FP16-pair store
+        if (use_tc && Aout) TBK_TRY(apply(Aout, y, tmpA));
+        if (use_tc) TBK_TRY(find_scale(Aout ? tmpA : y, h));
+        if (!Aout) TBK_TRY(round_to(y, ks, 0));
+        else if (!fuse && use_tc) TBK_TRY(round_to(tmpA, ks, 0));
+        else if (!fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, 0));
+      } else if (m < M) {
+        rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
+                     (fuse ? ell_bytes(Aout, false) : 0.0);
+        ks.km[0] = fuse ? m - 1 : m;
+        TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), F.grid, F.tiles, q,
+                         fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false,
+                         F.pair.n_cls > 0 ? &F.pair : nullptr));
+        if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
+      } else if (fuse) {
+        TBK_TRY(apply_to_store(Aout, x, tmpA, ks, M - 1));
       }
-      return TBK_OK;
     }
-    // complex64 recursions take the operator's products inside the step wherever H~ and
-    // the operator have joint row classes: one pass over the vectors' neighbours per block
-    // instead of two (FCC 128^3, 4 vectors: 77.9 us against 56.5 + 83.7)
-    bool fuse = false;
-    ClassSet32 pair;
-    int pgrid = grid, ptiles = n_tiles;
-    if (Aout && ((flags & TBK_MU_FUSED_OPS) || prec == TBK_PREC_MIXED)) {
-      TBK_TRY(same_ell_structure(Ht, Aout, &fuse, st));
-      if (fuse && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
-      if (fuse && prec == TBK_PREC_MIXED) TBK_TRY(pair_classes32(Ht, Aout, &pair, st));
-      if (pair.n_cls > 0) TBK_TRY(pair_config(Ht, Rc, pair, &pgrid, &ptiles));
-      else fuse = fuse && (flags & TBK_MU_FUSED_OPS);
-    }
-    if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
-    else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
-    // block 0; its values set the scale of an FP16-pair store
-    if (use_tc && Aout) TBK_TRY(apply(Aout, r[0], tmpA));
-    if (use_tc) TBK_TRY(find_scale(Aout ? tmpA : r[0], h));
-    if (!Aout) TBK_TRY(round_to(r[0], ks, 0));
-    else if (!fuse && use_tc) TBK_TRY(round_to(tmpA, ks, 0));
-    else if (!fuse) TBK_TRY(apply_to_store(Aout, r[0], tmpA, ks, 0));
-    for (int32_t m = 1; m < M; ++m) {
-      void* y = r[m % 3];
-      const void* x = r[(m - 1) % 3];
-      const void* pv = m >= 2 ? r[(m - 2) % 3] : nullptr;
-      rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
-                   (fuse ? ell_bytes(Aout, false) : 0.0);
-      ks.km[0] = fuse ? m - 1 : m;
-      TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), pgrid, ptiles, st,
-                       fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false,
-                       pair.n_cls > 0 ? &pair : nullptr));
-      if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
-    }
-    if (fuse) TBK_TRY(apply_to_store(Aout, r[(M - 1) % 3], tmpA, ks, M - 1));
     return TBK_OK;
   };
   // both sides at once: columns [0, Rc) carry the left side (BL v0), [Rc, 2 Rc)
@@ -944,6 +988,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   const int64_t ksplit = std::max<int64_t>(16384, (blk + 63) / 64);
   const int32_t nsplit = (int32_t)((blk + ksplit - 1) / ksplit);
   if (f64b) TBK_TRY(part.alloc(sizeof(double2) * (size_t)nsplit * M * M));
+  SecondStream second;
+  if (dual) TBK_TRY(second.create(st));
   cudaEvent_t ev[3];
   for (auto& e : ev) TBK_CUDA(cudaEventCreate(&e));
   KuboTiming tm;
@@ -953,8 +999,22 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     else TBK_TRY(random_block_any(prec, n, R, r0, Rc, seed, v0, st));
     auto blocks = [&]() -> int {
       if (both) return both_sides();
-      TBK_TRY(side(AL, BL, Ls.as<float2>(), 0));
-      return side(AR, BR, Rs.as<float2>(), 1);
+      if (!dual) {
+        TBK_TRY(side(0, 0, M + 1));
+        return side(1, 0, M + 1);
+      }
+      TBK_CUDA(cudaEventRecord(second.fork, st));
+      TBK_CUDA(cudaStreamWaitEvent(second.st, second.fork, 0));
+      for (int32_t m = 0; m <= M; ++m) {                 // issued in turn, so that neither side waits for the host
+        q = second.st;
+        const int s1 = side(1, m, m + 1);
+        q = st;
+        TBK_TRY(s1);
+        TBK_TRY(side(0, m, m + 1));
+      }
+      TBK_CUDA(cudaEventRecord(second.join, second.st));
+      TBK_CUDA(cudaStreamWaitEvent(st, second.join, 0));
+      return TBK_OK;
     };
     TBK_TRY(blocks());
     TBK_CUDA(cudaEventRecord(ev[1], st));
@@ -1047,7 +1107,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
         TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K, cudaMemcpyHostToDevice, st));
         if (split) {
           float* s = scales.as<float>() + side * M + m;
-          sc.find(stage.as<const double2>(), K, s, st);
+          sc.find(stage.as<const double2>(), K, s, 0, st);
           split_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<__half>(), m, M, K, s, sc.bad());
         } else {
           round_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<float2>(), m, M, K);

@@ -207,6 +207,7 @@ struct KStore {
   const void* vdiag[2] = {nullptr, nullptr};
   int32_t km[2] = {-1, -1};
   int32_t usev[2] = {0, 0};
+  int32_t vreal[2] = {0, 0};       // V's values are real although H's are complex
   int32_t kM = 0;
   int32_t halves = 1;
   // split: the stores are FP16 pairs (split_store.cuh), scaled by *scale[h]
@@ -234,6 +235,8 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
 // grid and tiles of a step with an operator product in the joint class form (complex64;
 // pair: pair_classes32 of A and the operator)
 int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles);
+// whether A's steps in a precision run in the class form (after step_config)
+bool has_row_classes(tbk_sparse_s* A, int prec);
 // ELL value / diagonal arrays of a precision (FP32, FP64 or double-float pairs)
 const void* ell_vals(const EllDev& E, int prec);
 const void* ell_diag(const EllDev& E, int prec);
@@ -242,7 +245,8 @@ const void* ell_diag(const EllDev& E, int prec);
 int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
             int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode = 2);
 // true when B's sliced ELL has A's slices, widths and columns (values may differ)
-int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st);
+// (b_real: B may hold real values where A's are complex; then set)
+int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st, bool* b_real = nullptr);
 int load_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, const double2* src, void* dst,
                    cudaStream_t st);
 int random_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t seed, void* dst,
