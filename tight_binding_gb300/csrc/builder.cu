@@ -512,19 +512,15 @@ __global__ void row_sort_kernel(int32_t n, const int32_t* __restrict__ rp, int32
   }
 }
 
+// one row per lane, one slice per warp
 __global__ void slice_width_kernel(int32_t n, int32_t n_slices, const int32_t* __restrict__ rp,
                                    const int32_t* __restrict__ rc, int32_t* __restrict__ width32) {
-  int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_slices) return;
-  int32_t w = 0;
-  for (int l = 0; l < 32; ++l) {
-    int32_t i = s * 32 + l;
-    if (i >= n) break;
-    int32_t cnt = 0;
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  int32_t cnt = 0;
+  if (i < n)
     for (int32_t p = rp[i]; p < rp[i + 1]; ++p) cnt += rc[p] != i ? 1 : 0;
-    w = max(w, cnt);
-  }
-  width32[s] = w * 32;
+  cnt = __reduce_max_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0 && (i >> 5) < n_slices) width32[i >> 5] = cnt * 32;
 }
 
 __global__ void ell_fill_kernel(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ rc,
@@ -633,7 +629,7 @@ int ensure_ell(tbk_sparse_s* A, cudaStream_t st) {
   TBK_CHECK_LAUNCH();
   TBK_TRY(w32.alloc(sizeof(int32_t) * (E.n_slices + 1)));
   TBK_CUDA(cudaMemsetAsync(w32.p, 0, sizeof(int32_t) * (E.n_slices + 1), st));
-  slice_width_kernel<<<(E.n_slices + T - 1) / T, T, 0, st>>>(n, E.n_slices, rp.as<int32_t>(), rc.as<int32_t>(),
+  slice_width_kernel<<<(n + T - 1) / T, T, 0, st>>>(n, E.n_slices, rp.as<int32_t>(), rc.as<int32_t>(),
                                                                w32.as<int32_t>());
   TBK_CHECK_LAUNCH();
   TBK_TRY(E.slice_off.alloc(sizeof(int32_t) * (E.n_slices + 1)));

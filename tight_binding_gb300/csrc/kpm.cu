@@ -70,24 +70,34 @@ __global__ void load_block_kernel(int32_t n, int32_t R, int32_t r0, int32_t rc, 
   }
 }
 
-// Device random-phase kets exp(2 pi i u)/sqrt(N), u = u01(seed, r, i), site-major.
-template <typename F>
-__global__ void random_block_kernel(int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t seed,
+// Device random-phase kets exp(2 pi i u)/sqrt(N), u = u01(seed, r, i), site-major.  Bound
+// by the FP64 pipe (the sincos): 1/sqrt(N) comes from the host, and indices of blocks
+// below 2^32 values divide in 32 bits.  152,306 x 4: 51 -> 36 us.
+template <typename F, typename I>
+__global__ void random_block_kernel(int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t seed, double inv,
                                     typename C2<F>::T* __restrict__ dst) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (int64_t)n * Rp) return;
-  int32_t i = (int32_t)(g / Rp), c = (int32_t)(g % Rp);
+  const int32_t i = (int32_t)((I)g / (I)Rp), c = (int32_t)((I)g % (I)Rp);
   typename C2<F>::T o;
   if (r0 + c < R) {
     double th = 6.283185307179586476925286766559 * u01(seed, (uint64_t)(r0 + c), (uint64_t)i);
     double s, cs;
     sincos(th, &s, &cs);
-    double inv = 1.0 / sqrt((double)n);
     o.x = (F)(cs * inv); o.y = (F)(s * inv);
   } else {
     o.x = 0; o.y = 0;
   }
   dst[g] = o;
+}
+template <typename F>
+static void random_block(int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t seed, void* dst, cudaStream_t st) {
+  const int64_t tot = (int64_t)n * Rp;
+  const unsigned g = (unsigned)((tot + 255) / 256);
+  const double inv = 1.0 / std::sqrt((double)n);
+  auto d = static_cast<typename C2<F>::T*>(dst);
+  if (tot < (1ll << 32)) random_block_kernel<F, uint32_t><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, inv, d);
+  else random_block_kernel<F, int64_t><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, inv, d);
 }
 
 // Fixed-order sum of the per-CTA partials of every (chunk, step, slot).
@@ -442,11 +452,9 @@ int load_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, const
 
 int random_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t seed, void* dst,
                      cudaStream_t st) {
-  const int64_t tot = (int64_t)n * Rp;
-  const unsigned g = (unsigned)((tot + 255) / 256);
-  if (prec == TBK_PREC_FP64) random_block_kernel<double><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, static_cast<double2*>(dst));
-  else if (prec == TBK_PREC_DD) random_block_kernel<dd><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, static_cast<dd2*>(dst));
-  else random_block_kernel<float><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, static_cast<float2*>(dst));
+  if (prec == TBK_PREC_FP64) random_block<double>(n, R, r0, Rp, seed, dst, st);
+  else if (prec == TBK_PREC_DD) random_block<dd>(n, R, r0, Rp, seed, dst, st);
+  else random_block<float>(n, R, r0, Rp, seed, dst, st);
   TBK_CHECK_LAUNCH();
   return TBK_OK;
 }
