@@ -64,8 +64,10 @@ enum {
                                      traffic, but the gathers are latency-bound on
                                      GB300 and it measures slower, so opt-in)     */
   TBK_FLAG_NO_GRAPH = 1 << 9,     /* never replay the recursion as a CUDA graph
-                                     (small single-chunk plans capture their
-                                     launch sequence on the second identical run) */
+                                     (single-chunk plans too large for the cooperative
+                                     recursion and of at most 64 MiB a block capture
+                                     their launch sequence on the second identical
+                                     run) */
   TBK_FLAG_PERSISTENT = 1 << 10,  /* small single-chunk plans: the whole recursion
                                      in one launch.  Complex64 vectors of an H~
                                      with row classes that fit one SM: one CTA
@@ -327,8 +329,9 @@ int tbk_kpm_run(tbk_kpm plan, int32_t n_mom, const double* bras, const double* k
 int tbk_kpm_run_random(tbk_kpm plan, int32_t n_mom, uint64_t seed, double* mu_out,
                        void* stream);
 /* Device time of the recursion kernels of the last run (CUDA events on the
- * launching stream), number of recursion launches and algorithmic DRAM bytes
- * per launch. */
+ * launching stream), number of recursion launches (of steps where a small
+ * recursion runs in one cooperative launch) and algorithmic DRAM bytes per
+ * launch. */
 int tbk_kpm_last_timing(tbk_kpm plan, double* ms_recursion, int32_t* launches,
                         double* bytes_per_launch);
 void tbk_kpm_destroy(tbk_kpm plan);

@@ -41,6 +41,7 @@ namespace tbk {
 #include "kpm_tma.cuh"
 #include "kpm_fused.cuh"
 #include "kpm_small.cuh"
+#include "kpm_persist.cuh"
 namespace tbk {
 
 // Column-major complex128 (Eigen) -> site-major work block of width Rp.
@@ -502,6 +503,8 @@ struct tbk_kpm_s {
   int small_state = 0;              // one-launch recursion: 0 undecided, 1 used, -1 not applicable
   SmallLayout slay{};
   bool cta = false;                 // the one-launch recursion is one CTA per vector (kpm_cta_kernel)
+  int persist = 0;                  // cooperative recursion (kpm_persist_kernel): 0 undecided, 1 used, -1 not
+  DevBuf meet;
   CtaLayout clay{};
 };
 
@@ -830,6 +833,66 @@ static int launch_small(tbk_kpm_s* P, bool braket, int32_t n_steps, cudaStream_t
   return c ? launch_small_t<float, true>(P, braket, n_steps, st) : launch_small_t<float, false>(P, braket, n_steps, st);
 }
 
+template <typename F>
+static void* persist_kernel_t(bool cplx, bool braket, bool cls) {
+  if (cplx) {
+    if (braket) return cls ? (void*)kpm_persist_kernel<F, true, true, true> : (void*)kpm_persist_kernel<F, true, true, false>;
+    return cls ? (void*)kpm_persist_kernel<F, true, false, true> : (void*)kpm_persist_kernel<F, true, false, false>;
+  }
+  if (braket) return cls ? (void*)kpm_persist_kernel<F, false, true, true> : (void*)kpm_persist_kernel<F, false, true, false>;
+  return cls ? (void*)kpm_persist_kernel<F, false, false, true> : (void*)kpm_persist_kernel<F, false, false, false>;
+}
+static void* persist_kernel(const tbk_kpm_s* P, bool braket) {
+  const bool cplx = P->H->ell.cplx != 0;
+  if (P->prec == TBK_PREC_FP64) return persist_kernel_t<double>(cplx, braket, P->use_cls);
+  if (P->prec == TBK_PREC_DD) return persist_kernel_t<dd>(cplx, braket, P->use_cls);
+  return persist_kernel_t<float>(cplx, braket, P->use_cls);
+}
+
+// Decides once per plan whether the cooperative recursion applies: one chunk of whole
+// lanes, one tile per CTA in the step kernels' own grid (so that the partial sums are
+// the same), all CTAs resident at once in both modes.
+static int plan_persist(tbk_kpm_s* P) {
+  if (P->persist != 0) return TBK_OK;
+  P->persist = -1;
+  const bool lanes = P->prec == TBK_PREC_FP64 || P->Rc % 2 == 0;
+  if (P->n_chunks != 1 || !lanes || P->n_tiles != P->grid ||
+      (P->flags & (TBK_FLAG_STAGED | TBK_FLAG_TWO_STEP | TBK_FLAG_PERSISTENT)))
+    return TBK_OK;
+  const size_t smem = P->use_cls ? class_smem(P->H->ell, P->prec) : 0;
+  for (int b = 0; b < 2; ++b) {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, persist_kernel(P, b == 1), kStepThreads, smem) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return TBK_OK;
+    }
+    if (P->grid > nb * sm_count()) return TBK_OK;
+  }
+  TBK_TRY(P->meet.alloc(sizeof(unsigned int)));
+  P->persist = 1;
+  return TBK_OK;
+}
+
+static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* part, cudaStream_t st) {
+  const EllDev& E = P->H->ell;
+  const ClassTab ct = class_tab(E, P->prec);
+  const size_t smem = P->use_cls ? class_smem(E, P->prec) : 0;
+  TBK_CUDA(cudaMemsetAsync(P->meet.p, 0, sizeof(unsigned int), st));
+  int32_t n = (int32_t)P->n, lpr = P->prec == TBK_PREC_FP64 ? P->Rc : P->Rc / 2;
+  const int32_t* so = E.slice_off.as<int32_t>();
+  const int32_t* co = E.col.as<int32_t>();
+  const void* ev = ell_vals(E, P->prec);
+  const void* dg = ell_diag(E, P->prec);
+  void *va = P->va.p, *vb = P->vb.p, *br = braket ? P->bras.p : nullptr;
+  unsigned int* meet = P->meet.as<unsigned int>();
+  int* err = P->err.as<int>();
+  uint32_t lim = kWaitLimit;
+  void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &meet, &err, &lim};
+  TBK_CUDA(cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st));
+  return TBK_OK;
+}
+
 // Runs all chunks.  kets_loader(r0, dst) fills the chunk's v0 (site-major);
 // bras_loader(r0, dst) fills the chunk's bras block (braket mode only).
 template <typename KL, typename BL>
@@ -841,6 +904,7 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
   const int32_t n_steps = doubling ? (n_mom <= 2 ? 1 : n_mom / 2 + 1) : n_mom - 1;
   const bool tma = P->use_tma && (P->flags & TBK_FLAG_STAGED);
   TBK_TRY(plan_small(P, tma));
+  TBK_TRY(plan_persist(P));
   TBK_TRY(plan_partials(P, n_steps));
   TBK_TRY(plan_mu(P, n_mom));
   if (braket && P->bras.bytes < P->va.bytes) {
@@ -921,6 +985,9 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
     if (small) {
       TBK_TRY(launch_small(P, braket, n_steps, st));
       launches += 1;
+    } else if (P->persist == 1 && (int64_t)n_steps * P->grid < (int64_t)INT32_MAX) {
+      TBK_TRY(launch_persist(P, braket, n_steps, P->part.as<double>(), st));
+      launches += n_steps;
     } else if (graphable) {
       tbk_kpm_s::GraphKey key;
       key.n_steps = n_steps;
