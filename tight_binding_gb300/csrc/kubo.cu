@@ -405,34 +405,37 @@ __global__ void __launch_bounds__(kDiagThreads) diag_sums_kernel(const double2* 
   if constexpr (BASTIN) p[2 * L + t] = d;
 }
 
-// The row chunks summed in order, then the series coefficients A, (BASTIN) B and I.
+// The row chunks summed, then the series coefficients A, (BASTIN) B and I: 32 q per CTA,
+// its 8 warps taking every 8th chunk (one thread per q waits for 5 loads a chunk, 20 us at
+// 32 chunks).
+constexpr int kCoefWarps = 8;
 template <bool BASTIN>
-__global__ void __launch_bounds__(kDiagThreads) series_coef_kernel(const double2* __restrict__ part, int32_t M,
-                                                                   int32_t chunks, double2* __restrict__ coef) {
-  const int32_t L = 2 * M - 1;
-  const int32_t q = blockIdx.x * kDiagThreads + threadIdx.x;
-  if (q >= L) return;
-  double2 u = make_double2(0.0, 0.0), d = u, vp = u, vm = u;
-#pragma unroll 4
-  for (int32_t c = 0; c < chunks; ++c) {
-    const double2* p = part + (int64_t)c * (BASTIN ? 3 : 2) * L;
-    const double2 a = p[q];
-    u.x += a.x;
-    u.y += a.y;
-    if (q < M) {
-      const double2 b = p[L + (M - 1) + q], e = p[L + (M - 1) - q];
-      vp.x += b.x;
-      vp.y += b.y;
-      vm.x += e.x;
-      vm.y += e.y;
+__global__ void __launch_bounds__(32 * kCoefWarps) series_coef_kernel(const double2* __restrict__ part, int32_t M,
+                                                                      int32_t chunks, double2* __restrict__ coef) {
+  const int32_t L = 2 * M - 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t q = blockIdx.x * 32 + lane;
+  double2 v[4] = {};                                       // U, D, V_q, V_-q
+  auto add = [](double2& s, double2 x) { s.x += x.x; s.y += x.y; };
+  if (q < L)
+    for (int32_t c = warp; c < chunks; c += kCoefWarps) {
+      const double2* p = part + (int64_t)c * (BASTIN ? 3 : 2) * L;
+      add(v[0], p[q]);
+      if constexpr (BASTIN) add(v[1], p[2 * L + q]);
+      if (q < M) {
+        add(v[2], p[L + (M - 1) + q]);
+        add(v[3], p[L + (M - 1) - q]);
+      }
     }
-    if constexpr (BASTIN) {
-      const double2 g = p[2 * L + q];
-      d.x += g.x;
-      d.y += g.y;
-    }
-  }
-  if (q == 0) vm = make_double2(0.0, 0.0);                 // the main diagonal counts once
+  __shared__ double2 sh[kCoefWarps][4][32];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) sh[warp][k][lane] = v[k];
+  __syncthreads();
+  if (warp != 0 || q >= L) return;
+  for (int w = 1; w < kCoefWarps; ++w)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) add(v[k], sh[w][k][lane]);
+  const double2 u = v[0], d = v[1], vp = v[2];
+  const double2 vm = q == 0 ? make_double2(0.0, 0.0) : v[3];        // the main diagonal counts once
   const double2 i = q == 0 ? vm : make_double2(vp.x - vm.x, vp.y - vm.y);
   coef[q] = make_double2(u.x + vp.x + vm.x, u.y + vp.y + vm.y);
   if constexpr (BASTIN) {
@@ -513,7 +516,7 @@ int moment_series(int32_t M, const double* mu, int32_t n_eps, const double* eps,
   const int32_t qb = (L + kDiagThreads - 1) / kDiagThreads;
   diag_sums_kernel<BASTIN><<<dim3(qb, chunks), kDiagThreads, 0, st>>>(dm.as<double2>(), M, part.as<double2>());
   TBK_CHECK_LAUNCH();
-  series_coef_kernel<BASTIN><<<qb, kDiagThreads, 0, st>>>(part.as<double2>(), M, chunks, coef.as<double2>());
+  series_coef_kernel<BASTIN><<<(L + 31) / 32, 32 * kCoefWarps, 0, st>>>(part.as<double2>(), M, chunks, coef.as<double2>());
   TBK_CHECK_LAUNCH();
   constexpr int kPer = kSeriesThreads / 32;
   series_eval_kernel<BASTIN><<<(n_eps + kPer - 1) / kPer, kSeriesThreads, 0, st>>>(coef.as<double2>(), M, n_eps,
