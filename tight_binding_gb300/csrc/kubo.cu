@@ -651,22 +651,41 @@ struct SecondStream {
   }
 };
 
-// Vectors per chunk: the widest whose two stored sides (per_vector bytes each vector)
-// fit the budget; 1 when none does.  The same in every recursion precision (the GEMM
-// then sums in the same order).  both: a power of two (the widths of the one recursion
-// that carries both sides).
-int pick_chunk(int R, bool both, double per_vector, double budget) {
+// Vectors per chunk of the block recursions (n_pad rows, M blocks a side, sel bytes a stored
+// value; both stored sides within the budget; 1 when no width fits).  A chunk costs the two
+// sides' steps, each a launch (4.5 us), the matrix (5 bytes a row) and 32 bytes a row and
+// vector, twice as fast where the three vectors stay in L2 beside the stores that pass
+// through it, then the GEMM's products; stores that the pool does not keep cost their
+// mapping every call (137 GB: 57 ms to free, 5 to allocate).  So large problems take narrow
+// chunks: FCC 128^3, M = 1024, R = 8: 648 ms at width 4, 625 at 2, 721 at 1 (complex64 lanes
+// carry two vectors: 1 is not taken while 2 fits); FCC 64^3: 96.7 at 8, 79.1 at 4, 76.1 at
+// 2; honeycomb 1024^2, M = 512: 243 at 8, 216 at 4 and 2; square 512^2 with a flux, R = 12:
+// 48.3 at 6, 42.2 at 4.  The same in every recursion precision (the GEMM then sums in the
+// same order).  both: a power of two (the widths of the one recursion that carries both
+// sides).
+int pick_chunk(int R, bool both, int32_t M, int64_t n_pad, double sel, double budget) {
+  const double per_vector = 2.0 * M * n_pad * sel;
   if (both) {
     int c = 1;
     while (c < R && c < 32) c <<= 1;
     while (c > 1 && per_vector * c > budget) c >>= 1;
     return c;
   }
+  constexpr double kStepMs = 4.5e-3, kRowMs = 0.8e-9, kL2Ms = 4e-9, kHbmMs = 8e-9, kGemmMs = 8e-12, kMapMs = 0.45e-9;
+  int best = 1;
+  double least = 0.0;
   for (int cap = 32; cap > 1; cap -= 2) {
-    const int w = step_width(TBK_PREC_MIXED, R, cap);
-    if (per_vector * w <= budget) return w;
+    const int w = step_width(TBK_PREC_MIXED, R, cap), chunks = (R + w - 1) / w;
+    const double bytes = per_vector * w, pooled = bytes + 12.0 * 16.0 * n_pad * w;
+    if (bytes > budget) continue;
+    const double value = (24.0 * n_pad * w <= 32e6 ? kL2Ms : kHbmMs) + M * kGemmMs;
+    const double ms = chunks * 2.0 * M * (kStepMs + n_pad * (kRowMs + w * value)) +
+                      (pooled > (double)kKuboPoolKeep ? kMapMs * bytes : 0.0);
+    if (best > 1 && ms >= least) continue;
+    best = w;
+    least = ms;
   }
-  return 1;
+  return best;
 }
 
 }  // namespace
@@ -696,8 +715,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   for (auto* o : ops) if (o) TBK_TRY(ensure_ell(o, st));
   trace.mark("ell");
   const int64_t n_pad = (int64_t)Ht->ell.n_slices * 32;
-  // default budget: 60% of the free device memory (more vectors per chunk stream
-  // the matrix fewer times)
+  // default budget: 60% of the free device memory
   double budget = block_budget_gb * 1e9;
   if (block_budget_gb <= 0) {
     size_t fr = 0, tot = 0;
@@ -710,7 +728,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
                    : (flags & TBK_MU_DD_RECURSION)  ? TBK_PREC_DD
                                                     : TBK_PREC_FP64;
   // chunk of random vectors: both stored sides within the budget
-  const int Rc = pick_chunk(R, (flags & TBK_MU_BOTH_SIDES) != 0, 2.0 * M * n_pad * sel, budget);
+  const int Rc = pick_chunk(R, (flags & TBK_MU_BOTH_SIDES) != 0, M, n_pad, sel, budget);
   if (2.0 * M * n_pad * Rc * sel > budget)
     return fail(TBK_ERR_BUDGET, "stored Chebyshev blocks need %.1f GB > budget %.1f GB", 2.0 * M * n_pad * sel / 1e9,
                 budget / 1e9);
