@@ -28,6 +28,23 @@ struct ClassTab {
 // shared-memory table of the class form: values, offsets, counts
 template <typename F, bool CPLX_H>
 constexpr int class_value_bytes() { return (CPLX_H ? 2 : 1) * (int)sizeof(F); }
+// Four consecutive class values in FP32 (o a multiple of 4, as the tables' width is).
+template <bool CPLX_H>
+__device__ __forceinline__ void load_smem4(const float* p, int32_t o, HVal<float, CPLX_H> (&h)[4]) {
+  if constexpr (CPLX_H) {
+    const float4 a = reinterpret_cast<const float4*>(p)[o / 2], b = reinterpret_cast<const float4*>(p)[o / 2 + 1];
+    h[0] = {a.x, a.y};
+    h[1] = {a.z, a.w};
+    h[2] = {b.x, b.y};
+    h[3] = {b.z, b.w};
+  } else {
+    const float4 a = reinterpret_cast<const float4*>(p)[o / 4];
+    h[0] = {a.x};
+    h[1] = {a.y};
+    h[2] = {a.z};
+    h[3] = {a.w};
+  }
+}
 template <typename F, bool CPLX_H>
 inline size_t class_smem_bytes(const ClassTab& ct) {
   const size_t ne = (size_t)ct.n_cls * ct.w;
@@ -230,6 +247,12 @@ kpm_step_kernel(
     add_c = HVal<F, true>{F(f * ks.addc[0]), F(f * ks.addc[1])};
   }
 
+  const CT* xl = x + sub * VPL;            // this lane's column of x
+  const uint32_t row_bytes = (uint32_t)(RW * sizeof(CT));
+  auto nb = [&](uint32_t c) { return ld_row<F, VPL>(xl, c, row_bytes); };
+  // rows are verified equal to their class, so r + offset is the row's column; the clamp only
+  // keeps a bad table inside the block
+  auto clamp = [&](int32_t c) { return min((uint32_t)c, (uint32_t)(n - 1)); };
   for (int32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const uint32_t c_cur = c_next;
     if constexpr (CLS) {
@@ -310,6 +333,10 @@ kpm_step_kernel(
       // instructions and registers); the wider types keep the predicates,
       // whose unconditional form holds more gathers in registers
       constexpr bool WHOLE = sizeof(F) == 4;
+      // the table read four entries at a time where the launch bound leaves registers
+      // for it (FCC 64^3 Kubo blocks 8.8 -> 8.1 us; the moments step spills: honeycomb
+      // 1024^2, R = 32: 242 -> 277)
+      constexpr bool VEC = KST == 2;
       int k0 = 0;
       if constexpr (is_f64<F> && KST != 2) {
         // FP64: whole groups, then single entries (a predicated product still
@@ -318,33 +345,50 @@ kpm_step_kernel(
           LaneV<F, VPL> xv[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            xv[u] = ld_ro<F, VPL>(x + ((int64_t)min(max(r + s_off[tb + k0 + u], 0), n - 1) * LPR + sub) * VPL);
+            xv[u] = nb(clamp(r + s_off[tb + k0 + u]));
 #pragma unroll
           for (int u = 0; u < 4; ++u) HVal<F, CPLX_H>::load_smem(s_val, tb + k0 + u).template fma<VPL>(xv[u], acc);
         }
 #pragma unroll 1
         for (; k0 < cnt; ++k0)
-          HVal<F, CPLX_H>::load_smem(s_val, tb + k0).template fma<VPL>(
-              ld_ro<F, VPL>(x + ((int64_t)min(max(r + s_off[tb + k0], 0), n - 1) * LPR + sub) * VPL), acc);
+          HVal<F, CPLX_H>::load_smem(s_val, tb + k0).template fma<VPL>(nb(clamp(r + s_off[tb + k0])), acc);
       }
       for (int k = k0; k < cnt; k += 4) {
         HVal<F, CPLX_H> h[4];
         LaneV<F, VPL> xv[4];
+        if constexpr (WHOLE && VEC) {
+          const int4 o = *reinterpret_cast<const int4*>(s_off + tb + k);
+          xv[0] = nb(clamp(r + o.x));
+          xv[1] = nb(clamp(r + o.y));
+          xv[2] = nb(clamp(r + o.z));
+          xv[3] = nb(clamp(r + o.w));
+          load_smem4<CPLX_H>(s_val, tb + k, h);
+        } else if constexpr (WHOLE) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const bool v = WHOLE || k + u < cnt;
-          // rows are verified equal to their class, so r + offset is the
-          // row's column; the clamp only keeps a bad table inside the block
-          const int32_t c = v ? min(max(r + s_off[tb + k + u], 0), n - 1) : r;
-          h[u] = v ? HVal<F, CPLX_H>::load_smem(s_val, tb + k + u) : HVal<F, CPLX_H>::zero();
-          xv[u] = v ? ld_ro<F, VPL>(x + ((int64_t)c * LPR + sub) * VPL) : xs;
+          for (int u = 0; u < 4; ++u) {
+            h[u] = HVal<F, CPLX_H>::load_smem(s_val, tb + k + u);
+            xv[u] = nb(clamp(r + s_off[tb + k + u]));
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const bool v = k + u < cnt;
+            h[u] = v ? HVal<F, CPLX_H>::load_smem(s_val, tb + k + u) : HVal<F, CPLX_H>::zero();
+            xv[u] = v ? ld_ro<F, VPL>(x + ((int64_t)clamp(r + s_off[tb + k + u]) * LPR + sub) * VPL) : xs;
+          }
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], acc);
         if constexpr (KST == 2) {
+          if constexpr (WHOLE && VEC) {
+            load_smem4<CPLX_H>(s_val2, tb + k, h);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (WHOLE || k + u < cnt) HVal<F, CPLX_H>::load_smem(s_val2, tb + k + u).template fma<VPL>(xv[u], vacc);
+            for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], vacc);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (WHOLE || k + u < cnt) HVal<F, CPLX_H>::load_smem(s_val2, tb + k + u).template fma<VPL>(xv[u], vacc);
+          }
         }
       }
     } else if (gather) {
@@ -365,7 +409,7 @@ kpm_step_kernel(
           LaneV<F, VPL> xv[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            xv[u] = ld_ro<F, VPL>(x + ((int64_t)__ldg(cp + (k0 + u) * 32) * LPR + sub) * VPL);
+            xv[u] = nb(__ldg(cp + (k0 + u) * 32));
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             ell_entry<F, VPL, CPLX_H, FOLD>(eval, off + l + (int64_t)(k0 + u) * 32, xv[u], acc);
@@ -373,7 +417,7 @@ kpm_step_kernel(
 #pragma unroll 1
         for (; k0 < w; ++k0)
           ell_entry<F, VPL, CPLX_H, FOLD>(eval, off + l + (int64_t)k0 * 32,
-                                          ld_ro<F, VPL>(x + ((int64_t)__ldg(cp + k0 * 32) * LPR + sub) * VPL), acc);
+                                          nb(__ldg(cp + k0 * 32)), acc);
       }
       // all of a row's gathers in flight together: predicated groups of 4
       for (int k = k0; k < w; k += 4) {
@@ -392,7 +436,11 @@ kpm_step_kernel(
         }
         LaneV<F, VPL> xv[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) xv[u] = ld_ro<F, VPL>(x + ((int64_t)c[u] * LPR + sub) * VPL);
+        for (int u = 0; u < 4; ++u) {
+          // complex FP32 values: square 700x512 with a flux, R = 4: 9.4 us a step, 10.1 by rows
+          if constexpr (CPLX_H && sizeof(F) == 4 && KST == 0 && R > 0) xv[u] = ld_ro<F, VPL>(x + ((int64_t)c[u] * LPR + sub) * VPL);
+          else xv[u] = nb(c[u]);
+        }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           if constexpr (FOLD) {
