@@ -38,25 +38,32 @@ namespace {
 
 // ------------------------------------------------------------------ CUDA-core GEMM
 // C[m][n] += sum_k conj(L[m][k]) R[n][k] for a K range per CTA (split-K), blocks in the
-// K-tiled layout; FP32 products, FP32 sums over 32 terms added into float-float pairs by
+// K-tiled layout; FP32 products, FP32 sums over 32 values of k added into float-float pairs by
 // TwoSum (48 bits, on the FP32 pipe: FP64 sums of the chunks took twice the time of the
-// products), FP64 partial tiles.  64 x 32 complex outputs per CTA, 4 x 2 per thread: 6
-// shared-memory reads for 32 FMAs, each one wavefront (rows 17 values apart), so the FMAs
-// bound it; the K tiles arrive by cp.async, three deep.  M = 200, K = 56,064: 2.20 ms with
-// 2 x 2 outputs per thread and FP64 sums, 0.86 ms so.
+// products), FP64 partial tiles.  64 x 32 complex outputs per CTA, 4 x 2 per thread.  What
+// bounds it: the FP32 pipe and the issue slots in front of it (86% busy with scalar code, whose
+// re += a b + c d is a product, an FMA and an addition).  So two neighbouring k share packed
+// FMAs, one in each half (32 of them for 12 shared-memory reads), and the real and imaginary
+// parts lie apart in shared memory, where a read then is a packed operand; rows are 34 words
+// apart (no bank conflicts); the K tiles arrive by cp.async, three deep.  The halves are added
+// before the TwoSum: 17 roundings of half a chunk's sum, where the scalar form made 32 of all
+// of it.  M = 200, K = 56,064: 2.20 ms with 2 x 2 outputs per thread and FP64 sums, 0.81 ms
+// scalar with 4 x 2, 0.68 ms so (53% of the issue slots, the FP32 pipe in front; 16-byte
+// shared-memory reads: 0.70).
 constexpr int kGT = 32;      // output tile (complex) per CTA side of the FP64 form, and n here
 constexpr int kGM = 64;      // m
 constexpr int kGStages = 3;
-constexpr int kGPitch = 17;  // a K tile's 16 values and one of padding
+constexpr int kGPitch = 34;  // a K tile's 16 real parts, its 16 imaginary parts and two of padding
 
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool real) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(real ? 8 : 0)
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(real ? 4 : 0)
                : "memory");
 }
-__device__ __forceinline__ void ff_add(float& hi, float& lo, float v) {      // TwoSum (Knuth)
-  const float s = __fadd_rn(hi, v), b = __fsub_rn(s, hi);
-  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(v, b)));
+// hi + lo += v in both halves: TwoSum (Knuth)
+__device__ __forceinline__ void ff_add2(uint64_t& hi, uint64_t& lo, uint64_t v) {
+  const uint64_t s = f2_add(hi, v), b = f2_sub(s, hi);
+  lo = f2_add(lo, f2_add(f2_sub(hi, f2_sub(s, b)), f2_sub(v, b)));
   hi = s;
 }
 
@@ -64,63 +71,74 @@ __device__ __forceinline__ void ff_add(float& hi, float& lo, float v) {      // 
 __global__ void __launch_bounds__(256) mu_gemm_cc_kernel(const float2* __restrict__ L, const float2* __restrict__ Rb,
                                                          int32_t M, int64_t tiles, int64_t tiles_split,
                                                          double2* __restrict__ part) {
-  __shared__ float2 sm[kGStages][kGM + kGT][kGPitch];
+  __shared__ __align__(16) float sm[kGStages][kGM + kGT][kGPitch];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int32_t m0 = blockIdx.y * kGM, n0 = blockIdx.x * kGT;
   const int64_t t0 = (int64_t)blockIdx.z * tiles_split, t1 = min(tiles, t0 + tiles_split);
   // 6 values of a stage per thread: value tx of rows ty, ty + 16, ...; rows past M read as zero
   auto load = [&](int64_t t) {
     if (t < t1) {
-      float2(*st)[kGPitch] = sm[(t - t0) % kGStages];
+      float(*st)[kGPitch] = sm[(t - t0) % kGStages];
 #pragma unroll
       for (int q = 0; q < (kGM + kGT) / 16; ++q) {
         const int row = ty + 16 * q;
         const bool left = row < kGM;
         const int32_t b = left ? m0 + row : n0 + row - kGM;
         const float2* src = (left ? L : Rb) + (t * M + min(b, M - 1)) * 16 + tx;
-        cp_async8(&st[row][tx], src, b < M);
+        cp_async4(&st[row][tx], &src->x, b < M);
+        cp_async4(&st[row][16 + tx], &src->y, b < M);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float hr[4][2], lr[4][2], hi[4][2], li[4][2], ar[4][2], ai[4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) hr[i][j] = lr[i][j] = hi[i][j] = li[i][j] = ar[i][j] = ai[i][j] = 0.f;
+  // sums over even | odd k; float-float sums of re | im
+  uint64_t ar[4][2] = {}, ai[4][2] = {}, hi[4][2] = {}, lo[4][2] = {};
   load(t0);
   load(t0 + 1);
   for (int64_t t = t0; t < t1; ++t) {
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    const float2(*st)[kGPitch] = sm[(t - t0) % kGStages];
+    const float(*st)[kGPitch] = sm[(t - t0) % kGStages];
+    auto pair = [&](int row, int at) { return *reinterpret_cast<const uint64_t*>(&st[row][at]); };
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float2 a[4], b[2];
+    for (int kk = 0; kk < 16; kk += 2) {
+      uint64_t ax[4], ay[4], bx[2], by[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = st[ty + 16 * i][kk];
+      for (int i = 0; i < 4; ++i) {
+        ax[i] = pair(ty + 16 * i, kk);
+        ay[i] = pair(ty + 16 * i, 16 + kk);
+      }
 #pragma unroll
-      for (int j = 0; j < 2; ++j) b[j] = st[kGM + tx + 16 * j][kk];
+      for (int j = 0; j < 2; ++j) {
+        bx[j] = pair(kGM + tx + 16 * j, kk);
+        by[j] = pair(kGM + tx + 16 * j, 16 + kk);
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2; ++j) {
+        const uint64_t nx = bx[j] ^ 0x8000000080000000ull;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int i = 0; i < 4; ++i) {
           // conj(a) * b
-          ar[i][j] += a[i].x * b[j].x + a[i].y * b[j].y;
-          ai[i][j] += a[i].x * b[j].y - a[i].y * b[j].x;
+          ar[i][j] = f2_fma(ax[i], bx[j], ar[i][j]);
+          ai[i][j] = f2_fma(ax[i], by[j], ai[i][j]);
+          ar[i][j] = f2_fma(ay[i], by[j], ar[i][j]);
+          ai[i][j] = f2_fma(ay[i], nx, ai[i][j]);
         }
+      }
     }
     load(t + 2);                 // over the stage that every thread left before this barrier
-    // FP32 sums cover two K tiles (32 terms) only: long FP32 accumulations lose accuracy
+    // FP32 sums cover two K tiles (32 values of k) only: long FP32 accumulations lose accuracy
     // where the sum is much smaller than its terms (mu_nm at large m, n)
     if (((t - t0) & 1) || t + 1 == t1) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          ff_add(hr[i][j], lr[i][j], ar[i][j]);
-          ff_add(hi[i][j], li[i][j], ai[i][j]);
-          ar[i][j] = ai[i][j] = 0.f;
+          float r0, r1, i0, i1;
+          f2_unpack(ar[i][j], r0, r1);
+          f2_unpack(ai[i][j], i0, i1);
+          ff_add2(hi[i][j], lo[i][j], f2_pack(__fadd_rn(r0, r1), __fadd_rn(i0, i1)));
+          ar[i][j] = ai[i][j] = 0;
         }
     }
   }
@@ -130,9 +148,11 @@ __global__ void __launch_bounds__(256) mu_gemm_cc_kernel(const float2* __restric
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int32_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      float hr, hm, lr, lm;
+      f2_unpack(hi[i][j], hr, hm);
+      f2_unpack(lo[i][j], lr, lm);
       if (m < M && n < M)
-        part[((int64_t)blockIdx.z * M + m) * M + n] = make_double2((double)hr[i][j] + (double)lr[i][j],
-                                                                   (double)hi[i][j] + (double)li[i][j]);
+        part[((int64_t)blockIdx.z * M + m) * M + n] = make_double2((double)hr + (double)lr, (double)hm + (double)lm);
     }
 }
 
@@ -146,15 +166,25 @@ __global__ void mu_split_reduce_kernel(const double2* __restrict__ part, int32_t
   acc[q].y += i;
 }
 
-// acc += L^H R of complex64 K-tiled stores.  K is split until the CTAs fill the SMs twice
-// over (three CTAs each), into at most 64 partial M x M blocks of 1,024 values of k or
-// more, and at least into those of 16,384 or K / 64.
+// acc += L^H R of complex64 K-tiled stores.  K is split into at most 64 partial M x M
+// blocks of 512 values of k or more, and at least into those of 16,384 or K / 64: within
+// that, the fewest splits whose CTAs (two per SM) leave at most a twentieth of their last
+// wave empty, or the split that leaves least (M = 32, K = 30,000: 105 -> 56 us; M = 128, K =
+// 65,536: 253 -> 245).
 int mu_gemm_cc(const float2* L, const float2* Rb, int32_t M, int64_t K, DevBuf* part, double2* acc, cudaStream_t st) {
   const int64_t tiles = (K + 15) / 16;
   const dim3 out((M + kGT - 1) / kGT, (M + kGM - 1) / kGM);
-  const int64_t want = (6LL * sm_count() + (int64_t)out.x * out.y - 1) / ((int64_t)out.x * out.y);
-  int64_t split = std::max<int64_t>(64, (tiles + std::min<int64_t>(want, 64) - 1) / std::min<int64_t>(want, 64));
-  split = std::min(split, std::max<int64_t>(1024, (tiles + 63) / 64));
+  const int64_t wave = 2LL * sm_count(), longest = std::max<int64_t>(1024, (tiles + 63) / 64);
+  int64_t split = longest;
+  double best = 0.0;
+  for (int64_t ns = (tiles + longest - 1) / longest; ns <= 64 && (ns == 1 || tiles / ns >= 32); ++ns) {
+    const int64_t units = (int64_t)out.x * out.y * ns, waves = (units + wave - 1) / wave;
+    const double eff = (double)units / (double)(waves * wave);
+    if (eff <= best + 1e-9) continue;
+    best = eff;
+    split = (tiles + ns - 1) / ns;
+    if (eff >= 0.95) break;
+  }
   const int32_t nsplit = (int32_t)((tiles + split - 1) / split);
   const size_t need = sizeof(double2) * (size_t)nsplit * M * M;
   if (part->bytes < need) TBK_TRY(part->alloc(need));
