@@ -323,7 +323,7 @@ int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int*
 
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
              int grid, int n_tiles, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots,
-             const ClassSet32* pair) {
+             const ClassSet32* pair, bool reverse) {
   StepArgs a;
   a.n = A->rows;
   a.n_tiles = n_tiles;
@@ -339,7 +339,7 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
   a.bras = nullptr;
   a.part = part;
   a.store = store_y ? 1 : 0;
-  a.reverse = 0;
+  a.reverse = reverse ? 1 : 0;
   a.gather = 1;
   a.pf_dist = 1;
   a.pipe = A->ell.max_width > 4;

@@ -684,15 +684,15 @@ struct SecondStream {
 // Vectors per chunk of the block recursions (n_pad rows, M blocks a side, sel bytes a stored
 // value; both stored sides within the budget; 1 when no width fits).  A chunk costs the two
 // sides' steps, each a launch (4.5 us), the matrix (5 bytes a row) and 32 bytes a row and
-// vector, twice as fast where the three vectors stay in L2 beside the stores that pass
-// through it, then the GEMM's products; stores that the pool does not keep cost their
-// mapping every call (137 GB: 57 ms to free, 5 to allocate).  So large problems take narrow
-// chunks: FCC 128^3, M = 1024, R = 8: 648 ms at width 4, 625 at 2, 721 at 1 (complex64 lanes
-// carry two vectors: 1 is not taken while 2 fits); FCC 64^3: 96.7 at 8, 79.1 at 4, 76.1 at
-// 2; honeycomb 1024^2, M = 512: 243 at 8, 216 at 4 and 2; square 512^2 with a flux, R = 12:
-// 48.3 at 6, 42.2 at 4.  The same in every recursion precision (the GEMM then sums in the
-// same order).  both: a power of two (the widths of the one recursion that carries both
-// sides).
+// vector, twice as fast where the two vectors stay in L2 beside the stores that pass through
+// it (FCC 64^3: 8.5 us a step at width 4, 20.7 at 8), then the GEMM's products; stores that
+// the pool does not keep cost their mapping every call (137 GB: 57 ms to free, 5 to
+// allocate).  So large problems take narrow chunks: FCC 128^3, M = 1024, R = 8: 648 ms at
+// width 4, 625 at 2, 721 at 1 (complex64 lanes carry two vectors: 1 is not taken while 2
+// fits); FCC 64^3: 96.7 at 8, 79.1 at 4, 76.1 at 2; honeycomb 1024^2, M = 512: 243 at 8, 216
+// at 4 and 2; square 512^2 with a flux, R = 12: 48.3 at 6, 42.2 at 4.  The same in every
+// recursion precision (the GEMM then sums in the same order).  both: a power of two (the
+// widths of the one recursion that carries both sides).
 int pick_chunk(int R, bool both, int32_t M, int64_t n_pad, double sel, double budget) {
   const double per_vector = 2.0 * M * n_pad * sel;
   if (both) {
@@ -706,9 +706,9 @@ int pick_chunk(int R, bool both, int32_t M, int64_t n_pad, double sel, double bu
   double least = 0.0;
   for (int cap = 32; cap > 1; cap -= 2) {
     const int w = step_width(TBK_PREC_MIXED, R, cap), chunks = (R + w - 1) / w;
-    const double bytes = per_vector * w, pooled = bytes + 12.0 * 16.0 * n_pad * w;
+    const double bytes = per_vector * w, pooled = bytes + 8.0 * 16.0 * n_pad * w;
     if (bytes > budget) continue;
-    const double value = (24.0 * n_pad * w <= 32e6 ? kL2Ms : kHbmMs) + M * kGemmMs;
+    const double value = (16.0 * n_pad * w <= 20e6 ? kL2Ms : kHbmMs) + M * kGemmMs;
     const double ms = chunks * 2.0 * M * (kStepMs + n_pad * (kRowMs + w * value)) +
                       (pooled > (double)kKuboPoolKeep ? kMapMs * bytes : 0.0);
     if (best > 1 && ms >= least) continue;
@@ -772,7 +772,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   DevBuf Ls, Rs, work, partd, part, macc, gdev, kstage;
   bool use_tc = !f64b && (flags & TBK_MU_TENSOR) != 0;   // FP16-pair stores and the tensor-core GEMM
   const int64_t blk16 = (blk + 31) / 32 * 32;           // K padded to whole tiles of either store (zeros)
-  if ((!tl_async_alloc || tl_async_alloc->scratch) && 2.0 * sel * blk16 * M + 12.0 * csz * blk <= (double)kKuboPoolKeep) {
+  if ((!tl_async_alloc || tl_async_alloc->scratch) && 2.0 * sel * blk16 * M + 8.0 * csz * blk <= (double)kKuboPoolKeep) {
     kctx.pool = kubo_pool();
     kctx.stream = st;
   }
@@ -799,7 +799,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   {
     const AsyncAllocCtx* outer = tl_async_alloc;
     if (kctx.pool) tl_async_alloc = &kctx;
-    const int a = work.alloc(csz * blk * (both ? 12 : dual ? 11 : 6));
+    const int a = work.alloc(csz * blk * (both ? 8 : dual ? 7 : 4));
     tl_async_alloc = outer;
     TBK_TRY(a);
   }
@@ -843,7 +843,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   trace.mark("alloc+classes");
   char* wb = work.as<char>();
   auto wblk = [&](int i) { return static_cast<void*>(wb + (size_t)i * blk * csz); };
-  void* v0 = wblk(5);
+  void* v0 = wblk(3);
   // algorithmic DRAM bytes of the block phase: vector blocks read / written,
   // matrix (ELL columns + values + diagonal) per pass, complex64 stores
   double rec_bytes = 0.0;
@@ -909,13 +909,17 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     TBK_CHECK_LAUNCH();
     return TBK_OK;
   };
+  // vectors past L2: every pass starts where the one before it ended (FCC 128^3, 2 vectors:
+  // 38.5 -> 37.5 us a step; honeycomb 1024^2, 4 vectors: 32.4 -> 30.6; inside L2 1% slower)
+  const bool zigzag = 2.0 * csz * blk > 32e6;
   // block m of `store` = A x, written by the product itself (no work block)
   auto apply_to_store = [&](tbk_sparse_s* A, const void* x, void* scratch, KStore ks, int32_t m) -> int {
     rec_bytes += vecb + ell_bytes(A, true) + stb;
     int g, t;
     TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
     ks.km[0] = m;
-    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, q, &ks, false);
+    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, q, &ks, false, nullptr, true, nullptr,
+                    zigzag && (m & 1) == 0);
   };
   // one side: store[m] = Aout T_m(H~) (Bin v0), m < M; each step writes its
   // complex64 block (Aout absent) or feeds the product that does
@@ -927,9 +931,9 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   auto side = [&](int h, int32_t m_begin, int32_t m_end) -> int {
     tbk_sparse_s* Aout = h ? AR : AL;
     tbk_sparse_s* Bin = h ? BR : BL;
-    const int w0 = dual && h ? 6 : 0;                     // this side's work blocks
-    void* r[3] = {wblk(w0), wblk(w0 + 1), wblk(w0 + 2)};
-    void* tmpA = wblk(w0 + 3);
+    const int w0 = dual && h ? 4 : 0;                     // this side's work blocks
+    void* r[2] = {wblk(w0), wblk(w0 + 1)};                // T_m over T_{m-2}: one block less in L2
+    void* tmpA = wblk(w0 + 2);
     const Fused& F = fused[h];
     const bool fuse = F.on;
     KStore ks;
@@ -943,9 +947,9 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         if (Bin) TBK_TRY(apply(Bin, v0, r[0]));
         else TBK_CUDA(cudaMemcpyAsync(r[0], v0, csz * blk, cudaMemcpyDeviceToDevice, q));
       }
-      void* y = r[m % 3];
-      const void* x = m >= 1 ? r[(m - 1) % 3] : nullptr;
-      const void* pv = m >= 2 ? r[(m - 2) % 3] : nullptr;
+      void* y = r[m & 1];
+      const void* x = m >= 1 ? r[(m - 1) & 1] : nullptr;
+      const void* pv = m >= 2 ? y : nullptr;
       if (f64b) {                                         // recursion, operator, complex128 store
         if (m == M) break;
         if (m >= 1) {
@@ -968,7 +972,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         ks.km[0] = fuse ? m - 1 : m;
         TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), F.grid, F.tiles, q,
                          fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false,
-                         F.pair.n_cls > 0 ? &F.pair : nullptr));
+                         F.pair.n_cls > 0 ? &F.pair : nullptr, zigzag && (m & 1)));
         if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
       } else if (fuse) {
         TBK_TRY(apply_to_store(Aout, x, tmpA, ks, M - 1));
@@ -981,8 +985,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // operator as block m and A T_{m-1} of a side with one as block m-1
   auto both_sides = [&]() -> int {
     const size_t b2 = csz * blk * 2;
-    char* base = wb + csz * blk * 6;                     // three 2 Rc-wide blocks after the six Rc-wide ones
-    void* r[3] = {base, base + b2, base + 2 * b2};
+    char* base = wb + csz * blk * 4;                     // two 2 Rc-wide blocks after the four Rc-wide ones
+    void* r[2] = {base, base + b2};
     void* half[2] = {wblk(0), wblk(1)};
     tbk_sparse_s* Bin[2] = {BL, BR};
     tbk_sparse_s* Aout[2] = {AL, AR};
@@ -1003,8 +1007,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       if (Bin[h]) TBK_TRY(apply(Bin[h], v0, half[h]));
       else TBK_CUDA(cudaMemcpyAsync(half[h], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
       if (use_tc) {
-        if (Aout[h]) TBK_TRY(apply(Aout[h], half[h], wblk(3)));
-        TBK_TRY(find_scale(Aout[h] ? wblk(3) : half[h], h));
+        if (Aout[h]) TBK_TRY(apply(Aout[h], half[h], wblk(2)));
+        TBK_TRY(find_scale(Aout[h] ? wblk(2) : half[h], h));
       }
       TBK_TRY(with_block(prec, half[h], [&](auto p) {
         using CT = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
@@ -1025,12 +1029,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       rec_bytes += 2 * (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + 2 * stb;
       for (int h = 0; h < 2; ++h) rec_bytes += Aout[h] ? ell_bytes(Aout[h], false) : 0.0;
       for (int h = 0; h < 2; ++h) ks.km[h] = Aout[h] ? m - 1 : m;
-      TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(m - 1) % 3], r[m % 3], m >= 2 ? r[(m - 2) % 3] : nullptr, m == 1,
+      TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(m - 1) & 1], r[m & 1], m >= 2 ? r[m & 1] : nullptr, m == 1,
                       partd.as<double>(), grid2, tiles2, st, ks));
     }
     if (AL || AR) {                                      // A T_{M-1} -> block M-1 (the new vector is not kept)
       for (int h = 0; h < 2; ++h) ks.km[h] = Aout[h] ? M - 1 : -1;
-      TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(M - 1) % 3], r[M % 3], M >= 2 ? r[(M - 2) % 3] : nullptr, M == 1,
+      TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(M - 1) & 1], r[M & 1], M >= 2 ? r[M & 1] : nullptr, M == 1,
                       partd.as<double>(), grid2, tiles2, st, ks));
     }
     return TBK_OK;

@@ -229,9 +229,10 @@ int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cuda
 // vop: with ks, store vop x instead of the output; vop must share A's ELL
 // structure (same_ell_structure) and precision arrays; pair: their joint classes
 // dots: form the moment partial sums (false: the step only feeds other work)
+// reverse: the tiles from the last to the first (what the pass before left in L2 first)
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
              int grid, int n_tiles, cudaStream_t st, const KStore* ks = nullptr, bool store_y = true,
-             tbk_sparse_s* vop = nullptr, bool dots = true, const ClassSet32* pair = nullptr);
+             tbk_sparse_s* vop = nullptr, bool dots = true, const ClassSet32* pair = nullptr, bool reverse = false);
 // grid and tiles of a step with an operator product in the joint class form (complex64;
 // pair: pair_classes32 of A and the operator)
 int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles);
