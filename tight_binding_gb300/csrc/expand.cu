@@ -150,6 +150,9 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
   TBK_CUDA(cudaMemsetAsync(vk.p, 0, vk.bytes, st));
   TBK_CUDA(cudaMemsetAsync(bc.p, 0, bc.bytes, st));                         // padding rows stay zero
   auto c_of = [&](int32_t k) { return make_double2(coef[2 * k], coef[2 * k + 1]); };
+  // vectors past L2: every step starts where the one before it ended (double-float: honeycomb
+  // 500^2, 9 vectors, t = 40: 21.8 -> 21.4 ms; 700x600, 4 vectors: 12.3 -> 12.0)
+  const bool zigzag = 3.0 * csz * cnt > 48e6;
   for (int32_t r0 = 0; r0 < R; r0 += Rc) {
     TBK_TRY(load_block_any(prec, n, R, r0, Rc, src.as<double2>(), vk.p, st));
     // Clenshaw: x = b_{k+1}, p = b_{k+2}; b_k is written over p
@@ -162,7 +165,8 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
     for (int32_t k = n_terms - 2; k >= 1; --k) {
       ks.addc[0] = coef[2 * k];
       ks.addc[1] = coef[2 * k + 1];
-      TBK_TRY(step_ks(Ht, Rc, prec, x, p, p, false, part.as<double>(), grid, n_tiles, st, ks, 3));
+      TBK_TRY(step_ks(Ht, Rc, prec, x, p, p, false, part.as<double>(), grid, n_tiles, st, ks, 3,
+                      zigzag && (k & 1)));
       std::swap(x, p);                                                      // x = b_k, p = b_{k+1}
     }
     if (n_terms >= 2) {

@@ -366,7 +366,7 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
 }
 
 int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode) {
+            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode, bool reverse) {
   StepArgs a;
   a.n = A->rows;
   a.n_tiles = n_tiles;
@@ -382,7 +382,7 @@ int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const voi
   a.bras = nullptr;
   a.part = part;
   a.store = 1;
-  a.reverse = 0;
+  a.reverse = reverse ? 1 : 0;
   a.gather = 1;
   a.pf_dist = 1;
   a.ks = ks;

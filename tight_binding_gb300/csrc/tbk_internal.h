@@ -244,7 +244,7 @@ const void* ell_diag(const EllDev& E, int prec);
 // one recursion step (not the first block's braket form) writing the K-tiled
 // stores described by ks (output or operator products per column group)
 int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode = 2);
+            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode = 2, bool reverse = false);
 // true when B's sliced ELL has A's slices, widths and columns (values may differ)
 // (b_real: B may hold real values where A's are complex; then set)
 int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st, bool* b_real = nullptr);
