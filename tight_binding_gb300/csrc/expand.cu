@@ -116,7 +116,7 @@ using namespace tbk;
 struct tbk_cheb_view_s {
   tbk_sparse_s* H = nullptr;
   int32_t n = 0, R = 0, Rc = 0, n_chunks = 0, prec = 0, i = 0;
-  int grid = 1, n_tiles = 1;
+  int grid = 1;
   std::vector<DevBuf> cur, nxt;      // per chunk: T_i v, T_{i+1} v (site-major)
   DevBuf acc, dst, part;
 };
@@ -135,8 +135,8 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
   ScratchScope scope(st);
   const int32_t n = Ht->rows;
   const int Rc = chunk_width(prec, R);
-  int grid = 1, n_tiles = 1;
-  TBK_TRY(step_config(Ht, Rc, prec, &grid, &n_tiles, st));
+  int grid = 1;
+  TBK_TRY(step_config(Ht, Rc, prec, &grid, st, false));
   const int64_t n_pad = (int64_t)Ht->ell.n_slices * 32;
   const size_t csz = prec == TBK_PREC_MIXED ? sizeof(float2) : prec == TBK_PREC_DD ? sizeof(dd2) : sizeof(double2);
   const int64_t cnt = n_pad * Rc;
@@ -165,7 +165,7 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
     for (int32_t k = n_terms - 2; k >= 1; --k) {
       ks.addc[0] = coef[2 * k];
       ks.addc[1] = coef[2 * k + 1];
-      TBK_TRY(step_ks(Ht, Rc, prec, x, p, p, false, part.as<double>(), grid, n_tiles, st, ks, 3,
+      TBK_TRY(step_ks(Ht, Rc, prec, x, p, p, false, part.as<double>(), grid, st, ks, 3,
                       zigzag && (k & 1)));
       std::swap(x, p);                                                      // x = b_k, p = b_{k+1}
     }
@@ -173,7 +173,7 @@ int tbk_cheb_expand(tbk_sparse Ht, int32_t n_terms, const double* coef, int32_t 
       // b_0 out of place (b_2 stays for the final combination)
       ks.addc[0] = coef[0];
       ks.addc[1] = coef[1];
-      TBK_TRY(step_ks(Ht, Rc, prec, x, bc.p, p, false, part.as<double>(), grid, n_tiles, st, ks, 3));
+      TBK_TRY(step_ks(Ht, Rc, prec, x, bc.p, p, false, part.as<double>(), grid, st, ks, 3));
       TBK_TRY(final_any(prec, cnt, bc.p, p, vk.p, c_of(0), acc.as<double2>(), st));
     } else {
       // one term: out = c_0 v  (= (b_0 - b_2 + c_0 v)/2 with b_0 = c_0 v, b_2 = 0)
@@ -204,7 +204,7 @@ int tbk_cheb_view_create(tbk_cheb_view* out, tbk_sparse Ht, int32_t R, const dou
   V->Rc = chunk_width(precision, R);
   V->n_chunks = (R + V->Rc - 1) / V->Rc;
   auto bail = [&](int rc) { delete V; return rc; };
-  int rc = step_config(Ht, V->Rc, precision, &V->grid, &V->n_tiles, st);
+  int rc = step_config(Ht, V->Rc, precision, &V->grid, st);
   if (rc != TBK_OK) return bail(rc);
   const int64_t cnt = (int64_t)Ht->ell.n_slices * 32 * V->Rc;
   const size_t csz = precision == TBK_PREC_MIXED ? sizeof(float2) : precision == TBK_PREC_DD ? sizeof(dd2) : sizeof(double2);
@@ -224,7 +224,7 @@ int tbk_cheb_view_create(tbk_cheb_view* out, tbk_sparse Ht, int32_t R, const dou
     // v_0 = v, v_1 = x v (the view's constructor)
     if ((rc = load_block_any(precision, V->n, R, c * V->Rc, V->Rc, src.as<double2>(), V->cur[c].p, st)) != TBK_OK ||
         (rc = step_any(Ht, V->Rc, precision, V->cur[c].p, V->nxt[c].p, nullptr, true, V->part.as<double>(), V->grid,
-                       V->n_tiles, st, nullptr, true, nullptr, false)) != TBK_OK)
+                       st, nullptr, true, nullptr, false)) != TBK_OK)
       return bail(rc);
   }
   if (cudaStreamSynchronize(st) != cudaSuccess) return bail(fail(TBK_ERR_CUDA, "tbk_cheb_view_create: sync failed"));
@@ -249,7 +249,7 @@ int tbk_cheb_view_next(tbk_cheb_view V, int32_t* index, double* block, void* str
     }
     // T_{i+2} = 2 x T_{i+1} - T_i, written over T_i; then cur <-> nxt
     TBK_TRY(step_any(V->H, V->Rc, V->prec, V->nxt[c].p, V->cur[c].p, V->cur[c].p, false, V->part.as<double>(),
-                     V->grid, V->n_tiles, st, nullptr, true, nullptr, false));
+                     V->grid, st, nullptr, true, nullptr, false));
     std::swap(V->cur[c], V->nxt[c]);
   }
   if (block)

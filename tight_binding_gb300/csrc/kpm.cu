@@ -292,16 +292,18 @@ static int step_occupancy(tbk_sparse_s* A, int Rc, int prec, bool sums, int thre
   return std::min(oc, oe);
 }
 
-// grid and tiles of the steps without sums (step_any, step_ks)
-int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st) {
+static int tiles_of(tbk_sparse_s* A, int Rc, int prec, int threads) {
+  const int rpt = rows_per_tile(prec, Rc, threads);
+  return (A->rows + rpt - 1) / rpt;
+}
+
+int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, cudaStream_t st, bool wide) {
   TBK_TRY(ensure_ell(A, st));
   if (prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(A, st));
   if (prec == TBK_PREC_MIXED) TBK_TRY(ensure_classes32(A, st));
   else TBK_TRY(ensure_classes(A, st));
-  const int threads = step_threads(A, Rc, prec, kWideThreads<4>);
-  const int rpt = rows_per_tile(prec, Rc, threads);
-  *n_tiles = (A->rows + rpt - 1) / rpt;
-  *grid = std::max(1, std::min(*n_tiles, sm_count() * step_occupancy(A, Rc, prec, false, threads)));
+  const int threads = wide ? step_threads(A, Rc, prec, kWideThreads<4>) : kStepThreads;
+  *grid = std::max(1, std::min(tiles_of(A, Rc, prec, threads), sm_count() * step_occupancy(A, Rc, prec, false, threads)));
   return TBK_OK;
 }
 
@@ -312,21 +314,19 @@ static int pair_threads(tbk_sparse_s* A, int Rc) {
   return lanes >= (int64_t)kWideThreads<2> * 2 * 2 * sm_count() ? kWideThreads<2> : kStepThreads;
 }
 
-int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles) {
-  const int threads = pair_threads(A, Rc), rpt = rows_per_tile(TBK_PREC_MIXED, Rc, threads);
-  *n_tiles = (A->rows + rpt - 1) / rpt;
+int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid) {
+  const int threads = pair_threads(A, Rc);
   // launch bounds: two CTAs of the wide size per SM
   const int per_sm = 2 * kWideThreads<2> / threads;
-  *grid = std::max(1, std::min(*n_tiles, sm_count() * per_sm));
+  *grid = std::max(1, std::min(tiles_of(A, Rc, TBK_PREC_MIXED, threads), sm_count() * per_sm));
   return TBK_OK;
 }
 
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-             int grid, int n_tiles, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots,
+             int grid, cudaStream_t st, const KStore* ks, bool store_y, tbk_sparse_s* vop, bool dots,
              const ClassSet32* pair, bool reverse) {
   StepArgs a;
   a.n = A->rows;
-  a.n_tiles = n_tiles;
   a.n_slices = A->ell.n_slices;
   a.err = nullptr;
   a.soff = A->ell.slice_off.as<int32_t>();
@@ -366,10 +366,9 @@ int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const vo
 }
 
 int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode, bool reverse) {
+            int grid, cudaStream_t st, const KStore& ks, int mode, bool reverse) {
   StepArgs a;
   a.n = A->rows;
-  a.n_tiles = n_tiles;
   a.n_slices = A->ell.n_slices;
   a.err = nullptr;
   a.soff = A->ell.slice_off.as<int32_t>();
@@ -398,8 +397,9 @@ static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const St
   } else if (has_classes(A->ell, prec) && a.kst != 2) {     // the class form where it applies
     a.cls = true;
     a.ct = class_tab(A->ell, prec);
-    a.threads = step_threads(A, Rc, prec, kWideThreads<4>);
+    if (a.kst != 0 && a.kst != 3) a.threads = step_threads(A, Rc, prec, kWideThreads<4>);   // kWideSteps
   }
+  a.n_tiles = tiles_of(A, Rc, prec, a.threads);            // of the kernel that runs: the grid strides over any number
   return launch_step_prec(prec, A->ell.cplx != 0, Rc, a, first, false, grid, st);
 }
 

@@ -827,14 +827,15 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     TBK_TRY(kstage.alloc(sizeof(double2) * (size_t)n * R));
     TBK_CUDA(cudaMemcpyAsync(kstage.p, kets, sizeof(double2) * (size_t)n * R, cudaMemcpyHostToDevice, st));
   }
-  int grid = 1, n_tiles = 1;
-  TBK_TRY(step_config(Ht, Rc, prec, &grid, &n_tiles, st));
-  int gmax = grid;
+  int grid = 1, grid_op = 1;                             // of the steps; with an operator product in the ELL form
+  TBK_TRY(step_config(Ht, Rc, prec, &grid, st));
+  TBK_TRY(step_config(Ht, Rc, prec, &grid_op, st, false));
+  int gmax = std::max(grid, grid_op);
   for (auto* o : ops)
-    if (o) { int g2, t2; TBK_TRY(step_config(o, Rc, prec, &g2, &t2, st)); gmax = std::max(gmax, g2); }
-  int grid2 = 1, tiles2 = 1;
+    if (o) { int g2; TBK_TRY(step_config(o, Rc, prec, &g2, st)); gmax = std::max(gmax, g2); }
+  int grid2 = 1;
   if (both) {
-    TBK_TRY(step_config(Ht, 2 * Rc, prec, &grid2, &tiles2, st));
+    TBK_TRY(step_config(Ht, 2 * Rc, prec, &grid2, st, false));
     gmax = std::max(gmax, grid2);
     if (prec == TBK_PREC_DD)
       for (tbk_sparse_s* o : {AL, AR}) if (o) TBK_TRY(ensure_ell_dd(o, st));
@@ -862,28 +863,31 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   struct Fused {
     bool on = false;
     ClassSet32 pair;
-    int grid = 1, tiles = 1;
+    int grid = 1;
   } fused[2];
   for (int h = 0; h < 2 && !both && !f64b; ++h) {
     tbk_sparse_s* Aout = h ? AR : AL;
     Fused& F = fused[h];
     F.grid = grid;
-    F.tiles = n_tiles;
     const bool mixed = prec == TBK_PREC_MIXED;
     if (!Aout || !((flags & TBK_MU_FUSED_OPS) || mixed)) continue;
     bool v_real = false;
     TBK_TRY(same_ell_structure(Ht, Aout, &F.on, st, mixed ? &v_real : nullptr));
     if (F.on && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
     if (F.on && mixed && !v_real) TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
-    if (F.pair.n_cls > 0) TBK_TRY(pair_config(Ht, Rc, F.pair, &F.grid, &F.tiles));
-    else F.on = F.on && ((flags & TBK_MU_FUSED_OPS) || !has_row_classes(Ht, prec));
+    if (F.pair.n_cls > 0) {
+      TBK_TRY(pair_config(Ht, Rc, F.pair, &F.grid));
+    } else {
+      F.on = F.on && ((flags & TBK_MU_FUSED_OPS) || !has_row_classes(Ht, prec));
+      if (F.on) F.grid = grid_op;
+    }
   }
   cudaStream_t q = st;                                   // the stream the side being issued runs on
   auto apply = [&](tbk_sparse_s* A, const void* x, void* y) -> int {   // y = A x
     rec_bytes += 2 * vecb + ell_bytes(A, true);
-    int g, t;
-    TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
-    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, t, q, nullptr, true, nullptr, false);
+    int g;
+    TBK_TRY(step_config(A, Rc, prec, &g, st));
+    return step_any(A, Rc, prec, x, y, nullptr, true, partd.as<double>(), g, q, nullptr, true, nullptr, false);
   };
   const unsigned gblk = (unsigned)std::min<int64_t>((blk + 255) / 256, 65535);
   auto round_to = [&](const void* src, const KStore& ks, int32_t m) -> int {
@@ -915,10 +919,10 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // block m of `store` = A x, written by the product itself (no work block)
   auto apply_to_store = [&](tbk_sparse_s* A, const void* x, void* scratch, KStore ks, int32_t m) -> int {
     rec_bytes += vecb + ell_bytes(A, true) + stb;
-    int g, t;
-    TBK_TRY(step_config(A, Rc, prec, &g, &t, st));
+    int g;
+    TBK_TRY(step_config(A, Rc, prec, &g, st));
     ks.km[0] = m;
-    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, t, q, &ks, false, nullptr, true, nullptr,
+    return step_any(A, Rc, prec, x, scratch, nullptr, true, partd.as<double>(), g, q, &ks, false, nullptr, true, nullptr,
                     zigzag && (m & 1) == 0);
   };
   // one side: store[m] = Aout T_m(H~) (Bin v0), m < M; each step writes its
@@ -954,7 +958,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         if (m == M) break;
         if (m >= 1) {
           rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true);
-          TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, n_tiles, q, nullptr, true, nullptr,
+          TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), grid, q, nullptr, true, nullptr,
                            false));
         }
         if (Aout) TBK_TRY(apply(Aout, y, tmpA));
@@ -970,7 +974,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
                      (fuse ? ell_bytes(Aout, false) : 0.0);
         ks.km[0] = fuse ? m - 1 : m;
-        TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), F.grid, F.tiles, q,
+        TBK_TRY(step_any(Ht, Rc, prec, x, y, pv, m == 1, partd.as<double>(), F.grid, q,
                          fuse || !Aout ? &ks : nullptr, true, fuse ? Aout : nullptr, false,
                          F.pair.n_cls > 0 ? &F.pair : nullptr, zigzag && (m & 1)));
         if (Aout && !fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, m));
@@ -1030,12 +1034,12 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       for (int h = 0; h < 2; ++h) rec_bytes += Aout[h] ? ell_bytes(Aout[h], false) : 0.0;
       for (int h = 0; h < 2; ++h) ks.km[h] = Aout[h] ? m - 1 : m;
       TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(m - 1) & 1], r[m & 1], m >= 2 ? r[m & 1] : nullptr, m == 1,
-                      partd.as<double>(), grid2, tiles2, st, ks));
+                      partd.as<double>(), grid2, st, ks));
     }
     if (AL || AR) {                                      // A T_{M-1} -> block M-1 (the new vector is not kept)
       for (int h = 0; h < 2; ++h) ks.km[h] = Aout[h] ? M - 1 : -1;
       TBK_TRY(step_ks(Ht, 2 * Rc, prec, r[(M - 1) & 1], r[M & 1], M >= 2 ? r[M & 1] : nullptr, M == 1,
-                      partd.as<double>(), grid2, tiles2, st, ks));
+                      partd.as<double>(), grid2, st, ks));
     }
     return TBK_OK;
   };

@@ -223,7 +223,9 @@ struct KStore {
 // or y = 2 H x - pv; moment partials into part[2 * grid].  Block loaders:
 // Eigen-layout kets / seeded random phases.
 int step_width(int prec, int R, int cap);   // chunk width of R vectors
-int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cudaStream_t st);
+// grid of the steps without moment sums; wide: those of step_any without an operator product
+// outside the class form (which may have more threads per CTA)
+int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, cudaStream_t st, bool wide = true);
 // ks: optional K-tiled store that receives the step's output as block km[0]
 // (store_y false: only there)
 // vop: with ks, store vop x instead of the output; vop must share A's ELL
@@ -231,11 +233,11 @@ int step_config(tbk_sparse_s* A, int Rc, int prec, int* grid, int* n_tiles, cuda
 // dots: form the moment partial sums (false: the step only feeds other work)
 // reverse: the tiles from the last to the first (what the pass before left in L2 first)
 int step_any(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-             int grid, int n_tiles, cudaStream_t st, const KStore* ks = nullptr, bool store_y = true,
+             int grid, cudaStream_t st, const KStore* ks = nullptr, bool store_y = true,
              tbk_sparse_s* vop = nullptr, bool dots = true, const ClassSet32* pair = nullptr, bool reverse = false);
-// grid and tiles of a step with an operator product in the joint class form (complex64;
+// grid of a step with an operator product in the joint class form (complex64;
 // pair: pair_classes32 of A and the operator)
-int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid, int* n_tiles);
+int pair_config(tbk_sparse_s* A, int Rc, const ClassSet32& pair, int* grid);
 // whether A's steps in a precision run in the class form (after step_config)
 bool has_row_classes(tbk_sparse_s* A, int prec);
 // ELL value / diagonal arrays of a precision (FP32, FP64 or double-float pairs)
@@ -244,7 +246,7 @@ const void* ell_diag(const EllDev& E, int prec);
 // one recursion step (not the first block's braket form) writing the K-tiled
 // stores described by ks (output or operator products per column group)
 int step_ks(tbk_sparse_s* A, int Rc, int prec, const void* x, void* y, const void* pv, bool first, double* part,
-            int grid, int n_tiles, cudaStream_t st, const KStore& ks, int mode = 2, bool reverse = false);
+            int grid, cudaStream_t st, const KStore& ks, int mode = 2, bool reverse = false);
 // true when B's sliced ELL has A's slices, widths and columns (values may differ)
 // (b_real: B may hold real values where A's are complex; then set)
 int same_ell_structure(tbk_sparse_s* A, tbk_sparse_s* B, bool* same, cudaStream_t st, bool* b_real = nullptr);
