@@ -382,7 +382,9 @@ enum {
   TBK_MU_FUSED_OPS = 8,             /* form the output operator's products inside the
                                        recursion step when it shares H~'s sparsity (as
                                        commutators do): same stored bits, one pass per
-                                       block instead of two; opt-in: the wider step holds
+                                       block instead of two.  Complex64 recursions do so
+                                       by themselves with joint row classes and in the
+                                       ELL form; in double-float the wider step holds
                                        more registers and measured no faster            */
   TBK_MU_BOTH_SIDES = 16,           /* with TBK_MU_FUSED_OPS: run the left and right
                                        recursions as one of twice the width (same bits;

@@ -36,8 +36,8 @@ def kubo_mu(Ht: SparseMatrix, AL=None, BL=None, AR=None, BR=None, M: int = 64, R
     sigma errors are the same as with the wider recursions), "dd" (double-float
     work blocks: FP64-class recursion on the FP32 pipe) or "fp64" (complex128).  fuse_ops:
     form AL / AR products inside the recursion step when they share H~'s
-    sparsity (same stored bits, one pass instead of two; opt-in, measured no
-    faster); both_sides (with fuse_ops): run the two sides as one recursion of
+    sparsity (same stored bits, one pass instead of two; complex64 does so by
+    itself where it is faster); both_sides (with fuse_ops): run the two sides as one recursion of
     twice the width (same bits).  fp64_blocks: the FP64 reference form —
     complex128 stored blocks and an FP64 GEMM (tensor, fuse_ops and both_sides
     are then ignored)."""
