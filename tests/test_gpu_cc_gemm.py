@@ -22,3 +22,18 @@ def test_edges(gpu, M, K):
     mu = tb.mu_from_blocks(L, R, tensor=False)
     err = np.abs(mu - L.conj() @ R.T)
     assert np.all(err <= np.sqrt(2) * np.sqrt(2) * BOUND * (np.abs(L) @ np.abs(R).T))
+
+
+@pytest.mark.parametrize("value", [np.inf, 1e39, 1e25, np.nan])
+def test_infinities(gpu, value):
+    """Infinities, values and products past FP32's range: infinite as their IEEE sums are, the
+    rest of the matrix as without them."""
+    rng = np.random.default_rng(3)
+    L, R = ((np.abs(rng.normal(size=(3, 100))) + 0j) for _ in range(2))
+    ref = L @ R.T
+    L[1, 37] = value
+    R[1, 37] = 1e25
+    mu = tb.mu_from_blocks(L, R, tensor=False)
+    assert np.isnan(mu[1, 1].real) if np.isnan(value) else np.isposinf(mu[1, 1].real)
+    keep = np.ix_([0, 2], [0, 2])
+    assert np.all(np.abs(mu[keep] - ref[keep]) <= 2 * (BOUND + 2.0 ** -23) * ref[keep].real)

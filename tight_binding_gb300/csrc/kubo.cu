@@ -151,8 +151,10 @@ __global__ void __launch_bounds__(256) mu_gemm_cc_kernel(const float2* __restric
       float hr, hm, lr, lm;
       f2_unpack(hi[i][j], hr, hm);
       f2_unpack(lo[i][j], lr, lm);
+      // an infinite sum's second part is NaN: the first alone then
       if (m < M && n < M)
-        part[((int64_t)blockIdx.z * M + m) * M + n] = make_double2((double)hr + (double)lr, (double)hm + (double)lm);
+        part[((int64_t)blockIdx.z * M + m) * M + n] =
+            make_double2(isfinite(hr) ? (double)hr + (double)lr : (double)hr, isfinite(hm) ? (double)hm + (double)lm : (double)hm);
     }
 }
 
