@@ -288,14 +288,38 @@ __global__ void round_cols_kernel(int64_t n_pad, int32_t Rc, int32_t c0, const C
   }
 }
 
-// The scale of an FP16-pair store (split_store.cuh) from n values: a power of two that
-// takes their root mean square to 2^6, or their maximum to 2^13 where that is less.  The
+// The largest row sum of |a_ij| (|re| + |im| of complex entries) of an operator: |A x| is at
+// most that many times |x|, in the maximum and, for a Hermitian or antihermitian A, in the
+// root mean square.  *gain is the FP32 bits of the largest so far (NaN above infinity).
+__global__ void __launch_bounds__(256) operator_gain_kernel(int32_t n, const int32_t* __restrict__ soff,
+                                                            const float* __restrict__ val,
+                                                            const float* __restrict__ diag, int vw,
+                                                            unsigned int* __restrict__ gain) {
+  const int32_t r = blockIdx.x * 256 + threadIdx.x;
+  float sum = 0.f;
+  if (r < n) {
+    const int64_t base = soff[r >> 5] + (r & 31);
+    const int32_t w = (soff[(r >> 5) + 1] - soff[r >> 5]) >> 5;
+    for (int q = 0; q < vw; ++q) {
+      sum += fabsf(diag[(int64_t)vw * r + q]);
+      for (int32_t k = 0; k < w; ++k) sum += fabsf(val[vw * (base + (int64_t)k * 32) + q]);
+    }
+  }
+  const unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(sum));
+  if ((threadIdx.x & 31) == 0 && m != 0u) atomicMax(gain, m);
+}
+
+// The scale of an FP16-pair store (split_store.cuh) of blocks gain x, from the n values of the
+// first x: a power of two that takes gain times their root mean square to 2^6, or gain times
+// their maximum to 2^13 where that is less.  Not from the first block itself: an operator that
+// (nearly) vanishes on the start vectors does not vanish on T_m of them.  gain null: 1.  The
 // last CTA to finish sums the others' partials in a fixed order.
 constexpr int kStatThreads = 256;
 template <typename CT>
 __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __restrict__ src, int64_t n,
                                                                    double* __restrict__ part,
                                                                    unsigned int* __restrict__ count,
+                                                                   const float* __restrict__ gain,
                                                                    float* __restrict__ scale, int* __restrict__ bad) {
   float big = 0.f;
   double sum = 0.0;
@@ -337,8 +361,8 @@ __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __r
   }
   block_reduce();
   if (threadIdx.x == 0) {
-    const double mx = s_big[0], rms = sqrt(s_sum[0] / (2.0 * (double)n));
-    float s = 1.f;
+    const double f = gain ? (double)*gain : 1.0, mx = f * s_big[0], rms = f * sqrt(s_sum[0] / (2.0 * (double)n));
+    float s = 1.f;                                       // zero blocks
     if (!(mx < (double)INFINITY)) *bad = 1;
     else if (mx > 0.0) s = ldexpf(1.f, max(-120, min(120, min(12 - ilogb(mx), 6 - ilogb(rms)))));
     *scale = s;
@@ -637,21 +661,30 @@ int with_block(int prec, const void* p, Fn&& f) {
 // Scratch of split_scale_kernel, the two sides' scales and the flag of values that do
 // not fit.
 struct SplitScales {
-  DevBuf part, words;          // words: scale of the left, of the right side; bad; count of each side
+  DevBuf part, words;          // words: scale of the left, of the right side; bad; count, gain of each side
   int alloc(cudaStream_t st) {
     TBK_TRY(part.alloc(sizeof(double) * 8 * sm_count()));
-    TBK_TRY(words.alloc(5 * sizeof(int)));
+    TBK_TRY(words.alloc(7 * sizeof(int)));
     TBK_CUDA(cudaMemsetAsync(words.p, 0, words.bytes, st));
     return TBK_OK;
   }
   float* scale(int h) const { return words.as<float>() + h; }
   int* bad() const { return words.as<int>() + 2; }
-  // h: the side, each with scratch of its own
+  // the output operator of side h
+  int set_operator(int h, const EllDev& E, cudaStream_t st) const {
+    operator_gain_kernel<<<(E.n_rows + 255) / 256, 256, 0, st>>>(E.n_rows, E.slice_off.as<int32_t>(), E.val32.as<float>(),
+                                                                 E.diag32.as<float>(), E.cplx ? 2 : 1,
+                                                                 words.as<unsigned int>() + 5 + h);
+    TBK_CHECK_LAUNCH();
+    return TBK_OK;
+  }
+  // h: the side, each with scratch of its own; gain: the stored blocks are its operator's products
   template <typename CT>
-  void find(const CT* src, int64_t n, float* out, int h, cudaStream_t st) const {
+  void find(const CT* src, int64_t n, float* out, int h, bool gain, cudaStream_t st) const {
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + kStatThreads - 1) / kStatThreads, 2 * sm_count()));
     split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, part.as<double>() + 4 * h * sm_count(),
-                                                       words.as<unsigned int>() + 3 + h, out, bad());
+                                                       words.as<unsigned int>() + 3 + h,
+                                                       gain ? words.as<float>() + 5 + h : nullptr, out, bad());
   }
 };
 
@@ -822,6 +855,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   TBK_TRY(zero_tail());
   SplitScales sc;
   if (use_tc) TBK_TRY(sc.alloc(st));
+  for (int h = 0; h < 2 && use_tc; ++h)
+    if (h ? AR : AL) TBK_TRY(sc.set_operator(h, (h ? AR : AL)->ell, st));
   TBK_CUDA(cudaMemsetAsync(work.p, 0, work.bytes, st));
   TBK_TRY(macc.alloc(sizeof(double2) * (size_t)M * M));
   TBK_CUDA(cudaMemsetAsync(macc.p, 0, macc.bytes, st));
@@ -901,8 +936,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         round_block_kernel<<<gblk, 256, 0, q>>>(p, ks.store[0], m, M, blk);
     });
   };
-  auto find_scale = [&](const void* src, int h) -> int {
-    return with_block(prec, src, [&](auto p) { sc.find(p, blk, sc.scale(h), h, q); });
+  auto find_scale = [&](const void* src, int h) -> int {   // of a side whose recursion starts from src
+    return with_block(prec, src, [&](auto p) { sc.find(p, blk, sc.scale(h), h, (h ? AR : AL) != nullptr, q); });
   };
   // FP64 reference form: block m of the complex128 store from a work block
   auto store64 = [&](const void* src, void* store, int32_t m) -> int {
@@ -966,11 +1001,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
         if (Aout) TBK_TRY(apply(Aout, y, tmpA));
         TBK_TRY(store64(Aout ? tmpA : y, ks.store[0], m));
       } else if (m == 0) {
-        // block 0; its values set the scale of an FP16-pair store
-        if (use_tc && Aout) TBK_TRY(apply(Aout, y, tmpA));
-        if (use_tc) TBK_TRY(find_scale(Aout ? tmpA : y, h));
+        if (use_tc) TBK_TRY(find_scale(y, h));
         if (!Aout) TBK_TRY(round_to(y, ks, 0));
-        else if (!fuse && use_tc) TBK_TRY(round_to(tmpA, ks, 0));
         else if (!fuse) TBK_TRY(apply_to_store(Aout, y, tmpA, ks, 0));
       } else if (m < M) {
         rec_bytes += (m >= 2 ? 3 : 2) * vecb + ell_bytes(Ht, true) + ((fuse || !Aout) ? stb : 0.0) +
@@ -1012,10 +1044,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     for (int h = 0; h < 2; ++h) {
       if (Bin[h]) TBK_TRY(apply(Bin[h], v0, half[h]));
       else TBK_CUDA(cudaMemcpyAsync(half[h], v0, csz * blk, cudaMemcpyDeviceToDevice, st));
-      if (use_tc) {
-        if (Aout[h]) TBK_TRY(apply(Aout[h], half[h], wblk(2)));
-        TBK_TRY(find_scale(Aout[h] ? wblk(2) : half[h], h));
-      }
+      if (use_tc) TBK_TRY(find_scale(half[h], h));
       TBK_TRY(with_block(prec, half[h], [&](auto p) {
         using CT = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
         pack_cols_kernel<CT><<<gblk, 256, 0, st>>>(n_pad, Rc, h * Rc, p, static_cast<CT*>(r[0]));
@@ -1168,7 +1197,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
         TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K, cudaMemcpyHostToDevice, st));
         if (split) {
           float* s = scales.as<float>() + side * M + m;
-          sc.find(stage.as<const double2>(), K, s, 0, st);
+          sc.find(stage.as<const double2>(), K, s, 0, false, st);
           split_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<__half>(), m, M, K, s, sc.bad());
         } else {
           round_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<float2>(), m, M, K);

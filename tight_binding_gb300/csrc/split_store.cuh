@@ -7,10 +7,12 @@
 // k % 32 (hi) and 32 + k % 32 (lo) of row (k / 32 * 2 + part) * M + m.  8 bytes per value,
 // as a complex64 store; a warp of the recursion writes whole 128-byte lines, and 128
 // consecutive blocks of a part are a contiguous box for TMA.
-// s is a power of two (exact).  FP16 spans 2^-24 .. 65504: s puts the root mean square of
-// the first block near 2^6 and its maximum at 2^13 at most, so later values may grow by
-// 2^10 (2^3 where the first block is one spike), and values down to 2^-9 of the root mean
-// square keep all 22 bits.  Values that do not fit (a recursion outside [-1, 1], infinities,
+// s is a power of two (exact).  FP16 spans 2^-24 .. 65504.  T_m of a matrix with spectrum
+// in [-1, 1] does not grow in the root mean square, so s follows from the start vector x of
+// the recursion and a bound g on what the output operator multiplies by: g times x's root mean
+// square lies near 2^6 and g times its maximum at 2^13 at most.  Later values may grow by 2^10
+// over the former (2^3 over the latter, where x is one spike), and values down to 2^-9 of it
+// keep all 22 bits.  Values that do not fit (a recursion outside [-1, 1], infinities,
 // NaN) set a flag, and the caller forms the chunk from complex64 stores instead.
 #pragma once
 #include <cuda_fp16.h>
