@@ -197,6 +197,10 @@ int tbk_sparse_info(tbk_sparse A, int32_t* rows, int32_t* cols, int64_t* nnz,
  * the matrix does not qualify.  The environment variable TBK_NO_CLASSES=1,
  * read when a matrix is first examined, keeps the ELL form (A/B comparisons). */
 int tbk_sparse_row_classes(tbk_sparse A, int32_t* n_classes, void* stream);
+/* *yes = 1 when A equals its adjoint to rounding (2^-50 of each entry): the
+ * condition for TBK_FLAG_DOUBLING, whose product rule needs T_n(H~) Hermitian.
+ * Columns must be sorted without duplicates; *yes = 0 where they are not. */
+int tbk_sparse_hermitian(tbk_sparse A, int32_t* yes, void* stream);
 /* Copies the CSC arrays to host buffers. */
 int tbk_sparse_download(tbk_sparse A, int32_t* col_ptr, int32_t* row_idx, double* values,
                         void* stream);

@@ -1105,6 +1105,36 @@ int pair_classes32(tbk_sparse_s* A, tbk_sparse_s* B, ClassSet32* out, cudaStream
   return class_set32(A->ell, A->ell.val32.as<float>(), B->ell.val32.as<float>(), out, st);
 }
 
+// Sets *no where A (CSC, sorted without duplicates) differs from its adjoint: one thread per column
+// looks up every entry's mirror image.  Entries that sum several hoppings add them in an order
+// of their own, so a few roundings count as equal; an entry without a mirror must be zero.
+__global__ void hermitian_kernel(int32_t n, const int32_t* __restrict__ cp, const int32_t* __restrict__ ri,
+                                 const double* __restrict__ v, int vw, int* __restrict__ no) {
+  const int32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  for (int32_t p = cp[j]; p < cp[j + 1]; ++p) {
+    const int32_t i = ri[p];
+    bool ok = i >= 0 && i < n && (p == cp[j] || ri[p - 1] < i);
+    if (ok) {
+      int32_t a = cp[i], b = cp[i + 1];
+      const int32_t end = b;
+      while (a < b) {
+        const int32_t m = (a + b) >> 1;
+        if (ri[m] < j) a = m + 1;
+        else b = m;
+      }
+      const bool found = a < end && ri[a] == j;
+      const double re = v[(int64_t)vw * p], im = vw == 2 ? v[(int64_t)vw * p + 1] : 0.0;
+      const double mr = found ? v[(int64_t)vw * a] : 0.0, mi = found && vw == 2 ? v[(int64_t)vw * a + 1] : 0.0;
+      ok = fabs(re - mr) + fabs(im + mi) <= 0x1p-50 * (fabs(re) + fabs(im));
+    }
+    if (!ok) {
+      *no = 1;
+      return;
+    }
+  }
+}
+
 }  // namespace tbk
 
 using namespace tbk;
@@ -1301,6 +1331,27 @@ int tbk_sparse_row_classes(tbk_sparse A, int32_t* n_classes, void* stream) {
   ScratchScope scope(as_stream(stream));
   TBK_TRY(ensure_classes(A, as_stream(stream)));
   *n_classes = A->ell.cls_state == 1 ? A->ell.n_cls : 0;
+  return TBK_OK;
+}
+
+int tbk_sparse_hermitian(tbk_sparse A, int32_t* yes, void* stream) {
+  if (!A || !yes) return fail(TBK_ERR_INVALID, "tbk_sparse_hermitian: null argument");
+  *yes = 0;
+  if (A->rows != A->cols) return TBK_OK;
+  cudaStream_t st = as_stream(stream);
+  ScratchScope scope(st);
+  DevBuf no;
+  TBK_TRY(no.alloc(sizeof(int)));
+  TBK_CUDA(cudaMemsetAsync(no.p, 0, sizeof(int), st));
+  if (A->cols > 0) {
+    hermitian_kernel<<<(A->cols + 127) / 128, 128, 0, st>>>(A->cols, A->col_ptr.as<int32_t>(), A->row_idx.as<int32_t>(),
+                                                            A->values.as<double>(), A->is_complex ? 2 : 1, no.as<int>());
+    TBK_CHECK_LAUNCH();
+  }
+  int h = 1;
+  TBK_CUDA(cudaMemcpyAsync(&h, no.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaStreamSynchronize(st));
+  *yes = h == 0;
   return TBK_OK;
 }
 

@@ -179,11 +179,12 @@ def kernel_seq(N: int, kernel: Kernel) -> np.ndarray:
 
 
 # -------------------------------------------------------------- Green's function
-def _doubles(precision) -> bool:
+def _doubles(Ht: SparseMatrix, precision) -> bool:
     """Whether moments of equal bras and kets come from half the steps by the product
     rule.  Not in complex64: mu_2n = 2 <v_n|v_n> - mu_0 carries the single-precision
-    sums' error of mu_0, <b|v_n> only that of the small moment itself."""
-    return _prec(precision) != capi.PREC_MIXED
+    sums' error of mu_0, <b|v_n> only that of the small moment itself.  Nor for a matrix
+    that is not Hermitian (a complex on-site energy): <v_n|v_n> is <v| T_n^+ T_n |v>."""
+    return _prec(precision) != capi.PREC_MIXED and Ht.is_hermitian()
 
 
 class GreenFunctionImag:
@@ -195,7 +196,7 @@ class GreenFunctionImag:
         same = bras is kets
         K = _block(kets, n)
         B = K if same else _block(bras, n)
-        solver = KpmSolver(G.scaled_HE, K.shape[1], precision=precision, doubling=same and _doubles(precision))
+        solver = KpmSolver(G.scaled_HE, K.shape[1], precision=precision, doubling=same and _doubles(G.scaled_HE, precision))
         self._finish(solver.run(G.N, B, K), kernel)
 
     @classmethod
@@ -204,7 +205,7 @@ class GreenFunctionImag:
         device: the vectors of bases_of_uniform_ampl_with_random_phases(n, R, seed)."""
         self = object.__new__(cls)
         self.G = G
-        solver = KpmSolver(G.scaled_HE, R, precision=precision, doubling=_doubles(precision))
+        solver = KpmSolver(G.scaled_HE, R, precision=precision, doubling=_doubles(G.scaled_HE, precision))
         self._finish(solver.run_random(G.N, seed), kernel)
         return self
 

@@ -78,6 +78,12 @@ class SparseMatrix:
         check(lib().tbk_sparse_row_classes(self._h, C.byref(n), None))
         return n.value
 
+    def is_hermitian(self) -> bool:
+        """Whether the matrix equals its adjoint (to 2^-50 of each entry)."""
+        y = C.c_int32()
+        check(lib().tbk_sparse_hermitian(self._h, C.byref(y), None))
+        return y.value != 0
+
     def nonZeros(self) -> int:  # Eigen spelling
         return self.nnz
 
