@@ -313,9 +313,10 @@ int tbk_cheb_braket_complex(int32_t n_rows, int64_t nnz, const int32_t* col_ptr,
  * library's workspace pool keeps on the current device (at most 256 MB; no
  * counterpart in the reference, which keeps nothing between calls). */
 void tbk_cheb_braket_release(void);
-/* Polls a bounded device wait of the TMA-staged step kernel (TBK_FLAG_STAGED)
- * makes before it gives up, records an error and lets the call return
- * TBK_ERR_TIMEOUT; polls < 0 restores the default (2^24), 0 gives up at once.
+/* Polls a bounded device wait of the TMA-staged step kernel (TBK_FLAG_STAGED) and
+ * of the cooperative recursion of small single-chunk plans makes before it gives
+ * up, records an error and lets the call return TBK_ERR_TIMEOUT; polls < 0 restores
+ * the default (2^24), 0 gives up at once.
  * No counterpart in the reference (its kernels have no waits): it exists so a
  * test can drive the failure path without hanging the GPU.  Copies already in
  * flight are always waited for with the default limit. */

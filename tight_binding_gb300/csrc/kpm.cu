@@ -144,7 +144,8 @@ __global__ void assemble_moments_kernel(const double* __restrict__ sums, int32_t
 
 
 constexpr int kTmaStages = 4;
-// polls of the staged kernel's ring waits before they give up (tbk_set_wait_limit)
+// polls of the staged kernel's ring waits and the cooperative recursion's meetings before they
+// give up (tbk_set_wait_limit)
 std::atomic<uint32_t> g_wait_limit{kWaitLimit};
 
 template <typename F, int R, bool CPLX_H, bool BRAKET>
@@ -887,7 +888,7 @@ static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* pa
   void *va = P->va.p, *vb = P->vb.p, *br = braket ? P->bras.p : nullptr;
   unsigned int* meet = P->meet.as<unsigned int>();
   int* err = P->err.as<int>();
-  uint32_t lim = kWaitLimit;
+  uint32_t lim = g_wait_limit.load(std::memory_order_relaxed);
   void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &meet, &err, &lim};
   TBK_CUDA(cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st));
   return TBK_OK;
