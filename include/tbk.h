@@ -63,11 +63,12 @@ enum {
                                      over memory (temporal blocking; 1/3 less DRAM
                                      traffic, but the gathers are latency-bound on
                                      GB300 and it measures slower, so opt-in)     */
-  TBK_FLAG_NO_GRAPH = 1 << 9,     /* never replay the recursion as a CUDA graph
-                                     (single-chunk plans too large for the cooperative
-                                     recursion and of at most 64 MiB a block capture
-                                     their launch sequence on the second identical
-                                     run) */
+  TBK_FLAG_NO_GRAPH = 1 << 9,     /* one launch per recursion step.  Otherwise small
+                                     single-chunk plans run in one cooperative
+                                     launch (the same bits), and larger ones of at
+                                     most 64 MiB a block capture their launch
+                                     sequence as a CUDA graph on the second
+                                     identical run                                */
   TBK_FLAG_PERSISTENT = 1 << 10,  /* small single-chunk plans: the whole recursion
                                      in one launch.  Complex64 vectors of an H~
                                      with row classes that fit one SM: one CTA

@@ -858,7 +858,7 @@ static int plan_persist(tbk_kpm_s* P) {
   P->persist = -1;
   const bool lanes = P->prec == TBK_PREC_FP64 || P->Rc % 2 == 0;
   if (P->n_chunks != 1 || !lanes || P->n_tiles != P->grid ||
-      (P->flags & (TBK_FLAG_STAGED | TBK_FLAG_TWO_STEP | TBK_FLAG_PERSISTENT)))
+      (P->flags & (TBK_FLAG_STAGED | TBK_FLAG_TWO_STEP | TBK_FLAG_PERSISTENT | TBK_FLAG_NO_GRAPH)))
     return TBK_OK;
   const size_t smem = P->use_cls ? class_smem(P->H->ell, P->prec) : 0;
   for (int b = 0; b < 2; ++b) {
@@ -889,7 +889,9 @@ static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* pa
   unsigned int* meet = P->meet.as<unsigned int>();
   int* err = P->err.as<int>();
   uint32_t lim = g_wait_limit.load(std::memory_order_relaxed);
-  void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &meet, &err, &lim};
+  int zigzag = (P->flags & TBK_FLAG_NO_L2_ZIGZAG) ? 0 : 1;
+  void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &zigzag, &meet, &err,
+                  &lim};
   TBK_CUDA(cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st));
   return TBK_OK;
 }
