@@ -875,7 +875,8 @@ static int plan_persist(tbk_kpm_s* P) {
   return TBK_OK;
 }
 
-static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* part, cudaStream_t st) {
+// *launched false: the stream has fewer SMs than the plan counted on (a green context)
+static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* part, cudaStream_t st, bool* launched) {
   const EllDev& E = P->H->ell;
   const ClassTab ct = class_tab(E, P->prec);
   const size_t smem = P->use_cls ? class_smem(E, P->prec) : 0;
@@ -892,7 +893,10 @@ static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* pa
   int zigzag = (P->flags & TBK_FLAG_NO_L2_ZIGZAG) ? 0 : 1;
   void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &zigzag, &meet, &err,
                   &lim};
-  TBK_CUDA(cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st));
+  const cudaError_t e = cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st);
+  *launched = e == cudaSuccess;
+  if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();
+  else TBK_CUDA(e);
   return TBK_OK;
 }
 
@@ -985,13 +989,15 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
     };
     const bool graphable = P->n_chunks == 1 && s == 0 && !tma && !(P->flags & TBK_FLAG_NO_GRAPH) &&
                            P->va.bytes <= kGraphBlockBytes;
+    bool issued = small;
     if (small) {
       TBK_TRY(launch_small(P, braket, n_steps, st));
       launches += 1;
     } else if (P->persist == 1 && (int64_t)n_steps * P->grid < (int64_t)INT32_MAX) {
-      TBK_TRY(launch_persist(P, braket, n_steps, P->part.as<double>(), st));
-      launches += n_steps;
-    } else if (graphable) {
+      TBK_TRY(launch_persist(P, braket, n_steps, P->part.as<double>(), st, &issued));
+      launches += issued ? n_steps : 0;
+    }
+    if (!issued && graphable) {
       tbk_kpm_s::GraphKey key;
       key.n_steps = n_steps;
       key.braket = braket;
@@ -1032,7 +1038,7 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
         TBK_TRY(issue(st, 0, x, y));
         launches += n_steps;
       }
-    } else {
+    } else if (!issued) {
       TBK_TRY(issue(st, s, x, y));
       launches += n_steps - s;
     }
