@@ -11,6 +11,7 @@
 // distance of the Ritz value.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "host_model.h"
@@ -27,6 +28,8 @@ namespace {
 //   w       = H u_j                          partial sums of <u_j|w>
 //   u_(j+1) = w / b_j - (alpha_j / b_j) u_j - (b_j / b_(j-1)) u_(j-1),
 //             alpha_j = <u_j|w> / b_j^2      partial sums of |u_(j+1)|^2
+// b_j has the size of H's entries, <u_j|w> that of their cube: entries far from 1 are brought
+// near it by a power of two in the update's coefficients (lz_scale), which costs nothing per row.
 // Each CTA of the update sums both sets of partials itself (fixed order, the same
 // value in every CTA).  GB300 starts one FP64 warp instruction every 64 clocks on
 // each quarter of an SM, so the kernels count FP64 instructions: 10 and 6 FMAs per
@@ -37,6 +40,26 @@ namespace {
 // round trips (48 us) per iteration; 10.7 ms now (22 + 21 us).
 constexpr int kLzThreads = 512;
 constexpr int kLzWarps = kLzThreads / 32;
+
+// Power of two for H from the upper word of its largest |entry|: 1 within 2^-200 .. 2^200
+__host__ __device__ inline int lz_scale_exponent(uint32_t top) {
+  const int e = (int)(top >> 20) - 1023;
+  if (top == 0u || e == 1024 || (e >= -200 && e <= 200)) return 0;    // zero matrix; infinities, NaN
+  return e < 0 ? (e < -1000 ? 1000 : -e) : -e < -1000 ? -1000 : -e;
+}
+__global__ void __launch_bounds__(kLzThreads) lanczos_max_kernel(const double* __restrict__ v, int64_t n,
+                                                                 uint32_t* __restrict__ top) {
+  __shared__ uint32_t sh;
+  if (threadIdx.x == 0) sh = 0;
+  __syncthreads();
+  uint32_t m = 0;
+  for (int64_t i = (int64_t)blockIdx.x * kLzThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kLzThreads)
+    m = max(m, (uint32_t)__double2hiint(v[i]) & 0x7fffffffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sh, m);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(top, sh);
+}
 
 __device__ __forceinline__ double lz_warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -128,12 +151,12 @@ __global__ void __launch_bounds__(kLzThreads) lanczos_product_kernel(
   if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
 
-// u_(j+1) over w; scal[2 j] = alpha_j, scal[2 j + 1] = b_j.  pnorm: |u_j|^2 partials of
-// the update before (j > 0).
+// u_(j+1) over w; scal[2 j] = alpha_j, scal[2 j + 1] = b_j, of H times its power of two (top).
+// pnorm: |u_j|^2 partials of the update before (j > 0).
 __global__ void __launch_bounds__(kLzThreads) lanczos_update_kernel(
     int32_t n, int32_t j, double2* __restrict__ w, const double2* __restrict__ u, const double2* __restrict__ up,
     const double* __restrict__ pdot, const double* __restrict__ pnorm, double* __restrict__ onorm,
-    double* __restrict__ scal) {
+    double* __restrict__ scal, const uint32_t* __restrict__ top) {
   __shared__ double sh[kLzWarps], sdot, snorm, coef[3];
   const int warp = threadIdx.x >> 5;
   if (warp == 0) {
@@ -145,8 +168,9 @@ __global__ void __launch_bounds__(kLzThreads) lanczos_update_kernel(
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    const double b = sqrt(snorm), inv = 1.0 / b, alpha = sdot * inv * inv;
-    coef[0] = inv;
+    const double f = __hiloint2double((1023 + lz_scale_exponent(*top)) << 20, 0);
+    const double b = sqrt(snorm), inv = 1.0 / b, alpha = sdot * f * inv * inv;
+    coef[0] = inv * f;
     coef[1] = -alpha * inv;
     coef[2] = j > 0 ? -b / scal[2 * j - 1] : 0.0;
     if (blockIdx.x == 0) {
@@ -256,7 +280,13 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kLzThreads - 1) / kLzThreads, 2 * sm_count()));
   TBK_TRY(part.alloc(sizeof(double) * grid));
   TBK_TRY(upart.alloc(sizeof(double) * 2 * grid));
-  TBK_TRY(scal.alloc(sizeof(double) * (2 * (size_t)k_max + 1)));
+  TBK_TRY(scal.alloc(sizeof(double) * (2 * (size_t)k_max + 2)));   // the scalars, b_k, the largest entry
+  uint32_t* top = reinterpret_cast<uint32_t*>(scal.as<double>() + 2 * (size_t)k_max + 1);
+  TBK_CUDA(cudaMemsetAsync(top, 0, sizeof(double), st));
+  const int64_t words = A->nnz * (A->is_complex ? 2 : 1);
+  lanczos_max_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((words + kLzThreads - 1) / kLzThreads, 2 * sm_count())),
+                       kLzThreads, 0, st>>>(A->values.as<double>(), words, top);
+  TBK_CHECK_LAUNCH();
   double2* v = vb[0].as<double2>();      // u_j
   double2* vp = vb[1].as<double2>();     // u_(j-1)
   double2* w = vb[2].as<double2>();
@@ -269,7 +299,8 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
                         : lanczos_product<false, false>(E, ct, v, w, part.as<double>(), grid, st)));
     double* in = upart.as<double>() + (j & 1) * grid;
     double* out = upart.as<double>() + ((j + 1) & 1) * grid;
-    lanczos_update_kernel<<<grid, kLzThreads, 0, st>>>(n, j, w, v, vp, part.as<double>(), in, out, scal.as<double>());
+    lanczos_update_kernel<<<grid, kLzThreads, 0, st>>>(n, j, w, v, vp, part.as<double>(), in, out, scal.as<double>(),
+                                                       top);
     TBK_CHECK_LAUNCH();
     double2* t = vp;
     vp = v;
@@ -279,9 +310,13 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
   lanczos_norm_kernel<<<1, 32, 0, st>>>(upart.as<double>() + (k_max & 1) * grid, grid,
                                                scal.as<double>() + 2 * (size_t)k_max);
   TBK_CHECK_LAUNCH();
-  std::vector<double> hs(2 * (size_t)k_max + 1);
+  std::vector<double> hs(2 * (size_t)k_max + 2);
   TBK_CUDA(cudaMemcpyAsync(hs.data(), scal.p, sizeof(double) * hs.size(), cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
+  uint32_t htop;
+  std::memcpy(&htop, &hs.back(), sizeof(htop));
+  if (const int e = lz_scale_exponent(htop))
+    for (double& x : hs) x = std::ldexp(x, -e);
   // T = tridiag(beta, alpha, beta); an invariant subspace (a vanishing norm) ends the
   // recursion there: the scalars after it are not used
   std::vector<double> alpha, beta;
