@@ -280,8 +280,9 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kLzThreads - 1) / kLzThreads, 2 * sm_count()));
   TBK_TRY(part.alloc(sizeof(double) * grid));
   TBK_TRY(upart.alloc(sizeof(double) * 2 * grid));
-  TBK_TRY(scal.alloc(sizeof(double) * (2 * (size_t)k_max + 2)));   // the scalars, b_k, the largest entry
-  uint32_t* top = reinterpret_cast<uint32_t*>(scal.as<double>() + 2 * (size_t)k_max + 1);
+  TBK_TRY(scal.alloc(sizeof(double) * (2 * (size_t)k_max + 2)));   // the largest entry, b_k, then the scalars
+  uint32_t* top = scal.as<uint32_t>();
+  double* ab = scal.as<double>() + 2;
   TBK_CUDA(cudaMemsetAsync(top, 0, sizeof(double), st));
   const int64_t words = A->nnz * (A->is_complex ? 2 : 1);
   lanczos_max_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((words + kLzThreads - 1) / kLzThreads, 2 * sm_count())),
@@ -292,39 +293,55 @@ int tbk_spectral_range(tbk_sparse A, int32_t iters, uint64_t seed, double* e_min
   double2* w = vb[2].as<double2>();
   // u_0: the seeded random phases (unit norm)
   TBK_TRY(random_block_any(TBK_PREC_FP64, n, 1, 0, 1, seed, v, st));
-  for (int32_t j = 0; j < k_max; ++j) {
+  // the scalars of k iterations, without H's power of two
+  std::vector<double> hs;
+  auto read = [&](int32_t k) -> int {
+    hs.resize(2 * (size_t)k + 2);
+    TBK_CUDA(cudaMemcpyAsync(hs.data(), scal.p, sizeof(double) * hs.size(), cudaMemcpyDeviceToHost, st));
+    TBK_CUDA(cudaStreamSynchronize(st));
+    uint32_t h;
+    std::memcpy(&h, hs.data(), sizeof(h));
+    if (const int e = lz_scale_exponent(h))
+      for (double& x : hs) x = std::ldexp(x, -e);
+    return TBK_OK;
+  };
+  // A vanishing norm after iteration j: an invariant subspace, the scalars after it are not used
+  auto ends = [&](int32_t j) { return !(hs[2 * j + 5] > 1e-13 * std::max(1.0, std::fabs(hs[2 * j + 2]))); };
+  // Looked for after 4, 16, 64 ... iterations (a read-back of some 15 us each), so that a matrix
+  // of few distinct eigenvalues does not run all of them
+  int32_t k_run = 0;
+  for (int32_t look = 4; k_run < k_max; ++k_run) {
+    const int32_t j = k_run;
+    if (j == look) {
+      TBK_TRY(read(j));
+      bool done = false;
+      for (int32_t i = 0; i + 1 < j && !done; ++i) done = ends(i);
+      if (done) break;
+      look = look > INT32_MAX / 4 ? INT32_MAX : 4 * look;
+    }
     TBK_TRY(cplx ? (cls ? lanczos_product<true, true>(E, ct, v, w, part.as<double>(), grid, st)
                         : lanczos_product<true, false>(E, ct, v, w, part.as<double>(), grid, st))
                  : (cls ? lanczos_product<false, true>(E, ct, v, w, part.as<double>(), grid, st)
                         : lanczos_product<false, false>(E, ct, v, w, part.as<double>(), grid, st)));
     double* in = upart.as<double>() + (j & 1) * grid;
     double* out = upart.as<double>() + ((j + 1) & 1) * grid;
-    lanczos_update_kernel<<<grid, kLzThreads, 0, st>>>(n, j, w, v, vp, part.as<double>(), in, out, scal.as<double>(),
-                                                       top);
+    lanczos_update_kernel<<<grid, kLzThreads, 0, st>>>(n, j, w, v, vp, part.as<double>(), in, out, ab, top);
     TBK_CHECK_LAUNCH();
     double2* t = vp;
     vp = v;
     v = w;
     w = t;
   }
-  lanczos_norm_kernel<<<1, 32, 0, st>>>(upart.as<double>() + (k_max & 1) * grid, grid,
-                                               scal.as<double>() + 2 * (size_t)k_max);
+  lanczos_norm_kernel<<<1, 32, 0, st>>>(upart.as<double>() + (k_run & 1) * grid, grid, scal.as<double>() + 1);
   TBK_CHECK_LAUNCH();
-  std::vector<double> hs(2 * (size_t)k_max + 2);
-  TBK_CUDA(cudaMemcpyAsync(hs.data(), scal.p, sizeof(double) * hs.size(), cudaMemcpyDeviceToHost, st));
-  TBK_CUDA(cudaStreamSynchronize(st));
-  uint32_t htop;
-  std::memcpy(&htop, &hs.back(), sizeof(htop));
-  if (const int e = lz_scale_exponent(htop))
-    for (double& x : hs) x = std::ldexp(x, -e);
-  // T = tridiag(beta, alpha, beta); an invariant subspace (a vanishing norm) ends the
-  // recursion there: the scalars after it are not used
+  TBK_TRY(read(k_run));
+  // T = tridiag(beta, alpha, beta)
   std::vector<double> alpha, beta;
   double bprev = 0.0;
-  for (int32_t j = 0; j < k_max; ++j) {
-    alpha.push_back(hs[2 * j]);
-    bprev = j + 1 < k_max ? hs[2 * j + 3] : hs[2 * (size_t)k_max];
-    if (j + 1 == k_max || !(bprev > 1e-13 * std::max(1.0, std::fabs(alpha.back())))) break;
+  for (int32_t j = 0; j < k_run; ++j) {
+    alpha.push_back(hs[2 * j + 2]);
+    bprev = j + 1 < k_run ? hs[2 * j + 5] : hs[1];
+    if (j + 1 == k_run || ends(j)) break;
     beta.push_back(bprev);
   }
   // extreme Ritz values of T_k (Gershgorin interval for the bisection)
