@@ -29,13 +29,18 @@
 //              need, and 128 x 128 complex float-float pairs would fill the register file.
 // What bounds it: shared memory, and the power cap on long runs.  The MMAs of 16 k read 3
 // x (12 + 16) KB and the TMA writes 32 KB in the 768 clocks of the 12 products at full
-// rate, 151 bytes a clock against 128.  FCC 128^3, M = 1024, R = 8: 286 ms, 1,478 TFLOP/s of
-// issued products, 76% of cuBLAS' bf16 burst rate and 86% of its sustained rate (641 ms
+// rate, 151 bytes a clock against 128.  FCC 128^3, M = 1024, R = 8: 268 ms, 1,578 TFLOP/s of
+// issued products, 81% of cuBLAS' bf16 burst rate and 92% of its sustained rate (638 ms
 // with complex64 stores split into TF32 pairs by converter warps, 70% of the TF32 rate;
 // 410 ms with a row-major partial tile, whose flush held the accumulators up); square
-// 256^2, M = 512, R = 16: 10.0 -> 3.9 ms.  Error against 64 bits of the latter's mu_nm
-// 1.2e-6 (2-norm; 2.0e-6 before: FP16 products take 16 k at a time, so a chunk of 128 k is
-// half as many FP32 accumulations).
+// 256^2, M = 512, R = 16: 10.2 -> 4.2 ms.
+// Error against 64 bits, relative to the largest |L_m||R_n|: K = 2^21 and 2^22, M = 2: 1.5e-6 for
+// equal blocks (2.2e-6 with the TF32 pairs, whose chunk sums went into float-float pairs: FP16
+// products take 16 k at a time, so a chunk of 128 k is half as many FP32 accumulations),
+// 1.6e-6 where the amplitude grows by e^12 along k (2.4e-6), 5.6e-7 for positive ones
+// (1.4e-6); 1.6e-6, 1.7e-6 and 6e-7 at M = 1024, K = 2^16 (2.3e-6, 2.4e-6, 1.5e-6).  The FP32 register
+// sum is some twentieth of that: with kFlush = 16, 8, 4 the errors are within 6% of these,
+// and the GEMM takes 8, 29, 80% longer (square 256^2: 10, 31, 75%).
 // Every mbarrier wait is bounded; on timeout the CTA records an error, waits
 // (bounded) for its copies and MMAs in flight and frees its tensor memory.
 #include <cuda.h>
