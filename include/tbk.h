@@ -425,7 +425,9 @@ int tbk_kubo_release(void);
  * stream): building the stored blocks, the mu GEMM (+ split-K reduction), the
  * real flops of the GEMM products issued (3 split-FP16 terms on the tensor
  * path), the algorithmic DRAM bytes of the block phase (work vectors read and
- * written, matrix per pass, complex64 stores), and the number of vector chunks. */
+ * written, matrix per pass, stores), and the number of vector chunks.  Where a
+ * tensor GEMM is discarded because values left FP16's range, its time counts in
+ * neither phase and the blocks, built again, count twice. */
 int tbk_kubo_last_timing(double* ms_blocks, double* ms_gemm, double* gemm_flops, double* block_bytes,
                          int32_t* chunks);
 /* mu_mn = sum_k conj(L_m[k]) R_n[k] for given blocks (host, M x K complex128

@@ -1123,8 +1123,13 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
       TBK_TRY(mu_gemm_tc(L, R_, M, blk, macc.as<double>(), &usable, st));
       if (!usable) {                                     // values past FP16's range: complex64 stores from here on
         use_tc = false;
+        float ms = 0.f;                                  // the blocks count twice, the GEMM so far not
+        TBK_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+        tm.ms_blocks += ms;
+        TBK_CUDA(cudaEventRecord(ev[0], st));
         TBK_TRY(zero_tail());
         TBK_TRY(blocks());
+        TBK_CUDA(cudaEventRecord(ev[1], st));
       }
     }
     if (!use_tc && !f64b)
@@ -1220,6 +1225,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
       TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
       TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
       TBK_TRY(upload(false));
+      TBK_CUDA(cudaEventRecord(ev[0], st));
     }
   }
   if (!formed) TBK_TRY(mu_gemm_cc(Ld.as<float2>(), Rd.as<float2>(), M, K, &part, acc.as<double2>(), st));
@@ -1231,7 +1237,7 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   for (auto& e : ev) cudaEventDestroy(e);
   KuboTiming tm;
   tm.ms_gemm = ms;
-  tm.gemm_flops = 8.0 * M * (double)M * (double)K * ((flags & TBK_MU_TENSOR) ? 3.0 : 1.0);
+  tm.gemm_flops = 8.0 * M * (double)M * (double)K * (formed ? 3.0 : 1.0);
   tm.block_bytes = 2.0 * M * (double)K * 8.0;
   tm.chunks = 1;
   {
