@@ -93,8 +93,18 @@ __global__ void green_imag_kernel(int n, const double* __restrict__ g, const dou
   dc z2 = cmul(zz, zz);
   dc s1 = csqrt_p({1.0 - z2.r, 0.0 - z2.i});
   dc s2 = {zz.r + s1.i, zz.i - s1.r};              // z - i s1
-  const dc f = cmul(cdiv({0.0, -2.0}, s1), series_sum(n, g, mu, s2));
-  if (k < nz && threadIdx.x % kSeriesLanes == 0) out[k] = scale * f.i;
+  double f = cmul(cdiv({0.0, -2.0}, s1), series_sum(n, g, mu, s2)).i;
+  // far outside [-1, 1] the powers up to w^max(n, 15) leave the range where alpha_n itself may
+  // not: term by term there
+  if (0.5f * log2f((float)(s2.r * s2.r + s2.i * s2.i)) * (float)max(n, kSeriesLanes) > 1000.f) {
+    dc sn = cdiv({0.0, -2.0}, s1);
+    f = g[0] * cdiv({0.0, -1.0}, s1).i * mu[0];
+    for (int m = 1; m < n; ++m) {
+      sn = cmul(sn, s2);
+      f += g[m] * sn.i * mu[m];
+    }
+  }
+  if (k < nz && threadIdx.x % kSeriesLanes == 0) out[k] = scale * f;
 }
 
 // DCT-III (REDFT01) of g*mu at x_k = cos((k+1/2) pi / N), times 1/sqrt(1-x^2).
