@@ -98,23 +98,26 @@ struct DevBuf {
   int alloc(size_t n) {
     release();
     if (n == 0) n = 16;
-    cudaError_t e = cudaErrorMemoryAllocation;
     const AsyncAllocCtx* c = tl_async_alloc;
-    if (c && (!c->scratch || n <= kScratchMax)) {
-      e = cudaMallocFromPoolAsync(&p, n, c->pool, c->stream);
-      if (e == cudaSuccess) {
-        if (c->scratch) scratch = true;
-        else ctx = c;
-      }
-    }
-    if (e != cudaSuccess && (!c || c->scratch)) {
-      cudaGetLastError();
-      e = cudaMalloc(&p, n);
-      if (e == cudaErrorMemoryAllocation) {        // what the pool keeps may be what is missing
+    auto attempt = [&]() -> cudaError_t {
+      if (c && (!c->scratch || n <= kScratchMax)) {
+        const cudaError_t e = cudaMallocFromPoolAsync(&p, n, c->pool, c->stream);
+        if (e == cudaSuccess) {
+          if (c->scratch) scratch = true;
+          else ctx = c;
+          return e;
+        }
         cudaGetLastError();
-        scratch_trim();
-        e = cudaMalloc(&p, n);
+        if (!c->scratch) return e;
       }
+      const cudaError_t e = cudaMalloc(&p, n);
+      if (e != cudaSuccess) cudaGetLastError();
+      return e;
+    };
+    cudaError_t e = attempt();
+    if (e == cudaErrorMemoryAllocation) {          // what the library's pool keeps may be what is missing
+      scratch_trim();
+      e = attempt();
     }
     if (e != cudaSuccess) { p = nullptr; return fail(TBK_ERR_NOMEM, "device allocation of %zu bytes: %s", n, cudaGetErrorString(e)); }
     bytes = n;
