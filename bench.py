@@ -496,13 +496,18 @@ def run_gpu(args):
         "parity": {"mixed_vs_fp64_rel_err_first_%d_moments" % m64: mixed_vs_fp64, "e2e_vs_resident_rel": e2e_err,
                    "full": full_parity},
     }
-    if not args.no_configs:
-        line["configs"] = other_configs(args)
+    line.update(configs_record(args, ws))
     print(json.dumps(line), flush=True)
     if ws > 1:
         dist.barrier()
         dist.destroy_process_group()
     return 0
+
+
+def configs_record(args, ws):
+    """{"configs": other_configs()} of a one-GPU job.  Not of a larger one: the Kubo legs' GEMM
+    loads with cluster multicast, which runs on one GPU only take."""
+    return {} if args.no_configs or ws > 1 else {"configs": other_configs(args)}
 
 
 def other_configs(args):
