@@ -197,6 +197,7 @@ kpm_step_kernel(
   Acc m0 = 0, m1 = 0;
   constexpr bool FOLD = kFoldStep<F> && !FIRST;
   static_assert(!(CLS && PIPE), "class form: no column pipeline");
+  static_assert(!(CLS && KST == 2 && sizeof(F) != 4), "class form: operator products in FP32 only");
 
   // class form: the table in shared memory (4-byte words: values, offsets, counts)
   extern __shared__ __align__(16) unsigned char cls_smem[];
@@ -336,9 +337,9 @@ kpm_step_kernel(
       // the table read four entries at a time where the launch bound leaves registers
       // for it (FCC 64^3 Kubo blocks 8.8 -> 8.1 us; the moments step spills: honeycomb
       // 1024^2, R = 32: 242 -> 277)
-      constexpr bool VEC = KST == 2;
+      constexpr bool VEC = CLS && KST == 2;
       int k0 = 0;
-      if constexpr (is_f64<F> && KST != 2) {
+      if constexpr (is_f64<F>) {
         // FP64: whole groups, then single entries (a predicated product still
         // takes its turn on the FP64 pipe)
         for (; k0 + 4 <= cnt; k0 += 4) {
@@ -356,7 +357,7 @@ kpm_step_kernel(
       for (int k = k0; k < cnt; k += 4) {
         HVal<F, CPLX_H> h[4];
         LaneV<F, VPL> xv[4];
-        if constexpr (WHOLE && VEC) {
+        if constexpr (VEC) {
           const int4 o = *reinterpret_cast<const int4*>(s_off + tb + k);
           xv[0] = nb(clamp(r + o.x));
           xv[1] = nb(clamp(r + o.y));
@@ -379,16 +380,10 @@ kpm_step_kernel(
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], acc);
-        if constexpr (KST == 2) {
-          if constexpr (WHOLE && VEC) {
-            load_smem4<CPLX_H>(s_val2, tb + k, h);
+        if constexpr (VEC) {
+          load_smem4<CPLX_H>(s_val2, tb + k, h);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], vacc);
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (WHOLE || k + u < cnt) HVal<F, CPLX_H>::load_smem(s_val2, tb + k + u).template fma<VPL>(xv[u], vacc);
-          }
+          for (int u = 0; u < 4; ++u) h[u].template fma<VPL>(xv[u], vacc);
         }
       }
     } else if (gather) {
@@ -577,8 +572,12 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
     } else if (a.kst == 5) {
       if (first) TBK_STEP(true, false, 5); else TBK_STEP(false, false, 5);
     } else if (a.kst == 2) {
-      if (CLS && !a.ct.val2) return fail(TBK_ERR_UNSUPPORTED, "operator product without its class values");
-      if (first) TBK_STEP(true, false, 2); else TBK_STEP(false, false, 2);
+      if constexpr (CLS && sizeof(F) != 4) {
+        return fail(TBK_ERR_UNSUPPORTED, "operator products in the class form are complex64");
+      } else {
+        if (CLS && !a.ct.val2) return fail(TBK_ERR_UNSUPPORTED, "operator product without its class values");
+        if (first) TBK_STEP(true, false, 2); else TBK_STEP(false, false, 2);
+      }
     }
     else { if (first) TBK_STEP(true, false, 1); else TBK_STEP(false, false, 1); }
   } else if (first) { if (braket) TBK_STEP(true, true, 0); else TBK_STEP(true, false, 0); }
