@@ -259,9 +259,12 @@ __global__ void store_block64_kernel(const CT* __restrict__ src, double2* __rest
 __device__ __forceinline__ float2 to_c64(double2 v) { return make_float2(__double2float_rn(v.x), __double2float_rn(v.y)); }
 __device__ __forceinline__ float2 to_c64(float2 v) { return v; }
 __device__ __forceinline__ float2 to_c64(dd2 v) { return make_float2(__fadd_rn(v.x.hi, v.x.lo), __fadd_rn(v.y.hi, v.y.lo)); }
+// (blockIdx.y: several blocks of n values in a row)
 template <typename CT>
 __global__ void round_block_kernel(const CT* __restrict__ src, float2* __restrict__ store, int32_t m, int32_t M,
                                    int64_t n) {
+  src += blockIdx.y * n;
+  m += blockIdx.y;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     store[((q >> 4) * M + m) * 16 + (q & 15)] = to_c64(src[q]);
 }
@@ -313,7 +316,8 @@ __global__ void __launch_bounds__(256) operator_gain_kernel(int32_t n, const int
 // first x: a power of two that takes gain times their root mean square to 2^6, or gain times
 // their maximum to 2^13 where that is less.  Not from the first block itself: an operator that
 // (nearly) vanishes on the start vectors does not vanish on T_m of them.  gain null: 1.  The
-// last CTA to finish sums the others' partials in a fixed order.
+// last CTA to finish sums the others' partials in a fixed order.  (blockIdx.y: several blocks of n
+// values in a row, each with a scale, partials and a counter of its own.)
 constexpr int kStatThreads = 256;
 template <typename CT>
 __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __restrict__ src, int64_t n,
@@ -321,6 +325,10 @@ __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __r
                                                                    unsigned int* __restrict__ count,
                                                                    const float* __restrict__ gain,
                                                                    float* __restrict__ scale, int* __restrict__ bad) {
+  src += blockIdx.y * n;
+  part += 2 * (int64_t)blockIdx.y * gridDim.x;
+  count += blockIdx.y;
+  scale += blockIdx.y;
   float big = 0.f;
   double sum = 0.0;
   for (int64_t q = (int64_t)blockIdx.x * kStatThreads + threadIdx.x; q < n; q += (int64_t)gridDim.x * kStatThreads) {
@@ -370,11 +378,13 @@ __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __r
   }
 }
 
-// work block -> block m of an FP16-pair store
+// work block -> block m of an FP16-pair store (blockIdx.y as above)
 template <typename CT>
 __global__ void split_block_kernel(const CT* __restrict__ src, __half* __restrict__ store, int32_t m, int32_t M,
                                    int64_t n, const float* __restrict__ scale, int* __restrict__ bad) {
-  const float s = __ldg(scale);
+  src += blockIdx.y * n;
+  m += blockIdx.y;
+  const float s = __ldg(scale + blockIdx.y);
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
     const float2 v = to_c64(src[q]);
     split_put(store, M, m, q, v.x, v.y, s, bad);
@@ -1180,32 +1190,47 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   ScratchScope scope(st);
   const bool tensor = (flags & TBK_MU_TENSOR) != 0;
   const int64_t K16 = (K + 31) / 32 * 32;                // whole tiles of either store
-  DevBuf stage, Ld, Rd, acc, part, scales;
-  SplitScales sc;
-  TBK_TRY(stage.alloc(sizeof(double2) * K));
+  // blocks go up several at a time: a copy and three launches for each of them took 29 us a
+  // block (392 blocks of 7 values: 12.7 ms -> 0.3 ms)
+  constexpr int64_t kStageBytes = 32 << 20;
+  const int32_t per = (int32_t)std::max<int64_t>(1, std::min<int64_t>({M, kStageBytes / (16 * K), 65535}));
+  // CTAs of a block: enough together to fill the GPU, partials for all
+  const int gs = (int)std::max<int64_t>(1, std::min<int64_t>((K + kStatThreads - 1) / kStatThreads,
+                                                             (2 * sm_count() + per - 1) / per));
+  DevBuf stage, Ld, Rd, acc, part, scales, stat;
+  TBK_TRY(stage.alloc(sizeof(double2) * K * per));
   TBK_TRY(Ld.alloc(sizeof(float2) * M * K16));
   TBK_TRY(Rd.alloc(sizeof(float2) * M * K16));
   TBK_TRY(acc.alloc(sizeof(double2) * (size_t)M * M));
   TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
   TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
   TBK_CUDA(cudaMemsetAsync(acc.p, 0, acc.bytes, st));
+  unsigned int* count = nullptr;
+  int* bad = nullptr;
   if (tensor) {
-    TBK_TRY(sc.alloc(st));
+    const size_t sums = sizeof(double) * 2 * gs * (size_t)per;
     TBK_TRY(scales.alloc(sizeof(float) * 2 * M));        // a scale for every block
+    TBK_TRY(stat.alloc(sums + sizeof(int) * ((size_t)per + 1)));
+    count = reinterpret_cast<unsigned int*>(stat.as<char>() + sums);
+    bad = reinterpret_cast<int*>(count + per);
+    TBK_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * ((size_t)per + 1), st));
   }
-  const unsigned gk = (unsigned)std::min<int64_t>((K + 255) / 256, 4096);
+  const unsigned gk = (unsigned)std::min<int64_t>((K + 255) / 256, std::max<int64_t>(1, 4096 / per));
   auto upload = [&](bool split) -> int {
     for (int side = 0; side < 2; ++side) {
       DevBuf& dst = side ? Rd : Ld;
       const double* src = side ? Rb : L;
-      for (int32_t m = 0; m < M; ++m) {
-        TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K, cudaMemcpyHostToDevice, st));
+      for (int32_t m = 0; m < M; m += per) {
+        const int32_t nb = std::min(per, M - m);
+        const double2* from = stage.as<double2>();
+        TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K * nb, cudaMemcpyHostToDevice, st));
         if (split) {
           float* s = scales.as<float>() + side * M + m;
-          sc.find(stage.as<const double2>(), K, s, 0, false, st);
-          split_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<__half>(), m, M, K, s, sc.bad());
+          split_scale_kernel<<<dim3(gs, nb), kStatThreads, 0, st>>>(from, K, stat.as<double>(), count, nullptr, s, bad);
+          TBK_CHECK_LAUNCH();
+          split_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, dst.as<__half>(), m, M, K, s, bad);
         } else {
-          round_block_kernel<<<gk, 256, 0, st>>>(stage.as<const double2>(), dst.as<float2>(), m, M, K);
+          round_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, dst.as<float2>(), m, M, K);
         }
         TBK_CHECK_LAUNCH();
       }
@@ -1218,8 +1243,8 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   TBK_CUDA(cudaEventRecord(ev[0], st));
   bool formed = false;
   if (tensor) {
-    const SplitStore ls{Ld.as<__half>(), scales.as<float>(), 1, sc.bad()};
-    const SplitStore rs{Rd.as<__half>(), scales.as<float>() + M, 1, sc.bad()};
+    const SplitStore ls{Ld.as<__half>(), scales.as<float>(), 1, bad};
+    const SplitStore rs{Rd.as<__half>(), scales.as<float>() + M, 1, bad};
     TBK_TRY(mu_gemm_tc(ls, rs, M, K, acc.as<double>(), &formed, st));
     if (!formed) {                                       // infinities or NaN: complex64 blocks
       TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
