@@ -54,30 +54,29 @@ __device__ __forceinline__ dc csqrt_p(dc z) {  // principal branch, as std::sqrt
   return {fabs(z.i) / (2.0 * s), signbit(z.i) ? -s : s};
 }
 
-// sum_m c_m w^m, c_0 = g_0 mu_0 / 2, c_m = g_m mu_m, by kSeriesLanes lanes of a warp: lane l
-// takes m = l, l + kSeriesLanes, ... by Horner's rule in w^kSeriesLanes (5 FP64 instructions a
-// term) and multiplies by w^l; every lane of the group returns the sum.  One thread per
-// point runs n dependent steps on an FP64 pipe that starts a warp instruction every 64
-// clocks, with most of the GPU idle: 512 moments, 1,000 energies 110 us; 1,024 moments, 512
-// energies 212 us; so 24 us
-// for the former.
-constexpr int kSeriesLanes = 16;
+// sum_m c_m w^m, c_0 = g_0 mu_0 / 2, c_m = g_m mu_m, by L lanes of a warp: lane l takes m = l,
+// l + L, ... by Horner's rule in w^L (5 FP64 instructions a term) and multiplies by w^l; every lane
+// of the group returns the sum.  One thread per point runs n dependent steps on an FP64 pipe
+// that starts a warp instruction every 64 clocks, with most of the GPU idle: 512 moments, 1,000
+// energies 110 us; 24 us with 16 lanes.  But the powers of w are work per lane, and a few warps
+// an SM keep the pipe busy: series_lanes.
+template <int L>
 __device__ dc series_sum(int n, const double* __restrict__ g, const double* __restrict__ mu, dc w) {
-  const int l = threadIdx.x & (kSeriesLanes - 1);
-  dc q = w, wl = {1.0, 0.0};                       // w^l by its bits, q = w^kSeriesLanes
+  const int l = threadIdx.x & (L - 1);
+  dc q = w, wl = {1.0, 0.0};                       // w^l by its bits, q = w^L
 #pragma unroll
-  for (int b = 1; b < kSeriesLanes; b <<= 1) {
+  for (int b = 1; b < L; b <<= 1) {
     if (l & b) wl = cmul(wl, q);
     q = cmul(q, q);
   }
   dc p = {0.0, 0.0};
-  for (int m = l + (n - 1 - l) / kSeriesLanes * kSeriesLanes; m >= 0 && l < n; m -= kSeriesLanes) {
-    const double c = m == 0 ? 0.5 * (g[0] * mu[0]) : g[m] * mu[m];
-    p = {fma(p.r, q.r, fma(-p.i, q.i, c)), fma(p.r, q.i, p.i * q.r)};
-  }
-  p = cmul(p, wl);
+  auto term = [&](double c) { p = {fma(p.r, q.r, fma(-p.i, q.i, c)), fma(p.r, q.i, p.i * q.r)}; };
+#pragma unroll 4
+  for (int m = l + (n - 1 - l) / L * L; m >= L; m -= L) term(g[m] * mu[m]);
+  if (l < n) term(l == 0 ? 0.5 * (g[0] * mu[0]) : g[l] * mu[l]);
+  if constexpr (L > 1) p = cmul(p, wl);
 #pragma unroll
-  for (int o = kSeriesLanes / 2; o > 0; o >>= 1) {
+  for (int o = L / 2; o > 0; o >>= 1) {
     p.r += __shfl_xor_sync(0xffffffffu, p.r, o);
     p.i += __shfl_xor_sync(0xffffffffu, p.i, o);
   }
@@ -85,18 +84,19 @@ __device__ dc series_sum(int n, const double* __restrict__ g, const double* __re
 }
 
 // f(z) = sum_n g_n Im(alpha_n(z)) mu_n with alpha_0 = -i / s1, alpha_k = -2 i (z - i s1)^k / s1
+template <int L>
 __global__ void green_imag_kernel(int n, const double* __restrict__ g, const double* __restrict__ mu, int nz,
                                   const double* __restrict__ z, double scale, double* __restrict__ out) {
-  const int k = (blockIdx.x * blockDim.x + threadIdx.x) / kSeriesLanes;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   const int kk = min(k, nz - 1);                   // whole warps take part in the sums
   dc zz = {z[2 * kk], z[2 * kk + 1]};
   dc z2 = cmul(zz, zz);
   dc s1 = csqrt_p({1.0 - z2.r, 0.0 - z2.i});
   dc s2 = {zz.r + s1.i, zz.i - s1.r};              // z - i s1
-  double f = cmul(cdiv({0.0, -2.0}, s1), series_sum(n, g, mu, s2)).i;
-  // far outside [-1, 1] the powers up to w^max(n, 15) leave the range where alpha_n itself may
+  double f = cmul(cdiv({0.0, -2.0}, s1), series_sum<L>(n, g, mu, s2)).i;
+  // far outside [-1, 1] the powers up to w^max(n, L) leave the range where alpha_n itself may
   // not: term by term there
-  if (0.5f * log2f((float)(s2.r * s2.r + s2.i * s2.i)) * (float)max(n, kSeriesLanes) > 1000.f) {
+  if (0.5f * log2f((float)(s2.r * s2.r + s2.i * s2.i)) * (float)max(n, L) > 1000.f) {
     dc sn = cdiv({0.0, -2.0}, s1);
     f = g[0] * cdiv({0.0, -1.0}, s1).i * mu[0];
     for (int m = 1; m < n; ++m) {
@@ -104,7 +104,7 @@ __global__ void green_imag_kernel(int n, const double* __restrict__ g, const dou
       f += g[m] * sn.i * mu[m];
     }
   }
-  if (k < nz && threadIdx.x % kSeriesLanes == 0) out[k] = scale * f;
+  if (k < nz && threadIdx.x % L == 0) out[k] = scale * f;
 }
 
 // DCT-III (REDFT01) of g*mu at x_k = cos((k+1/2) pi / N), times 1/sqrt(1-x^2).
@@ -129,8 +129,31 @@ __global__ void green_fft_kernel(int n, const double* __restrict__ g, const doub
 }
 
 constexpr int kSeriesThreads = 128;
-static unsigned series_grid(int points) {
-  return (unsigned)(((int64_t)points * kSeriesLanes + kSeriesThreads - 1) / kSeriesThreads);
+// Lanes per point: the least of a model of both costs, the chain of n / L terms (0.29 us each) and
+// the FP64 pipe's work of 5 instructions a term and 150 a lane (root, division, powers of w) at
+// 0.6 T/s.  1, 4, 16 lanes, whole calls: 512 moments, 1,000 points 126, 63, 49 us, 10,000 points
+// 136, 114, 133, 200,000 points 1049, 1140, 1763; 64 moments, 20,000 points 74, 75, 135; 2,048
+// moments, 10,000 points 418, 305, 275.
+static int series_lanes(int n, int points) {
+  int best = 1;
+  double least = 0.0;
+  for (int lanes : {1, 4, 16}) {
+    const double us = 0.29 * n / lanes + points * (150.0 * lanes + 5.0 * n) / 6e5;
+    if (lanes > 1 && us >= least) continue;
+    best = lanes;
+    least = us;
+  }
+  return best;
+}
+static int green_imag(int n, const double* g, const double* mu, int nz, const double* z, double scale, double* out,
+                      cudaStream_t st) {
+  const int lanes = series_lanes(n, nz);
+  const unsigned grid = (unsigned)(((int64_t)nz * lanes + kSeriesThreads - 1) / kSeriesThreads);
+  if (lanes == 16) green_imag_kernel<16><<<grid, kSeriesThreads, 0, st>>>(n, g, mu, nz, z, scale, out);
+  else if (lanes == 4) green_imag_kernel<4><<<grid, kSeriesThreads, 0, st>>>(n, g, mu, nz, z, scale, out);
+  else green_imag_kernel<1><<<grid, kSeriesThreads, 0, st>>>(n, g, mu, nz, z, scale, out);
+  TBK_CHECK_LAUNCH();
+  return TBK_OK;
 }
 
 template <typename T>
@@ -188,9 +211,7 @@ int tbk_green_imag_eval(int32_t n, const double* g, const double* mu, int32_t n_
   TBK_TRY(upload(dm, mu, n, st));
   TBK_TRY(upload(dz, z, 2 * (size_t)n_z, st));
   TBK_TRY(dout.alloc(sizeof(double) * n_z));
-  green_imag_kernel<<<series_grid(n_z), kSeriesThreads, 0, st>>>(n, dg.as<double>(), dm.as<double>(), n_z, dz.as<double>(),
-                                                       1.0, dout.as<double>());
-  TBK_CHECK_LAUNCH();
+  TBK_TRY(green_imag(n, dg.as<double>(), dm.as<double>(), n_z, dz.as<double>(), 1.0, dout.as<double>(), st));
   TBK_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double) * n_z, cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
   return TBK_OK;
@@ -236,9 +257,7 @@ int tbk_dos_from_moments(int32_t n, const double* mu, int32_t kind, double p0, d
   TBK_TRY(dout.alloc(sizeof(double) * n_e));
   const double pi = 3.14159265358979323846;
   // rho = -1/R/pi * f(e), TB/functions.h:28
-  green_imag_kernel<<<series_grid(n_e), kSeriesThreads, 0, st>>>(n, dg.as<double>(), dm.as<double>(), n_e, dz.as<double>(),
-                                                       -1.0 / R / pi, dout.as<double>());
-  TBK_CHECK_LAUNCH();
+  TBK_TRY(green_imag(n, dg.as<double>(), dm.as<double>(), n_e, dz.as<double>(), -1.0 / R / pi, dout.as<double>(), st));
   TBK_CUDA(cudaMemcpyAsync(rho, dout.p, sizeof(double) * n_e, cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
   return TBK_OK;
