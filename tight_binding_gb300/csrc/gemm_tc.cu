@@ -337,13 +337,15 @@ __global__ void __launch_bounds__(kThreads, 1) mu_tc_kernel(const __grid_constan
 
 // acc += (split-K partials summed in order) / (s_m s_n), one CTA row of tile rows per
 // output column; nothing where the stores are marked unusable (the caller then forms the
-// chunk from complex64 stores).
+// chunk from complex64 stores).  The mark goes to *bad_out beside the kernel's error, for one
+// read-back.
 __global__ void __launch_bounds__(kTM) mu_tc_reduce_kernel(const double* __restrict__ part, int32_t M, int32_t n_tiles_p,
                                                            int32_t tiles, int32_t nsplit, const float* __restrict__ sl,
                                                            int32_t sl_stride, const float* __restrict__ sr,
                                                            int32_t sr_stride, const int* __restrict__ bad,
-                                                           double2* __restrict__ acc) {
+                                                           int* __restrict__ bad_out, double2* __restrict__ acc) {
   const int32_t n = blockIdx.x, mt = blockIdx.y, m = mt * kTM + threadIdx.x;
+  if (n == 0 && m == 0) *bad_out = *bad;
   if (m >= M || *bad) return;
   const int64_t tile = (int64_t)mt * n_tiles_p + n / kTN, step = (int64_t)tiles * kAccCols * kTM;
   const double* p = part + (tile * kAccCols + n % kTN) * kTM + threadIdx.x;
@@ -424,8 +426,8 @@ int mu_gemm_tc(const SplitStore& L, const SplitStore& Rb, int32_t M, int64_t K, 
   nsplit = (int)((tiles_k + tiles_split - 1) / tiles_split);
   DevBuf part, errb;
   TBK_TRY(part.alloc(sizeof(double) * (size_t)nsplit * tiles * kAccCols * kTM));
-  TBK_TRY(errb.alloc(sizeof(int)));
-  TBK_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
+  TBK_TRY(errb.alloc(2 * sizeof(int)));
+  TBK_CUDA(cudaMemsetAsync(errb.p, 0, 2 * sizeof(int), st));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, nsplit);
   cfg.blockDim = dim3(kThreads);
@@ -442,11 +444,10 @@ int mu_gemm_tc(const SplitStore& L, const SplitStore& Rb, int32_t M, int64_t K, 
                               part.as<double>(), errb.as<int>()));
   mu_tc_reduce_kernel<<<dim3(M, m_tiles), kTM, 0, st>>>(part.as<double>(), M, n_tiles, tiles, nsplit, L.scale,
                                                         L.scale_stride, Rb.scale, Rb.scale_stride, L.bad,
-                                                        reinterpret_cast<double2*>(mu_acc));
+                                                        errb.as<int>() + 1, reinterpret_cast<double2*>(mu_acc));
   TBK_CHECK_LAUNCH();
   int h[2] = {0, 0};
-  TBK_CUDA(cudaMemcpyAsync(&h[0], errb.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  TBK_CUDA(cudaMemcpyAsync(&h[1], L.bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(h, errb.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
   if (h[0]) return fail(TBK_ERR_TIMEOUT, "tensor-core mu_nm kernel gave up waiting (code %d)", h[0]);
   *usable = h[1] == 0;

@@ -337,39 +337,44 @@ __global__ void __launch_bounds__(kStatThreads) split_scale_kernel(const CT* __r
     big = (v.x != v.x || v.y != v.y) ? INFINITY : fmaxf(big, m);
     sum += (double)v.x * v.x + (double)v.y * v.y;
   }
-  __shared__ double s_sum[kStatThreads], s_big[kStatThreads];
+  __shared__ double s_sum[kStatThreads / 32];
+  __shared__ float s_big[kStatThreads / 32];
   __shared__ bool last;
-  auto block_reduce = [&]() {
+  auto block_reduce = [&](double& v, float& m) {          // valid in warp 0
     __syncthreads();
-    for (int o = kStatThreads / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) {
-        s_sum[threadIdx.x] += s_sum[threadIdx.x + o];
-        s_big[threadIdx.x] = fmax(s_big[threadIdx.x], s_big[threadIdx.x + o]);
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int o = 16; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       }
+      if (pass == 1) break;
+      if ((threadIdx.x & 31) == 0) { s_sum[threadIdx.x >> 5] = v; s_big[threadIdx.x >> 5] = m; }
       __syncthreads();
+      if (threadIdx.x >= 32) break;
+      const bool in = threadIdx.x < kStatThreads / 32;
+      v = in ? s_sum[threadIdx.x] : 0.0;
+      m = in ? s_big[threadIdx.x] : 0.f;
     }
   };
-  s_sum[threadIdx.x] = sum;
-  s_big[threadIdx.x] = big;
-  block_reduce();
+  block_reduce(sum, big);
   if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = s_sum[0];
-    part[2 * blockIdx.x + 1] = s_big[0];
+    part[2 * blockIdx.x] = sum;
+    part[2 * blockIdx.x + 1] = big;
     __threadfence();
     last = atomicAdd(count, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  s_sum[threadIdx.x] = 0.0;
-  s_big[threadIdx.x] = 0.0;
+  sum = 0.0;
+  big = 0.f;
   for (int b = threadIdx.x; b < (int)gridDim.x; b += kStatThreads) {
-    s_sum[threadIdx.x] += __ldcg(part + 2 * b);
-    s_big[threadIdx.x] = fmax(s_big[threadIdx.x], __ldcg(part + 2 * b + 1));
+    sum += __ldcg(part + 2 * b);
+    big = fmaxf(big, (float)__ldcg(part + 2 * b + 1));
   }
-  block_reduce();
+  block_reduce(sum, big);
   if (threadIdx.x == 0) {
-    const double f = gain ? (double)*gain : 1.0, mx = f * s_big[0], rms = f * sqrt(s_sum[0] / (2.0 * (double)n));
+    const double f = gain ? (double)*gain : 1.0, mx = f * big, rms = f * sqrt(sum / (2.0 * (double)n));
     float s = 1.f;                                       // zero blocks
     if (!(mx < (double)INFINITY)) *bad = 1;
     else if (mx > 0.0) s = ldexpf(1.f, max(-120, min(120, min(12 - ilogb(mx), 6 - ilogb(rms)))));
@@ -671,20 +676,19 @@ int with_block(int prec, const void* p, Fn&& f) {
 // Scratch of split_scale_kernel, the two sides' scales and the flag of values that do
 // not fit.
 struct SplitScales {
-  DevBuf part, words;          // words: scale of the left, of the right side; bad; count, gain of each side
+  DevBuf buf;                  // 7 words: scale of the left, of the right side; bad; count, gain of each side; the partials
   int alloc(cudaStream_t st) {
-    TBK_TRY(part.alloc(sizeof(double) * 8 * sm_count()));
-    TBK_TRY(words.alloc(7 * sizeof(int)));
-    TBK_CUDA(cudaMemsetAsync(words.p, 0, words.bytes, st));
+    TBK_TRY(buf.alloc(sizeof(double) * (4 + 8 * sm_count())));
+    TBK_CUDA(cudaMemsetAsync(buf.p, 0, 4 * sizeof(double), st));
     return TBK_OK;
   }
-  float* scale(int h) const { return words.as<float>() + h; }
-  int* bad() const { return words.as<int>() + 2; }
+  float* scale(int h) const { return buf.as<float>() + h; }
+  int* bad() const { return buf.as<int>() + 2; }
   // the output operator of side h
   int set_operator(int h, const EllDev& E, cudaStream_t st) const {
     operator_gain_kernel<<<(E.n_rows + 255) / 256, 256, 0, st>>>(E.n_rows, E.slice_off.as<int32_t>(), E.val32.as<float>(),
                                                                  E.diag32.as<float>(), E.cplx ? 2 : 1,
-                                                                 words.as<unsigned int>() + 5 + h);
+                                                                 buf.as<unsigned int>() + 5 + h);
     TBK_CHECK_LAUNCH();
     return TBK_OK;
   }
@@ -692,17 +696,19 @@ struct SplitScales {
   template <typename CT>
   void find(const CT* src, int64_t n, float* out, int h, bool gain, cudaStream_t st) const {
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + kStatThreads - 1) / kStatThreads, 2 * sm_count()));
-    split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, part.as<double>() + 4 * h * sm_count(),
-                                                       words.as<unsigned int>() + 3 + h,
-                                                       gain ? words.as<float>() + 5 + h : nullptr, out, bad());
+    split_scale_kernel<CT><<<g, kStatThreads, 0, st>>>(src, n, buf.as<double>() + 4 + 4 * h * sm_count(),
+                                                       buf.as<unsigned int>() + 3 + h,
+                                                       gain ? buf.as<float>() + 5 + h : nullptr, out, bad());
   }
 };
 
 // Blocks of up to this size leave much of the GPU idle in one recursion: both sides of
 // square 256x256 with a flux, M = 512, 16 vectors (8 MB a block), took 9.8 ms one after the
 // other, the operator's products in a pass of their own, and take 7.9 ms on two streams;
-// honeycomb 91x77, M = 200, 3 vectors, 1.25 and 0.75 ms.
+// honeycomb 91x77, M = 200, 3 vectors, 1.25 and 0.75 ms.  The stream costs some 20 us a call: whole
+// calls of 1 and 2 streams, square 80x80, 8 vectors, M = 4: 261, 262 us; 12: 333, 309; 24: 427, 367.
 constexpr double kDualBlock = 16e6;
+constexpr int64_t kDualSteps = 8;     // steps a side
 
 // A stream beside the caller's, of its priority, for the length of a call
 struct SecondStream {
@@ -840,7 +846,8 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     both = same;
   }
   // small blocks: the two sides' recursions run side by side on two streams
-  const bool dual = !both && !f64b && (double)csz * blk <= kDualBlock;
+  const int64_t steps = (int64_t)M * ((R + Rc - 1) / Rc);   // of one side
+  const bool dual = !both && !f64b && (double)csz * blk <= kDualBlock && steps >= kDualSteps;
   {
     const AsyncAllocCtx* outer = tl_async_alloc;
     if (kctx.pool) tl_async_alloc = &kctx;
@@ -906,7 +913,11 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
   // Complex64 recursions take the operator's products inside the step wherever H~ and the
   // operator have joint row classes: one pass over the vectors' neighbours per block
   // instead of two (FCC 128^3, 4 vectors: 77.9 us against 56.5 + 83.7); and where H~ runs in
-  // the ELL form anyway, whose columns they then load once (a flux).
+  // the ELL form anyway, whose columns they then load once (a flux).  Comparing the matrices and
+  // finding the classes costs some 60 us an operator, a product of its own 3 us a step or more:
+  // whole calls with and without, honeycomb 31x29, 3 vectors, M = 4: 365, 255 us; 24: 496, 455; 32:
+  // 539, 535; 48: 636, 684; 100: 964, 1205.
+  constexpr int64_t kFuseSteps = 32;
   struct Fused {
     bool on = false;
     ClassSet32 pair;
@@ -917,7 +928,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     Fused& F = fused[h];
     F.grid = grid;
     const bool mixed = prec == TBK_PREC_MIXED;
-    if (!Aout || !((flags & TBK_MU_FUSED_OPS) || mixed)) continue;
+    if (!Aout || !((flags & TBK_MU_FUSED_OPS) || (mixed && steps >= kFuseSteps))) continue;
     bool v_real = false;
     TBK_TRY(same_ell_structure(Ht, Aout, &F.on, st, mixed ? &v_real : nullptr));
     if (F.on && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
