@@ -430,7 +430,7 @@ __global__ void mu_kernel_scale_kernel(double2* __restrict__ mu, const double* _
 // where e = cos th and s = sin th.  As M x M sums per energy the two were bound by
 // the FP64 pipe (6 FMAs per moment and energy): M = 512, 1,024 energies took 4.00 +
 // 0.94 ms in their kernels, 5.62 ms for both calls with the host copies; as series
-// both calls take 0.72 ms, nearly all of it copies and allocations.
+// both calls take 0.25 ms, nearly all of it copies and launches.
 constexpr int kDiagThreads = 128;
 constexpr int kDiagRows = 16;       // rows of mu per CTA: M = 512 gives 256 CTAs
 constexpr int kSeriesThreads = 128; // evaluation: one warp per energy
@@ -575,26 +575,26 @@ int moment_series(int32_t M, const double* mu, int32_t n_eps, const double* eps,
                   cudaStream_t st) {
   ScratchScope scope(st);
   const int32_t L = 2 * M - 1, chunks = (M + kDiagRows - 1) / kDiagRows, planes = BASTIN ? 3 : 2;
+  const size_t mb = sizeof(double2) * (size_t)M * M, cb = sizeof(double2) * (size_t)planes * L;
   const size_t ob = sizeof(double) * (BASTIN ? 2 : 1) * (size_t)n_eps;
-  DevBuf dm, de, dz, part, coef;
-  TBK_TRY(dm.alloc(sizeof(double2) * (size_t)M * M));
-  TBK_TRY(de.alloc(sizeof(double) * n_eps));
-  TBK_TRY(dz.alloc(ob));
-  TBK_TRY(part.alloc(sizeof(double2) * (size_t)chunks * planes * L));
-  TBK_TRY(coef.alloc(sizeof(double2) * (size_t)planes * L));
-  TBK_CUDA(cudaMemcpyAsync(dm.p, mu, sizeof(double2) * (size_t)M * M, cudaMemcpyHostToDevice, st));
-  TBK_CUDA(cudaMemcpyAsync(de.p, eps, sizeof(double) * n_eps, cudaMemcpyHostToDevice, st));
+  DevBuf ws;                                             // one workspace: mu, partials, coefficients, results, energies
+  TBK_TRY(ws.alloc(mb + cb * (chunks + 1) + ob + sizeof(double) * n_eps));
+  double2* dm = ws.as<double2>();
+  double2* part = dm + (size_t)M * M;
+  double2* coef = part + (size_t)chunks * planes * L;
+  double* dz = reinterpret_cast<double*>(coef + (size_t)planes * L);
+  double* de = dz + (BASTIN ? 2 : 1) * (size_t)n_eps;
+  TBK_CUDA(cudaMemcpyAsync(dm, mu, mb, cudaMemcpyHostToDevice, st));
+  TBK_CUDA(cudaMemcpyAsync(de, eps, sizeof(double) * n_eps, cudaMemcpyHostToDevice, st));
   const int32_t qb = (L + kDiagThreads - 1) / kDiagThreads;
-  diag_sums_kernel<BASTIN><<<dim3(qb, chunks), kDiagThreads, 0, st>>>(dm.as<double2>(), M, part.as<double2>());
+  diag_sums_kernel<BASTIN><<<dim3(qb, chunks), kDiagThreads, 0, st>>>(dm, M, part);
   TBK_CHECK_LAUNCH();
-  series_coef_kernel<BASTIN><<<(L + 31) / 32, 32 * kCoefWarps, 0, st>>>(part.as<double2>(), M, chunks, coef.as<double2>());
+  series_coef_kernel<BASTIN><<<(L + 31) / 32, 32 * kCoefWarps, 0, st>>>(part, M, chunks, coef);
   TBK_CHECK_LAUNCH();
   constexpr int kPer = kSeriesThreads / 32;
-  series_eval_kernel<BASTIN><<<(n_eps + kPer - 1) / kPer, kSeriesThreads, 0, st>>>(coef.as<double2>(), M, n_eps,
-                                                                                   de.as<double>(), norm,
-                                                                                   dz.as<double>());
+  series_eval_kernel<BASTIN><<<(n_eps + kPer - 1) / kPer, kSeriesThreads, 0, st>>>(coef, M, n_eps, de, norm, dz);
   TBK_CHECK_LAUNCH();
-  TBK_CUDA(cudaMemcpyAsync(out, dz.p, ob, cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(out, dz, ob, cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
   return TBK_OK;
 }
