@@ -932,7 +932,7 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     bool v_real = false;
     TBK_TRY(same_ell_structure(Ht, Aout, &F.on, st, mixed ? &v_real : nullptr));
     if (F.on && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
-    if (F.on && mixed && !v_real) TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
+    if (F.on && mixed && !v_real && steps >= kFuseSteps) TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
     if (F.pair.n_cls > 0) {
       TBK_TRY(pair_config(Ht, Rc, F.pair, &F.grid));
     } else {
@@ -1208,40 +1208,37 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   // CTAs of a block: enough together to fill the GPU, partials for all
   const int gs = (int)std::max<int64_t>(1, std::min<int64_t>((K + kStatThreads - 1) / kStatThreads,
                                                              (2 * sm_count() + per - 1) / per));
-  DevBuf stage, Ld, Rd, acc, part, scales, stat;
-  TBK_TRY(stage.alloc(sizeof(double2) * K * per));
-  TBK_TRY(Ld.alloc(sizeof(float2) * M * K16));
-  TBK_TRY(Rd.alloc(sizeof(float2) * M * K16));
-  TBK_TRY(acc.alloc(sizeof(double2) * (size_t)M * M));
-  TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
-  TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
-  TBK_CUDA(cudaMemsetAsync(acc.p, 0, acc.bytes, st));
-  unsigned int* count = nullptr;
-  int* bad = nullptr;
-  if (tensor) {
-    const size_t sums = sizeof(double) * 2 * gs * (size_t)per;
-    TBK_TRY(scales.alloc(sizeof(float) * 2 * M));        // a scale for every block
-    TBK_TRY(stat.alloc(sums + sizeof(int) * ((size_t)per + 1)));
-    count = reinterpret_cast<unsigned int*>(stat.as<char>() + sums);
-    bad = reinterpret_cast<int*>(count + per);
-    TBK_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * ((size_t)per + 1), st));
-  }
+  // zeroed: both stores, the sums, the scale search's mark and counters; not zeroed: its partials, the
+  // scales, the stage
+  const size_t store = sizeof(float2) * M * K16, sums = sizeof(double2) * (size_t)M * M;
+  const size_t stat = sizeof(double) * 2 * gs * (size_t)per, scal = (sizeof(float) * 2 * M + 15) / 16 * 16;
+  DevBuf zero, work, part;
+  TBK_TRY(zero.alloc(2 * store + sums + sizeof(int) * ((size_t)per + 1)));
+  TBK_TRY(work.alloc(stat + scal + sizeof(double2) * K * per));
+  TBK_CUDA(cudaMemsetAsync(zero.p, 0, zero.bytes, st));
+  void* Ld = zero.p;
+  void* Rd = zero.as<char>() + store;
+  double2* acc = reinterpret_cast<double2*>(zero.as<char>() + 2 * store);
+  int* bad = reinterpret_cast<int*>(acc + (size_t)M * M);
+  unsigned int* count = reinterpret_cast<unsigned int*>(bad + 1);
+  float* scales = reinterpret_cast<float*>(work.as<char>() + stat);   // one for every block
+  double2* stage = reinterpret_cast<double2*>(work.as<char>() + stat + scal);
   const unsigned gk = (unsigned)std::min<int64_t>((K + 255) / 256, std::max<int64_t>(1, 4096 / per));
   auto upload = [&](bool split) -> int {
     for (int side = 0; side < 2; ++side) {
-      DevBuf& dst = side ? Rd : Ld;
+      void* dst = side ? Rd : Ld;
       const double* src = side ? Rb : L;
       for (int32_t m = 0; m < M; m += per) {
         const int32_t nb = std::min(per, M - m);
-        const double2* from = stage.as<double2>();
-        TBK_CUDA(cudaMemcpyAsync(stage.p, src + 2 * (int64_t)m * K, sizeof(double2) * K * nb, cudaMemcpyHostToDevice, st));
+        const double2* from = stage;
+        TBK_CUDA(cudaMemcpyAsync(stage, src + 2 * (int64_t)m * K, sizeof(double2) * K * nb, cudaMemcpyHostToDevice, st));
         if (split) {
-          float* s = scales.as<float>() + side * M + m;
-          split_scale_kernel<<<dim3(gs, nb), kStatThreads, 0, st>>>(from, K, stat.as<double>(), count, nullptr, s, bad);
+          float* s = scales + side * M + m;
+          split_scale_kernel<<<dim3(gs, nb), kStatThreads, 0, st>>>(from, K, work.as<double>(), count, nullptr, s, bad);
           TBK_CHECK_LAUNCH();
-          split_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, dst.as<__half>(), m, M, K, s, bad);
+          split_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, static_cast<__half*>(dst), m, M, K, s, bad);
         } else {
-          round_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, dst.as<float2>(), m, M, K);
+          round_block_kernel<<<dim3(gk, nb), 256, 0, st>>>(from, static_cast<float2*>(dst), m, M, K);
         }
         TBK_CHECK_LAUNCH();
       }
@@ -1254,19 +1251,18 @@ int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, 
   TBK_CUDA(cudaEventRecord(ev[0], st));
   bool formed = false;
   if (tensor) {
-    const SplitStore ls{Ld.as<__half>(), scales.as<float>(), 1, bad};
-    const SplitStore rs{Rd.as<__half>(), scales.as<float>() + M, 1, bad};
-    TBK_TRY(mu_gemm_tc(ls, rs, M, K, acc.as<double>(), &formed, st));
+    const SplitStore ls{static_cast<__half*>(Ld), scales, 1, bad};
+    const SplitStore rs{static_cast<__half*>(Rd), scales + M, 1, bad};
+    TBK_TRY(mu_gemm_tc(ls, rs, M, K, reinterpret_cast<double*>(acc), &formed, st));
     if (!formed) {                                       // infinities or NaN: complex64 blocks
-      TBK_CUDA(cudaMemsetAsync(Ld.p, 0, Ld.bytes, st));
-      TBK_CUDA(cudaMemsetAsync(Rd.p, 0, Rd.bytes, st));
+      TBK_CUDA(cudaMemsetAsync(Ld, 0, 2 * store, st));
       TBK_TRY(upload(false));
       TBK_CUDA(cudaEventRecord(ev[0], st));
     }
   }
-  if (!formed) TBK_TRY(mu_gemm_cc(Ld.as<float2>(), Rd.as<float2>(), M, K, &part, acc.as<double2>(), st));
+  if (!formed) TBK_TRY(mu_gemm_cc(static_cast<float2*>(Ld), static_cast<float2*>(Rd), M, K, &part, acc, st));
   TBK_CUDA(cudaEventRecord(ev[1], st));
-  TBK_CUDA(cudaMemcpyAsync(mu_out, acc.p, sizeof(double2) * (size_t)M * M, cudaMemcpyDeviceToHost, st));
+  TBK_CUDA(cudaMemcpyAsync(mu_out, acc, sizeof(double2) * (size_t)M * M, cudaMemcpyDeviceToHost, st));
   TBK_CUDA(cudaStreamSynchronize(st));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ev[0], ev[1]);
