@@ -932,7 +932,9 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     bool v_real = false;
     TBK_TRY(same_ell_structure(Ht, Aout, &F.on, st, mixed ? &v_real : nullptr));
     if (F.on && prec == TBK_PREC_DD) TBK_TRY(ensure_ell_dd(Aout, st));
-    if (F.on && mixed && !v_real && steps >= kFuseSteps) TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
+    // (joint classes are at least H~'s: none where it has none)
+    if (F.on && mixed && !v_real && steps >= kFuseSteps && has_row_classes(Ht, prec))
+      TBK_TRY(pair_classes32(Ht, Aout, &F.pair, st));
     if (F.pair.n_cls > 0) {
       TBK_TRY(pair_config(Ht, Rc, F.pair, &F.grid));
     } else {
