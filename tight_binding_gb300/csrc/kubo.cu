@@ -741,11 +741,12 @@ struct SecondStream {
 // allocate).  So large problems take narrow chunks: FCC 128^3, M = 1024, R = 8: 648 ms at
 // width 4, 625 at 2, 721 at 1 (complex64 lanes carry two vectors: 1 is not taken while 2
 // fits); FCC 64^3: 96.7 at 8, 79.1 at 4, 76.1 at 2; honeycomb 1024^2, M = 512: 243 at 8, 216
-// at 4 and 2; square 512^2 with a flux, R = 12: 48.3 at 6, 42.2 at 4.  The wider recursions are bound
-// by arithmetic, whatever the width, and the FP64 GEMM of the reference form wants long K: wide
-// chunks (honeycomb 305x310, M = 301, R = 16, double-float: 31.9 ms at 16, 42.5 at 6; Lieb
-// 276x274, M = 60, R = 16, complex128 blocks: 143 ms at 4, 123 at 16).  both: a power of two (the
-// widths of the one recursion that carries both sides).
+// at 4 and 2; square 512^2 with a flux, R = 12: 48.3 at 6, 42.2 at 4.  Double-float and FP64
+// recursions, both alike so that their GEMMs sum in the same order, take powers of two only (the
+// kernels of other widths cost them more than they save: honeycomb 305x310, M = 301, R = 16,
+// double-float, 42.5 ms at 6).  The FP64 GEMM of the reference form wants long K: wide chunks (Lieb
+// 276x274, M = 60, R = 16: 143 ms at 4, 122 at 16).  both: a power of two (the widths of the one
+// recursion that carries both sides).
 int pick_chunk(int R, bool both, int prec, bool f64b, int32_t M, int64_t n_pad, double sel, double budget) {
   const double per_vector = 2.0 * M * n_pad * sel;
   if (both) {
@@ -755,14 +756,13 @@ int pick_chunk(int R, bool both, int prec, bool f64b, int32_t M, int64_t n_pad, 
     return c;
   }
   constexpr double kStepMs = 4.5e-3, kRowMs = 0.8e-9, kL2Ms = 4e-9, kHbmMs = 8e-9, kGemmMs = 8e-12, kMapMs = 0.45e-9;
-  const double kPipeMs = prec == TBK_PREC_FP64 ? 40e-9 : 13e-9;   // FP64 pipe; packed FP32
   int best = 1;
   double least = 0.0;
   for (int cap = 32; cap > 1; cap -= 2) {
     const int w = step_width(TBK_PREC_MIXED, R, cap), chunks = (R + w - 1) / w;
     const double bytes = per_vector * w, pooled = bytes + 8.0 * 16.0 * n_pad * w;
-    if (bytes > budget) continue;
-    const double value = (prec != TBK_PREC_MIXED || f64b ? kPipeMs : 16.0 * n_pad * w <= 20e6 ? kL2Ms : kHbmMs) + M * kGemmMs;
+    if (bytes > budget || (prec != TBK_PREC_MIXED && (w & (w - 1)))) continue;
+    const double value = (!f64b && 16.0 * n_pad * w <= 20e6 ? kL2Ms : kHbmMs) + M * kGemmMs;
     const double ms = chunks * 2.0 * M * (kStepMs + n_pad * (kRowMs + w * value)) +
                       (pooled > (double)kKuboPoolKeep ? kMapMs * bytes : 0.0);
     if (best > 1 && ms >= least) continue;
