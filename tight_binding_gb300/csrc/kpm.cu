@@ -101,16 +101,17 @@ static void random_block(int32_t n, int32_t R, int32_t r0, int32_t Rp, uint64_t 
   else random_block_kernel<F, int64_t><<<g, 256, 0, st>>>(n, R, r0, Rp, seed, inv, d);
 }
 
-// Fixed-order sum of the per-CTA partials of every (chunk, step, slot).
+// Fixed-order sum of the per-CTA partials of every (chunk, step, slot).  mirror: CTA b ran tile b in odd
+// steps too, where a step kernel's CTA b runs the last tile but b.
 __global__ void reduce_partials_kernel(const double* __restrict__ part, int32_t n_chunks, int32_t n_steps,
-                                       int32_t nblk, double* __restrict__ sums) {
+                                       int32_t nblk, int mirror, double* __restrict__ sums) {
   const int32_t step = blockIdx.x, slot = blockIdx.y;
   double acc = 0.0;
   __shared__ double sh[256];
   for (int32_t ch = 0; ch < n_chunks; ++ch) {
     const double* p = part + (((int64_t)ch * n_steps + step) * 2 + slot) * nblk;
     double a = 0.0;
-    for (int32_t b = threadIdx.x; b < nblk; b += blockDim.x) a += p[b];
+    for (int32_t b = threadIdx.x; b < nblk; b += blockDim.x) a += p[mirror && (step & 1) ? nblk - 1 - b : b];
     sh[threadIdx.x] = a;
     __syncthreads();
     for (int o = blockDim.x / 2; o > 0; o >>= 1) {
@@ -890,9 +891,7 @@ static int launch_persist(tbk_kpm_s* P, bool braket, int32_t n_steps, double* pa
   unsigned int* meet = P->meet.as<unsigned int>();
   int* err = P->err.as<int>();
   uint32_t lim = g_wait_limit.load(std::memory_order_relaxed);
-  int zigzag = (P->flags & TBK_FLAG_NO_L2_ZIGZAG) ? 0 : 1;
-  void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &zigzag, &meet, &err,
-                  &lim};
+  void* args[] = {&n, &n_steps, &lpr, &so, &co, &ev, &dg, const_cast<ClassTab*>(&ct), &va, &vb, &br, &part, &meet, &err, &lim};
   const cudaError_t e = cudaLaunchCooperativeKernel(persist_kernel(P, braket), dim3(P->grid), dim3(kStepThreads), args, smem, st);
   *launched = e == cudaSuccess;
   if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();
@@ -926,6 +925,7 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
   const bool cplx = P->H->ell.cplx != 0;
   float ms_total = 0.f;
   int32_t launches = 0;
+  bool mirror = false;
   const bool small = P->small_state == 1;
   const int32_t nblk = small ? P->R * P->slay.cs : G;    // partials per (step, slot)
   for (int32_t ch = 0; ch < P->n_chunks; ++ch) {
@@ -995,6 +995,7 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
       launches += 1;
     } else if (P->persist == 1 && (int64_t)n_steps * P->grid < (int64_t)INT32_MAX) {
       TBK_TRY(launch_persist(P, braket, n_steps, P->part.as<double>(), st, &issued));
+      mirror = issued && !(P->flags & TBK_FLAG_NO_L2_ZIGZAG);
       launches += issued ? n_steps : 0;
     }
     if (!issued && graphable) {
@@ -1049,7 +1050,7 @@ static int kpm_run_impl(tbk_kpm_s* P, int32_t n_mom, bool braket, KL&& kets_load
     ms_total += ms;
   }
   reduce_partials_kernel<<<dim3(n_steps, 2), 256, 0, st>>>(P->part.as<double>(), P->n_chunks, n_steps, nblk,
-                                                          P->sums.as<double>());
+                                                          mirror ? 1 : 0, P->sums.as<double>());
   TBK_CHECK_LAUNCH();
   assemble_moments_kernel<<<(n_mom + 255) / 256, 256, 0, st>>>(P->sums.as<double>(), n_mom, doubling ? 1 : 0,
                                                                P->mu.as<double>());

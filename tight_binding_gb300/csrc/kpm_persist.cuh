@@ -6,8 +6,9 @@
 // (through L2, where the other CTAs wrote them) and writes v_{s+1}.  Between steps the CTAs
 // meet at a counter in global memory; the step's moment sums run between a CTA's
 // arrival and its wait.  The arithmetic, its order and the partial sums are those of
-// kpm_step_kernel with one tile per CTA: the same bits.  (Where that sweeps odd steps from the
-// last tile to the first, CTA b's sums belong to the last tile but b: zigzag.)
+// kpm_step_kernel with one tile per CTA: the same bits.  (That sweeps odd steps from the last
+// tile to the first, so its CTA b has the sums of the last tile but b: the reduction reads these
+// backwards.)
 // What bounds a step: the L2 round trip of the gathers, the FP64 pipe and the meeting.
 // us a step against one launch per step (graph replay): square 64x64, R = 8, braket FP64
 // 3.99 -> 2.52, double-float 3.78 -> 2.65, complex64 3.65 -> 2.28; 170x160, R = 8, complex64
@@ -80,7 +81,7 @@ template <typename F, bool CPLX_H, bool BRAKET, bool CLS>
 __global__ void __launch_bounds__(kStepThreads) kpm_persist_kernel(
     int32_t n, int32_t n_steps, int32_t lpr, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
     const F* __restrict__ eval, const F* __restrict__ diag, const ClassTab ct, typename C2<F>::T* va,
-    typename C2<F>::T* vb, const typename C2<F>::T* __restrict__ bras, double* __restrict__ part, int zigzag,
+    typename C2<F>::T* vb, const typename C2<F>::T* __restrict__ bras, double* __restrict__ part,
     unsigned int* __restrict__ meet, int* __restrict__ err, uint32_t wait_limit) {
   using CT = typename C2<F>::T;
   using HV = HVal<F, CPLX_H>;
@@ -180,7 +181,6 @@ __global__ void __launch_bounds__(kStepThreads) kpm_persist_kernel(
       atomicAdd(meet, 1u);
     }
     double* p = part + (int64_t)s * 2 * gridDim.x;
-    if (zigzag && (s & 1)) p += (int)gridDim.x - 1 - 2 * (int)blockIdx.x;   // the sums go to p[slot * grid + blockIdx.x]
     if (!BRAKET || first) step_sums<F, true>(m0, m1, p);
     else step_sums<F, false>(m0, m1, p);
     if constexpr (FOLD) {
