@@ -287,10 +287,11 @@ static int step_threads(tbk_sparse_s* A, int Rc, int prec, int wide) {
 // CTAs per SM of A's form.  FP64: the smaller of both forms', so that they group their
 // partial sums alike and give the same bits.
 static int step_occupancy(tbk_sparse_s* A, int Rc, int prec, bool sums, int threads = kStepThreads) {
+  const StepKind kind{sums, class_tab(A->ell, prec).w > 8};
   const bool cplx = A->ell.cplx != 0, cls = has_classes(A->ell, prec);
   const int oc = cls || prec == TBK_PREC_FP64
-                     ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec), sums, threads) : 64;
-  const int oe = !cls || prec == TBK_PREC_FP64 ? occupancy_prec(prec, cplx, Rc, sums) : 64;
+                     ? occupancy_cls_prec(prec, cplx, Rc, class_smem(A->ell, prec), kind, threads) : 64;
+  const int oe = !cls || prec == TBK_PREC_FP64 ? occupancy_prec(prec, cplx, Rc, kind) : 64;
   return std::min(oc, oe);
 }
 
@@ -408,20 +409,20 @@ static int step_dispatch(tbk_sparse_s* A, int Rc, int prec, bool first, const St
 int launch_step_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
-int occupancy_f32(bool cplx, int R, bool sums);
-int occupancy_f64(bool cplx, int R, bool sums);
-int occupancy_dd(bool cplx, int R, bool sums);
+int occupancy_f32(bool cplx, int R, StepKind kind);
+int occupancy_f64(bool cplx, int R, StepKind kind);
+int occupancy_dd(bool cplx, int R, StepKind kind);
 int launch_step_cls_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
 int launch_step_cls_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid, cudaStream_t st);
-int occupancy_cls_f32(bool cplx, int R, size_t smem, bool sums, int threads);
-int occupancy_cls_f64(bool cplx, int R, size_t smem, bool sums);
-int occupancy_cls_dd(bool cplx, int R, size_t smem, bool sums);
+int occupancy_cls_f32(bool cplx, int R, size_t smem, StepKind kind, int threads);
+int occupancy_cls_f64(bool cplx, int R, size_t smem, StepKind kind);
+int occupancy_cls_dd(bool cplx, int R, size_t smem, StepKind kind);
 
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums, int threads) {
-  if (prec == TBK_PREC_FP64) return occupancy_cls_f64(cplx, R, smem, sums);
-  if (prec == TBK_PREC_DD) return occupancy_cls_dd(cplx, R, smem, sums);
-  return occupancy_cls_f32(cplx, R, smem, sums, threads);
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, StepKind kind, int threads) {
+  if (prec == TBK_PREC_FP64) return occupancy_cls_f64(cplx, R, smem, kind);
+  if (prec == TBK_PREC_DD) return occupancy_cls_dd(cplx, R, smem, kind);
+  return occupancy_cls_f32(cplx, R, smem, kind, threads);
 }
 
 int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid,
@@ -436,10 +437,10 @@ int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, 
   return launch_step_f32(cplx, R, a, first, braket, grid, st);
 }
 
-int occupancy_prec(int prec, bool cplx, int R, bool sums) {
-  if (prec == TBK_PREC_FP64) return occupancy_f64(cplx, R, sums);
-  if (prec == TBK_PREC_DD) return occupancy_dd(cplx, R, sums);
-  return occupancy_f32(cplx, R, sums);
+int occupancy_prec(int prec, bool cplx, int R, StepKind kind) {
+  if (prec == TBK_PREC_FP64) return occupancy_f64(cplx, R, kind);
+  if (prec == TBK_PREC_DD) return occupancy_dd(cplx, R, kind);
+  return occupancy_f32(cplx, R, kind);
 }
 
 int load_block_any(int prec, int32_t n, int32_t R, int32_t r0, int32_t Rp, const double2* src, void* dst,
@@ -861,6 +862,9 @@ static int plan_persist(tbk_kpm_s* P) {
   if (P->n_chunks != 1 || !lanes || P->n_tiles != P->grid ||
       (P->flags & (TBK_FLAG_STAGED | TBK_FLAG_TWO_STEP | TBK_FLAG_PERSISTENT | TBK_FLAG_NO_GRAPH)))
     return TBK_OK;
+  // double-float: two CTAs an SM at most (honeycomb 200x200, R = 2, 313 tiles: 6.57 us a step, 5.89 in
+  // launches of their own)
+  if (P->prec == TBK_PREC_DD && P->grid > 2 * sm_count()) return TBK_OK;
   const size_t smem = P->use_cls ? class_smem(P->H->ell, P->prec) : 0;
   for (int b = 0; b < 2; ++b) {
     int nb = 0;

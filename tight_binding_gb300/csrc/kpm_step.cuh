@@ -78,10 +78,10 @@ __device__ __forceinline__ void step_sums(F m0, F m1, double* __restrict__ part)
     if (threadIdx.x % kStepWarps == 0) part[slot * gridDim.x + blockIdx.x] = d;
   }
 }
-// Complex64 steps call it out of line: inlined, its FP64 registers change how the row
-// loop is scheduled (both 40 registers; honeycomb 701x600 with vacancies, ELL form:
-// R = 32 122.0 -> 108.8 us a step, R = 16 66.1 -> 59.7; honeycomb 1024x1024, class form,
-// R = 32 253.2 -> 248.8).  The wider types run 2-6% faster with it inlined.
+// Complex64 steps call it out of line, but for the brakets below: inlined, its FP64 registers change
+// how the row loop is scheduled (doubling: honeycomb 701x600 with vacancies, ELL form, R = 32 122.0 ->
+// 108.8 us a step; honeycomb 1024x1024, class form, R = 32 249.7 -> 239.2; braket with a flux, R = 32,
+// square 900x900 185 -> 163).  The wider types run 2-6% faster with it inlined.
 template <bool kTwo>
 __device__ __noinline__ void step_sums_call(float m0, float m1, double* __restrict__ part) {
   step_sums<float, kTwo>(m0, m1, part);
@@ -135,15 +135,32 @@ constexpr bool kWideSteps = CLS && sizeof(F) == 4 && KST != 0 && KST != 3;
 template <int KST>
 constexpr int kWideThreads = KST == 2 ? 512 : 768;
 
-// Steps bound by arithmetic may take more registers than the compiler gives them by
-// itself: fewer warps with more gathers each in flight run faster (honeycomb 1024x1024,
-// R = 32: FP64 braket 1,483 -> 1,364 us, double-float doubling 795 -> 744-762 us).  FP64: 4
-// CTAs per SM in both forms, which then keep one grid and so the same bits (3 would give
-// the class form 1,227 us, the ELL form, R = 32 with vacancies, 577 against 484).  Double-float:
-// any number in the class form's moment steps; not in the ELL form (701x600 with
-// vacancies, R = 20: 200 -> 216 us) nor in its Clenshaw steps.  0: not stated.
-template <typename F, int KST, bool CLS>
-constexpr int kMinCtas = kWideSteps<F, KST, CLS> ? 2 : is_f64<F> ? 4 : (CLS && is_dd<F> && KST == 0) ? 1 : 0;
+// Rows of more than 8 entries in the double-float class form (PIPE there)
+template <typename F, int R, bool CLS>
+constexpr bool kWideRows = CLS && is_dd<F> && R >= 16;
+// CTAs per SM that the registers must leave room for (0: not stated).  What is best is between
+// the number of warps and the gathers that each has in flight, and left to itself the compiler
+// swings either way with small changes around the row loop.  us a step:
+// FP64: 4 in both forms, which then keep one grid and so the same bits (honeycomb 1024x1024, R = 32,
+//   braket 1,483 -> 1,364; 3 would give the class form 1,227, the ELL form 577 against 484).
+// Double-float, class form: 3 (not stated, as before 60-64 registers, | 1: 88-106 | 3): honeycomb
+//   512x512, R = 8, braket 48.5 | 56.3 | 50.5; 1024x1024, R = 32, doubling 791 | 753 | 737, braket 889
+//   | 799 | 729; R = 4, doubling 97 | 106 | 101.  Rows of more than 8 entries, R >= 16: 1 (FCC 100^3,
+//   R = 32, doubling 843 | 673 | 708).  ELL form of real matrices: 3 (FCC 64^3 with vacancies, R = 32,
+//   doubling 242 not stated, 187 with 3), but for short rows of run-time widths (square 900x900 with
+//   vacancies, R = 6, 60 -> 67); complex ones not stated.
+// Complex64 braket: 6, which is 40 registers, where the compiler takes 32 (class form, and the ELL form
+//   with few entries a row: FCC 64^3, R = 32, 61.4 -> 56; square 900x900 with a flux, R = 32, 164 -> 147, with
+//   vacancies 148 -> 127), but for widths 1, 2 and run-time ones (flux, R = 2, 11.3 -> 14.4 with it).
+template <typename F, int R, bool CPLX_H, bool BRAKET, int KST, bool PIPE, bool CLS>
+constexpr int min_ctas() {
+  if (kWideSteps<F, KST, CLS>) return 2;
+  if (is_f64<F>) return 4;
+  if (KST != 0) return 0;
+  if (is_dd<F>) return CLS ? (PIPE ? 1 : 3) : CPLX_H || (R == 0 && !PIPE) ? 0 : 3;
+  if (BRAKET) return CLS || (!PIPE && R >= 4) ? 6 : 0;
+  return 0;
+}
 
 // One recursion step over all rows, x = v_s, y = v_{s-1} on entry.
 //   FIRST: y = H x                    else: y = 2 H x - y  (v_{s+1} over v_{s-1})
@@ -163,7 +180,7 @@ constexpr int kMinCtas = kWideSteps<F, KST, CLS> ? 2 : is_f64<F> ? 4 : (CLS && i
 //   KST = 5: as 1, into an FP16-pair store (ks.split; KST = 2 looks at it itself).
 //   KST = 4: a plain step whose moments nothing reads (the Kubo recursion
 //   ahead of an operator product).  Only KST = 0 forms the moment sums.
-//   PIPE: rows wider than one group of 4 gathers (ELL width > 4, e.g. FCC's
+//   PIPE (of the ELL form; see kWideRows): rows wider than one group of 4 gathers (ELL width > 4, e.g. FCC's
 //   12 neighbours) load the next group's columns while this group's gathers
 //   are in flight: 4 dependent memory round trips per 12-neighbour row instead
 //   of 6 (1.8x on the FCC Kubo recursion).  Narrow rows keep the plain loop,
@@ -176,7 +193,7 @@ constexpr int kMinCtas = kWideSteps<F, KST, CLS> ? 2 : is_f64<F> ? 4 : (CLS && i
 //   R: vectors per row, a power of two; 0: any other width, LPR lanes per row given
 //   at run time (rows stay whole within a CTA, a few threads at its end idle).
 template <typename F, int R, bool CPLX_H, bool FIRST, bool BRAKET, int KST = 0, bool PIPE = false, bool CLS = false>
-__global__ void __launch_bounds__(kWideSteps<F, KST, CLS> ? kWideThreads<KST> : kStepThreads, kMinCtas<F, KST, CLS>)
+__global__ void __launch_bounds__(kWideSteps<F, KST, CLS> ? kWideThreads<KST> : kStepThreads, min_ctas<F, R, CPLX_H, BRAKET, KST, PIPE, CLS>())
 kpm_step_kernel(
     int32_t n, int32_t n_tiles, const int32_t* __restrict__ soff, const int32_t* __restrict__ ecol,
     const F* __restrict__ eval, const F* __restrict__ diag, const typename C2<F>::T* __restrict__ x,
@@ -196,7 +213,6 @@ kpm_step_kernel(
   const int sub = threadIdx.x % LPR;
   Acc m0 = 0, m1 = 0;
   constexpr bool FOLD = kFoldStep<F> && !FIRST;
-  static_assert(!(CLS && PIPE), "class form: no column pipeline");
   static_assert(!(CLS && KST == 2 && sizeof(F) != 4), "class form: operator products in FP32 only");
 
   // class form: the table in shared memory (4-byte words: values, offsets, counts)
@@ -503,7 +519,7 @@ kpm_step_kernel(
     }
   }
   if constexpr (KST == 0) {
-    if constexpr (sizeof(F) == 4) step_sums_call<!BRAKET || FIRST>(m0, m1, part);
+    if constexpr (sizeof(F) == 4 && !(BRAKET && (CLS || (!CPLX_H && !PIPE && R >= 4)))) step_sums_call<!BRAKET || FIRST>(m0, m1, part);
     else step_sums<F, !BRAKET || FIRST>(m0, m1, part);
   }
 }
@@ -545,6 +561,14 @@ inline int launch_step_r(const StepArgs& a, bool first, bool braket, int grid, c
   auto dg = static_cast<const F*>(a.diag);
 #define TBK_STEP(FI, BR, KS)                                                                          \
   do {                                                                                                \
+    if constexpr (kWideRows<F, R, CLS> && KS == 0 && !FI) {                                           \
+      if (a.ct.w > 8) {                                                                               \
+        kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, true, true><<<grid, kStepThreads, smem, st>>>(      \
+            a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
+            a.ct, a.lpr);                                                                             \
+        break;                                                                                        \
+      }                                                                                               \
+    }                                                                                                 \
     if constexpr (CLS)                                                                                \
       kpm_step_kernel<F, R, CPLX_H, FI, BR, KS, false, true><<<grid, kWideSteps<F, KS, true> ? a.threads : kStepThreads, smem, st>>>( \
           a.n, a.n_tiles, a.soff, a.ecol, ev, dg, x, y, pv, b, a.part, a.store, a.reverse, a.gather, a.pf_dist, a.ks, \
@@ -609,11 +633,16 @@ inline int launch_step(int R, const StepArgs& a, bool first, bool braket, int gr
 }
 
 
+// of the steps that form moment sums or not; in rows of more than 8 entries
+struct StepKind { bool sums = false, wide = false; };
 // threads: of a wide step (kWideSteps)
 template <typename F, bool CPLX_H, int R, bool CLS = false>
-inline int occupancy_blocks(size_t smem, bool sums, int threads = kStepThreads) {
+inline int occupancy_blocks(size_t smem, StepKind kind, int threads = kStepThreads) {
   int nb = 0;
-  if (sums)
+  if (kind.sums && kind.wide && kWideRows<F, R, CLS>)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &nb, kpm_step_kernel<F, R, CPLX_H, false, false, 0, kWideRows<F, R, CLS>, CLS>, kStepThreads, smem);
+  else if (kind.sums)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kpm_step_kernel<F, R, CPLX_H, false, false, 0, false, CLS>,
                                                   kStepThreads, smem);
   else
@@ -623,25 +652,25 @@ inline int occupancy_blocks(size_t smem, bool sums, int threads = kStepThreads) 
 }
 
 template <typename F, bool CLS>
-inline int occupancy_r(bool cplx, int R, size_t smem, bool sums, int threads = kStepThreads) {
+inline int occupancy_r(bool cplx, int R, size_t smem, StepKind kind, int threads = kStepThreads) {
   switch (R) {
-    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 1, CLS>(smem, sums, threads);
-    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 2, CLS>(smem, sums, threads);
-    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 4, CLS>(smem, sums, threads);
-    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 8, CLS>(smem, sums, threads);
-    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 16, CLS>(smem, sums, threads);
-    case 32: case 64: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 32, CLS>(smem, sums, threads);
-    default: return cplx ? occupancy_blocks<F, true, 0, CLS>(smem, sums, threads) : occupancy_blocks<F, false, 0, CLS>(smem, sums, threads);
+    case 1: return cplx ? occupancy_blocks<F, true, 1, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 1, CLS>(smem, kind, threads);
+    case 2: return cplx ? occupancy_blocks<F, true, 2, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 2, CLS>(smem, kind, threads);
+    case 4: return cplx ? occupancy_blocks<F, true, 4, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 4, CLS>(smem, kind, threads);
+    case 8: return cplx ? occupancy_blocks<F, true, 8, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 8, CLS>(smem, kind, threads);
+    case 16: return cplx ? occupancy_blocks<F, true, 16, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 16, CLS>(smem, kind, threads);
+    case 32: case 64: return cplx ? occupancy_blocks<F, true, 32, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 32, CLS>(smem, kind, threads);
+    default: return cplx ? occupancy_blocks<F, true, 0, CLS>(smem, kind, threads) : occupancy_blocks<F, false, 0, CLS>(smem, kind, threads);
   }
 }
 
 // per-precision entry points (TBK_PREC_*); a.cls selects the class form
 int launch_step_prec(int prec, bool cplx, int R, const StepArgs& a, bool first, bool braket, int grid,
                      cudaStream_t st);
-// CTAs per SM; sums: of the steps that form moment sums
-int occupancy_prec(int prec, bool cplx, int R, bool sums);
+// CTAs per SM
+int occupancy_prec(int prec, bool cplx, int R, StepKind kind);
 // the same of the class-form kernel with its shared-memory table
-int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, bool sums, int threads = kStepThreads);
+int occupancy_cls_prec(int prec, bool cplx, int R, size_t smem, StepKind kind, int threads = kStepThreads);
 // whether a matrix runs in the class form in a precision
 bool has_classes(const EllDev& E, int prec);
 // the class table of a matrix in a precision (ct.n_cls == 0: no class form)

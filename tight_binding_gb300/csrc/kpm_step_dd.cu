@@ -7,6 +7,6 @@ int launch_step_dd(bool cplx, int R, const StepArgs& a, bool first, bool braket,
   return cplx ? launch_step<dd, true>(R, a, first, braket, grid, st) : launch_step<dd, false>(R, a, first, braket, grid, st);
 }
 
-int occupancy_dd(bool cplx, int R, bool sums) { return occupancy_r<dd, false>(cplx, R, 0, sums); }
+int occupancy_dd(bool cplx, int R, StepKind kind) { return occupancy_r<dd, false>(cplx, R, 0, kind); }
 
 }  // namespace tbk

@@ -9,6 +9,6 @@ int launch_step_cls_dd(bool cplx, int R, const StepArgs& a, bool first, bool bra
               : launch_step<dd, false, true>(R, a, first, braket, grid, st);
 }
 
-int occupancy_cls_dd(bool cplx, int R, size_t smem, bool sums) { return occupancy_r<dd, true>(cplx, R, smem, sums); }
+int occupancy_cls_dd(bool cplx, int R, size_t smem, StepKind kind) { return occupancy_r<dd, true>(cplx, R, smem, kind); }
 
 }  // namespace tbk

@@ -7,6 +7,6 @@ int launch_step_f32(bool cplx, int R, const StepArgs& a, bool first, bool braket
   return cplx ? launch_step<float, true>(R, a, first, braket, grid, st) : launch_step<float, false>(R, a, first, braket, grid, st);
 }
 
-int occupancy_f32(bool cplx, int R, bool sums) { return occupancy_r<float, false>(cplx, R, 0, sums); }
+int occupancy_f32(bool cplx, int R, StepKind kind) { return occupancy_r<float, false>(cplx, R, 0, kind); }
 
 }  // namespace tbk

@@ -9,8 +9,8 @@ int launch_step_cls_f32(bool cplx, int R, const StepArgs& a, bool first, bool br
               : launch_step<float, false, true>(R, a, first, braket, grid, st);
 }
 
-int occupancy_cls_f32(bool cplx, int R, size_t smem, bool sums, int threads) {
-  return occupancy_r<float, true>(cplx, R, smem, sums, threads);
+int occupancy_cls_f32(bool cplx, int R, size_t smem, StepKind kind, int threads) {
+  return occupancy_r<float, true>(cplx, R, smem, kind, threads);
 }
 
 }  // namespace tbk

@@ -7,6 +7,6 @@ int launch_step_f64(bool cplx, int R, const StepArgs& a, bool first, bool braket
   return cplx ? launch_step<double, true>(R, a, first, braket, grid, st) : launch_step<double, false>(R, a, first, braket, grid, st);
 }
 
-int occupancy_f64(bool cplx, int R, bool sums) { return occupancy_r<double, false>(cplx, R, 0, sums); }
+int occupancy_f64(bool cplx, int R, StepKind kind) { return occupancy_r<double, false>(cplx, R, 0, kind); }
 
 }  // namespace tbk

@@ -9,6 +9,6 @@ int launch_step_cls_f64(bool cplx, int R, const StepArgs& a, bool first, bool br
               : launch_step<double, false, true>(R, a, first, braket, grid, st);
 }
 
-int occupancy_cls_f64(bool cplx, int R, size_t smem, bool sums) { return occupancy_r<double, true>(cplx, R, smem, sums); }
+int occupancy_cls_f64(bool cplx, int R, size_t smem, StepKind kind) { return occupancy_r<double, true>(cplx, R, smem, kind); }
 
 }  // namespace tbk
