@@ -378,7 +378,7 @@ int tbk_dos_from_moments(int32_t n, const double* mu, int32_t kernel_kind, doubl
  * Kubo conductivities from double-Chebyshev moments.
  * ========================================================================= */
 enum {
-  TBK_MU_CUDA_CORE = 0,             /* mu_nm GEMM on CUDA cores (FP32 chunks, FP64 sums) */
+  TBK_MU_CUDA_CORE = 0,             /* mu_nm GEMM on CUDA cores (FP32 chunks, float-float sums, FP64 partials) */
   TBK_MU_TENSOR = 1,                /* mu_nm GEMM on tcgen05 (FP16-pair stores; complex64
                                        stores and CUDA cores where values leave FP16's
                                        range)                                          */
@@ -388,9 +388,9 @@ enum {
   TBK_MU_FUSED_OPS = 8,             /* form the output operator's products inside the
                                        recursion step when it shares H~'s sparsity (as
                                        commutators do): same stored bits, one pass per
-                                       block instead of two.  Complex64 recursions do so
-                                       by themselves with joint row classes and in the
-                                       ELL form; in double-float the wider step holds
+                                       block instead of two.  Complex64 recursions of 32
+                                       steps or more do so by themselves with joint row
+                                       classes and in the ELL form; in double-float the wider step holds
                                        more registers and measured no faster            */
   TBK_MU_BOTH_SIDES = 16,           /* with TBK_MU_FUSED_OPS: run the left and right
                                        recursions as one of twice the width (same bits;
@@ -431,7 +431,8 @@ int tbk_kubo_release(void);
 int tbk_kubo_last_timing(double* ms_blocks, double* ms_gemm, double* gemm_flops, double* block_bytes,
                          int32_t* chunks);
 /* mu_mn = sum_k conj(L_m[k]) R_n[k] for given blocks (host, M x K complex128
- * row-major each, rounded to complex64 on the device): the contraction of
+ * row-major each, rounded on the device to complex64, FP16 pairs of 22 bits
+ * under TBK_MU_TENSOR): the contraction of
  * TB/snippets.h:337-342 on caller-supplied Chebyshev blocks.  flags: TBK_MU_*
  * (TBK_MU_TENSOR: tcgen05 split-FP16 GEMM, every block with its own scale).  mu_out: host M x M complex128. */
 int tbk_mu_from_blocks(int32_t M, int64_t K, const double* L, const double* Rb, int32_t flags,

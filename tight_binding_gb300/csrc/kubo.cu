@@ -12,8 +12,8 @@
 // consecutive blocks is contiguous (one coalesced 128-byte row per block) for
 // the mu GEMM.  For the tensor-core GEMM they are FP16 (hi, lo) pairs of the same
 // size (split_store.cuh).  They are produced by the fused recursion
-// step of kpm.cu on a three-block ring (the outer operator AL/AR applied after
-// each step), each stored value rounded once.
+// step of kpm.cu, in place on two blocks (T_m over T_{m-2}); the outer operator AL/AR
+// is applied inside the step or after it, and each stored value rounded once.
 // Random vectors are processed in chunks so that both sides fit the block
 // budget; mu accumulates over chunks in FP64 on the device.  The Gamma
 // contractions (FP64) and the Bastin integration follow TB/snippets.h:343-449.
@@ -817,9 +817,9 @@ int tbk_kubo_mu(tbk_sparse Ht, tbk_sparse AL, tbk_sparse BL, tbk_sparse AR, tbk_
     return fail(TBK_ERR_BUDGET, "stored Chebyshev blocks need %.1f GB > budget %.1f GB", 2.0 * M * n_pad * sel / 1e9,
                 budget / 1e9);
   const int64_t blk = n_pad * Rc;                       // complex entries per block
-  // stored blocks: complex64.  Recursion and operator applications: complex128
-  // work blocks by default (the Chebyshev recursion accumulates rounding error
-  // near the band edges, where the Kubo weights 1/(1-e^2)^2 are largest; each
+  // stored blocks: complex64 or FP16 pairs.  Recursion and operator applications:
+  // complex128 work blocks by default (the Chebyshev recursion accumulates rounding
+  // error near the band edges, where the Kubo weights 1/(1-e^2)^2 are largest; each
   // stored value is rounded to complex64 exactly once); TBK_MU_MIXED_RECURSION
   // runs them in complex64 with FP32 H~ (HBM-bound instead of FP64-pipe-bound).
   const size_t csz = prec == TBK_PREC_MIXED ? sizeof(float2) : sizeof(double2);

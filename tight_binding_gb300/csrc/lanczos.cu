@@ -37,7 +37,7 @@ namespace {
 // few against the rows, and the scalars formed by one thread.
 // 1,025,280-site honeycomb, 200 iterations: 21.9 ms with a 38 us product (the step
 // kernel, with a norm it did not need), an 18 us update, a 6 us scaling and two host
-// round trips (48 us) per iteration; 10.7 ms now (22 + 21 us).
+// round trips (48 us) per iteration; 10.0 ms now (22 + 21 us).
 constexpr int kLzThreads = 512;
 constexpr int kLzWarps = kLzThreads / 32;
 

@@ -32,7 +32,7 @@ def kubo_mu(Ht: SparseMatrix, AL=None, BL=None, AR=None, BR=None, M: int = 64, R
             fp64_blocks: bool = False) -> np.ndarray:
     """mu_mn = sum conj(g_m AL T_m BL r) (g_n AR T_n BR r); operators None = identity.
     recursion: "mixed" (default: complex64 work blocks, FP32 H~; the stored
-    blocks are complex64 either way, and against the FP64 reference form the
+    blocks are complex64 either way, FP16 pairs of 22 bits with tensor=True, and against the FP64 reference form the
     sigma errors are the same as with the wider recursions), "dd" (double-float
     work blocks: FP64-class recursion on the FP32 pipe) or "fp64" (complex128).  fuse_ops:
     form AL / AR products inside the recursion step when they share H~'s
@@ -64,7 +64,8 @@ def kubo_release() -> None:
 
 
 def mu_from_blocks(L: np.ndarray, R: np.ndarray, tensor: bool = True) -> np.ndarray:
-    """mu_mn = sum_k conj(L[m, k]) R[n, k] on the GPU (blocks rounded to complex64)."""
+    """mu_mn = sum_k conj(L[m, k]) R[n, k] on the GPU (blocks rounded to complex64,
+    with tensor=True to FP16 pairs of 22 bits under a scale of each block's own)."""
     L = np.ascontiguousarray(L, dtype=np.complex128)
     R = np.ascontiguousarray(R, dtype=np.complex128)
     M, K = L.shape
